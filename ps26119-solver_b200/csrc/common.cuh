@@ -335,6 +335,19 @@ class PinnedBuf {
   std::size_t n_ = 0, bytes_ = 0;
 };
 
+// A timing-free event of the current device.
+class Event {
+ public:
+  Event() { B200_CHECK(cudaEventCreateWithFlags(&ev_, cudaEventDisableTiming)); }
+  ~Event() { cudaEventDestroy(ev_); }
+  Event(const Event&) = delete;
+  Event& operator=(const Event&) = delete;
+  cudaEvent_t get() const { return ev_; }
+
+ private:
+  cudaEvent_t ev_ = nullptr;
+};
+
 constexpr int kBlock = 256;
 constexpr unsigned kFull = 0xffffffffu;
 

@@ -10,6 +10,8 @@
 //   fp32 copies saf / satf and of the scaled vectors for mixed precision.
 #pragma once
 
+#include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -30,36 +32,97 @@ static __global__ void k_absmax(long long n, const double* v, unsigned long long
   B200_FOR(i, n) mx = std_max(mx, fabs(v[i]));
   warp_max_atomic(key, mx);
 }
-static __global__ void k_prod_terms(int n, const double* a, const double* b, double* t) {
-  B200_FOR(i, n) t[i] = a[i] * b[i];
-}
-// w[j] -= al*v[j] + bprev*vprev[j]; t[j] = w[j]² (csr.cpp:108-112)
-static __global__ void k_lanczos_update(int n, double* w, const double* v, const double* vprev, double al, double bprev,
-                                 double* t) {
-  B200_FOR(j, n) {
-    w[j] -= al * v[j] + bprev * vprev[j];
-    t[j] = w[j] * w[j];
+// ---------------------------------------------------------------------- Lanczos
+// The start vector is the reference's xorshift64* stream: entry j comes from the generator's state
+// after j + 1 updates. An update is linear over GF(2), so a thread jumps to its place with the powers
+// kStartRun·2^k of the update's matrix (the state's bits select columns to xor) and then steps through
+// kStartRun entries; the reference walks the stream from its seed. terms receives v[j]².
+constexpr int kStartRun = 32;
+constexpr int kStartPowers = 27;  // 32·2^27 entries and more
+static __global__ void k_lanczos_start(int n, const unsigned long long* jump, double* v, double* terms) {
+  const long long run = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+  const long long j0 = run * kStartRun;
+  if (j0 >= n) return;
+  unsigned long long s = 0x9E3779B97F4A7C15ULL;
+  for (int k = 0; k < kStartPowers && (run >> k) != 0; ++k) {
+    if (!((run >> k) & 1)) continue;
+    unsigned long long to = 0;
+    for (int b = 0; b < 64; ++b) to ^= ((s >> b) & 1ULL) ? __ldg(jump + k * 64 + b) : 0ULL;
+    s = to;
+  }
+  for (long long j = j0; j < j0 + kStartRun && j < n; ++j) {
+    s ^= s >> 12, s ^= s << 25, s ^= s >> 27;
+    const double e = static_cast<double>((s * 0x2545F4914F6CDD1DULL) >> 11) / 9007199254740992.0 * 2.0 - 1.0;
+    v[j] = e;
+    terms[j] = e * e;
   }
 }
-static __global__ void k_lanczos_next(int n, const double* w, double* v, double* vprev, double bn) {
+// The jump matrices: column b of power k is the state that bit b becomes after kStartRun·2^k updates.
+inline const std::vector<unsigned long long>& lanczos_jumps() {
+  static const std::vector<unsigned long long> all = [] {
+    using Cols = std::array<unsigned long long, 64>;
+    auto apply = [](const Cols& m, unsigned long long x) {
+      unsigned long long y = 0;
+      for (int b = 0; b < 64; ++b)
+        if ((x >> b) & 1) y ^= m[static_cast<std::size_t>(b)];
+      return y;
+    };
+    Cols m;
+    for (int b = 0; b < 64; ++b) {
+      unsigned long long s = 1ULL << b;
+      s ^= s >> 12, s ^= s << 25, s ^= s >> 27;
+      m[static_cast<std::size_t>(b)] = s;
+    }
+    auto square = [&] {
+      Cols q;
+      for (std::size_t b = 0; b < 64; ++b) q[b] = apply(m, m[b]);
+      m = q;
+    };
+    for (int k = 1; k < kStartRun; k <<= 1) square();
+    std::vector<unsigned long long> out;
+    for (int k = 0; k < kStartPowers; ++k, square()) out.insert(out.end(), m.begin(), m.end());
+    return out;
+  }();
+  return all;
+}
+static __global__ void k_lanczos_normalise(int n, double* v, double* vprev, const double* sq) {
+  const double nv = sqrt(*sq);
   B200_FOR(j, n) {
-    vprev[j] = v[j];
-    v[j] = w[j] / bn;
+    v[j] = v[j] / nv;
+    vprev[j] = 0.0;
   }
 }
-// The same two steps with α and β read from the device, where the sums left them: α = *al,
-// β_prev = sqrt(*bsq_prev) (0 without one), β = sqrt(*bsq) — sqrt correctly rounded, as the
-// host's std::sqrt. `hist` receives (α, β²) of step k for the host's later replay.
-static __global__ void k_lanczos_update_dev(int n, double* w, const double* v, const double* vprev, const double* al,
-                                            const double* bsq_prev, double* t) {
-  const double a = *al, bp = bsq_prev ? sqrt(*bsq_prev) : 0.0;
-  B200_FOR(j, n) {
-    w[j] -= a * v[j] + bp * vprev[j];
-    t[j] = w[j] * w[j];
+// After w = Ãᵀt: the terms of α = wᵀv and their tile sums (reduce.cuh) on the way.
+struct EpiLanczosW : AlwaysActive {
+  const double* v;
+  double *w, *terms, *stat;
+  struct Acc {
+    double term = 0.0;
+  };
+  __device__ void operator()(int j, double s, Acc& acc) const {
+    w[j] = s;
+    acc.term = s * v[j];
+    terms[j] = acc.term;
   }
+  __device__ void flush(const Acc& acc) const { x_leave_stat(stat, acc.term); }
+};
+// w[j] -= al*v[j] + bprev*vprev[j]; terms[j] = w[j]² (csr.cpp:108-112), with α and β_prev² read
+// from the device, where the sums left them (sqrt correctly rounded, as the host's std::sqrt).
+// Launched with one thread per entry in blocks of kXTile, for the tile sums.
+static __global__ void __launch_bounds__(kXTile) k_lanczos_update(int n, double* w, const double* v, const double* vprev,
+                                                                  const double* ab, double* terms, double* stat) {
+  const int j = blockIdx.x * kXTile + threadIdx.x;
+  double term = 0.0;
+  if (j < n) {
+    const double e = w[j] - (ab[0] * v[j] + sqrt(ab[1]) * vprev[j]);
+    w[j] = e;
+    term = e * e;
+    terms[j] = term;
+  }
+  x_leave_stat(stat, term);
 }
-static __global__ void k_lanczos_next_dev(int n, const double* w, double* v, double* vprev, const double* ab,
-                                          double* hist) {
+// The next Lanczos vector, w/β; hist receives (α, β²) of this step for the host's later replay.
+static __global__ void k_lanczos_next(int n, const double* w, double* v, double* vprev, const double* ab, double* hist) {
   const double bn = sqrt(ab[1]);
   if (blockIdx.x == 0 && threadIdx.x == 0) hist[0] = ab[0], hist[1] = ab[1];
   B200_FOR(j, n) {
@@ -67,7 +130,6 @@ static __global__ void k_lanczos_next_dev(int n, const double* w, double* v, dou
     v[j] = w[j] / bn;
   }
 }
-
 
 struct ScaledDevice {
   int m = 0, n = 0, sense = 1;
@@ -237,105 +299,148 @@ struct ScaledDevice {
   template <class T> const T* rl() const;
   template <class T> const T* ru() const;
 
-  // ‖Ã‖₂ by Lanczos on ÃᵀÃ (csr.cpp:86-132). The start vector is the reference's xorshift64*
-  // stream, generated and normalised on the host in the reference's order; the products run
-  // on the device; α and β are reduced in the selected order and stay on the device, where the
-  // next step's update reads them. The host reads them back once per batch of steps (21, then
-  // 8 at a time) and replays the reference's per-step decisions on them (Sturm bisection,
-  // breakdown and stagnation tests) in step order: the result and the number of steps that
-  // count are the sequential loop's; steps run past the stopping one are discarded.
+  // ‖Ã‖₂ by Lanczos on ÃᵀÃ (csr.cpp:86-132), on the device: the reference's start vector, the
+  // products, and α and β reduced in the reference's order. α and β stay on the device, where the
+  // next step's update reads them; the host reads them back a batch of steps at a time (21, then 8)
+  // and replays the reference's per-step decisions on them (Sturm bisection, breakdown and
+  // stagnation tests) in step order while the device runs the next batch. The result and the number
+  // of steps that count are the sequential loop's; steps run past the stopping one are discarded.
   double lanczos(cudaStream_t st, unsigned* err = nullptr) {
     if (n == 0 || nnz == 0) return 0.0;
     const int K = 400;
     const double rel_tol = 1e-12;
-    std::vector<double> hv(static_cast<std::size_t>(n));
-    std::uint64_t state = 0x9E3779B97F4A7C15ULL;
-    double nv = 0;
-    for (int j = 0; j < n; ++j) {
-      state ^= state >> 12, state ^= state << 25, state ^= state >> 27;
-      hv[j] = static_cast<double>((state * 0x2545F4914F6CDD1DULL) >> 11) / 9007199254740992.0 * 2.0 - 1.0;
-      nv += hv[j] * hv[j];
-    }
-    nv = std::sqrt(nv);
-    for (double& e : hv) e /= nv;
     lanczos_launched = 0;
     DevBuf<double> v(n), vprev(n), w(n), t(m), terms(n);
-    B200_CHECK(cudaMemcpyAsync(v.get(), hv.data(), hv.size() * sizeof(double), cudaMemcpyHostToDevice, st));
-    B200_CHECK(cudaMemsetAsync(vprev.get(), 0, static_cast<std::size_t>(n) * sizeof(double), st));
     DevBuf<double> out(2), hist(2 * static_cast<std::size_t>(K));
+    DevBuf<unsigned long long> jump;
+    jump.upload(lanczos_jumps().data(), lanczos_jumps().size(), st);
     SumPlan pal, pbn;
     pal.add(terms.get(), 0, n, 0.0, SumOrder::kSeq, out.get());
     pbn.add(terms.get(), 0, n, 0.0, SumOrder::kSeq, out.get() + 1);
     pal.build(true, nullptr, st);  // α and β enter η = 0.998/‖Ã‖₂: always the reference's order
     pbn.build(true, nullptr, st);
-    std::vector<double> alpha, beta, h(2 * static_cast<std::size_t>(K));
-    double theta = 0, theta_old = -1;
-    int stagnant = 0;
-    int done = 0;  // steps launched
-    for (;;) {
-      const int batch = std::min(K - done, done == 0 ? 21 : 8);
-      for (int k = done; k < done + batch; ++k) {
+    k_lanczos_start<<<grid_for((n + kStartRun - 1) / kStartRun, 64), 64, 0, st>>>(n, jump.get(), v.get(), terms.get());
+    B200_LAUNCH_CHECK();
+    pbn.launch(st);
+    k_lanczos_normalise<<<grid_for(n), kBlock, 0, st>>>(n, v.get(), vprev.get(), out.get() + 1);
+    B200_LAUNCH_CHECK();
+    B200_CHECK(cudaMemsetAsync(out.get() + 1, 0, sizeof(double), st));  // no β before the first step
+    kernels += 2 + pbn.kernel_count();
+    const int tiles = (n + kXTile - 1) / kXTile;
+    auto launch = [&](int from, int to) {
+      for (int k = from; k < to; ++k) {
         launch_slab_tma<double>(m, a_rp.get(), a_col.get(), sa.get(), v.get(), EpiStore<double>{{}, t.get()}, st,
                                 nullptr, err);
-        launch_slab_tma<double>(n, M.col_start, t_ri.get(), sat.get(), t.get(), EpiStore<double>{{}, w.get()}, st,
-                                nullptr, err);
-        k_prod_terms<<<grid_for(n), kBlock, 0, st>>>(n, w.get(), v.get(), terms.get());
-        B200_LAUNCH_CHECK();
-        pal.launch(st);
+        launch_slab_tma<double>(n, t_rp.get(), t_ri.get(), sat.get(), t.get(),
+                                EpiLanczosW{{}, v.get(), w.get(), terms.get(), pal.stat()}, st, nullptr, err);
+        pal.launch(st, true);
         // β of the previous step is still in out[1]: this step's β² overwrites it only below
-        k_lanczos_update_dev<<<grid_for(n), kBlock, 0, st>>>(n, w.get(), v.get(), vprev.get(), out.get(),
-                                                              k > 0 ? out.get() + 1 : nullptr, terms.get());
+        k_lanczos_update<<<tiles, kXTile, 0, st>>>(n, w.get(), v.get(), vprev.get(), out.get(), terms.get(), pbn.stat());
         B200_LAUNCH_CHECK();
-        pbn.launch(st);
-        k_lanczos_next_dev<<<grid_for(n), kBlock, 0, st>>>(n, w.get(), v.get(), vprev.get(), out.get(),
-                                                            hist.get() + 2 * k);
+        pbn.launch(st, true);
+        k_lanczos_next<<<grid_for(n), kBlock, 0, st>>>(n, w.get(), v.get(), vprev.get(), out.get(), hist.get() + 2 * k);
         B200_LAUNCH_CHECK();
-        kernels += 5 + pal.kernel_count() + pbn.kernel_count();
+        kernels += 6;
       }
-      lanczos_launched = done + batch;
-      B200_CHECK(cudaMemcpyAsync(h.data() + 2 * done, hist.get() + 2 * done, 2 * batch * sizeof(double),
+      lanczos_launched = to;
+    };
+    PinnedBuf<double> h;
+    h.alloc(2 * static_cast<std::size_t>(K));
+    Event landed[2];
+    std::vector<double> alpha, beta;
+    double theta = 0, theta_old = -1;
+    int stagnant = 0;
+    int from = 0, to = std::min(K, 21), slot = 0;
+    auto fetch = [&](int a, int b, int s) {
+      B200_CHECK(cudaMemcpyAsync(h.get() + 2 * a, hist.get() + 2 * a, 2 * static_cast<std::size_t>(b - a) * sizeof(double),
                                  cudaMemcpyDeviceToHost, st));
-      B200_CHECK(cudaStreamSynchronize(st));
-      for (int k = done; k < done + batch; ++k) {  // the reference's loop body, step by step
-        const double al = h[2 * k], bn = std::sqrt(h[2 * k + 1]);
-        alpha.push_back(al);
-        theta = tridiag_max_eig(alpha, beta, static_cast<int>(alpha.size()));
-        if (bn <= 1e-14 * std_max(1.0, theta)) return std::sqrt(std_max(theta, 0.0)) * (1.0 + 1e-4);
-        beta.push_back(bn);
-        if (theta - theta_old <= rel_tol * theta) {
-          if (++stagnant >= 5 && k >= 20) return std::sqrt(std_max(theta, 0.0)) * (1.0 + 1e-4);
-        } else {
-          stagnant = 0;
-        }
+      B200_CHECK(cudaEventRecord(landed[s].get(), st));
+    };
+    launch(from, to);
+    fetch(from, to, slot);
+    for (bool done = false; !done;) {
+      // The device goes on while the host looks at this batch, where a step is cheap against the
+      // host's look or the run is long; else the steps past the stop would cost more than the wait.
+      const bool ahead = n <= (1 << 18) || to >= 100;
+      const int next = std::min(K, to + 8);
+      auto go_on = [&] {
+        if (next > to) launch(to, next), fetch(to, next, slot ^ 1);
+      };
+      if (ahead) go_on();
+      B200_CHECK(cudaEventSynchronize(landed[slot].get()));
+      for (int k = from; k < to; ++k) alpha.push_back(h[2 * k]), beta.push_back(std::sqrt(h[2 * k + 1]));
+      double thetas[21];
+      tridiag_max_eigs(alpha.data(), beta.data(), from + 1, to - from, thetas);
+      for (int k = from; k < to && !done; ++k) {  // the reference's loop body, step by step
+        const double bn = beta[static_cast<std::size_t>(k)];
+        theta = thetas[k - from];
+        if (bn <= 1e-14 * std_max(1.0, theta)) done = true;
+        else if (theta - theta_old <= rel_tol * theta) done = ++stagnant >= 5 && k >= 20;
+        else stagnant = 0;
         theta_old = theta;
       }
-      done += batch;
-      if (done >= K) return std::sqrt(std_max(theta, 0.0)) * (1.0 + 1e-4);
+      if (to >= K) done = true;
+      if (!done && !ahead) go_on();
+      from = to, to = next, slot ^= 1;
     }
+    B200_CHECK(cudaStreamSynchronize(st));  // the steps past the stop, before their buffers go back
+    return std::sqrt(std_max(theta, 0.0)) * (1.0 + 1e-4);
   }
 
-  // Largest eigenvalue of the Lanczos tridiagonal by Sturm bisection (csr.cpp:54-84).
-  static double tridiag_max_eig(const std::vector<double>& a, const std::vector<double>& b, int k) {
-    double lo = 1e300, hi = -1e300;
-    for (int i = 0; i < k; ++i) {
-      const double r = (i > 0 ? std::fabs(b[i - 1]) : 0.0) + (i + 1 < k ? std::fabs(b[i]) : 0.0);
-      lo = std_min(lo, a[i] - r);
-      hi = std_max(hi, a[i] + r);
-    }
-    for (int it = 0; it < 200 && hi - lo > 1e-15 * std_max(1.0, std::fabs(hi)); ++it) {
-      const double mid = 0.5 * (lo + hi);
-      int c = 0;
-      double d = 1.0;
-      for (int i = 0; i < k; ++i) {
-        const double bb = i > 0 ? b[i - 1] * b[i - 1] : 0.0;
-        d = (a[i] - mid) - (i > 0 ? bb / d : 0.0);
-        if (d == 0.0) d = -1e-300;
-        if (d < 0) ++c;
+  // Largest eigenvalues of the leading k0, k0 + 1, …, k0 + count − 1 rows of the Lanczos tridiagonal
+  // (a, b), each by the reference's Sturm bisection (csr.cpp:54-84). One bisection is a chain of
+  // divisions; up to 8 of them go through the recurrence side by side.
+  static void tridiag_max_eigs(const double* a, const double* b, int k0, int count, double* out) {
+    constexpr int L = 8;
+    for (int f = 0; f < count; f += L) {
+      const int c = std::min(L, count - f);
+      double lo[L], hi[L], mid[L], d[L];
+      int k[L], it[L], neg[L];
+      bool open[L];
+      for (int q = 0; q < L; ++q) {
+        k[q] = k0 + f + std::min(q, c - 1), it[q] = 0, lo[q] = 1e300, hi[q] = -1e300;
+        for (int i = 0; i < k[q]; ++i) {
+          const double r = (i > 0 ? std::fabs(b[i - 1]) : 0.0) + (i + 1 < k[q] ? std::fabs(b[i]) : 0.0);
+          lo[q] = std_min(lo[q], a[i] - r);
+          hi[q] = std_max(hi[q], a[i] + r);
+        }
       }
-      if (c == k) hi = mid;
-      else lo = mid;
+      for (;;) {
+        bool any = false;
+        for (int q = 0; q < L; ++q) {
+          open[q] = q < c && it[q] < 200 && hi[q] - lo[q] > 1e-15 * std_max(1.0, std::fabs(hi[q]));
+          any = any || open[q];
+          mid[q] = 0.5 * (lo[q] + hi[q]);
+          neg[q] = 0, d[q] = 1.0;
+        }
+        if (!any) break;
+        const int shortest = k[0], longest = k[c - 1];
+        for (int i = 0; i < shortest; ++i) {
+          const double ai = a[i], bb = i > 0 ? b[i - 1] * b[i - 1] : 0.0;
+          for (int q = 0; q < L; ++q) {
+            d[q] = (ai - mid[q]) - (i > 0 ? bb / d[q] : 0.0);
+            d[q] = d[q] == 0.0 ? -1e-300 : d[q];
+            neg[q] += d[q] < 0 ? 1 : 0;
+          }
+        }
+        for (int i = shortest; i < longest; ++i) {
+          const double ai = a[i], bb = i > 0 ? b[i - 1] * b[i - 1] : 0.0;
+          for (int q = 0; q < c; ++q) {
+            if (i >= k[q]) continue;
+            d[q] = (ai - mid[q]) - (i > 0 ? bb / d[q] : 0.0);
+            if (d[q] == 0.0) d[q] = -1e-300;
+            if (d[q] < 0) ++neg[q];
+          }
+        }
+        for (int q = 0; q < L; ++q) {
+          if (!open[q]) continue;
+          ++it[q];
+          if (neg[q] == k[q]) hi[q] = mid[q];
+          else lo[q] = mid[q];
+        }
+      }
+      for (int q = 0; q < c; ++q) out[f + q] = hi[q];
     }
-    return hi;
   }
 
  private:

@@ -6,8 +6,8 @@
 //          host loops, e.g. kkt_general, cpu_backend.cpp:226-284); kChunk64 = 64 contiguous
 //          chunks summed sequentially, then the 64 partials in order (la::parallel_sum,
 //          parallel.h:169-188, used by Backend::dot / diff_norm2). Each chain's result is the
-//          sequential chain's bit for bit, computed in parallel (k_xstat / k_xagg / k_xchain
-//          below): the order is exactly i = lo, lo+1, … as far as rounding can tell.
+//          sequential chain's bit for bit, computed in parallel (k_xstat / k_xwalk below): the
+//          order is exactly i = lo, lo+1, … as far as rounding can tell.
 //   fast:  a fixed two-level tree (kTreeBlocks blocks per sum, block tree, then one block
 //          combines the partials) — deterministic run to run, but a different rounding.
 // Maxima never go through a SumPlan: they are taken with integer atomics on non-negative
@@ -55,69 +55,81 @@ __device__ __forceinline__ double block_sum_fixed(double v, double* sh) {
 // tie, k = f or f + 1, whichever makes S + k even. So inside such a run the chain is an integer
 // walk whose only dependence on the past is the parity of S: a run of terms is summarised by its
 // effect for each of the two parities (XRun), and effects compose associatively. So:
-//   k_xstat   per tile of kXTile terms: an approximate fp64 sum and the approximate range of the
-//             tile's running sums (any order; only used to guess each tile's binade);
-//   k_xagg    per tile: the guessed binade's u from the approximate start (the approximate sums
-//             of the chain's earlier tiles), then the tile's XRun (exact int64: change of S, its
-//             lowest and highest running value, parity after, per parity before); a term with
-//             |t/u| ≥ 2^51 (or non-finite) marks the tile;
-//   k_xgroup  per group of kXGroup consecutive tiles of a long chain: the composition of the
-//             tiles' XRuns when all of them count in one grid with no split and no bad term;
-//   k_xchain  one warp per chain walks its groups, then its tiles, in order with the EXACT s: a
-//             run of whole groups is committed like one tile (below) as far as every running S
-//             provably stays inside the binade; the first group that is not is walked tile by
-//             tile. A tile is committed
+//   k_xstat   per tile of kXTile terms (one warp): an approximate fp64 sum, in any order; only used
+//             to guess each tile's binade. A kernel that produces the terms may leave it itself.
+//   k_xwalk   one block per group of kXGroup consecutive tiles, one warp per tile: the guessed
+//             binade's u from the approximate start (the approximate sums of the chain's earlier
+//             tiles), then the tile's XRun (exact int64: change of S, its lowest and highest running
+//             value, parity after, per parity before); a term with |t/u| ≥ 2^51 (or non-finite)
+//             marks the tile. The block composes its tiles' XRuns into the group's when all of them
+//             count in one grid with no split and no bad term. The block that finishes last of a
+//             chain's then walks the chain with the EXACT s, with one warp: a run of whole groups
+//             is committed like one tile (below) as far as every running S provably stays inside
+//             the binade; the first group that is not is walked tile by tile. A tile is committed
 //             as s ← (S0 + K[S0 mod 2])·u when s = S0·u lies in the guessed binade and every
 //             running S stays within [2^52 + 1, 2^53 − 1] (then each exact partial sum lies inside
-//             the binade, at least u/2 from its ends, and rounds to that grid); any other tile is
-//             walked in windows of 256 terms with the same exact test per term (a warp scan of
-//             the lanes' XRuns), committing the valid prefix and adding the first failing term
-//             with one plain fp64 addition (so binade changes, zeros, subnormals, infinities and
-//             NaN get exactly the sequential chain's arithmetic).
+//             the binade, at least u/2 from its ends, and rounds to that grid). A tile whose running
+//             sum changes binade once is committed in three parts; the terms of any other tile are
+//             added one by one (x_add), so that binade changes, zeros, subnormals, infinities and
+//             NaN get exactly the sequential chain's arithmetic. A chain of at most kXShort terms is
+//             added one by one from the start.
 // The approximations only choose between two exact paths; the result never depends on them.
-constexpr int kXTile = 2048;    // terms per tile (8 per thread of a 256-thread block)
-constexpr int kXPer = 8;        // terms per thread (tiles) and per lane (windows)
-constexpr int kXThreads = kXTile / kXPer;
+//
+// What bounds it: latency. A dependent fp64 addition takes 8.3 cycles, 10.4 with its operand from
+// shared memory, so a tile added one by one takes 1.4 us, and the walk of a chain pays that for its
+// first tile (the sum starts at zero) and for the few tiles that cross a binade more than once; every
+// other step is a warp scan over 32 tiles (0.4 us). Tiles of 256 terms, one warp's, keep the tiles
+// that must be added one by one cheap. Measured, 15,000 terms: 24 us a launch; three launches over
+// tiles of 2,048 terms, the first tile walked in windows of 256 with a scan and a restart per binade
+// crossing, took 68 us.
+constexpr int kXPer = 8;              // terms per lane
+constexpr int kXTile = 32 * kXPer;    // terms per tile (one warp)
+constexpr int kXGroup = 32;           // tiles per group (one block)
+constexpr int kXWarps = 16;           // warps per block of k_xwalk
+constexpr long long kXShort = 1024;   // chains up to this long are added one by one by a warp
 
 struct XChain {
   const double* t;
   long long lo, hi;  // terms t[lo, hi)
   double init;
   double* out;
-  int tile0, ntiles;    // this chain's tiles in the tile arrays (ntiles = 0: windows only)
-  int group0, ngroups;  // its groups of kXGroup tiles in the group array (ngroups = 0: none)
+  int tile0, ntiles;    // this chain's tiles in the tile arrays (ntiles = 0: added one by one)
+  int group0, ngroups;  // its groups of kXGroup tiles
+  int job;              // its kChunk64 job (−1: *out is the chain's own result)
 };
-constexpr int kXGroup = 32;  // tiles per group (one warp lane per tile)
-constexpr int kXChainWarps = 4;  // warps per block of k_xchain / k_xgroup
-struct XTileStat {
-  double sum, pmin, pmax;  // approximate: Σ t, min / max of the running sums from the tile start
-  int bad;                 // a non-finite term
-  int pad;
+// A kChunk64 job: the chains of its chunks leave their sums in part[0, chunks); the chain that
+// finishes last adds them in order (la::parallel_sum).
+struct XJob {
+  const double* part;
+  int chunks;
+  double init;
+  double* out;
 };
 // The effect of a run of terms on S (the partial sum in units of u), for S even (index 0) and
 // odd (1) at the run's start: K the change of S, mn / mx the lowest / highest running change
 // over positions 1…len (LLONG_MAX / LLONG_MIN for an empty run), out the parity after; bad: a
-// term the integer form cannot take (|t/u| ≥ 2^51 or non-finite).
-struct XRun {
+// term the integer form cannot take (|t/u| ≥ 2^51 or non-finite); ties: a term is a tie, so that the
+// two parities may differ (without one they agree, and a run is plain integer sums).
+struct alignas(16) XRun {
   long long K[2], mn[2], mx[2];
   int out[2];
-  int bad;
+  int bad, ties;
 };
 // A tile's summary: its terms before `split` counted in the grid u (the binade of the tile's
 // approximate start), the term at `split` (where the approximate running sum leaves that binade;
 // split = −1: it never does) added as a plain fp64 addition, the terms after it counted in the
 // grid u1 of the binade the running sum moved to. u = 0: no usable guess (bad is set).
-struct XTileAgg {
+struct alignas(16) XTileAgg {
   double u, u1;
+  double at;  // the term at `split`
   XRun pre, suf;
   int split;
-  int pad;
 };
 // A group of kXGroup consecutive tiles of one chain that all count in the same grid u with no
 // split and no bad term: the composition of their runs. u = 0: the group cannot be taken whole.
-struct XGroupAgg {
-  double u;
+struct alignas(16) XGroupAgg {
   XRun run;
+  double u;
 };
 
 constexpr long long kX52 = 1LL << 52, kX53 = 1LL << 53;
@@ -128,13 +140,14 @@ __device__ __forceinline__ XRun x_identity() {
   r.mn[0] = r.mn[1] = LLONG_MAX;
   r.mx[0] = r.mx[1] = LLONG_MIN;
   r.out[0] = 0, r.out[1] = 1;
-  r.bad = 0;
+  r.bad = r.ties = 0;
   return r;
 }
 // a then b (selects instead of indexing with a.out[p], so everything stays in registers)
 __device__ __forceinline__ XRun x_compose(const XRun& a, const XRun& b) {
   XRun r;
   r.bad = a.bad | b.bad;
+  r.ties = a.ties | b.ties;
 #pragma unroll
   for (int p = 0; p < 2; ++p) {
     const bool q = a.out[p] != 0;
@@ -146,6 +159,10 @@ __device__ __forceinline__ XRun x_compose(const XRun& a, const XRun& b) {
   }
   return r;
 }
+__device__ __forceinline__ int x_pack(const XRun& v) { return v.out[0] | (v.out[1] << 1) | (v.bad << 2) | (v.ties << 3); }
+__device__ __forceinline__ void x_unpack(XRun& r, int packed) {
+  r.out[0] = packed & 1, r.out[1] = (packed >> 1) & 1, r.bad = (packed >> 2) & 1, r.ties = (packed >> 3) & 1;
+}
 __device__ __forceinline__ XRun x_shfl_down(const XRun& v, int off) {
   XRun r;
 #pragma unroll
@@ -154,8 +171,7 @@ __device__ __forceinline__ XRun x_shfl_down(const XRun& v, int off) {
     r.mn[p] = __shfl_down_sync(kFull, v.mn[p], off);
     r.mx[p] = __shfl_down_sync(kFull, v.mx[p], off);
   }
-  const int packed = __shfl_down_sync(kFull, v.out[0] | (v.out[1] << 1) | (v.bad << 2), off);
-  r.out[0] = packed & 1, r.out[1] = (packed >> 1) & 1, r.bad = packed >> 2;
+  x_unpack(r, __shfl_down_sync(kFull, x_pack(v), off));
   return r;
 }
 __device__ __forceinline__ XRun x_shfl_up(const XRun& v, int off) {
@@ -166,8 +182,7 @@ __device__ __forceinline__ XRun x_shfl_up(const XRun& v, int off) {
     r.mn[p] = __shfl_up_sync(kFull, v.mn[p], off);
     r.mx[p] = __shfl_up_sync(kFull, v.mx[p], off);
   }
-  const int packed = __shfl_up_sync(kFull, v.out[0] | (v.out[1] << 1) | (v.bad << 2), off);
-  r.out[0] = packed & 1, r.out[1] = (packed >> 1) & 1, r.bad = packed >> 2;
+  x_unpack(r, __shfl_up_sync(kFull, x_pack(v), off));
   return r;
 }
 
@@ -180,17 +195,24 @@ __device__ __forceinline__ bool x_binade(double v, int& e) {
   e = ef - 1023;
   return e >= -970 && e <= 1023;
 }
+// The sign and exponent of v: two numbers of which one lies in a binade lie in the same one, with the
+// same sign, where these agree.
+__device__ __forceinline__ int x_top(double v) { return __double2hiint(v) >> 20; }
 __device__ __forceinline__ double x_pow2(int p) {  // 2^p, p in [−1022, 1023]
   return __longlong_as_double(static_cast<long long>(p + 1023) << 52);
 }
 // A term in units of u (inv_u = 1/u, powers of two: t·inv_u is exact unless it under/overflows):
-// false for |t/u| ≥ 2^51 or a non-finite t; else kf = rint(t/u), or floor(t/u) for a tie.
+// false for |t/u| ≥ 2^51 or a non-finite t; else kf = rint(t/u), or floor(t/u) for a tie. Adding and
+// taking away 1.5·2^52 rounds to an integer, and leaves it in the low bits of the sum.
 __device__ __forceinline__ bool x_term(double t, double inv_u, long long& kf, bool& tie) {
+  constexpr double kMagic = 6755399441055744.0;  // 1.5·2^52
   const double q = t * inv_u;
   if (!(fabs(q) < 2251799813685248.0)) return false;  // 2^51; also NaN / inf
-  const double f = floor(q);
-  tie = q - f == 0.5;
-  kf = static_cast<long long>(tie ? f : rint(q));
+  const double m = q + kMagic;
+  kf = __double_as_longlong(m) - __double_as_longlong(kMagic);
+  const double d = q - (m - kMagic);
+  tie = fabs(d) == 0.5;
+  if (d == -0.5) --kf;
   return true;
 }
 // The step of S with parity `par` for a term (kf, tie): returns k; par becomes S + k's parity.
@@ -204,54 +226,66 @@ __device__ __forceinline__ long long x_step(long long kf, bool tie, int& par) {
   }
   return k;
 }
-// The XRun of up to kXPer terms v[0, cnt).
-__device__ __forceinline__ XRun x_run_of(const double* v, int cnt, double inv_u) {
-  XRun r = x_identity();
-  long long kf[kXPer];
-  bool tie[kXPer];
-#pragma unroll
-  for (int q = 0; q < kXPer; ++q)
-    if (q < cnt && !x_term(v[q], inv_u, kf[q], tie[q])) r.bad = 1, kf[q] = 0, tie[q] = false;
-#pragma unroll
-  for (int p = 0; p < 2; ++p) {
-    int par = p;
-    long long K = 0;
-#pragma unroll
-    for (int q = 0; q < kXPer; ++q)
-      if (q < cnt) {
-        K += x_step(kf[q], tie[q], par);
-        r.mn[p] = min(r.mn[p], K);
-        r.mx[p] = max(r.mx[p], K);
-      }
-    r.K[p] = K;
-    r.out[p] = par;
-  }
-  return r;
-}
-// The XRun of the terms v[q] whose bit q is set in `mask` (the others left out).
-__device__ __forceinline__ XRun x_run_masked(const double* v, unsigned mask, double inv_u) {
+// The XRun of a warp's terms (lane l holds terms 8l … 8l+7; those whose bit q is set in `mask`, the
+// others left out), valid in lane 0. Without a tie both parities make the same steps, and the run is
+// integer sums: about a sixth of the general form's instructions.
+__device__ __forceinline__ XRun x_warp_run(const double* v, unsigned mask, double inv_u) {
+  const int lane = threadIdx.x & 31;
   XRun r = x_identity();
   long long kf[kXPer];
   bool tie[kXPer];
 #pragma unroll
   for (int q = 0; q < kXPer; ++q) {
     kf[q] = 0, tie[q] = false;
-    if (((mask >> q) & 1u) && !x_term(v[q], inv_u, kf[q], tie[q])) r.bad = 1, kf[q] = 0, tie[q] = false;
+    if ((mask >> q) & 1u) {
+      if (!x_term(v[q], inv_u, kf[q], tie[q])) r.bad = 1, kf[q] = 0, tie[q] = false;
+      r.ties |= tie[q] ? 1 : 0;
+    }
   }
+  if (__any_sync(kFull, r.ties)) {
 #pragma unroll
-  for (int p = 0; p < 2; ++p) {
-    int par = p;
-    long long K = 0;
+    for (int p = 0; p < 2; ++p) {
+      int par = p;
+      long long K = 0;
 #pragma unroll
-    for (int q = 0; q < kXPer; ++q)
-      if ((mask >> q) & 1u) {
-        K += x_step(kf[q], tie[q], par);
-        r.mn[p] = min(r.mn[p], K);
-        r.mx[p] = max(r.mx[p], K);
-      }
-    r.K[p] = K;
-    r.out[p] = par;
+      for (int q = 0; q < kXPer; ++q)
+        if ((mask >> q) & 1u) {
+          K += x_step(kf[q], tie[q], par);
+          r.mn[p] = min(r.mn[p], K);
+          r.mx[p] = max(r.mx[p], K);
+        }
+      r.K[p] = K;
+      r.out[p] = par;
+    }
+    for (int off = 1; off < 32; off <<= 1) {  // ordered reduction (lane order)
+      const XRun o = x_shfl_down(r, off);
+      if ((lane & (2 * off - 1)) == 0 && lane + off < 32) r = x_compose(r, o);
+    }
+    return r;
   }
+  long long K = 0, mn = LLONG_MAX, mx = LLONG_MIN;
+#pragma unroll
+  for (int q = 0; q < kXPer; ++q)
+    if ((mask >> q) & 1u) {
+      K += kf[q];
+      mn = min(mn, K);
+      mx = max(mx, K);
+    }
+  long long inc = K;
+  for (int off = 1; off < 32; off <<= 1) {
+    const long long o = __shfl_up_sync(kFull, inc, off);
+    if (lane >= off) inc += o;
+  }
+  if (mask) mn += inc - K, mx += inc - K;
+  for (int off = 16; off > 0; off >>= 1) {
+    mn = min(mn, __shfl_xor_sync(kFull, mn, off));
+    mx = max(mx, __shfl_xor_sync(kFull, mx, off));
+  }
+  r.K[0] = r.K[1] = __shfl_sync(kFull, inc, 31);
+  r.mn[0] = r.mn[1] = mn;
+  r.mx[0] = r.mx[1] = mx;
+  r.out[0] = static_cast<int>(r.K[0] & 1), r.out[1] = r.out[0] ^ 1;
+  r.bad = __any_sync(kFull, r.bad) ? 1 : 0;
   return r;
 }
 // |S| inside [2^52 + 1, 2^53 − 1] with the sign of S0.
@@ -259,36 +293,16 @@ __device__ __forceinline__ bool x_inside(long long S0, long long S) {
   return S0 > 0 ? (S >= kX52 + 1 && S <= kX53 - 1) : (S <= -(kX52 + 1) && S >= -(kX53 - 1));
 }
 
-template <class T, class Op>
-__device__ __forceinline__ T x_block_reduce(T v, Op op, T* sh) {  // result valid in every thread
-  for (int off = 16; off > 0; off >>= 1) v = op(v, __shfl_xor_sync(kFull, v, off));
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  __syncthreads();
-  if (lane == 0) sh[wid] = v;
-  __syncthreads();
-  v = sh[0];
-  for (int w = 1; w < nw; ++w) v = op(v, sh[w]);
+// A struct of 16-byte words another block wrote, read past this SM's L1.
+template <class S>
+__device__ __forceinline__ S x_load(const S* p) {
+  static_assert(sizeof(S) % 16 == 0, "whole 16-byte words");
+  S v;
+  const uint4* src = reinterpret_cast<const uint4*>(p);
+  uint4* dst = reinterpret_cast<uint4*>(&v);
+#pragma unroll
+  for (unsigned k = 0; k < sizeof(S) / 16; ++k) dst[k] = __ldcg(src + k);
   return v;
-}
-// Exclusive prefix of per-thread values over the block (thread order), and the block total.
-template <class T>
-__device__ __forceinline__ T x_block_excl(T v, T& total, T* sh) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  T inc = v;
-  for (int off = 1; off < 32; off <<= 1) {
-    const T o = __shfl_up_sync(kFull, inc, off);
-    if (lane >= off) inc += o;
-  }
-  __syncthreads();
-  if (lane == 31) sh[wid] = inc;
-  __syncthreads();
-  T before = T(0);
-  total = T(0);
-  for (int w = 0; w < nw; ++w) {
-    if (w < wid) before += sh[w];
-    total += sh[w];
-  }
-  return before + inc - v;
 }
 
 __device__ __forceinline__ void x_tile_range(const XChain& c, int tile, long long& a, long long& b) {
@@ -296,120 +310,157 @@ __device__ __forceinline__ void x_tile_range(const XChain& c, int tile, long lon
   b = a + kXTile < c.hi ? a + kXTile : c.hi;
 }
 
-static __global__ void __launch_bounds__(kXThreads) k_xstat(const XChain* ch, const int* tile_chain,
-                                                            XTileStat* st, const int* skip) {
-  __shared__ double shd[32];
-  __shared__ int shi[32];
-  if (skip && *skip) return;
-  const int tile = blockIdx.x;
-  const XChain c = ch[tile_chain[tile]];
-  long long a, b;
-  x_tile_range(c, tile, a, b);
-  const long long i0 = a + static_cast<long long>(threadIdx.x) * kXPer;
-  double run = 0.0, mn = INFINITY, mx = -INFINITY;
-  int bad = 0;
+// s + t[a] + t[a+1] + … + t[b−1], one rounding per addition in that order; every lane of the warp
+// calls it with the same s and returns the same sum. The terms come in chunks of kXTile through the
+// warp's shared buffer `sh` (16-byte aligned), the next chunk on its way while one is added. Places
+// past the end hold −0.0, which leaves every s as it is (−0.0 included).
+__device__ __forceinline__ double x_add(const double* t, long long a, long long b, double s, double* sh) {
+  const int lane = threadIdx.x & 31;
+  double nx[kXPer];
 #pragma unroll
-  for (int q = 0; q < kXPer; ++q)
-    if (i0 + q < b) {
-      const double v = c.t[i0 + q];
-      bad |= !isfinite(v);
-      run += v;
-      mn = fmin(mn, run), mx = fmax(mx, run);
+  for (int q = 0; q < kXPer; ++q) nx[q] = a + q * 32 + lane < b ? __ldcg(t + a + q * 32 + lane) : -0.0;
+  for (long long pos = a; pos < b; pos += kXTile) {
+    __syncwarp();  // the previous chunk has been read
+#pragma unroll
+    for (int q = 0; q < kXPer; ++q) sh[q * 32 + lane] = nx[q];
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < kXPer; ++q) {
+      const long long i = pos + kXTile + q * 32 + lane;
+      nx[q] = i < b ? __ldcg(t + i) : -0.0;
     }
-  double total;
-  const double before = x_block_excl(run, total, shd);
-  mn += before, mx += before;
-  mn = x_block_reduce(mn, [](double x, double y) { return fmin(x, y); }, shd);
-  mx = x_block_reduce(mx, [](double x, double y) { return fmax(x, y); }, shd);
-  bad = x_block_reduce(bad, [](int x, int y) { return x | y; }, shi);
-  if (threadIdx.x == 0) st[tile] = XTileStat{total, mn, mx, bad, 0};
+    const int cnt = b - pos < kXTile ? static_cast<int>(b - pos) : kXTile;
+    const double2* p = reinterpret_cast<const double2*>(sh);
+    double2 v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] = p[q];
+    for (int i = 0; i < cnt; i += 8) {  // 8 terms ahead in registers (wrapping at the buffer's end)
+      double2 w[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) w[q] = p[((i >> 1) + 4 + q) & (kXTile / 2 - 1)];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) s += v[q].x, s += v[q].y;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) v[q] = w[q];
+    }
+  }
+  return s;
 }
 
-// Ordered reduction of the block's per-thread runs (thread order); the result in thread 0.
-__device__ __forceinline__ XRun x_block_ordered(XRun r, XRun* sh) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+static __global__ void __launch_bounds__(256) k_xstat(const XChain* ch, const int* tile_chain, int ntiles,
+                                                      double* stat, const int* skip) {
+  if (skip && *skip) return;
+  const int tile = static_cast<int>((blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) >> 5);
+  const int lane = threadIdx.x & 31;
+  if (tile >= ntiles) return;
+  const XChain& c = ch[tile_chain[tile]];
+  long long a, b;
+  x_tile_range(c, tile, a, b);
+  double v[kXPer], s = 0.0;
+#pragma unroll
+  for (int q = 0; q < kXPer; ++q) v[q] = a + q * 32 + lane < b ? c.t[a + q * 32 + lane] : 0.0;
+#pragma unroll
+  for (int q = 0; q < kXPer; ++q) s += v[q];
+  for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(kFull, s, off);
+  if (lane == 0) stat[tile] = s;
+}
+// A producer's own tile sum: called by every thread of a block of kXTile threads whose thread i
+// made term i of tile blockIdx.x; stat may be null (a chain that needs none).
+__device__ __forceinline__ void x_leave_stat(double* stat, double term) {
+  __shared__ double sh[kXTile / 32];
+  if (!stat) return;
+  for (int off = 16; off > 0; off >>= 1) term += __shfl_xor_sync(kFull, term, off);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = term;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double s = sh[0];
+    for (int w = 1; w < kXTile / 32; ++w) s += sh[w];
+    stat[blockIdx.x] = s;
+  }
+}
+
+// The composition of the warp's runs in lane order, valid in lane 0.
+__device__ __forceinline__ XRun x_warp_ordered(XRun r) {
+  const int lane = threadIdx.x & 31;
+  if (!__any_sync(kFull, r.ties)) {
+    long long inc = r.K[0], mn = r.mn[0], mx = r.mx[0];
+    for (int off = 1; off < 32; off <<= 1) {
+      const long long o = __shfl_up_sync(kFull, inc, off);
+      if (lane >= off) inc += o;
+    }
+    if (mn != LLONG_MAX) mn += inc - r.K[0], mx += inc - r.K[0];
+    for (int off = 16; off > 0; off >>= 1) {
+      mn = min(mn, __shfl_xor_sync(kFull, mn, off));
+      mx = max(mx, __shfl_xor_sync(kFull, mx, off));
+    }
+    r.K[0] = r.K[1] = __shfl_sync(kFull, inc, 31);
+    r.mn[0] = r.mn[1] = mn;
+    r.mx[0] = r.mx[1] = mx;
+    r.out[0] = static_cast<int>(r.K[0] & 1), r.out[1] = r.out[0] ^ 1;
+    r.bad = __any_sync(kFull, r.bad) ? 1 : 0;
+    return r;
+  }
   for (int off = 1; off < 32; off <<= 1) {
     const XRun o = x_shfl_down(r, off);
     if ((lane & (2 * off - 1)) == 0 && lane + off < 32) r = x_compose(r, o);
   }
-  __syncthreads();
-  if (lane == 0) sh[wid] = r;
-  __syncthreads();
-  if (threadIdx.x == 0)
-    for (int w = 1; w < kXThreads / 32; ++w) r = x_compose(r, sh[w]);
   return r;
 }
 
-static __global__ void __launch_bounds__(kXThreads) k_xagg(const XChain* ch, const int* tile_chain,
-                                                           const XTileStat* st, XTileAgg* ag, const int* skip) {
-  __shared__ double shd[32];
-  __shared__ int shi[32];
-  __shared__ XRun shr[kXThreads / 32];
-  __shared__ double sh_at_split;
-  if (skip && *skip) return;
-  const int tile = blockIdx.x;
-  const XChain c = ch[tile_chain[tile]];
-  long long a, b;
-  x_tile_range(c, tile, a, b);
-  // the approximate running sum at the tile's start (the approximate sums of the earlier tiles)
-  double pre = 0.0;
-  for (int k = c.tile0 + static_cast<int>(threadIdx.x); k < tile; k += blockDim.x) pre += st[k].sum;
-  pre = x_block_reduce(pre, [](double x, double y) { return x + y; }, shd);
-  const double s0 = c.init + pre;
-  int e0;
+// The summary of the terms t[a, b) (one tile, one warp; lane l holds terms 8l … 8l+7) for a chain
+// whose approximate sum before them is s0; valid in lane 0.
+__device__ __forceinline__ XTileAgg x_tile_agg(const double* __restrict__ t, long long a, long long b, double s0) {
+  const int lane = threadIdx.x & 31;
   XTileAgg g;
-  g.u = g.u1 = 0.0;
+  g.u = g.u1 = g.at = 0.0;
   g.split = -1;
-  g.pad = 0;
   g.pre = g.suf = x_identity();
-  if (!x_binade(s0, e0)) {  // uniform over the block
-    if (threadIdx.x == 0) g.pre.bad = 1, ag[tile] = g;
-    return;
+  int e0;
+  if (!x_binade(s0, e0)) {  // uniform over the warp
+    g.pre.bad = 1;
+    return g;
   }
-  const long long i0 = a + static_cast<long long>(threadIdx.x) * kXPer;
+  const long long i0 = a + static_cast<long long>(lane) * kXPer;
   double v[kXPer];
   double run = 0.0;
 #pragma unroll
-  for (int q = 0; q < kXPer; ++q) {
-    v[q] = i0 + q < b ? c.t[i0 + q] : 0.0;
-    run += v[q];
+  for (int q = 0; q < kXPer; ++q) v[q] = i0 + q < b ? t[i0 + q] : 0.0;
+#pragma unroll
+  for (int q = 0; q < kXPer; ++q) run += v[q];
+  double inc = run;
+  for (int off = 1; off < 32; off <<= 1) {
+    const double o = __shfl_up_sync(kFull, inc, off);
+    if (lane >= off) inc += o;
   }
-  // approximate running sums: the first position whose running sum leaves e0's binade
-  double total;
-  const double before = x_block_excl(run, total, shd);
-  const int base = static_cast<int>(threadIdx.x) * kXPer;
+  const double start = s0 + (inc - run);
+  // the first position whose approximate running sum leaves e0's binade
+  const int base = lane * kXPer;
+  const int top0 = x_top(s0);
   int first = INT_MAX;
-  double acc = s0 + before;
+  double acc = start, at = 0.0, term = 0.0;
 #pragma unroll
   for (int q = 0; q < kXPer; ++q)
     if (i0 + q < b) {
       acc += v[q];
-      int e;
-      if (first == INT_MAX && !(x_binade(acc, e) && e == e0 && (acc > 0) == (s0 > 0))) first = base + q;
+      if (first == INT_MAX && x_top(acc) != top0) first = base + q, at = acc, term = v[q];
     }
-  const int split = x_block_reduce(first, [](int x, int y) { return x < y ? x : y; }, shi);
+  const int split = __reduce_min_sync(kFull, first);
   // the binade after the split: all later approximate running sums must share it
-  int e1 = e0, ok1 = 1;
+  int e1 = e0;
+  bool ok1 = true;
   if (split != INT_MAX) {
-    if (split >= base && split < base + kXPer) {
-      double acc2 = s0 + before;
-#pragma unroll
-      for (int q = 0; q < kXPer; ++q)
-        if (q <= split - base) acc2 += v[q];
-      sh_at_split = acc2;
-    }
-    __syncthreads();
-    const double after = sh_at_split;
-    ok1 = x_binade(after, e1) ? 1 : 0;
-    double acc3 = s0 + before;
+    const double after = __shfl_sync(kFull, at, split / kXPer);
+    ok1 = x_binade(after, e1);
+    const int top1 = x_top(after);
+    bool same = true;
+    acc = start;
 #pragma unroll
     for (int q = 0; q < kXPer; ++q)
       if (i0 + q < b) {
-        acc3 += v[q];
-        int e;
-        if (base + q > split && !(x_binade(acc3, e) && e == e1 && (acc3 > 0) == (after > 0))) ok1 = 0;
+        acc += v[q];
+        if (base + q > split && x_top(acc) != top1) same = false;
       }
-    ok1 = x_block_reduce(ok1, [](int x, int y) { return x & y; }, shi);
+    ok1 = __all_sync(kFull, same) && ok1;
   }
   unsigned mpre = 0, msuf = 0;
 #pragma unroll
@@ -418,108 +469,19 @@ static __global__ void __launch_bounds__(kXThreads) k_xagg(const XChain* ch, con
       if (base + q < split) mpre |= 1u << q;
       else if (split != INT_MAX && base + q > split) msuf |= 1u << q;
     }
-  const XRun rp = x_block_ordered(x_run_masked(v, mpre, x_pow2(52 - e0)), shr);
-  XRun rs = x_identity();
-  if (split != INT_MAX && ok1) rs = x_block_ordered(x_run_masked(v, msuf, x_pow2(52 - e1)), shr);
-  if (threadIdx.x == 0) {
-    g.u = x_pow2(e0 - 52);
-    g.pre = rp;
-    if (split != INT_MAX) {
-      g.split = split;
-      g.u1 = ok1 ? x_pow2(e1 - 52) : 0.0;
-      g.suf = rs;
-      if (!ok1) g.suf.bad = 1;
+  g.u = x_pow2(e0 - 52);
+  g.pre = x_warp_run(v, mpre, x_pow2(52 - e0));
+  if (split != INT_MAX) {
+    g.split = split;
+    g.at = __shfl_sync(kFull, term, split / kXPer);
+    if (ok1) {
+      g.u1 = x_pow2(e1 - 52);
+      g.suf = x_warp_run(v, msuf, x_pow2(52 - e1));
+    } else {
+      g.suf.bad = 1;
     }
-    ag[tile] = g;
   }
-}
-
-// The chain over t[a, b) from the exact partial sum s, by windows of 32·kXPer terms (all 32 lanes
-// call it with the same s and return the same s). The next window's terms are requested before
-// the current one is evaluated, so a run of valid windows waits on memory once.
-__device__ __forceinline__ void x_load_window(const double* __restrict__ t, long long pos, long long b,
-                                              double (&v)[kXPer]) {
-  const long long i0 = pos + static_cast<long long>(threadIdx.x & 31) * kXPer;
-#pragma unroll
-  for (int q = 0; q < kXPer; ++q) v[q] = i0 + q < b ? t[i0 + q] : 0.0;
-}
-__device__ __forceinline__ double x_window_walk(const double* __restrict__ t, long long a, long long b, double s) {
-  const int lane = threadIdx.x & 31;
-  long long pos = a;
-  double v[kXPer], nx[kXPer];
-  x_load_window(t, pos, b, v);
-  while (pos < b) {
-    int e;
-    if (!x_binade(s, e)) {  // zero, subnormal, inf or NaN: a plain sequential run of up to 32 terms
-      const long long rem = b - pos;
-      const int cnt = rem < 32 ? static_cast<int>(rem) : 32;
-      const double w = lane < cnt ? t[pos + lane] : 0.0;
-      for (int j = 0; j < cnt; ++j) s += __shfl_sync(kFull, w, j);
-      pos += cnt;
-      x_load_window(t, pos, b, v);
-      continue;
-    }
-    x_load_window(t, pos + 32LL * kXPer, b, nx);  // the next window, if this one is valid
-    const double u = x_pow2(e - 52), inv_u = x_pow2(52 - e);
-    const long long S0 = static_cast<long long>(s * inv_u);
-    const int p0 = static_cast<int>(S0 & 1);
-    const long long i0 = pos + static_cast<long long>(lane) * kXPer;
-    int cnt = 0;
-#pragma unroll
-    for (int q = 0; q < kXPer; ++q) cnt += i0 + q < b ? 1 : 0;
-    XRun inc = x_run_of(v, cnt, inv_u);  // warp inclusive scan in lane order
-    for (int off = 1; off < 32; off <<= 1) {
-      const XRun o = x_shfl_up(inc, off);
-      if (lane >= off) inc = x_compose(o, inc);
-    }
-    XRun ex = x_shfl_up(inc, 1);
-    if (lane == 0) ex = x_identity();
-    // this lane's terms with its exact incoming state: the first invalid position
-    long long run = p0 ? ex.K[1] : ex.K[0], committed = run;
-    int par = p0 ? ex.out[1] : ex.out[0], first = kXPer;
-    double vf = 0.0;
-#pragma unroll
-    for (int q = 0; q < kXPer; ++q) {
-      if (q < cnt && first == kXPer) {
-        long long kf;
-        bool tie;
-        bool ok = x_term(v[q], inv_u, kf, tie);
-        if (ok) {
-          int p2 = par;
-          const long long k = x_step(kf, tie, p2);
-          ok = x_inside(S0, S0 + run + k);
-          if (ok) run += k, par = p2;
-        }
-        if (!ok) first = q, committed = run, vf = v[q];
-      }
-    }
-    const unsigned fail = __ballot_sync(kFull, first < kXPer);
-    if (fail == 0) {
-      const long long total = __shfl_sync(kFull, p0 ? inc.K[1] : inc.K[0], 31);
-      s = static_cast<double>(S0 + total) * u;
-      pos = pos + 32LL * kXPer < b ? pos + 32LL * kXPer : b;
-#pragma unroll
-      for (int q = 0; q < kXPer; ++q) v[q] = nx[q];
-      continue;
-    }
-    const int fl = __ffs(fail) - 1;
-    const int fq = __shfl_sync(kFull, first, fl);
-    committed = __shfl_sync(kFull, committed, fl);
-    vf = __shfl_sync(kFull, vf, fl);
-    s = static_cast<double>(S0 + committed) * u;  // the valid prefix (nothing when it is empty)
-    s += vf;                                      // the failing term, as the sequential chain adds it
-    const long long f = static_cast<long long>(fl) * kXPer + fq;
-    pos += f + 1;
-    if (f < kXPer) {  // little progress: a plain run of up to 32 terms before the next window
-      const long long rem = b - pos;
-      const int n2 = rem <= 0 ? 0 : (rem < 32 ? static_cast<int>(rem) : 32);
-      const double w = lane < n2 ? t[pos + lane] : 0.0;
-      for (int j = 0; j < n2; ++j) s += __shfl_sync(kFull, w, j);
-      pos += n2;
-    }
-    x_load_window(t, pos, b, v);
-  }
-  return s;
+  return g;
 }
 
 // Commits the run r (counted in the grid u) onto the exact s when s lies in u's binade and every
@@ -536,171 +498,194 @@ __device__ __forceinline__ bool x_commit(double& s, double u, const XRun& r) {
   return true;
 }
 
-// One warp per group of kXGroup tiles: lane l composes tile l's run in order (an ordered warp
-// reduction); the group is whole when every tile counts in lane 0's grid, has no split and no bad
-// term. group_chain[g]: the chain of group g.
-static __global__ void __launch_bounds__(32 * kXChainWarps) k_xgroup(const XChain* ch, const int* group_chain,
-                                                                      int ngroups, const XTileAgg* ag,
-                                                                      XGroupAgg* gg, const int* skip) {
-  if (skip && *skip) return;
-  const int g = static_cast<int>((blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) >> 5);
+// One warp: lanes from … cnt−1 hold consecutive runs r counted in the grid u (usable where `ok`).
+// Commits onto s every run up to the first that is not usable, not in s's binade, or whose running
+// S leaves it, and returns that lane (cnt: all committed).
+__device__ __forceinline__ int x_commit_lanes(double& s, XRun r, double u, bool ok, int from, int cnt) {
   const int lane = threadIdx.x & 31;
-  if (g >= ngroups) return;
-  const XChain c = ch[group_chain[g]];
-  const int tile = c.tile0 + (g - c.group0) * kXGroup + lane;
-  const bool mine = tile < c.tile0 + c.ntiles;
-  XRun r = x_identity();
-  double u = 0.0;
-  bool ok = true;
-  if (mine) {
-    const XTileAgg& G = ag[tile];
-    r = G.pre;
-    u = G.u;
-    ok = !G.pre.bad && G.split < 0 && G.u != 0.0;
-  }
-  const double u0 = __shfl_sync(kFull, u, 0);
-  ok = __all_sync(kFull, !mine || (ok && u == u0)) != 0;
-  for (int off = 1; off < 32; off <<= 1) {  // ordered reduction: lane 0 ends with tiles 0 … 31
-    const XRun o = x_shfl_down(r, off);
-    if ((lane & (2 * off - 1)) == 0 && lane + off < 32) r = x_compose(r, o);
-  }
-  if (lane == 0) {
-    XGroupAgg out;
-    out.u = ok ? u0 : 0.0;
-    out.run = r;
-    gg[g] = out;
-  }
-}
-
-// One warp per chain (4 warps per block): tiles in order, the rest walked in windows. The tile
-// summaries are brought into shared memory 32 at a time; the lanes take one tile each and a warp
-// scan of their XRuns gives every tile its exact incoming S, so one step commits every tile up
-// to the first one that is not valid for the exact s or whose running sum changes binade. Such a
-// tile is taken on its own: its part before the change, the changing term as a plain addition,
-// its part after; what does not commit is walked in windows.
-static __global__ void __launch_bounds__(32 * kXChainWarps) k_xchain(const XChain* ch, int nch, const XTileAgg* ag,
-                                                                      const XGroupAgg* gg, const int* skip) {
-  __shared__ XTileAgg sg[kXChainWarps][32];
-  if (skip && *skip) return;
-  const int warp = static_cast<int>((blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) >> 5);
-  const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
-  if (warp >= nch) return;
-  const XChain c = ch[warp];
-  double s = c.init;
-  if (c.ntiles == 0) {
-    s = x_window_walk(c.t, c.lo, c.hi, s);
+  int e;
+  const bool have = x_binade(s, e);
+  const double us = have ? x_pow2(e - 52) : 0.0;
+  const long long S0 = have ? static_cast<long long>(s * x_pow2(52 - e)) : 0;
+  const int p0 = static_cast<int>(S0 & 1);
+  const bool mine = lane >= from && lane < cnt;
+  ok = ok && mine && have && u == us && !r.bad;
+  const unsigned unusable = __ballot_sync(kFull, mine && !ok);
+  if (unusable && __ffs(unusable) - 1 == from) return from;
+  if (!mine) r = x_identity();
+  long long Kb, total;  // the change of S before this lane's run, and over all
+  bool valid = false;
+  if (!__any_sync(kFull, r.ties)) {
+    long long inc = r.K[0];
+    for (int off = 1; off < 32; off <<= 1) {
+      const long long o = __shfl_up_sync(kFull, inc, off);
+      if (lane >= off) inc += o;
+    }
+    Kb = inc - r.K[0];
+    total = __shfl_sync(kFull, inc, 31);
+    if (ok) valid = x_inside(S0, S0 + Kb + r.mn[0]) && x_inside(S0, S0 + Kb + r.mx[0]);
   } else {
-    int g0 = 0;  // the next tile, a multiple of kXGroup
-    while (g0 < c.ntiles) {
-      if (gg && c.ngroups > 0) {
-        // whole groups first: up to 32 groups (32 · kXGroup tiles) per scan, committed up to the
-        // first group that is not whole, not in this binade, or whose running sum leaves it
-        const int gi = g0 / kXGroup;
-        const int cntg = c.ngroups - gi < 32 ? c.ngroups - gi : 32;
-        int e;
-        const bool have = x_binade(s, e);
-        const double u = have ? x_pow2(e - 52) : 0.0;
-        const long long S0 = have ? static_cast<long long>(s * x_pow2(52 - e)) : 0;
-        const int p0 = static_cast<int>(S0 & 1);
-        XRun r = x_identity();
-        bool mine_ok = false;
-        if (lane < cntg) {
-          const XGroupAgg& G = gg[c.group0 + gi + lane];
-          mine_ok = have && G.u == u && !G.run.bad;
-          r = G.run;
-        }
-        XRun inc = r;
-        for (int off = 1; off < 32; off <<= 1) {
-          const XRun o = x_shfl_up(inc, off);
-          if (lane >= off) inc = x_compose(o, inc);
-        }
-        XRun ex = x_shfl_up(inc, 1);
-        if (lane == 0) ex = x_identity();
-        const long long Kb = p0 ? ex.K[1] : ex.K[0];
-        const int pb = p0 ? ex.out[1] : ex.out[0];
-        bool valid = false;
-        if (mine_ok) {
-          const long long mn = pb ? r.mn[1] : r.mn[0], mx = pb ? r.mx[1] : r.mx[0];
-          valid = x_inside(S0, S0 + Kb + mn) && x_inside(S0, S0 + Kb + mx);
-        }
-        const unsigned bad = __ballot_sync(kFull, lane < cntg && !valid);
-        const int f = bad ? __ffs(bad) - 1 : cntg;  // first group not committed
-        if (f > 0) {
-          const long long K = f < 32 ? __shfl_sync(kFull, Kb, f & 31) : __shfl_sync(kFull, p0 ? inc.K[1] : inc.K[0], 31);
-          s = static_cast<double>(S0 + K) * u;
-        }
-        g0 += f * kXGroup;
-        if (f == cntg) continue;  // every loaded group taken: the next 32 groups
-      }
-      if (g0 >= c.ntiles) break;
-      // tiles g0 … g0 + 31 one by one
-      const int cnt = c.ntiles - g0 < 32 ? c.ntiles - g0 : 32;
-      __syncwarp();
-      if (lane < cnt) sg[wl][lane] = ag[c.tile0 + g0 + lane];
-      __syncwarp();
-      int j = 0;
-      while (j < cnt) {
-        int e;
-        const bool have = x_binade(s, e);
-        const double u = have ? x_pow2(e - 52) : 0.0;
-        const long long S0 = have ? static_cast<long long>(s * x_pow2(52 - e)) : 0;
-        const int p0 = static_cast<int>(S0 & 1);
-        // lane l >= j: tile l's run if it stays in this binade; lanes below j: nothing
-        XRun r = x_identity();
-        bool mine_ok = false;
-        if (lane >= j && lane < cnt) {
-          const XTileAgg& G = sg[wl][lane];
-          mine_ok = have && !G.pre.bad && G.split < 0 && G.u == u;
-          r = G.pre;
-        }
-        XRun inc = r;
-        for (int off = 1; off < 32; off <<= 1) {
-          const XRun o = x_shfl_up(inc, off);
-          if (lane >= off) inc = x_compose(o, inc);
-        }
-        XRun ex = x_shfl_up(inc, 1);
-        if (lane == 0) ex = x_identity();
-        const long long Kb = p0 ? ex.K[1] : ex.K[0];
-        const int pb = p0 ? ex.out[1] : ex.out[0];
-        bool valid = false;
-        if (mine_ok) {
-          const long long mn = pb ? r.mn[1] : r.mn[0], mx = pb ? r.mx[1] : r.mx[0];
-          valid = x_inside(S0, S0 + Kb + mn) && x_inside(S0, S0 + Kb + mx);
-        }
-        const unsigned bad = __ballot_sync(kFull, lane >= j && lane < cnt && !valid);
-        const int f = bad ? __ffs(bad) - 1 : cnt;  // first tile not committed
-        if (f > j) {  // tiles j … f−1: S0 plus the exclusive change at tile f (or the total)
-          const long long K = f < 32 ? __shfl_sync(kFull, Kb, f & 31) : __shfl_sync(kFull, p0 ? inc.K[1] : inc.K[0], 31);
-          s = static_cast<double>(S0 + K) * u;
-        }
-        if (f < cnt) {  // tile f on its own
-          long long a, b;
-          x_tile_range(c, c.tile0 + g0 + f, a, b);
-          long long resume = a;
-          if (lane == 0) {
-            const XTileAgg& G = sg[wl][f];
-            double s2 = s;
-            if (x_commit(s2, G.u, G.pre)) {
-              if (G.split < 0) {
-                resume = b;
-              } else {
-                s2 += c.t[a + G.split];  // the term that changes the binade, as the chain adds it
-                resume = a + G.split + 1;
-                if (x_commit(s2, G.u1, G.suf)) resume = b;
-              }
-              s = s2;
-            }
-          }
-          s = __shfl_sync(kFull, s, 0);
-          resume = __shfl_sync(kFull, resume, 0);
-          if (resume < b) s = x_window_walk(c.t, resume, b, s);
-        }
-        j = f + 1;
-      }
-      g0 += 32;
+    XRun inc = r;
+    for (int off = 1; off < 32; off <<= 1) {
+      const XRun o = x_shfl_up(inc, off);
+      if (lane >= off) inc = x_compose(o, inc);
+    }
+    XRun ex = x_shfl_up(inc, 1);
+    if (lane == 0) ex = x_identity();
+    Kb = p0 ? ex.K[1] : ex.K[0];
+    const int pb = p0 ? ex.out[1] : ex.out[0];
+    total = __shfl_sync(kFull, p0 ? inc.K[1] : inc.K[0], 31);
+    if (ok) {
+      const long long mn = pb ? r.mn[1] : r.mn[0], mx = pb ? r.mx[1] : r.mx[0];
+      valid = x_inside(S0, S0 + Kb + mn) && x_inside(S0, S0 + Kb + mx);
     }
   }
-  if (lane == 0) *c.out = s;
+  const unsigned bad = __ballot_sync(kFull, mine && !valid);
+  const int f = bad ? __ffs(bad) - 1 : cnt;  // the first run not committed
+  const long long upto = __shfl_sync(kFull, Kb, f & 31);
+  if (f > from) s = static_cast<double>(S0 + (f < 32 ? upto : total)) * us;
+  return f;
+}
+
+// The chain c from its tiles' and groups' summaries (one warp; sg: room for 32 tile summaries).
+__device__ __forceinline__ double x_walk(const XChain& c, const XTileAgg* ag, const XGroupAgg* gg, XTileAgg* sg,
+                                         double* sh) {
+  const int lane = threadIdx.x & 31;
+  double s = c.init;
+  int g0 = 0;  // the next group
+  while (g0 < c.ngroups) {
+    // whole groups first, up to 32 per scan
+    const int cntg = c.ngroups - g0 < 32 ? c.ngroups - g0 : 32;
+    XGroupAgg G;
+    G.u = 0.0;
+    G.run = x_identity();
+    if (lane < cntg) G = x_load(gg + c.group0 + g0 + lane);
+    const int f = x_commit_lanes(s, G.run, G.u, G.u != 0.0, 0, cntg);
+    g0 += f;
+    if (f == cntg) continue;
+    // the group that was not taken whole: its tiles
+    const int t0 = g0 * kXGroup, cnt = c.ntiles - t0 < kXGroup ? c.ntiles - t0 : kXGroup;
+    __syncwarp();
+    if (lane < cnt) sg[lane] = x_load(ag + c.tile0 + t0 + lane);
+    __syncwarp();
+    int j = 0;
+    while (j < cnt) {
+      XRun r = x_identity();
+      double u = 0.0;
+      bool ok = false;
+      if (lane < cnt) r = sg[lane].pre, u = sg[lane].u, ok = sg[lane].split < 0 && u != 0.0;
+      const int k = x_commit_lanes(s, r, u, ok, j, cnt);
+      if (k < cnt) {  // tile k on its own
+        long long a, b;
+        x_tile_range(c, c.tile0 + t0 + k, a, b);
+        const XTileAgg& T = sg[k];
+        long long resume = a;
+        double s2 = s;
+        if (x_commit(s2, T.u, T.pre)) {
+          if (T.split < 0) {
+            resume = b;
+          } else {
+            s2 += T.at;  // the term that changes the binade, as the chain adds it
+            resume = a + T.split + 1;
+            if (x_commit(s2, T.u1, T.suf)) resume = b;
+          }
+          s = s2;
+        }
+        if (resume < b) s = x_add(c.t, resume, b, s, sh);
+      }
+      j = k + 1;
+    }
+    ++g0;
+  }
+  return s;
+}
+
+// Blocks [0, ngroups): one group of tiles each (group_chain: its chain). The blocks after them:
+// one chain of at most kXShort terms per warp (short_chain). chain_done / job_done count a chain's
+// finished groups and a job's finished chains; the last one goes on, and sets its counter back to
+// zero for the next launch.
+static __global__ void __launch_bounds__(32 * kXWarps) k_xwalk(const XChain* __restrict__ ch, const XJob* jobs,
+                                                               const int* group_chain, int ngroups,
+                                                               const int* short_chain, int nshort, const double* stat,
+                                                               XTileAgg* ag, XGroupAgg* gg, unsigned* chain_done,
+                                                               unsigned* job_done, const int* skip) {
+  __shared__ XTileAgg sg[kXGroup];
+  __shared__ alignas(16) double sh_add[kXWarps][kXTile];
+  __shared__ double sh_sum[kXWarps];
+  if (skip && *skip) return;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  int ci;
+  double s;
+  if (static_cast<int>(blockIdx.x) < ngroups) {
+    const int g = blockIdx.x;
+    ci = group_chain[g];
+    const XChain c = ch[ci];
+    const int t0 = (g - c.group0) * kXGroup, cnt = c.ntiles - t0 < kXGroup ? c.ntiles - t0 : kXGroup;
+    // the approximate sum before this group, then before each of its tiles
+    double pre = 0.0;
+    for (int k = threadIdx.x; k < t0; k += blockDim.x) pre += stat[c.tile0 + k];
+    for (int off = 16; off > 0; off >>= 1) pre += __shfl_xor_sync(kFull, pre, off);
+    if (lane == 0) sh_sum[w] = pre;
+    const double mine = lane < cnt ? stat[c.tile0 + t0 + lane] : 0.0;
+    double inc = mine;
+    for (int off = 1; off < 32; off <<= 1) {
+      const double o = __shfl_up_sync(kFull, inc, off);
+      if (lane >= off) inc += o;
+    }
+    __syncthreads();
+    pre = c.init;
+    for (int k = 0; k < kXWarps; ++k) pre += sh_sum[k];
+    for (int k = w; k < cnt; k += kXWarps) {
+      const double s0 = pre + __shfl_sync(kFull, inc - mine, k);
+      long long a, b;
+      x_tile_range(c, c.tile0 + t0 + k, a, b);
+      const XTileAgg T = x_tile_agg(c.t, a, b, s0);
+      if (lane == 0) sg[k] = T, ag[c.tile0 + t0 + k] = T;
+    }
+    __threadfence();
+    __syncthreads();
+    if (w != 0) return;
+    XRun r = x_identity();
+    double u = 0.0;
+    bool ok = true;
+    if (lane < cnt) r = sg[lane].pre, u = sg[lane].u, ok = !r.bad && sg[lane].split < 0 && u != 0.0;
+    const double u0 = __shfl_sync(kFull, u, 0);
+    ok = __all_sync(kFull, lane >= cnt || (ok && u == u0)) != 0;
+    r = x_warp_ordered(r);
+    unsigned last = 0;
+    if (lane == 0) {
+      XGroupAgg G;
+      G.u = ok ? u0 : 0.0;
+      G.run = r;
+      gg[g] = G;
+      __threadfence();
+      last = atomicAdd(chain_done + ci, 1u) + 1u == static_cast<unsigned>(c.ngroups) ? 1u : 0u;
+      if (last) chain_done[ci] = 0u;
+    }
+    if (!__shfl_sync(kFull, last, 0)) return;
+    __threadfence();
+    s = x_walk(c, ag, gg, sg, sh_add[0]);
+  } else {
+    const int k = (static_cast<int>(blockIdx.x) - ngroups) * kXWarps + w;
+    if (k >= nshort) return;
+    ci = short_chain[k];
+    s = x_add(ch[ci].t, ch[ci].lo, ch[ci].hi, ch[ci].init, sh_add[w]);
+  }
+  const XChain& c = ch[ci];
+  unsigned last = 0;
+  if (lane == 0) {
+    *c.out = s;
+    if (c.job >= 0) {
+      __threadfence();
+      last = atomicAdd(job_done + c.job, 1u) + 1u == static_cast<unsigned>(jobs[c.job].chunks) ? 1u : 0u;
+      if (last) job_done[c.job] = 0u;
+    }
+  }
+  if (!__shfl_sync(kFull, last, 0)) return;
+  __threadfence();
+  const XJob& J = jobs[c.job];
+  s = x_add(J.part, 0, J.chunks, J.init, sh_add[w]);
+  if (lane == 0) *J.out = s;
 }
 
 static __global__ void k_tree1(const TreeSeg* segs, int nseg, double* partials, const int* skip) {
@@ -742,56 +727,52 @@ class SumPlan {
     exact_ = exact;
     skip_ = skip;
     if (exact) {
-      std::vector<XChain> phase1, phase2;
-      std::vector<int> tile_chain;
+      std::vector<XChain> chains;
+      std::vector<XJob> jobs;
+      std::vector<int> tile_chain, group_chain, short_chain;
       long long nchunk_jobs = 0;
       for (const Job& j : jobs_)
         if (j.order == SumOrder::kChunk64) ++nchunk_jobs;
       partials_.alloc(static_cast<std::size_t>(nchunk_jobs > 0 ? nchunk_jobs * kChunks : 1));
-      auto chain = [&](const double* t, long long lo, long long hi, double init, double* out) {
-        XChain c{t, lo, hi, init, out, static_cast<int>(tile_chain.size()), 0, 0, 0};
-        const long long n = hi - lo;
-        if (n >= 2LL * kXTile) {  // long chains go by tiles; short ones by windows only
-          c.ntiles = static_cast<int>((n + kXTile - 1) / kXTile);
-          for (int k = 0; k < c.ntiles; ++k) tile_chain.push_back(static_cast<int>(phase1.size()));
+      auto chain = [&](const double* t, long long lo, long long hi, double init, double* out, int job) {
+        XChain c{t, lo, hi, init, out, static_cast<int>(tile_chain.size()), 0, static_cast<int>(group_chain.size()), 0, job};
+        const int id = static_cast<int>(chains.size());
+        if (hi - lo > kXShort) {
+          c.ntiles = static_cast<int>((hi - lo + kXTile - 1) / kXTile);
+          c.ngroups = (c.ntiles + kXGroup - 1) / kXGroup;
+          tile_chain.insert(tile_chain.end(), static_cast<std::size_t>(c.ntiles), id);
+          group_chain.insert(group_chain.end(), static_cast<std::size_t>(c.ngroups), id);
+        } else {
+          short_chain.push_back(id);
         }
-        phase1.push_back(c);
+        chains.push_back(c);
       };
-      long long slot = 0;
       for (const Job& j : jobs_) {
         const long long n = j.hi - j.lo;
         if (j.order == SumOrder::kSeq) {
-          chain(j.t, j.lo, j.hi, j.init, j.out);
-        } else {
+          chain(j.t, j.lo, j.hi, j.init, j.out, -1);
+        } else {  // parallel_sum: the chunks' sums added in order
           const long long chunks = n < kChunks ? (n < 1 ? 1 : n) : kChunks;
-          double* part = partials_.get() + slot * kChunks;
+          double* part = partials_.get() + static_cast<long long>(jobs.size()) * kChunks;
           for (long long c = 0; c < chunks; ++c)
-            chain(j.t, j.lo + n * c / chunks, j.lo + n * (c + 1) / chunks, 0.0, part + c);
-          // parallel_sum: s = 0; s += part[c] in order — then the caller's init (0 for dots)
-          phase2.push_back({part, 0, chunks, j.init, j.out, 0, 0, 0, 0});
-          ++slot;
+            chain(j.t, j.lo + n * c / chunks, j.lo + n * (c + 1) / chunks, 0.0, part + c, static_cast<int>(jobs.size()));
+          jobs.push_back({part, static_cast<int>(chunks), j.init, j.out});
         }
       }
       ntiles_ = static_cast<int>(tile_chain.size());
-      // chains of more than one group of tiles also get group summaries (k_xgroup)
-      std::vector<int> group_chain;
-      for (std::size_t k = 0; k < phase1.size(); ++k) {
-        XChain& c = phase1[k];
-        if (c.ntiles <= kXGroup) continue;
-        c.group0 = static_cast<int>(group_chain.size());
-        c.ngroups = (c.ntiles + kXGroup - 1) / kXGroup;
-        for (int g = 0; g < c.ngroups; ++g) group_chain.push_back(static_cast<int>(k));
-      }
       ngroups_ = static_cast<int>(group_chain.size());
-      upload(group_chain, group_chain_, st);
-      group_agg_.alloc(static_cast<std::size_t>(ngroups_ > 0 ? ngroups_ : 1) * sizeof(XGroupAgg));
-      upload(phase1, seg1_, st);
-      upload(phase2, seg2_, st);
+      nshort_ = static_cast<int>(short_chain.size());
+      upload(chains, chains_, st);
+      upload(jobs, xjobs_, st);
       upload(tile_chain, tile_chain_, st);
-      tile_stat_.alloc(static_cast<std::size_t>(ntiles_ > 0 ? ntiles_ : 1) * sizeof(XTileStat));
+      upload(group_chain, group_chain_, st);
+      upload(short_chain, short_chain_, st);
+      stat_.alloc(static_cast<std::size_t>(ntiles_ > 0 ? ntiles_ : 1));
       tile_agg_.alloc(static_cast<std::size_t>(ntiles_ > 0 ? ntiles_ : 1) * sizeof(XTileAgg));
-      n1_ = static_cast<int>(phase1.size());
-      n2_ = static_cast<int>(phase2.size());
+      group_agg_.alloc(static_cast<std::size_t>(ngroups_ > 0 ? ngroups_ : 1) * sizeof(XGroupAgg));
+      done_.alloc(chains.size() + jobs.size() + 1);
+      B200_CHECK(cudaMemsetAsync(done_.get(), 0, (chains.size() + jobs.size() + 1) * sizeof(unsigned), st));
+      nchains_ = static_cast<int>(chains.size());
     } else {
       std::vector<TreeSeg> tree;
       for (const Job& j : jobs_) tree.push_back({j.t, j.lo, j.hi, j.init, j.out});
@@ -800,30 +781,24 @@ class SumPlan {
       partials_.alloc(static_cast<std::size_t>(nt_ > 0 ? nt_ : 1) * kTreeBlocks);
     }
   }
-  void launch(cudaStream_t st) const {
+  // The tile sums a producer may leave itself (x_leave_stat) before launch(st, true): of the plan's
+  // only chain, starting at its first term. Null when the chain needs none.
+  double* stat() { return exact_ && ntiles_ > 0 ? stat_.get() : nullptr; }
+  void launch(cudaStream_t st, bool have_stat = false) const {
     if (exact_) {
-      const XChain* c1 = reinterpret_cast<const XChain*>(seg1_.get());
-      const int* tc = reinterpret_cast<const int*>(tile_chain_.get());
-      XTileStat* ts = reinterpret_cast<XTileStat*>(tile_stat_.get());
-      XTileAgg* ta = reinterpret_cast<XTileAgg*>(tile_agg_.get());
-      XGroupAgg* tg = ngroups_ > 0 ? reinterpret_cast<XGroupAgg*>(group_agg_.get()) : nullptr;
-      if (ntiles_ > 0) {
-        k_xstat<<<ntiles_, kXThreads, 0, st>>>(c1, tc, ts, skip_);
-        k_xagg<<<ntiles_, kXThreads, 0, st>>>(c1, tc, ts, ta, skip_);
+      const XChain* ch = reinterpret_cast<const XChain*>(chains_.get());
+      if (ntiles_ > 0 && !have_stat) {
+        k_xstat<<<(ntiles_ + 7) / 8, 256, 0, st>>>(ch, reinterpret_cast<const int*>(tile_chain_.get()), ntiles_,
+                                                   stat_.get(), skip_);
         B200_LAUNCH_CHECK();
       }
-      if (ngroups_ > 0) {
-        k_xgroup<<<(ngroups_ + kXChainWarps - 1) / kXChainWarps, 32 * kXChainWarps, 0, st>>>(
-            c1, reinterpret_cast<const int*>(group_chain_.get()), ngroups_, ta, tg, skip_);
-        B200_LAUNCH_CHECK();
-      }
-      if (n1_ > 0) {
-        k_xchain<<<(n1_ + kXChainWarps - 1) / kXChainWarps, 32 * kXChainWarps, 0, st>>>(c1, n1_, ta, tg, skip_);
-        B200_LAUNCH_CHECK();
-      }
-      if (n2_ > 0) {
-        k_xchain<<<(n2_ + kXChainWarps - 1) / kXChainWarps, 32 * kXChainWarps, 0, st>>>(
-            reinterpret_cast<const XChain*>(seg2_.get()), n2_, ta, nullptr, skip_);
+      const int blocks = ngroups_ + (nshort_ + kXWarps - 1) / kXWarps;
+      if (blocks > 0) {
+        k_xwalk<<<blocks, 32 * kXWarps, 0, st>>>(
+            ch, reinterpret_cast<const XJob*>(xjobs_.get()), reinterpret_cast<const int*>(group_chain_.get()), ngroups_,
+            reinterpret_cast<const int*>(short_chain_.get()), nshort_, stat_.get(),
+            reinterpret_cast<XTileAgg*>(tile_agg_.get()), reinterpret_cast<XGroupAgg*>(group_agg_.get()), done_.get(),
+            done_.get() + nchains_, skip_);
         B200_LAUNCH_CHECK();
       }
     } else if (nt_ > 0) {
@@ -835,7 +810,7 @@ class SumPlan {
     }
   }
   int kernel_count() const {
-    return exact_ ? 2 * (ntiles_ > 0) + (ngroups_ > 0) + (n1_ > 0) + (n2_ > 0) : (nt_ > 0 ? 2 : 0);
+    return exact_ ? (ntiles_ > 0) + (ngroups_ + nshort_ > 0) : (nt_ > 0 ? 2 : 0);
   }
   bool empty() const { return jobs_.empty(); }
 
@@ -859,10 +834,11 @@ class SumPlan {
   std::vector<Job> jobs_;
   bool exact_ = false;
   const int* skip_ = nullptr;
-  DevBuf<unsigned char> seg1_, seg2_, tseg_, tile_chain_, group_chain_;
-  mutable DevBuf<unsigned char> tile_stat_, tile_agg_, group_agg_;
-  mutable DevBuf<double> partials_;
-  int n1_ = 0, n2_ = 0, nt_ = 0, ntiles_ = 0, ngroups_ = 0;
+  DevBuf<unsigned char> chains_, xjobs_, tseg_, tile_chain_, group_chain_, short_chain_;
+  mutable DevBuf<unsigned char> tile_agg_, group_agg_;
+  mutable DevBuf<double> partials_, stat_;
+  mutable DevBuf<unsigned> done_;
+  int nchains_ = 0, nshort_ = 0, nt_ = 0, ntiles_ = 0, ngroups_ = 0;
 };
 
 }  // namespace b200
