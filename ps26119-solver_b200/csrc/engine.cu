@@ -35,6 +35,7 @@
 #include "engine.hpp"
 #include "parallel.hpp"
 #include "problem.cuh"
+#include "resident.cuh"
 #include "tune.hpp"
 
 namespace b200 {
@@ -97,9 +98,20 @@ double slot_max(const double* h, int s) { return h[s]; }  // bit pattern of a no
 template <class T>
 struct IterVecs {
   DevBuf<T> x, x0, xh, xb, dx, ddx, y, y0, yh, yb, dy, adx, ddy;
+  // resident epochs (resident.cuh): the points after a Halpern cycle's first step, the cells of x̄ and y
+  DevBuf<T> xh0, xb0, yh0, yb0;
+  DevBuf<Cell<T>> xcell, ycell;
   void alloc(int n, int m) {
     for (DevBuf<T>* v : {&x, &x0, &xh, &xb, &dx, &ddx}) v->alloc(static_cast<std::size_t>(n));
     for (DevBuf<T>* v : {&y, &y0, &yh, &yb, &dy, &adx, &ddy}) v->alloc(static_cast<std::size_t>(m));
+  }
+  void alloc_resident(int n, int m, cudaStream_t st) {
+    for (DevBuf<T>* v : {&xh0, &xb0}) v->alloc(static_cast<std::size_t>(n));
+    for (DevBuf<T>* v : {&yh0, &yb0}) v->alloc(static_cast<std::size_t>(m));
+    xcell.alloc(static_cast<std::size_t>(n)), ycell.alloc(static_cast<std::size_t>(m));
+    // tag 0 everywhere: the first epoch's tags start above it
+    B200_CHECK(cudaMemsetAsync(xcell.get(), 0, static_cast<std::size_t>(n) * sizeof(Cell<T>), st));
+    B200_CHECK(cudaMemsetAsync(ycell.get(), 0, static_cast<std::size_t>(m) * sizeof(Cell<T>), st));
   }
 };
 
@@ -110,7 +122,9 @@ __global__ void k_diff(long long n, const T* a, const T* b, T* out) {  // out = 
 
 class Engine {
  public:
-  Engine(const DeviceModel& M, const EngineOptions& o, cudaStream_t st) : M_(M), o_(o), st_(st) {
+  // grouped: the epochs are launched by a GroupScheduler
+  Engine(const DeviceModel& M, const EngineOptions& o, cudaStream_t st, bool grouped)
+      : M_(M), o_(o), st_(st), grouped_(grouped) {
     for (auto& e : ev_) B200_CHECK(cudaEventCreate(&e));
   }
   ~Engine() {
@@ -201,7 +215,11 @@ class Engine {
   template <class T> void capture_epoch();
   template <class T> void capture_check(int variant);
   template <class T> void launch_residual(bool with_restart_terms, const int* skip, SumPlan& plan,
-                                          cudaStream_t sums_on = nullptr);
+                                          cudaStream_t sums_on = nullptr, bool resident_first = false);
+  template <class T> void plan_resident(int max_row, int max_col);
+  template <class T> void launch_resident_epoch();
+  template <class T> void launch_resident_pdlp(int cur);
+  bool resident() const { return shape_[mixed_now_ ? 1 : 0].blocks > 0; }
   template <class T> void launch_kkt_scaled(const T* xs, const T* ys, cudaStream_t on = nullptr);
   void launch_kkt_original(cudaStream_t on = nullptr);
   void make_side_streams();
@@ -237,6 +255,9 @@ class Engine {
   DeviceModel M_;
   const EngineOptions& o_;
   cudaStream_t st_;
+  bool grouped_;
+  ResidentShape shape_[2];  // resident epochs in fp64 / fp32 (blocks = 0: the step kernels)
+  unsigned tag_ = 1;        // the next resident epoch's first tag
   DevBuf<unsigned> stage_err_;  // this solve's bulk-copy timeouts (see count_stage_timeout)
   clock::time_point t0_;
   ScaledDevice sp_;
@@ -312,10 +333,26 @@ void Engine::setup() {
   if (n > 0) k_slab_table<<<grid_for(slab_count(n)), kBlock, 0, st_>>>(n, M_.col_start, slab_t_.get());
   B200_LAUNCH_CHECK();
   kernels_ += 2;
-  cap_a_ = fed_tile_capacity(slab_max_nnz(slab_a_.get(), slab_count(m), st_));
-  cap_t_ = fed_tile_capacity(slab_max_nnz(slab_t_.get(), slab_count(n), st_));
+  // the largest slabs (the kernels' tile capacities), rows and columns
+  int ext[4] = {0, 0, 0, 0};
+  {
+    DevBuf<int> d(4);
+    B200_CHECK(cudaMemsetAsync(d.get(), 0, sizeof ext, st_));
+    if (m > 0) k_extents<<<std::min(grid_for(m), 8 * sm_count()), kBlock, 0, st_>>>(m, sp_.a_rp.get(), d.get());
+    if (n > 0) k_extents<<<std::min(grid_for(n), 8 * sm_count()), kBlock, 0, st_>>>(n, sp_.t_rp.get(), d.get() + 2);
+    B200_LAUNCH_CHECK();
+    kernels_ += 2;
+    B200_CHECK(cudaMemcpyAsync(ext, d.get(), sizeof ext, cudaMemcpyDeviceToHost, st_));
+    B200_CHECK(cudaStreamSynchronize(st_));
+  }
+  cap_a_ = fed_tile_capacity(ext[0]);
+  cap_t_ = fed_tile_capacity(ext[2]);
   vd_.alloc(n, m);
   if (o_.mixed) vf_.alloc(n, m);
+  if (!grouped_ && tune_forced() < 0) {  // a forced step-kernel variant runs the step kernels
+    plan_resident<double>(ext[1], ext[3]);
+    if (o_.mixed) plan_resident<float>(ext[1], ext[3]);
+  }
   params_.alloc(1);
   hparams_.alloc(1);
   res_.alloc(kNumSlots);
@@ -457,8 +494,10 @@ void Engine::build_plans() {
 // The residual: dx = x̄ − x̂, adx = Ã dx, dy = ȳ − ŷ and the terms of the five dots.
 // sums_on: the stream of the dots' sums (nullptr: the engine's; another stream must already wait for
 // the engine's stream, and the caller joins it back).
+// resident_first: of the points that a resident epoch left after its first step.
 template <class T>
-void Engine::launch_residual(bool with_restart_terms, const int* skip, SumPlan& plan, cudaStream_t sums_on) {
+void Engine::launch_residual(bool with_restart_terms, const int* skip, SumPlan& plan, cudaStream_t sums_on,
+                             bool resident_first) {
   IterVecs<T>& v = vecs<T>();
   const int m = M_.m, n = M_.n;
   double* px = rt_.get();
@@ -466,10 +505,11 @@ void Engine::launch_residual(bool with_restart_terms, const int* skip, SumPlan& 
   double* py = dxn + n;
   double* cross = py + m;
   double* dyn = cross + m;
-  k_res_x<T><<<grid_for(n), kBlock, 0, st_>>>(n, v.xb.get(), v.xh.get(), v.x0.get(), v.dx.get(), px,
-                                              with_restart_terms ? dxn : nullptr, skip);
+  const bool f = resident_first;
+  k_res_x<T><<<grid_for(n), kBlock, 0, st_>>>(n, (f ? v.xb0 : v.xb).get(), (f ? v.xh0 : v.xh).get(), v.x0.get(),
+                                              v.dx.get(), px, with_restart_terms ? dxn : nullptr, skip);
   B200_LAUNCH_CHECK();
-  EpiResY<T> e{v.yb.get(), v.yh.get(), v.y0.get(), v.dy.get(), v.adx.get(), py, cross,
+  EpiResY<T> e{(f ? v.yb0 : v.yb).get(), (f ? v.yh0 : v.yh).get(), v.y0.get(), v.dy.get(), v.adx.get(), py, cross,
                with_restart_terms ? dyn : nullptr, skip};
   launch_slab_tma<T>(m, sp_.a_rp.get(), sp_.a_col.get(), sp_.A_val<T>(), v.dx.get(), e, st_, nullptr, err());
   cudaStream_t ss = st_;
@@ -983,8 +1023,60 @@ void Engine::begin_epoch() {
   L_.fresh = L_.inner == 0;
 }
 
+// Whether this solve's epochs are resident in precision T, and their buffers: the rule is that the
+// matrix and the updates' vectors fit the SMs' shared memory (resident_shape).
+template <class T>
+void Engine::plan_resident(int max_row, int max_col) {
+  ResidentShape& s = shape_[std::is_same<T, float>::value ? 1 : 0];
+  s = resident_shape<T, ResidentR2h<T>>(M_.m, M_.n, M_.nnz, max_row, max_col);
+  if (s.blocks > 0) vecs<T>().alloc_resident(M_.n, M_.m, st_);
+}
+
+template <class T>
+void Engine::launch_resident_epoch() {
+  IterVecs<T>& v = vecs<T>();
+  const StepParams& hp = *hparams_.get();
+  ResidentPart<T, ResidentR2h<T>> p{
+      M_.m, M_.n, 0, shape_[std::is_same<T, float>::value ? 1 : 0].blocks, sp_.t_rp.get(), sp_.t_ri.get(), sp_.a_rp.get(),
+      sp_.a_col.get(), sp_.At_val<T>(), sp_.A_val<T>(), v.xcell.get(), v.ycell.get(), tag_, err(),
+      {v.x.get(), v.xh.get(), v.xb.get(), v.y.get(), v.yh.get(), v.yb.get(), v.x0.get(), sp_.c<T>(), sp_.l<T>(), sp_.u<T>(),
+       v.y0.get(), sp_.rl<T>(), sp_.ru<T>(), v.xh0.get(), v.xb0.get(), v.yh0.get(), v.yb0.get(), hp.tau, hp.sigma, hp.rho,
+       hp.inner0, hp.K}};
+  B200_CHECK(cudaEventRecord(ev_[0], st_));
+  launch_resident(p, shape_[std::is_same<T, float>::value ? 1 : 0], st_);
+  B200_CHECK(cudaEventRecord(ev_[1], st_));
+  tag_ += static_cast<unsigned>(hp.K) + 1;
+  ++kernels_;
+  if (L_.fresh) launch_residual<T>(false, nullptr, plan_r0_, nullptr, true);
+}
+
+template <class T>
+void Engine::launch_resident_pdlp(int cur) {
+  IterVecs<T>& v = vecs<T>();
+  const StepParams& hp = *hparams_.get();
+  const bool odd = (hp.K & 1) != 0;
+  T* xs[2] = {v.x.get(), v.xh.get()};
+  T* ys[2] = {v.y.get(), v.yh.get()};
+  const int out = odd ? 1 - cur : cur;  // the buffers alternate from step to step
+  ResidentPart<T, ResidentPdlp<T>> p{
+      M_.m, M_.n, 0, shape_[std::is_same<T, float>::value ? 1 : 0].blocks, sp_.t_rp.get(), sp_.t_ri.get(), sp_.a_rp.get(),
+      sp_.a_col.get(), sp_.At_val<T>(), sp_.A_val<T>(), v.xcell.get(), v.ycell.get(), tag_, err(),
+      {xs[cur], sp_.c<T>(), sp_.l<T>(), sp_.u<T>(), ys[cur], sp_.rl<T>(), sp_.ru<T>(), v.dx.get(), v.dy.get(), xs[out],
+       xs[1 - out], v.xb.get(), ys[out], ys[1 - out], hp.tau, hp.sigma, hp.inner0, hp.K}};
+  B200_CHECK(cudaEventRecord(ev_[0], st_));
+  launch_resident(p, shape_[std::is_same<T, float>::value ? 1 : 0], st_);
+  B200_CHECK(cudaEventRecord(ev_[1], st_));
+  tag_ += static_cast<unsigned>(hp.K) + 1;
+  ++kernels_;
+}
+
 void Engine::launch_epoch() {
   const int pidx = mixed_now_ ? 1 : 0;
+  if (resident()) {
+    if (mixed_now_) launch_resident_epoch<float>();
+    else launch_resident_epoch<double>();
+    return;
+  }
   if (mixed_now_) capture_epoch<float>();
   else capture_epoch<double>();
   B200_CHECK(cudaGraphLaunch(g_epoch_[pidx], st_));
@@ -1105,6 +1197,7 @@ EngineResult Engine::run(const DeviceOutputs& out) {
   if (start(out)) return R_;
   const int K = o_.check_every;
   for (;;) {
+    const bool stepped_resident = resident();
     begin_epoch();
     launch_epoch();
     launch_check();
@@ -1112,7 +1205,7 @@ EngineResult Engine::run(const DeviceOutputs& out) {
     {  // the iteration kernels' time, from the events inside the epoch graph
       float a = 0, b = 0;
       B200_CHECK(cudaEventElapsedTime(&a, ev_[0], ev_[1]));
-      B200_CHECK(cudaEventElapsedTime(&b, ev_[2], ev_[3]));
+      if (!stepped_resident) B200_CHECK(cudaEventElapsedTime(&b, ev_[2], ev_[3]));
       iter_ms_ += a + b;
       iter_launches_ += 2LL * K;
     }
@@ -1347,10 +1440,15 @@ EngineResult Engine::run_pdlp(const DeviceOutputs& out) {
     hp.skip_r0 = 1;
     B200_CHECK(cudaMemcpyAsync(params_.get(), &hp, sizeof(StepParams), cudaMemcpyHostToDevice, st_));
     const int pidx = mixed_now_ ? 1 : 0;
-    if (mixed_now_) capture_pdlp_epoch<float>(cur);
-    else capture_pdlp_epoch<double>(cur);
-    B200_CHECK(cudaGraphLaunch(g_pdlp_[pidx][cur], st_));
-    kernels_ += pdlp_kernels_[pidx][cur];
+    if (resident()) {
+      if (mixed_now_) launch_resident_pdlp<float>(cur);
+      else launch_resident_pdlp<double>(cur);
+    } else {
+      if (mixed_now_) capture_pdlp_epoch<float>(cur);
+      else capture_pdlp_epoch<double>(cur);
+      B200_CHECK(cudaGraphLaunch(g_pdlp_[pidx][cur], st_));
+      kernels_ += pdlp_kernels_[pidx][cur];
+    }
     it += K;
     inner += K;
     cur = (cur + K) & 1;
@@ -1651,7 +1749,6 @@ EngineResult run_engine(const DeviceModel& M, const EngineOptions& opt, const De
   EngineResult R;
   unsigned timeouts = 0;
   {
-    auto e = std::make_unique<Engine>(M, opt, st);
     // Large LPs keep their own kernels: they fill the device alone, and in lockstep with a
     // group their epochs would wait for everyone's checks. Small ones (launch-bound alone) join
     // the group. The limit is PS26119_GROUP_MAX_NNZ nonzeros (default 100,000).
@@ -1659,7 +1756,9 @@ EngineResult run_engine(const DeviceModel& M, const EngineOptions& opt, const De
       const char* e = std::getenv("PS26119_GROUP_MAX_NNZ");
       return e && *e ? std::atoll(e) : 100000LL;
     }();
-    if (t_grouped && !opt.pdlp && opt.check_every == 64 && M.nnz <= group_max_nnz) {
+    const bool grouped = t_grouped && !opt.pdlp && opt.check_every == 64 && M.nnz <= group_max_nnz;
+    auto e = std::make_unique<Engine>(M, opt, st, grouped);
+    if (grouped) {
       // setup here, on this caller's stream; the epochs in the device's group
       if (e->start(out)) {
         R = e->result();

@@ -17,8 +17,6 @@
 #include <cstddef>
 #include <cstdint>
 #include <type_traits>
-#include <vector>
-
 #include "common.cuh"
 
 namespace b200 {
@@ -788,15 +786,19 @@ static __global__ void k_slab_table(int rows, const int* rp, int2* out) {
 }
 inline int slab_count(int rows) { return rows <= 0 ? 0 : (rows + kSlabRows - 1) / kSlabRows; }
 
-// The largest slab's nonzero count, from a slab table (synchronises `st`; setup only).
-inline long long slab_max_nnz(const int2* table, int nb, cudaStream_t st) {
-  if (nb <= 0) return 0;
-  std::vector<int2> h(static_cast<std::size_t>(nb));
-  B200_CHECK(cudaMemcpyAsync(h.data(), table, h.size() * sizeof(int2), cudaMemcpyDeviceToHost, st));
-  B200_CHECK(cudaStreamSynchronize(st));
-  long long mx = 0;
-  for (const int2& r : h) mx = std::max<long long>(mx, static_cast<long long>(r.y) - r.x);
-  return mx;
+// The most nonzeros of a slab (out[0]) and of a row (out[1]); out zeroed before.
+static __global__ void k_extents(int rows, const int* __restrict__ rp, int* out) {
+  int slab = 0, row = 0;
+  B200_FOR(r, rows) {
+    const int i = static_cast<int>(r), a = rp[i];
+    row = max(row, rp[i + 1] - a);
+    if (i % kSlabRows == 0) slab = max(slab, rp[min(i + kSlabRows, rows)] - a);
+  }
+  slab = __reduce_max_sync(kFull, slab), row = __reduce_max_sync(kFull, row);
+  if ((threadIdx.x & 31) == 0) {
+    if (slab > 0) atomicMax(out, slab);
+    if (row > 0) atomicMax(out + 1, row);
+  }
 }
 
 // Number of bulk-copy waits that ran out since the library was loaded (host side).
