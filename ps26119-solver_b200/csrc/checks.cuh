@@ -35,41 +35,30 @@ __device__ __forceinline__ unsigned long long* max_slot(double* res, int s) {
 }
 
 // ---------------------------------------------------------------------- residual
-// dx = x̄ − x̂ written as the reference's axpby(−1, x̂, 1, dx) with dx = x̄; terms Δx², and the
-// restart distance (x̂ − x0)² (diff_norm2, evaluated in fp64 of the working values).
+// Of a Halpern cycle's first step: dx = x̄ − x̂ written as the reference's axpby(−1, x̂, 1, dx) with
+// dx = x̄; terms Δx².
 template <class T>
-static __global__ void k_res_x(int n, const T* __restrict__ xb, const T* __restrict__ xh, const T* __restrict__ x0,
-                        T* __restrict__ dx, double* t_px, double* t_dxn, const int* skip) {
+static __global__ void k_res_x(int n, const T* __restrict__ xb, const T* __restrict__ xh, T* __restrict__ dx,
+                               double* t_px, const int* skip) {
   if (skip && *skip) return;
   B200_FOR(j, n) {
     const T d = static_cast<T>(-1.0) * xh[j] + static_cast<T>(1.0) * xb[j];
     dx[j] = d;
     t_px[j] = static_cast<double>(d) * static_cast<double>(d);
-    if (t_dxn) {
-      const double e = static_cast<double>(xh[j]) - static_cast<double>(x0[j]);
-      t_dxn[j] = e * e;
-    }
   }
 }
-// Epilogue after adx = Ã·dx: dy = ȳ − ŷ, terms Δy², Δyᵀ(AΔx), (ŷ − y0)².
+// Epilogue after adx = Ã·dx: dy = ȳ − ŷ, terms Δy², Δyᵀ(AΔx).
 template <class T>
 struct EpiResY {
-  const T *yb, *yh, *y0;
-  T *dy, *adx;
-  double *t_py, *t_cross, *t_dyn;
+  const T *yb, *yh;
+  double *t_py, *t_cross;
   const int* skip;
   __device__ bool active() const { return !(skip && *skip); }
   __device__ void operator()(int i, double s) const {
     const T ax = static_cast<T>(s);
-    adx[i] = ax;
     const T d = static_cast<T>(-1.0) * yh[i] + static_cast<T>(1.0) * yb[i];
-    dy[i] = d;
     t_py[i] = static_cast<double>(d) * static_cast<double>(d);
     t_cross[i] = static_cast<double>(d) * static_cast<double>(ax);
-    if (t_dyn) {
-      const double e = static_cast<double>(yh[i]) - static_cast<double>(y0[i]);
-      t_dyn[i] = e * e;
-    }
   }
 };
 
@@ -231,6 +220,264 @@ struct EpiRayRows : AlwaysActive {
   }
   __device__ void flush(const Acc& a) const { warp_max_atomic(max_slot(res, slot_pviol), a.pviol); }
 };
+
+// ---------------------------------------------------------------------- a check in three kernels
+// Everything a check evaluates on the way to its sums, for r²HPDHG: the residual's Δ, the unscaled point,
+// the ray directions (kRays ≥ 1: of the last step; 2: of the drift since the restart anchor as well) and
+// their products. k_check_points makes the points, one thread per column and per row, and packs what the
+// products gather: X[j] = {x, Δx̃, d, d₂}, Y[i] = {y, r, r₂, 0}, 32 bytes, one sector. k_check_products then
+// walks every row and every column once for all of them. Each value is the one that the kernels above
+// compute, sums in the same order; the terms go to the same arrays.
+// What bounds it: for LPs up to some 100k rows the number of dependent launches (up to 15 in the longest
+// chain before, 4 now); for large ones the gathers (one of 32 bytes per nonzero and side, against five to
+// seven of 8). A check with the host's part, fp64: 10k rows 87 -> 33 us, 100k 157 -> 71, 1M 560 -> 389.
+template <class T>
+struct CheckVecs {
+  int n, m;
+  const T *xb, *xh, *x0, *yb, *yh, *y0;
+  const double *col_scale, *row_scale;
+  double bound_scale, obj_scale, sense;
+  const double *c, *cl, *cu, *rl, *ru;
+  double4 *X, *Y;
+  double *t_px, *t_dxn, *t_py, *t_cross, *t_dyn;  // residual and restart distances
+  double *k_rp2, *k_d, *k_rd2, *k_p;              // KKT (rows at [0, m), columns at [m, m + n))
+  double *r_obj, *r_mag, *r_cd, *r_cmag;          // rays
+  double *q_obj, *q_mag, *q_cd, *q_cmag;          // drift rays
+  double* res;
+};
+__device__ __forceinline__ double ray_dual(double v, double lo, double up) {  // engine.cpp:88-96
+  if (!isfinite(lo)) v = std_min(v, 0.0);
+  if (!isfinite(up)) v = std_max(v, 0.0);
+  return v;
+}
+__device__ __forceinline__ double ray_primal(double v, double lo, double up) {  // engine.cpp:130-137
+  if (isfinite(lo)) v = std_max(v, 0.0);
+  if (isfinite(up)) v = std_min(v, 0.0);
+  return v;
+}
+template <class T, int kRays>
+static __global__ void __launch_bounds__(kBlock) k_check_points(const __grid_constant__ CheckVecs<T> v, int col_blocks) {
+  const bool cols = static_cast<int>(blockIdx.x) < col_blocks;
+  const int k = (static_cast<int>(blockIdx.x) - (cols ? 0 : col_blocks)) * kBlock + static_cast<int>(threadIdx.x);
+  double mx = 0.0, mx2 = 0.0;
+  if (cols) {
+    if (k < v.n) {
+      const T xh = v.xh[k], x0 = v.x0[k];
+      const T d = static_cast<T>(-1.0) * xh + static_cast<T>(1.0) * v.xb[k];
+      const double e = static_cast<double>(xh) - static_cast<double>(x0), dd = static_cast<double>(d);
+      const double sc = v.col_scale[k], lo = v.cl[k], up = v.cu[k];
+      double4 X;
+      X.x = std_min(std_max(sc * static_cast<double>(xh) / v.bound_scale, lo), up);
+      X.y = dd, X.z = X.w = 0.0;
+      v.t_px[k] = dd * dd;
+      v.t_dxn[k] = e * e;
+      if constexpr (kRays >= 1) {
+        X.z = ray_primal(sc * dd / v.bound_scale, lo, up);
+        mx = fabs(X.z);
+      }
+      if constexpr (kRays == 2) {
+        const T g = static_cast<T>(-1.0) * x0 + static_cast<T>(1.0) * xh;
+        X.w = ray_primal(sc * static_cast<double>(g) / v.bound_scale, lo, up);
+        mx2 = fabs(X.w);
+      }
+      v.X[k] = X;
+    }
+    if constexpr (kRays >= 1) warp_max_atomic(max_slot(v.res, kMaxDabs), mx);
+    if constexpr (kRays == 2) warp_max_atomic(max_slot(v.res, kMaxDabs2), mx2);
+  } else {
+    if (k < v.m) {
+      const T yh = v.yh[k], y0 = v.y0[k];
+      const T d = static_cast<T>(-1.0) * yh + static_cast<T>(1.0) * v.yb[k];
+      const double e = static_cast<double>(yh) - static_cast<double>(y0), dd = static_cast<double>(d);
+      const double sc = v.row_scale[k];
+      double4 Y;
+      Y.x = sc * static_cast<double>(yh) / v.obj_scale;
+      Y.y = Y.z = 0.0, Y.w = 0.0;
+      v.t_py[k] = dd * dd;
+      v.t_dyn[k] = e * e;
+      if constexpr (kRays >= 1) {
+        Y.y = ray_dual(sc * dd / v.obj_scale, v.rl[k], v.ru[k]);
+        mx = fabs(Y.y);
+      }
+      if constexpr (kRays == 2) {
+        const T g = static_cast<T>(-1.0) * y0 + static_cast<T>(1.0) * yh;
+        Y.z = ray_dual(sc * static_cast<double>(g) / v.obj_scale, v.rl[k], v.ru[k]);
+        mx2 = fabs(Y.z);
+      }
+      v.Y[k] = Y;
+    }
+    if constexpr (kRays >= 1) warp_max_atomic(max_slot(v.res, kMaxRmax), mx);
+    if constexpr (kRays == 2) warp_max_atomic(max_slot(v.res, kMaxRmax2), mx2);
+  }
+}
+
+// A packed point: its first two values, or all four.
+template <bool kAll>
+__device__ __forceinline__ double4 load_packed(const double4* p) {
+  const double2 a = __ldg(reinterpret_cast<const double2*>(p));
+  double2 b = make_double2(0.0, 0.0);
+  if constexpr (kAll) b = __ldg(reinterpret_cast<const double2*>(p) + 1);
+  return make_double4(a.x, a.y, b.x, b.y);
+}
+// A ray's row terms (EpiRayRows) and column terms (k_ray_cols).
+__device__ __forceinline__ double ray_row(double ad, double r, double lo, double up, double& obj, double& mag) {
+  double viol = 0.0;
+  if (isfinite(lo)) viol = std_max(viol, -ad);
+  if (isfinite(up)) viol = std_max(viol, ad);
+  obj = r > 0 ? lo * r : (r < 0 ? up * r : 0.0);
+  mag = fabs(obj);
+  return viol;
+}
+__device__ __forceinline__ double ray_col(double g, double gabs, double lo, double up, double& obj, double& mag) {
+  const double lam = -g;
+  double viol = 0.0;
+  obj = mag = 0.0;
+  if (lam > 0) {
+    if (isfinite(lo)) obj = lo * lam, mag = gabs * fabs(lo);
+    else viol = lam;
+  } else if (lam < 0) {
+    if (isfinite(up)) obj = up * lam, mag = gabs * fabs(up);
+    else viol = -lam;
+  }
+  return viol;
+}
+// Rows of A (blocks [0, row_blocks)): original values a0 and scaled values as on one index list; columns
+// (the blocks after them): the caller's CSC.
+template <class T, int kRays>
+static __global__ void __launch_bounds__(kBlock) k_check_products(const __grid_constant__ CheckVecs<T> v, int row_blocks,
+                                                                  const int* __restrict__ rp, const int* __restrict__ col,
+                                                                  const double* __restrict__ a0, const T* __restrict__ as,
+                                                                  const int* __restrict__ cp, const int* __restrict__ ri,
+                                                                  const double* __restrict__ av) {
+  constexpr int GB = 4;  // entries whose gathers are in flight together
+  const bool rows = static_cast<int>(blockIdx.x) < row_blocks;
+  const int k = (static_cast<int>(blockIdx.x) - (rows ? 0 : row_blocks)) * kBlock + static_cast<int>(threadIdx.x);
+  double pmax = 0.0, dmax = 0.0, viol = 0.0, viol2 = 0.0;
+  if (rows) {
+    if (k < v.m) {
+      const int b = rp[k], e = rp[k + 1];
+      double ax = 0.0, adx = 0.0, ad = 0.0, ad2 = 0.0;
+      for (int p = b; p < e; p += GB) {
+        double4 g[GB];
+        double w[GB], ws[GB];
+#pragma unroll
+        for (int q = 0; q < GB; ++q) {
+          const int at = p + q < e ? p + q : p;
+          g[q] = load_packed<(kRays >= 1)>(v.X + col[at]);
+          w[q] = a0[at], ws[q] = static_cast<double>(as[at]);
+        }
+#pragma unroll
+        for (int q = 0; q < GB; ++q)
+          if (p + q < e) {  // each sum in CSR order
+            ax += w[q] * g[q].x;
+            adx += ws[q] * g[q].y;
+            if constexpr (kRays >= 1) ad += w[q] * g[q].z;
+            if constexpr (kRays == 2) ad2 += w[q] * g[q].w;
+          }
+      }
+      const double lo = v.rl[k], up = v.ru[k];
+      const double4 Y = v.Y[k];
+      const T dy = static_cast<T>(-1.0) * v.yh[k] + static_cast<T>(1.0) * v.yb[k];
+      v.t_cross[k] = static_cast<double>(dy) * static_cast<double>(static_cast<T>(adx));
+      const double out = ax < lo ? lo - ax : (ax > up ? ax - up : 0.0);
+      v.k_rp2[k] = out * out;
+      pmax = elem_viol(ax, lo, up);
+      const double yi = Y.x;
+      double d = 0.0, rd = 0.0;
+      if (yi > 0) {
+        if (isfinite(lo)) d = yi * lo;
+        else rd = yi * yi, dmax = yi;
+      } else if (yi < 0) {
+        if (isfinite(up)) d = yi * up;
+        else rd = yi * yi, dmax = -yi;
+      }
+      v.k_d[k] = d;
+      v.k_rd2[k] = rd;
+      if constexpr (kRays >= 1) {
+        double obj, mag;
+        viol = ray_row(ad, Y.y, lo, up, obj, mag);
+        v.r_obj[k] = obj, v.r_mag[k] = mag;
+        if constexpr (kRays == 2) {
+          viol2 = ray_row(ad2, Y.z, lo, up, obj, mag);
+          v.q_obj[k] = obj, v.q_mag[k] = mag;
+        }
+      }
+    }
+    if constexpr (kRays >= 1) warp_max_atomic(max_slot(v.res, kMaxPviol), viol);
+    if constexpr (kRays == 2) warp_max_atomic(max_slot(v.res, kMaxPviol2), viol2);
+  } else {
+    if (k < v.n) {
+      const int b = cp[k], e = cp[k + 1];
+      double aty = 0.0, gr = 0.0, ga = 0.0, gr2 = 0.0, ga2 = 0.0;
+      for (int p = b; p < e; p += GB) {
+        double4 g[GB];
+        double w[GB];
+#pragma unroll
+        for (int q = 0; q < GB; ++q) {
+          const int at = p + q < e ? p + q : p;
+          g[q] = load_packed<kRays == 2>(v.Y + ri[at]);
+          w[q] = av[at];
+        }
+#pragma unroll
+        for (int q = 0; q < GB; ++q)
+          if (p + q < e) {
+            aty += w[q] * g[q].x;
+            if constexpr (kRays >= 1) {
+              const double t = w[q] * g[q].y;
+              gr += t, ga += fabs(t);
+            }
+            if constexpr (kRays == 2) {
+              const double t = w[q] * g[q].z;
+              gr2 += t, ga2 += fabs(t);
+            }
+          }
+      }
+      const double lo = v.cl[k], up = v.cu[k], c = v.c[k];
+      const double4 X = v.X[k];
+      const long long at = static_cast<long long>(v.m) + k;
+      const double cj = v.sense * c;
+      v.k_p[at] = cj * X.x;
+      pmax = elem_viol(X.x, lo, up);
+      const double lam = cj - aty;
+      double z;
+      if (isfinite(lo) && isfinite(up)) z = lam;
+      else if (isfinite(lo)) z = std_max(lam, 0.0);
+      else if (isfinite(up)) z = std_min(lam, 0.0);
+      else z = 0.0;
+      v.k_rd2[at] = (lam - z) * (lam - z);
+      dmax = fabs(lam - z);
+      v.k_d[at] = z > 0 ? z * lo : (z < 0 ? z * up : 0.0);
+      if constexpr (kRays >= 1) {
+        double obj, mag;
+        viol = ray_col(gr, ga, lo, up, obj, mag);
+        v.r_obj[at] = obj, v.r_mag[at] = mag;
+        v.r_cd[k] = v.sense * c * X.z;
+        v.r_cmag[k] = fabs(c * X.z);
+        if constexpr (kRays == 2) {
+          viol2 = ray_col(gr2, ga2, lo, up, obj, mag);
+          v.q_obj[at] = obj, v.q_mag[at] = mag;
+          v.q_cd[k] = v.sense * c * X.w;
+          v.q_cmag[k] = fabs(c * X.w);
+        }
+      }
+    }
+    if constexpr (kRays >= 1) warp_max_atomic(max_slot(v.res, kMaxDviol), viol);
+    if constexpr (kRays == 2) warp_max_atomic(max_slot(v.res, kMaxDviol2), viol2);
+  }
+  warp_max_atomic(max_slot(v.res, kMaxPmax), pmax);
+  warp_max_atomic(max_slot(v.res, kMaxDmax), dmax);
+}
+// The results go to the host's pinned block, and the maxima back to zero for the next check.
+static __global__ void k_check_publish(double* res, double* host) {
+  const int k = threadIdx.x;
+  if (k >= kNumSlots) return;
+  host[k] = res[k];
+  if (k >= kMaxPmax) res[k] = 0.0;
+}
+// One packed component as a vector (an infeasibility ray).
+static __global__ void k_unpack(int len, const double4* P, int which, double* out) {
+  B200_FOR(i, len) out[i] = which == 0 ? P[i].x : which == 1 ? P[i].y : which == 2 ? P[i].z : P[i].w;
+}
 
 // ---------------------------------------------------------------------- finish
 // y = sense · y_min; z_j = c_j − Σ a_ij y_i with the subtractions in CSC order (engine.cpp:283-286)

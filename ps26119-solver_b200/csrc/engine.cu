@@ -97,13 +97,13 @@ double slot_max(const double* h, int s) { return h[s]; }  // bit pattern of a no
 
 template <class T>
 struct IterVecs {
-  DevBuf<T> x, x0, xh, xb, dx, ddx, y, y0, yh, yb, dy, adx, ddy;
+  DevBuf<T> x, x0, xh, xb, dx, y, y0, yh, yb, dy;
   // resident epochs (resident.cuh): the points after a Halpern cycle's first step, the cells of x̄ and y
   DevBuf<T> xh0, xb0, yh0, yb0;
   DevBuf<Cell<T>> xcell, ycell;
   void alloc(int n, int m) {
-    for (DevBuf<T>* v : {&x, &x0, &xh, &xb, &dx, &ddx}) v->alloc(static_cast<std::size_t>(n));
-    for (DevBuf<T>* v : {&y, &y0, &yh, &yb, &dy, &adx, &ddy}) v->alloc(static_cast<std::size_t>(m));
+    for (DevBuf<T>* v : {&x, &x0, &xh, &xb, &dx}) v->alloc(static_cast<std::size_t>(n));
+    for (DevBuf<T>* v : {&y, &y0, &yh, &yb, &dy}) v->alloc(static_cast<std::size_t>(m));
   }
   void alloc_resident(int n, int m, cudaStream_t st) {
     for (DevBuf<T>* v : {&xh0, &xb0}) v->alloc(static_cast<std::size_t>(n));
@@ -147,8 +147,7 @@ class Engine {
       if (e) cudaEventDestroy(e);
     for (auto& e : fork_)
       if (e) cudaEventDestroy(e);
-    for (auto& q : side_)
-      if (q) cudaStreamDestroy(q);
+    if (side_) cudaStreamDestroy(side_);
 #ifdef B200_TEARDOWN_TRACE
     std::fprintf(stderr, "teardown: graphs+events %.1f ms\n",
                  std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - tt0).count());
@@ -214,15 +213,15 @@ class Engine {
   template <class T> IterVecs<T>& vecs();
   template <class T> void capture_epoch();
   template <class T> void capture_check(int variant);
-  template <class T> void launch_residual(bool with_restart_terms, const int* skip, SumPlan& plan,
-                                          cudaStream_t sums_on = nullptr, bool resident_first = false);
+  template <class T> void launch_first_residual(const int* skip);
+  template <class T, int kRays> void launch_check_kernels();
   template <class T> void plan_resident(int max_row, int max_col);
   template <class T> void launch_resident_epoch();
   template <class T> void launch_resident_pdlp(int cur);
   bool resident() const { return shape_[mixed_now_ ? 1 : 0].blocks > 0; }
-  template <class T> void launch_kkt_scaled(const T* xs, const T* ys, cudaStream_t on = nullptr);
-  void launch_kkt_original(cudaStream_t on = nullptr);
-  void make_side_streams();
+  template <class T> void launch_kkt_scaled(const T* xs, const T* ys);
+  void launch_kkt_original();
+  void make_side_stream();
   template <class T> void launch_ray(const T* dx, const T* dy, double* r, double* d, int drift);
   Kkt read_kkt(const double* h) const;
   Status ray_verdict(const double* h, int which, const Kkt& k, std::string& why) const;
@@ -269,8 +268,10 @@ class Engine {
   PinnedBuf<StepParams> hparams_;
   DevBuf<double> res_;
   PinnedBuf<double> hres_;
+  DevBuf<double4> X4_, Y4_;  // a check's packed points
   DevBuf<double> rt_, kt_, rayt_, xo_, yo_, r1_, d1_, r2_, d2_, objt_;
-  SumPlan plan_r0_, plan_res_, plan_pid_, plan_kkt_, plan_ray1_, plan_ray2_, plan_obj_, plan_chk_;
+  SumPlan plan_r0_, plan_pid_, plan_kkt_, plan_ray1_, plan_ray2_, plan_obj_, plan_chk_;
+  SumPlan plan_check_[3];  // a check's sums (residual, KKT, rays), by its variant
   cudaGraphExec_t g_epoch_[2] = {nullptr, nullptr};
   cudaGraphExec_t g_check_[2][3] = {{nullptr, nullptr, nullptr}, {nullptr, nullptr, nullptr}};
   cudaGraphExec_t g_pdlp_[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};         // [precision][phase]
@@ -285,11 +286,10 @@ class Engine {
   SumPlan plan_dist_;
   long long epoch_kernels_[2] = {0, 0}, check_kernels_[2][3] = {{0, 0, 0}, {0, 0, 0}};
   cudaEvent_t ev_[4] = {nullptr, nullptr, nullptr, nullptr};
-  // The check graph's side branches: side_[0] runs the KKT statistics, side_[1] the residual's
-  // and restart distances' sums, while the engine's stream runs the ray tests (fork_[0..3]: the
-  // forks and joins that order them).
-  cudaStream_t side_[2] = {nullptr, nullptr};
-  cudaEvent_t fork_[4] = {nullptr, nullptr, nullptr, nullptr};
+  // The check graph's side branch: the restart distances' reference-order sums run beside the
+  // products and their sums (fork_[0], fork_[1]: the fork and the join).
+  cudaStream_t side_ = nullptr;
+  cudaEvent_t fork_[2] = {nullptr, nullptr};
   long long kernels_ = 0;  // counted launches (graph kernel nodes per replay)
   long long capture_count_ = 0;
   bool capturing_ = false;
@@ -361,7 +361,8 @@ void Engine::setup() {
   const std::size_t mm = static_cast<std::size_t>(m), nn = static_cast<std::size_t>(n);
   rt_.alloc(2 * nn + 3 * mm);
   kt_.alloc(4 * (mm + nn));
-  rayt_.alloc(2 * (mm + nn) + 2 * nn);
+  rayt_.alloc((o_.pdlp ? 1 : 2) * (2 * (mm + nn) + 2 * nn));
+  if (!o_.pdlp) X4_.alloc(nn), Y4_.alloc(mm);
   xo_.alloc(nn), yo_.alloc(mm), r1_.alloc(mm), d1_.alloc(nn), r2_.alloc(mm), d2_.alloc(nn);
   objt_.alloc(mm + 2 * nn);
   build_plans();
@@ -453,9 +454,6 @@ void Engine::build_plans() {
   plan_r0_.add(px, 0, n, 0.0, SumOrder::kChunk64, R + kPx0);
   plan_r0_.add(py, 0, m, 0.0, SumOrder::kChunk64, R + kPy0);
   plan_r0_.add(cross, 0, m, 0.0, SumOrder::kChunk64, R + kCross0);
-  plan_res_.add(px, 0, n, 0.0, SumOrder::kChunk64, R + kPx);
-  plan_res_.add(py, 0, m, 0.0, SumOrder::kChunk64, R + kPy);
-  plan_res_.add(cross, 0, m, 0.0, SumOrder::kChunk64, R + kCross);
   // the restart distances enter the PID primal weight ω (and so every later step): always the
   // reference's order, whatever the mode (positive terms: the exact chains are cheap on them)
   plan_pid_.add(dxn, 0, n, 0.0, SumOrder::kChunk64, R + kDxn2);
@@ -476,58 +474,58 @@ void Engine::build_plans() {
   plan_ray2_.add(T0 + L, 0, L, 0.0, SumOrder::kSeq, R + kRayMag2);
   plan_ray2_.add(T0 + 2 * L, 0, n, 0.0, SumOrder::kSeq, R + kRayCd2);
   plan_ray2_.add(T0 + 2 * L + n, 0, n, 0.0, SumOrder::kSeq, R + kRayCmag2);
+  if (!o_.pdlp)
+    for (int v = 0; v < 3; ++v) {
+      SumPlan& p = plan_check_[v];
+      p.add(px, 0, n, 0.0, SumOrder::kChunk64, R + kPx);
+      p.add(py, 0, m, 0.0, SumOrder::kChunk64, R + kPy);
+      p.add(cross, 0, m, 0.0, SumOrder::kChunk64, R + kCross);
+      p.add(K0, 0, m, 0.0, SumOrder::kSeq, R + kRp2);
+      p.add(K0 + L, 0, L, 0.0, SumOrder::kSeq, R + kD);
+      p.add(K0 + 2 * L, 0, L, 0.0, SumOrder::kSeq, R + kRd2);
+      p.add(K0 + 3 * L, m, L, 0.0, SumOrder::kSeq, R + kP);
+      for (int ray = 0; ray < v; ++ray) {
+        const double* t = T0 + ray * (2 * L + 2 * n);
+        p.add(t, 0, L, 0.0, SumOrder::kSeq, R + (ray ? kRayObj2 : kRayObj));
+        p.add(t + L, 0, L, 0.0, SumOrder::kSeq, R + (ray ? kRayMag2 : kRayMag));
+        p.add(t + 2 * L, 0, n, 0.0, SumOrder::kSeq, R + (ray ? kRayCd2 : kRayCd));
+        p.add(t + 2 * L + n, 0, n, 0.0, SumOrder::kSeq, R + (ray ? kRayCmag2 : kRayCmag));
+      }
+      p.build(o_.exact, nullptr, st_);
+    }
   // finish: objective = offset + Σ c x (Model::objective_value), check sums (solution_checker)
   double* O = objt_.get();
   plan_obj_.add(O, 0, n, M_.offset, SumOrder::kSeq, R + kObjective);
   plan_chk_.add(O + n, 0, L, 0.0, SumOrder::kSeq, R + kChkDual);
   plan_chk_.add(O, 0, n, 0.0, SumOrder::kSeq, R + kChkPrimal);
   plan_r0_.build(o_.exact, skip_r0_flag(params_.get()), st_);
-  plan_res_.build(o_.exact, nullptr, st_);
   plan_pid_.build(true, nullptr, st_);
   plan_kkt_.build(o_.exact, nullptr, st_);
-  plan_ray1_.build(o_.exact, nullptr, st_);
-  plan_ray2_.build(o_.exact, nullptr, st_);
+  if (o_.pdlp) plan_ray1_.build(o_.exact, nullptr, st_), plan_ray2_.build(o_.exact, nullptr, st_);
   plan_obj_.build(o_.exact, nullptr, st_);
   plan_chk_.build(o_.exact, nullptr, st_);
 }
 
-// The residual: dx = x̄ − x̂, adx = Ã dx, dy = ȳ − ŷ and the terms of the five dots.
-// sums_on: the stream of the dots' sums (nullptr: the engine's; another stream must already wait for
-// the engine's stream, and the caller joins it back).
-// resident_first: of the points that a resident epoch left after its first step.
+// The residual of a Halpern cycle's first step: dx = x̄ − x̂, adx = Ã dx, dy = ȳ − ŷ and the terms of its
+// three dots. skip: see SumPlan; resident epochs have left the points of that step in buffers of their own.
 template <class T>
-void Engine::launch_residual(bool with_restart_terms, const int* skip, SumPlan& plan, cudaStream_t sums_on,
-                             bool resident_first) {
+void Engine::launch_first_residual(const int* skip) {
   IterVecs<T>& v = vecs<T>();
   const int m = M_.m, n = M_.n;
   double* px = rt_.get();
-  double* dxn = px + n;
-  double* py = dxn + n;
-  double* cross = py + m;
-  double* dyn = cross + m;
-  const bool f = resident_first;
-  k_res_x<T><<<grid_for(n), kBlock, 0, st_>>>(n, (f ? v.xb0 : v.xb).get(), (f ? v.xh0 : v.xh).get(), v.x0.get(),
-                                              v.dx.get(), px, with_restart_terms ? dxn : nullptr, skip);
+  double* py = px + 2 * n;
+  const bool f = v.xh0.get() != nullptr;
+  k_res_x<T><<<grid_for(n), kBlock, 0, st_>>>(n, (f ? v.xb0 : v.xb).get(), (f ? v.xh0 : v.xh).get(), v.dx.get(), px,
+                                              skip);
   B200_LAUNCH_CHECK();
-  EpiResY<T> e{(f ? v.yb0 : v.yb).get(), (f ? v.yh0 : v.yh).get(), v.y0.get(), v.dy.get(), v.adx.get(), py, cross,
-               with_restart_terms ? dyn : nullptr, skip};
+  EpiResY<T> e{(f ? v.yb0 : v.yb).get(), (f ? v.yh0 : v.yh).get(), py, py + m, skip};
   launch_slab_tma<T>(m, sp_.a_rp.get(), sp_.a_col.get(), sp_.A_val<T>(), v.dx.get(), e, st_, nullptr, err());
-  cudaStream_t ss = st_;
-  if (sums_on) {
-    B200_CHECK(cudaEventRecord(fork_[2], st_));
-    B200_CHECK(cudaStreamWaitEvent(sums_on, fork_[2], 0));
-    ss = sums_on;
-  }
-  plan.launch(ss);
-  B200_COUNT(2 + plan.kernel_count());
-  if (with_restart_terms) {
-    plan_pid_.launch(ss);
-    B200_COUNT(plan_pid_.kernel_count());
-  }
+  plan_r0_.launch(st_);
+  B200_COUNT(2 + plan_r0_.kernel_count());
 }
 
-void Engine::launch_kkt_original(cudaStream_t on) {
-  const cudaStream_t s = on ? on : st_;
+void Engine::launch_kkt_original() {
+  const cudaStream_t s = st_;
   const int m = M_.m, n = M_.n;
   const long long L = static_cast<long long>(m) + n;
   double* K0 = kt_.get();
@@ -541,23 +539,60 @@ void Engine::launch_kkt_original(cudaStream_t on) {
 }
 
 template <class T>
-void Engine::launch_kkt_scaled(const T* xs, const T* ys, cudaStream_t on) {
-  const cudaStream_t s = on ? on : st_;
+void Engine::launch_kkt_scaled(const T* xs, const T* ys) {
+  const cudaStream_t s = st_;
   const int m = M_.m, n = M_.n;
   k_unscale_x<T><<<grid_for(n), kBlock, 0, s>>>(n, xs, sp_.col_scale.get(), sp_.bound_scale, M_.col_lower,
                                                 M_.col_upper, xo_.get());
   k_unscale_y<T><<<grid_for(m), kBlock, 0, s>>>(m, ys, sp_.row_scale.get(), sp_.obj_scale, yo_.get());
   B200_LAUNCH_CHECK();
   B200_COUNT(2);
-  launch_kkt_original(s);
+  launch_kkt_original();
 }
 
-// The check graph's two side streams and its fork / join events, made once per engine outside
-// any capture.
-void Engine::make_side_streams() {
-  if (side_[0]) return;
-  for (auto& q : side_) B200_CHECK(cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking));
+// The check graph's side stream and its fork / join events, made once per engine outside any
+// capture.
+void Engine::make_side_stream() {
+  if (side_) return;
+  B200_CHECK(cudaStreamCreateWithFlags(&side_, cudaStreamNonBlocking));
   for (auto& e : fork_) B200_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+}
+
+// A check's kernels (checks.cuh) in the capture: the points; the restart distances' sums on the side
+// stream beside the products and their sums; the results to the host.
+template <class T, int kRays>
+void Engine::launch_check_kernels() {
+  IterVecs<T>& v = vecs<T>();
+  const int m = M_.m, n = M_.n;
+  const long long L = static_cast<long long>(m) + n;
+  double* px = rt_.get();
+  double* K0 = kt_.get();
+  double* T0 = rayt_.get();
+  double* T1 = T0 + 2 * L + 2 * n;
+  CheckVecs<T> c{n, m, v.xb.get(), v.xh.get(), v.x0.get(), v.yb.get(), v.yh.get(), v.y0.get(), sp_.col_scale.get(),
+                 sp_.row_scale.get(), sp_.bound_scale, sp_.obj_scale, static_cast<double>(M_.sense), M_.c, M_.col_lower,
+                 M_.col_upper, M_.row_lower, M_.row_upper, X4_.get(), Y4_.get(), px, px + n, px + 2 * n, px + 2 * n + m,
+                 px + 2 * n + 2 * m, K0, K0 + L, K0 + 2 * L, K0 + 3 * L, T0, T0 + L, T0 + 2 * L, T0 + 2 * L + n, T1, T1 + L,
+                 T1 + 2 * L, T1 + 2 * L + n, res_.get()};
+  const int cb = (n + kBlock - 1) / kBlock, rb = (m + kBlock - 1) / kBlock;
+  if (cb + rb > 0) {
+    k_check_points<T, kRays><<<cb + rb, kBlock, 0, st_>>>(c, cb);
+    B200_LAUNCH_CHECK();
+  }
+  B200_CHECK(cudaEventRecord(fork_[0], st_));
+  B200_CHECK(cudaStreamWaitEvent(side_, fork_[0], 0));
+  plan_pid_.launch(side_);
+  B200_CHECK(cudaEventRecord(fork_[1], side_));
+  if (cb + rb > 0) {
+    k_check_products<T, kRays><<<cb + rb, kBlock, 0, st_>>>(c, rb, sp_.a_rp.get(), sp_.a_col.get(), sp_.a_v0.get(),
+                                                            sp_.A_val<T>(), M_.col_start, M_.row_index, M_.value);
+    B200_LAUNCH_CHECK();
+  }
+  plan_check_[kRays].launch(st_);
+  B200_CHECK(cudaStreamWaitEvent(st_, fork_[1], 0));
+  k_check_publish<<<1, 64, 0, st_>>>(res_.get(), hres_.get());
+  B200_LAUNCH_CHECK();
+  B200_COUNT(3 + plan_pid_.kernel_count() + plan_check_[kRays].kernel_count());
 }
 
 template <class T>
@@ -635,7 +670,7 @@ void Engine::capture_epoch() {
   B200_CHECK(cudaEventRecordWithFlags(ev_[0], st_, cudaEventRecordExternal));
   step(0);
   B200_CHECK(cudaEventRecordWithFlags(ev_[1], st_, cudaEventRecordExternal));
-  launch_residual<T>(false, r0_skip, plan_r0_);  // r⁰ after the first step of a Halpern cycle
+  launch_first_residual<T>(r0_skip);  // r⁰ after the first step of a Halpern cycle
   B200_CHECK(cudaEventRecordWithFlags(ev_[2], st_, cudaEventRecordExternal));
   for (int s = 1; s < K; ++s) step(s);
   B200_CHECK(cudaEventRecordWithFlags(ev_[3], st_, cudaEventRecordExternal));
@@ -652,40 +687,15 @@ template <class T>
 void Engine::capture_check(int variant) {
   const int idx = std::is_same<T, float>::value ? 1 : 0;
   if (g_check_[idx][variant]) return;
-  IterVecs<T>& v = vecs<T>();
   cudaGraph_t g;
-  slab_prepare<T, EpiResY<T>, B200_STAGE_TMA != 0>();
-  slab_prepare<double, EpiKktRows, B200_STAGE_TMA != 0>();
-  slab_prepare<double, EpiKktCols, false>();
-  slab_prepare<double, EpiRayRows, B200_STAGE_TMA != 0>();
-  make_side_streams();
+  make_side_stream();
   capturing_ = true;
   capture_count_ = 0;
   auto capture_scope = std::make_unique<CaptureScope>();  // no device-wide syncs elsewhere meanwhile
   B200_CHECK(cudaStreamBeginCapture(st_, cudaStreamCaptureModeThreadLocal));
-  clear_maxima();
-  // Three branches that share no buffer and write disjoint result slots: the KKT statistics of
-  // (x̂, ŷ) on side_[0]; the residual's kernels on the engine's stream, then their sums and the
-  // restart distances on side_[1] while the ray tests (which read dx, dy) run on the engine's
-  // stream. Each branch's order is the serial one, so every value is the same; the short sum
-  // kernels of one branch overlap the matrix products of another.
-  B200_CHECK(cudaEventRecord(fork_[0], st_));
-  B200_CHECK(cudaStreamWaitEvent(side_[0], fork_[0], 0));
-  launch_kkt_scaled<T>(v.xh.get(), v.yh.get(), side_[0]);
-  B200_CHECK(cudaEventRecord(fork_[1], side_[0]));
-  launch_residual<T>(true, nullptr, plan_res_, side_[1]);
-  B200_CHECK(cudaEventRecord(fork_[3], side_[1]));
-  if (variant >= 1) launch_ray<T>(v.dx.get(), v.dy.get(), r1_.get(), d1_.get(), 0);
-  if (variant == 2) {
-    k_diff<T><<<grid_for(M_.n), kBlock, 0, st_>>>(M_.n, v.xh.get(), v.x0.get(), v.ddx.get());
-    k_diff<T><<<grid_for(M_.m), kBlock, 0, st_>>>(M_.m, v.yh.get(), v.y0.get(), v.ddy.get());
-    B200_LAUNCH_CHECK();
-    capture_count_ += 2;
-    launch_ray<T>(v.ddx.get(), v.ddy.get(), r2_.get(), d2_.get(), 1);
-  }
-  B200_CHECK(cudaStreamWaitEvent(st_, fork_[1], 0));  // join the KKT branch
-  B200_CHECK(cudaStreamWaitEvent(st_, fork_[3], 0));  // join the sums branch
-  B200_CHECK(cudaMemcpyAsync(hres_.get(), res_.get(), kNumSlots * sizeof(double), cudaMemcpyDeviceToHost, st_));
+  if (variant == 0) launch_check_kernels<T, 0>();
+  else if (variant == 1) launch_check_kernels<T, 1>();
+  else launch_check_kernels<T, 2>();
   const cudaError_t e = cudaStreamEndCapture(st_, &g);
   capture_scope.reset();
   capturing_ = false;
@@ -878,6 +888,11 @@ void Engine::finish_p(EngineResult& R, Status status, const T* xs, const T* ys, 
     kernels_ += 2;
     if (ytmp.get()) B200_CHECK(cudaStreamSynchronize(st_));
   }
+  if (status == Status::Infeasible && X4_.get() && ray_test > 0)  // a check left its rays packed
+    k_unpack<<<grid_for(m), kBlock, 0, st_>>>(m, Y4_.get(), ray_test, (ray_test == 2 ? r2_ : r1_).get());
+  if (status == Status::Unbounded && X4_.get() && ray_test > 0)
+    k_unpack<<<grid_for(n), kBlock, 0, st_>>>(n, X4_.get(), ray_test + 1, (ray_test == 2 ? d2_ : d1_).get());
+  B200_LAUNCH_CHECK();
   if (status == Status::Infeasible && out.dual_ray)
     B200_CHECK(cudaMemcpyAsync(out.dual_ray, ray_test == 2 ? r2_.get() : r1_.get(), m * sizeof(double),
                                cudaMemcpyDeviceToDevice, st_));
@@ -993,6 +1008,7 @@ bool Engine::start(const DeviceOutputs& out) {
       finish_run(Status::Optimal, false, "warm start already optimal", 0);
       return true;
     }
+    clear_maxima();  // the first check finds them at zero
   }
   const long long m = M_.m, n = M_.n;
   if (mixed_now_) {
@@ -1047,7 +1063,7 @@ void Engine::launch_resident_epoch() {
   B200_CHECK(cudaEventRecord(ev_[1], st_));
   tag_ += static_cast<unsigned>(hp.K) + 1;
   ++kernels_;
-  if (L_.fresh) launch_residual<T>(false, nullptr, plan_r0_, nullptr, true);
+  if (L_.fresh) launch_first_residual<T>(nullptr);
 }
 
 template <class T>
@@ -1089,8 +1105,8 @@ void Engine::launch_r0(cudaStream_t on) {
   if (!L_.fresh) return;
   const cudaStream_t own = st_;
   st_ = on;  // launched on the group's stream, between the group's step 0 and step 1
-  if (mixed_now_) launch_residual<float>(false, nullptr, plan_r0_);
-  else launch_residual<double>(false, nullptr, plan_r0_);
+  if (mixed_now_) launch_first_residual<float>(nullptr);
+  else launch_first_residual<double>(nullptr);
   st_ = own;
 }
 

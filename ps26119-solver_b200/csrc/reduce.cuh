@@ -688,29 +688,34 @@ static __global__ void __launch_bounds__(32 * kXWarps) k_xwalk(const XChain* __r
   if (lane == 0) *J.out = s;
 }
 
-static __global__ void k_tree1(const TreeSeg* segs, int nseg, double* partials, const int* skip) {
+// The fixed tree: kTreeBlocks blocks per sum, the block that finishes last adds the partials (done: a
+// counter per sum, back to zero for the next launch).
+static __global__ void __launch_bounds__(kBlock) k_tree(const TreeSeg* segs, double* partials, unsigned* done,
+                                                        const int* skip) {
   __shared__ double sh[32];
+  __shared__ bool last;
   if (skip && *skip) return;
   const int s = blockIdx.x / kTreeBlocks, b = blockIdx.x % kTreeBlocks;
-  if (s >= nseg) return;
   const TreeSeg g = segs[s];
   const long long len = g.hi - g.lo;
   const long long a = g.lo + len * b / kTreeBlocks, e = g.lo + len * (b + 1) / kTreeBlocks;
   double acc = 0.0;
   for (long long i = a + threadIdx.x; i < e; i += blockDim.x) acc += g.t[i];
   acc = block_sum_fixed(acc, sh);
-  if (threadIdx.x == 0) partials[static_cast<long long>(s) * kTreeBlocks + b] = acc;
-}
-
-static __global__ void k_tree2(const TreeSeg* segs, int nseg, const double* partials, const int* skip) {
-  __shared__ double sh[32];
-  if (skip && *skip) return;
-  const int s = blockIdx.x;
-  if (s >= nseg) return;
-  double acc = 0.0;
-  for (int i = threadIdx.x; i < kTreeBlocks; i += blockDim.x) acc += partials[static_cast<long long>(s) * kTreeBlocks + i];
+  double* part = partials + static_cast<long long>(s) * kTreeBlocks;
+  if (threadIdx.x == 0) {
+    part[b] = acc;
+    __threadfence();
+    last = atomicAdd(done + s, 1u) + 1u == static_cast<unsigned>(kTreeBlocks);
+    if (last) done[s] = 0u;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  acc = 0.0;
+  for (int i = threadIdx.x; i < kTreeBlocks; i += blockDim.x) acc += __ldcg(part + i);
   acc = block_sum_fixed(acc, sh);
-  if (threadIdx.x == 0) *segs[s].out = segs[s].init + acc;
+  if (threadIdx.x == 0) *g.out = g.init + acc;
 }
 
 // A fixed set of sums over fixed term arrays. Built once (descriptors live on the device),
@@ -779,6 +784,8 @@ class SumPlan {
       upload(tree, tseg_, st);
       nt_ = static_cast<int>(tree.size());
       partials_.alloc(static_cast<std::size_t>(nt_ > 0 ? nt_ : 1) * kTreeBlocks);
+      done_.alloc(tree.size() + 1);
+      B200_CHECK(cudaMemsetAsync(done_.get(), 0, (tree.size() + 1) * sizeof(unsigned), st));
     }
   }
   // The tile sums a producer may leave itself (x_leave_stat) before launch(st, true): of the plan's
@@ -802,15 +809,13 @@ class SumPlan {
         B200_LAUNCH_CHECK();
       }
     } else if (nt_ > 0) {
-      k_tree1<<<nt_ * kTreeBlocks, kBlock, 0, st>>>(reinterpret_cast<const TreeSeg*>(tseg_.get()), nt_,
-                                                    partials_.get(), skip_);
-      B200_LAUNCH_CHECK();
-      k_tree2<<<nt_, kBlock, 0, st>>>(reinterpret_cast<const TreeSeg*>(tseg_.get()), nt_, partials_.get(), skip_);
+      k_tree<<<nt_ * kTreeBlocks, kBlock, 0, st>>>(reinterpret_cast<const TreeSeg*>(tseg_.get()), partials_.get(),
+                                                   done_.get(), skip_);
       B200_LAUNCH_CHECK();
     }
   }
   int kernel_count() const {
-    return exact_ ? (ntiles_ > 0) + (ngroups_ + nshort_ > 0) : (nt_ > 0 ? 2 : 0);
+    return exact_ ? (ntiles_ > 0) + (ngroups_ + nshort_ > 0) : (nt_ > 0 ? 1 : 0);
   }
   bool empty() const { return jobs_.empty(); }
 
