@@ -369,6 +369,15 @@ inline int sm_count() {
   return v;
 }
 
+// Programmatic dependent launch (sm_90+): a kernel launched with the programmatic-serialisation
+// attribute may start while the kernel before it in the stream is still running; it must not
+// touch that kernel's outputs (or anything a kernel still running may read or write) before
+// pdl_wait(), which returns once every earlier kernel has completed and its writes are visible.
+// pdl_allow_next() lets the next such kernel be scheduled once every block of this one has issued
+// it. In a kernel launched without the attribute both are no-ops.
+__device__ __forceinline__ void pdl_allow_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Grid-stride helper over [0, n).
 #define B200_FOR(i, n) \
   for (std::int64_t i = blockIdx.x * static_cast<std::int64_t>(blockDim.x) + threadIdx.x; i < (n); \

@@ -57,35 +57,35 @@ __device__ __forceinline__ double block_sum_fixed(double v, double* sh) {
 // effect for each of the two parities (XRun), and effects compose associatively. So:
 //   k_xstat   per tile of kXTile terms (one warp): an approximate fp64 sum, in any order; only used
 //             to guess each tile's binade. A kernel that produces the terms may leave it itself.
-//   k_xwalk   one block per group of kXGroup consecutive tiles, one warp per tile: the guessed
-//             binade's u from the approximate start (the approximate sums of the chain's earlier
-//             tiles), then the tile's XRun (exact int64: change of S, its lowest and highest running
-//             value, parity after, per parity before); a term with |t/u| ≥ 2^51 (or non-finite)
-//             marks the tile. The block composes its tiles' XRuns into the group's when all of them
-//             count in one grid with no split and no bad term. The block that finishes last of a
-//             chain's then walks the chain with the EXACT s, with one warp: a run of whole groups
-//             is committed like one tile (below) as far as every running S provably stays inside
-//             the binade; the first group that is not is walked tile by tile. A tile is committed
-//             as s ← (S0 + K[S0 mod 2])·u when s = S0·u lies in the guessed binade and every
-//             running S stays within [2^52 + 1, 2^53 − 1] (then each exact partial sum lies inside
-//             the binade, at least u/2 from its ends, and rounds to that grid). A tile whose running
-//             sum changes binade once is committed in three parts; the terms of any other tile are
-//             added one by one (x_add), so that binade changes, zeros, subnormals, infinities and
-//             NaN get exactly the sequential chain's arithmetic. A chain of at most kXShort terms is
-//             added one by one from the start.
+//   k_xwalk   one warp per tile, kXWarps tiles per block: the guessed binade's u from the approximate
+//             start (the approximate sums of the chain's earlier tiles), then the tile's XRun (exact
+//             int64: change of S, its lowest and highest running value, parity after, per parity
+//             before); a term with |t/u| ≥ 2^51 (or non-finite) marks the tile. A tile whose running sum
+//             changes binade once is summarised in three parts: the run before the term that changes it,
+//             that term, the run after it in the new grid. The block that finishes last of a group of
+//             kXGroup tiles composes the tiles' summaries into the group's, of the same form. The block
+//             that finishes last of a chain's walks the chain with the EXACT s, with one warp: a run of
+//             groups is committed as s ← (S0 + K[S0 mod 2])·u as far as s = S0·u lies in their binade and
+//             every running S provably stays within [2^52 + 1, 2^53 − 1] (then each exact partial sum
+//             lies inside the binade, at least u/2 from its ends, and rounds to that grid); a group that
+//             changes binade is committed by its three parts; any other one is walked by its tiles in the
+//             same way; and the terms of a tile that cannot be committed are added one by one (x_add), so
+//             that zeros, subnormals, infinities and NaN get exactly the sequential chain's arithmetic.
+//             A chain of at most kXShort terms is added one by one from the start.
 // The approximations only choose between two exact paths; the result never depends on them.
 //
 // What bounds it: latency. A dependent fp64 addition takes 8.3 cycles, 10.4 with its operand from
 // shared memory, so a tile added one by one takes 1.4 us, and the walk of a chain pays that for its
-// first tile (the sum starts at zero) and for the few tiles that cross a binade more than once; every
-// other step is a warp scan over 32 tiles (0.4 us). Tiles of 256 terms, one warp's, keep the tiles
-// that must be added one by one cheap. Measured, 15,000 terms: 24 us a launch; three launches over
-// tiles of 2,048 terms, the first tile walked in windows of 256 with a scan and a restart per binade
-// crossing, took 68 us.
+// first tile (the sum starts at zero) and for the few tiles that cross a binade more than once; the
+// other steps are one check over 32 summaries held by the warp's lanes, and a hand-over per crossing.
+// Tiles of 256 terms, one warp's, keep the tiles that must be added one by one cheap. Measured, 15,000
+// terms: 18.5 us a launch (24 with summaries read from shared memory and scanned anew at every crossing,
+// 16 warps of a block on 32 tiles); three launches over tiles of 2,048 terms, the first tile walked in
+// windows of 256 with a scan and a restart per binade crossing, took 68 us.
 constexpr int kXPer = 8;              // terms per lane
 constexpr int kXTile = 32 * kXPer;    // terms per tile (one warp)
-constexpr int kXGroup = 32;           // tiles per group (one block)
-constexpr int kXWarps = 16;           // warps per block of k_xwalk
+constexpr int kXGroup = 32;           // tiles per group (one warp lane each)
+constexpr int kXWarps = 8;            // warps per block of k_xwalk, tiles per block
 constexpr long long kXShort = 1024;   // chains up to this long are added one by one by a warp
 
 struct XChain {
@@ -95,6 +95,7 @@ struct XChain {
   double* out;
   int tile0, ntiles;    // this chain's tiles in the tile arrays (ntiles = 0: added one by one)
   int group0, ngroups;  // its groups of kXGroup tiles
+  int block0;           // its first block of kXWarps tiles
   int job;              // its kChunk64 job (−1: *out is the chain's own result)
 };
 // A kChunk64 job: the chains of its chunks leave their sums in part[0, chunks); the chain that
@@ -118,20 +119,14 @@ struct alignas(16) XRun {
 // A tile's summary: its terms before `split` counted in the grid u (the binade of the tile's
 // approximate start), the term at `split` (where the approximate running sum leaves that binade;
 // split = −1: it never does) added as a plain fp64 addition, the terms after it counted in the
-// grid u1 of the binade the running sum moved to. u = 0: no usable guess (bad is set).
+// grid u1 of the binade the running sum moved to. u = 0: no usable guess (bad is set). A group's summary
+// has the same form (its split is the tile that changes binade).
 struct alignas(16) XTileAgg {
   double u, u1;
   double at;  // the term at `split`
   XRun pre, suf;
   int split;
 };
-// A group of kXGroup consecutive tiles of one chain that all count in the same grid u with no
-// split and no bad term: the composition of their runs. u = 0: the group cannot be taken whole.
-struct alignas(16) XGroupAgg {
-  XRun run;
-  double u;
-};
-
 constexpr long long kX52 = 1LL << 52, kX53 = 1LL << 53;
 
 __device__ __forceinline__ XRun x_identity() {
@@ -498,191 +493,199 @@ __device__ __forceinline__ bool x_commit(double& s, double u, const XRun& r) {
   return true;
 }
 
-// One warp: lanes from … cnt−1 hold consecutive runs r counted in the grid u (usable where `ok`).
-// Commits onto s every run up to the first that is not usable, not in s's binade, or whose running
-// S leaves it, and returns that lane (cnt: all committed).
-__device__ __forceinline__ int x_commit_lanes(double& s, XRun r, double u, bool ok, int from, int cnt) {
-  const int lane = threadIdx.x & 31;
-  int e;
-  const bool have = x_binade(s, e);
-  const double us = have ? x_pow2(e - 52) : 0.0;
-  const long long S0 = have ? static_cast<long long>(s * x_pow2(52 - e)) : 0;
-  const int p0 = static_cast<int>(S0 & 1);
-  const bool mine = lane >= from && lane < cnt;
-  ok = ok && mine && have && u == us && !r.bad;
-  const unsigned unusable = __ballot_sync(kFull, mine && !ok);
-  if (unusable && __ffs(unusable) - 1 == from) return from;
-  if (!mine) r = x_identity();
-  long long Kb, total;  // the change of S before this lane's run, and over all
-  bool valid = false;
-  if (!__any_sync(kFull, r.ties)) {
-    long long inc = r.K[0];
-    for (int off = 1; off < 32; off <<= 1) {
-      const long long o = __shfl_up_sync(kFull, inc, off);
-      if (lane >= off) inc += o;
-    }
-    Kb = inc - r.K[0];
-    total = __shfl_sync(kFull, inc, 31);
-    if (ok) valid = x_inside(S0, S0 + Kb + r.mn[0]) && x_inside(S0, S0 + Kb + r.mx[0]);
-  } else {
-    XRun inc = r;
-    for (int off = 1; off < 32; off <<= 1) {
-      const XRun o = x_shfl_up(inc, off);
-      if (lane >= off) inc = x_compose(o, inc);
-    }
-    XRun ex = x_shfl_up(inc, 1);
-    if (lane == 0) ex = x_identity();
-    Kb = p0 ? ex.K[1] : ex.K[0];
-    const int pb = p0 ? ex.out[1] : ex.out[0];
-    total = __shfl_sync(kFull, p0 ? inc.K[1] : inc.K[0], 31);
-    if (ok) {
-      const long long mn = pb ? r.mn[1] : r.mn[0], mx = pb ? r.mx[1] : r.mx[0];
-      valid = x_inside(S0, S0 + Kb + mn) && x_inside(S0, S0 + Kb + mx);
-    }
+// Commits a whole summary, its change of binade included; returns false (s unchanged) where it cannot.
+__device__ __forceinline__ bool x_commit(double& s, const XTileAgg& T) {
+  double s2 = s;
+  if (!x_commit(s2, T.u, T.pre)) return false;
+  if (T.split >= 0) {
+    s2 += T.at;  // the term that changes the binade, as the chain adds it
+    if (!x_commit(s2, T.u1, T.suf)) return false;
   }
-  const unsigned bad = __ballot_sync(kFull, mine && !valid);
-  const int f = bad ? __ffs(bad) - 1 : cnt;  // the first run not committed
-  const long long upto = __shfl_sync(kFull, Kb, f & 31);
-  if (f > from) s = static_cast<double>(S0 + (f < 32 ? upto : total)) * us;
-  return f;
+  s = s2;
+  return true;
 }
 
-// The chain c from its tiles' and groups' summaries (one warp; sg: room for 32 tile summaries).
-__device__ __forceinline__ double x_walk(const XChain& c, const XTileAgg* ag, const XGroupAgg* gg, XTileAgg* sg,
-                                         double* sh) {
+// One warp walks cnt consecutive summaries, lane l holding T of the l-th, with the exact s. other(k, s)
+// returns the sum after the k-th where its summary cannot be committed. Every step commits all summaries
+// up to the first that changes binade, is not in s's binade, or whose running S would leave it. Without
+// ties a run's K does not depend on what came before, so one prefix sum over the lanes serves all steps
+// (across a change of grid the sum means nothing, but a step only uses differences within one).
+template <class F>
+__device__ __forceinline__ double x_walk_lanes(double s, const XTileAgg& T, int cnt, F&& other) {
+  const int lane = threadIdx.x & 31;
+  const bool here = lane < cnt;
+  const bool plain = here && !T.pre.bad && T.split < 0 && T.u != 0.0;
+  const unsigned ties = __ballot_sync(kFull, here && T.pre.ties);
+  long long inc = here ? T.pre.K[0] : 0;
+  for (int off = 1; off < 32; off <<= 1) {
+    const long long o = __shfl_up_sync(kFull, inc, off);
+    if (lane >= off) inc += o;
+  }
+  const long long before = inc - (here ? T.pre.K[0] : 0);
+  int j = 0;
+  while (j < cnt) {
+    int e;
+    const bool have = x_binade(s, e);
+    const double u = have ? x_pow2(e - 52) : 0.0;
+    const unsigned stop = __ballot_sync(kFull, lane >= j && !(plain && have && T.u == u));
+    int f = stop ? __ffs(stop) - 1 : 32;  // the first that cannot be committed with those before it
+    if (f > j) {
+      const long long S0 = static_cast<long long>(s * x_pow2(52 - e));
+      const bool in = lane >= j && lane < f;
+      bool valid;
+      long long K;  // the change of S up to and with this lane's run
+      if ((ties & ((f < 32 ? (1u << f) : 0u) - (1u << j))) == 0) {
+        const long long Kb = before - __shfl_sync(kFull, before, j);
+        K = Kb + T.pre.K[0];
+        valid = x_inside(S0, S0 + Kb + T.pre.mn[0]) && x_inside(S0, S0 + Kb + T.pre.mx[0]);
+      } else {
+        const int p0 = static_cast<int>(S0 & 1);
+        XRun run = in ? T.pre : x_identity();
+        for (int off = 1; off < 32; off <<= 1) {
+          const XRun o = x_shfl_up(run, off);
+          if (lane >= off) run = x_compose(o, run);
+        }
+        XRun ex = x_shfl_up(run, 1);
+        if (lane == 0) ex = x_identity();
+        const long long Kb = p0 ? ex.K[1] : ex.K[0];
+        const bool pb = (p0 ? ex.out[1] : ex.out[0]) != 0;
+        K = p0 ? run.K[1] : run.K[0];
+        valid = x_inside(S0, S0 + Kb + (pb ? T.pre.mn[1] : T.pre.mn[0])) &&
+                x_inside(S0, S0 + Kb + (pb ? T.pre.mx[1] : T.pre.mx[0]));
+      }
+      const unsigned bad = __ballot_sync(kFull, in && !valid);
+      if (bad) f = __ffs(bad) - 1;
+      if (f > j) s = static_cast<double>(S0 + __shfl_sync(kFull, K, f - 1)) * u;
+    }
+    if (f >= cnt) break;
+    double s2 = s;
+    const int done = lane == f && x_commit(s2, T) ? 1 : 0;
+    s2 = __shfl_sync(kFull, s2, f);
+    s = __shfl_sync(kFull, done, f) ? s2 : other(f, s);
+    j = f + 1;
+  }
+  return s;
+}
+__device__ __forceinline__ XTileAgg x_no_summary() {
+  XTileAgg T;
+  T.u = T.u1 = T.at = 0.0;
+  T.pre = T.suf = x_identity();
+  T.split = -1;
+  return T;
+}
+
+// The chain c from its tiles' and groups' summaries (one warp).
+__device__ __forceinline__ double x_walk(const XChain& c, const XTileAgg* ag, const XTileAgg* gg, double* sh) {
   const int lane = threadIdx.x & 31;
   double s = c.init;
-  int g0 = 0;  // the next group
-  while (g0 < c.ngroups) {
-    // whole groups first, up to 32 per scan
+  for (int g0 = 0; g0 < c.ngroups; g0 += 32) {
     const int cntg = c.ngroups - g0 < 32 ? c.ngroups - g0 : 32;
-    XGroupAgg G;
-    G.u = 0.0;
-    G.run = x_identity();
-    if (lane < cntg) G = x_load(gg + c.group0 + g0 + lane);
-    const int f = x_commit_lanes(s, G.run, G.u, G.u != 0.0, 0, cntg);
-    g0 += f;
-    if (f == cntg) continue;
-    // the group that was not taken whole: its tiles
-    const int t0 = g0 * kXGroup, cnt = c.ntiles - t0 < kXGroup ? c.ntiles - t0 : kXGroup;
-    __syncwarp();
-    if (lane < cnt) sg[lane] = x_load(ag + c.tile0 + t0 + lane);
-    __syncwarp();
-    int j = 0;
-    while (j < cnt) {
-      XRun r = x_identity();
-      double u = 0.0;
-      bool ok = false;
-      if (lane < cnt) r = sg[lane].pre, u = sg[lane].u, ok = sg[lane].split < 0 && u != 0.0;
-      const int k = x_commit_lanes(s, r, u, ok, j, cnt);
-      if (k < cnt) {  // tile k on its own
+    const XTileAgg G = lane < cntg ? x_load(gg + c.group0 + g0 + lane) : x_no_summary();
+    s = x_walk_lanes(s, G, cntg, [&](int g, double sg) {
+      const int t0 = (g0 + g) * kXGroup, cnt = c.ntiles - t0 < kXGroup ? c.ntiles - t0 : kXGroup;
+      const XTileAgg T = lane < cnt ? x_load(ag + c.tile0 + t0 + lane) : x_no_summary();
+      return x_walk_lanes(sg, T, cnt, [&](int k, double st) {
         long long a, b;
         x_tile_range(c, c.tile0 + t0 + k, a, b);
-        const XTileAgg& T = sg[k];
-        long long resume = a;
-        double s2 = s;
-        if (x_commit(s2, T.u, T.pre)) {
-          if (T.split < 0) {
-            resume = b;
-          } else {
-            s2 += T.at;  // the term that changes the binade, as the chain adds it
-            resume = a + T.split + 1;
-            if (x_commit(s2, T.u1, T.suf)) resume = b;
-          }
-          s = s2;
-        }
-        if (resume < b) s = x_add(c.t, resume, b, s, sh);
-      }
-      j = k + 1;
-    }
-    ++g0;
+        return x_add(c.t, a, b, st, sh);
+      });
+    });
   }
   return s;
 }
 
-// Blocks [0, ngroups): one group of tiles each (group_chain: its chain). The blocks after them:
-// one chain of at most kXShort terms per warp (short_chain). chain_done / job_done count a chain's
-// finished groups and a job's finished chains; the last one goes on, and sets its counter back to
+// The summary of a group of tiles, lane l holding T of the l-th (valid in lane 0): all tiles in one grid
+// and none that changes binade, or one that does, with the tiles before it in its first grid and those
+// after it in its second. Else u = 0.
+__device__ __forceinline__ XTileAgg x_group(const XTileAgg& T, int cnt) {
+  const int lane = threadIdx.x & 31;
+  const bool here = lane < cnt;
+  const unsigned splits = __ballot_sync(kFull, here && T.split >= 0);
+  const int k = splits ? __ffs(splits) - 1 : 31;  // the last lane in the first grid
+  XTileAgg G = x_no_summary();
+  const double u0 = __shfl_sync(kFull, T.u, 0), u1 = splits ? __shfl_sync(kFull, T.u1, k) : u0;
+  bool ok = !here || (!T.pre.bad && T.u != 0.0 && T.u == (lane <= k ? u0 : u1));
+  if (lane == k && splits) ok = ok && !T.suf.bad && T.u1 != 0.0;
+  if (!__all_sync(kFull, ok) || __popc(splits) > 1) {
+    G.pre.bad = 1;
+    return G;
+  }
+  G.u = u0;
+  G.pre = x_warp_ordered(here && lane <= k ? T.pre : x_identity());
+  if (splits) {
+    G.u1 = u1, G.split = k;
+    G.at = __shfl_sync(kFull, T.at, k);
+    G.suf = x_warp_ordered(lane == k ? T.suf : (here && lane > k ? T.pre : x_identity()));
+  }
+  return G;
+}
+
+// Blocks [0, nblocks): kXWarps tiles of one chain each (block_chain: the chain). The blocks after them:
+// one chain of at most kXShort terms per warp (short_chain). done: counters of a group's finished blocks,
+// a chain's finished groups and a job's finished chains; the last one goes on, and sets its counter back to
 // zero for the next launch.
-static __global__ void __launch_bounds__(32 * kXWarps) k_xwalk(const XChain* __restrict__ ch, const XJob* jobs,
-                                                               const int* group_chain, int ngroups,
-                                                               const int* short_chain, int nshort, const double* stat,
-                                                               XTileAgg* ag, XGroupAgg* gg, unsigned* chain_done,
+static __global__ void __launch_bounds__(32 * kXWarps) k_xwalk(const XChain* __restrict__ ch, const XJob* __restrict__ jobs,
+                                                               const int* __restrict__ block_chain, int nblocks,
+                                                               const int* __restrict__ short_chain, int nshort,
+                                                               const double* stat, XTileAgg* ag, XTileAgg* gg,
+                                                               unsigned* group_done, unsigned* chain_done,
                                                                unsigned* job_done, const int* skip) {
-  __shared__ XTileAgg sg[kXGroup];
   __shared__ alignas(16) double sh_add[kXWarps][kXTile];
   __shared__ double sh_sum[kXWarps];
-  if (skip && *skip) return;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  int ci;
+  const bool tiled = static_cast<int>(blockIdx.x) < nblocks;
+  const int ks = (static_cast<int>(blockIdx.x) - nblocks) * kXWarps + w;
+  const int ci = tiled ? block_chain[blockIdx.x] : ks < nshort ? short_chain[ks] : -1;
+  XChain c;
+  if (ci >= 0) c = ch[ci];
+  pdl_wait();
+  if (skip && *skip) return;
   double s;
-  if (static_cast<int>(blockIdx.x) < ngroups) {
-    const int g = blockIdx.x;
-    ci = group_chain[g];
-    const XChain c = ch[ci];
-    const int t0 = (g - c.group0) * kXGroup, cnt = c.ntiles - t0 < kXGroup ? c.ntiles - t0 : kXGroup;
-    // the approximate sum before this group, then before each of its tiles
-    double pre = 0.0;
-    for (int k = threadIdx.x; k < t0; k += blockDim.x) pre += stat[c.tile0 + k];
+  // counts one more at *counter; true in every lane of the warp that made it `of`
+  auto last_of = [&](unsigned* counter, int of) {
+    unsigned last = 0;
+    if (lane == 0) {
+      __threadfence();
+      last = atomicAdd(counter, 1u) + 1u == static_cast<unsigned>(of) ? 1u : 0u;
+      if (last) *counter = 0u;
+    }
+    last = __shfl_sync(kFull, last, 0);
+    if (last) __threadfence();
+    return last != 0;
+  };
+  if (tiled) {
+    const int k0 = (static_cast<int>(blockIdx.x) - c.block0) * kXWarps, k = k0 + w;
+    const double mine = lane < w && k0 + lane < c.ntiles ? stat[c.tile0 + k0 + lane] : 0.0;
+    double pre = 0.0;  // the approximate sum before this block's tiles
+    for (int q = threadIdx.x; q < k0; q += 32 * kXWarps) pre += stat[c.tile0 + q];
     for (int off = 16; off > 0; off >>= 1) pre += __shfl_xor_sync(kFull, pre, off);
     if (lane == 0) sh_sum[w] = pre;
-    const double mine = lane < cnt ? stat[c.tile0 + t0 + lane] : 0.0;
-    double inc = mine;
-    for (int off = 1; off < 32; off <<= 1) {
-      const double o = __shfl_up_sync(kFull, inc, off);
-      if (lane >= off) inc += o;
-    }
     __syncthreads();
-    pre = c.init;
-    for (int k = 0; k < kXWarps; ++k) pre += sh_sum[k];
-    for (int k = w; k < cnt; k += kXWarps) {
-      const double s0 = pre + __shfl_sync(kFull, inc - mine, k);
+    double s0 = mine;
+    for (int off = 16; off > 0; off >>= 1) s0 += __shfl_xor_sync(kFull, s0, off);
+    s0 += c.init;
+    for (int q = 0; q < kXWarps; ++q) s0 += sh_sum[q];
+    if (k < c.ntiles) {
       long long a, b;
-      x_tile_range(c, c.tile0 + t0 + k, a, b);
+      x_tile_range(c, c.tile0 + k, a, b);
       const XTileAgg T = x_tile_agg(c.t, a, b, s0);
-      if (lane == 0) sg[k] = T, ag[c.tile0 + t0 + k] = T;
+      if (lane == 0) ag[c.tile0 + k] = T;
     }
     __threadfence();
     __syncthreads();
     if (w != 0) return;
-    XRun r = x_identity();
-    double u = 0.0;
-    bool ok = true;
-    if (lane < cnt) r = sg[lane].pre, u = sg[lane].u, ok = !r.bad && sg[lane].split < 0 && u != 0.0;
-    const double u0 = __shfl_sync(kFull, u, 0);
-    ok = __all_sync(kFull, lane >= cnt || (ok && u == u0)) != 0;
-    r = x_warp_ordered(r);
-    unsigned last = 0;
-    if (lane == 0) {
-      XGroupAgg G;
-      G.u = ok ? u0 : 0.0;
-      G.run = r;
-      gg[g] = G;
-      __threadfence();
-      last = atomicAdd(chain_done + ci, 1u) + 1u == static_cast<unsigned>(c.ngroups) ? 1u : 0u;
-      if (last) chain_done[ci] = 0u;
-    }
-    if (!__shfl_sync(kFull, last, 0)) return;
-    __threadfence();
-    s = x_walk(c, ag, gg, sg, sh_add[0]);
+    const int g = k0 / kXGroup, t0 = g * kXGroup, cnt = c.ntiles - t0 < kXGroup ? c.ntiles - t0 : kXGroup;
+    if (!last_of(group_done + c.group0 + g, (cnt + kXWarps - 1) / kXWarps)) return;
+    const XTileAgg G = x_group(lane < cnt ? x_load(ag + c.tile0 + t0 + lane) : x_no_summary(), cnt);
+    if (lane == 0) gg[c.group0 + g] = G;
+    if (!last_of(chain_done + ci, c.ngroups)) return;
+    s = x_walk(c, ag, gg, sh_add[0]);
   } else {
-    const int k = (static_cast<int>(blockIdx.x) - ngroups) * kXWarps + w;
-    if (k >= nshort) return;
-    ci = short_chain[k];
-    s = x_add(ch[ci].t, ch[ci].lo, ch[ci].hi, ch[ci].init, sh_add[w]);
+    if (ci < 0) return;
+    s = x_add(c.t, c.lo, c.hi, c.init, sh_add[w]);
   }
-  const XChain& c = ch[ci];
-  unsigned last = 0;
-  if (lane == 0) {
-    *c.out = s;
-    if (c.job >= 0) {
-      __threadfence();
-      last = atomicAdd(job_done + c.job, 1u) + 1u == static_cast<unsigned>(jobs[c.job].chunks) ? 1u : 0u;
-      if (last) job_done[c.job] = 0u;
-    }
-  }
-  if (!__shfl_sync(kFull, last, 0)) return;
-  __threadfence();
+  if (lane == 0) *c.out = s;
+  if (c.job < 0 || !last_of(job_done + c.job, jobs[c.job].chunks)) return;
   const XJob& J = jobs[c.job];
   s = x_add(J.part, 0, J.chunks, J.init, sh_add[w]);
   if (lane == 0) *J.out = s;
@@ -734,19 +737,22 @@ class SumPlan {
     if (exact) {
       std::vector<XChain> chains;
       std::vector<XJob> jobs;
-      std::vector<int> tile_chain, group_chain, short_chain;
+      ngroups_ = 0;
+      std::vector<int> tile_chain, block_chain, short_chain;
       long long nchunk_jobs = 0;
       for (const Job& j : jobs_)
         if (j.order == SumOrder::kChunk64) ++nchunk_jobs;
       partials_.alloc(static_cast<std::size_t>(nchunk_jobs > 0 ? nchunk_jobs * kChunks : 1));
       auto chain = [&](const double* t, long long lo, long long hi, double init, double* out, int job) {
-        XChain c{t, lo, hi, init, out, static_cast<int>(tile_chain.size()), 0, static_cast<int>(group_chain.size()), 0, job};
+        XChain c{t, lo, hi, init, out, static_cast<int>(tile_chain.size()), 0, ngroups_, 0,
+                 static_cast<int>(block_chain.size()), job};
         const int id = static_cast<int>(chains.size());
         if (hi - lo > kXShort) {
           c.ntiles = static_cast<int>((hi - lo + kXTile - 1) / kXTile);
           c.ngroups = (c.ntiles + kXGroup - 1) / kXGroup;
           tile_chain.insert(tile_chain.end(), static_cast<std::size_t>(c.ntiles), id);
-          group_chain.insert(group_chain.end(), static_cast<std::size_t>(c.ngroups), id);
+          ngroups_ += c.ngroups;
+          block_chain.insert(block_chain.end(), static_cast<std::size_t>((c.ntiles + kXWarps - 1) / kXWarps), id);
         } else {
           short_chain.push_back(id);
         }
@@ -765,18 +771,19 @@ class SumPlan {
         }
       }
       ntiles_ = static_cast<int>(tile_chain.size());
-      ngroups_ = static_cast<int>(group_chain.size());
+      nblocks_ = static_cast<int>(block_chain.size());
       nshort_ = static_cast<int>(short_chain.size());
       upload(chains, chains_, st);
       upload(jobs, xjobs_, st);
       upload(tile_chain, tile_chain_, st);
-      upload(group_chain, group_chain_, st);
+      upload(block_chain, block_chain_, st);
       upload(short_chain, short_chain_, st);
       stat_.alloc(static_cast<std::size_t>(ntiles_ > 0 ? ntiles_ : 1));
       tile_agg_.alloc(static_cast<std::size_t>(ntiles_ > 0 ? ntiles_ : 1) * sizeof(XTileAgg));
-      group_agg_.alloc(static_cast<std::size_t>(ngroups_ > 0 ? ngroups_ : 1) * sizeof(XGroupAgg));
-      done_.alloc(chains.size() + jobs.size() + 1);
-      B200_CHECK(cudaMemsetAsync(done_.get(), 0, (chains.size() + jobs.size() + 1) * sizeof(unsigned), st));
+      group_agg_.alloc(static_cast<std::size_t>(ngroups_ > 0 ? ngroups_ : 1) * sizeof(XTileAgg));
+      const std::size_t counters = static_cast<std::size_t>(ngroups_) + chains.size() + jobs.size();
+      done_.alloc(counters + 1);
+      B200_CHECK(cudaMemsetAsync(done_.get(), 0, (counters + 1) * sizeof(unsigned), st));
       nchains_ = static_cast<int>(chains.size());
     } else {
       std::vector<TreeSeg> tree;
@@ -799,14 +806,25 @@ class SumPlan {
                                                    stat_.get(), skip_);
         B200_LAUNCH_CHECK();
       }
-      const int blocks = ngroups_ + (nshort_ + kXWarps - 1) / kXWarps;
+      const int blocks = nblocks_ + (nshort_ + kXWarps - 1) / kXWarps;
       if (blocks > 0) {
-        k_xwalk<<<blocks, 32 * kXWarps, 0, st>>>(
-            ch, reinterpret_cast<const XJob*>(xjobs_.get()), reinterpret_cast<const int*>(group_chain_.get()), ngroups_,
-            reinterpret_cast<const int*>(short_chain_.get()), nshort_, stat_.get(),
-            reinterpret_cast<XTileAgg*>(tile_agg_.get()), reinterpret_cast<XGroupAgg*>(group_agg_.get()), done_.get(),
-            done_.get() + nchains_, skip_);
-        B200_LAUNCH_CHECK();
+        // its descriptors load while the kernel that makes the terms ends (programmatic dependent launch)
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(static_cast<unsigned>(blocks));
+        cfg.blockDim = dim3(32 * kXWarps);
+        cfg.stream = st;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        unsigned* done = done_.get();
+        B200_CHECK(cudaLaunchKernelEx(&cfg, k_xwalk, ch, reinterpret_cast<const XJob*>(xjobs_.get()),
+                                      reinterpret_cast<const int*>(block_chain_.get()), nblocks_,
+                                      reinterpret_cast<const int*>(short_chain_.get()), nshort_,
+                                      static_cast<const double*>(stat_.get()), reinterpret_cast<XTileAgg*>(tile_agg_.get()),
+                                      reinterpret_cast<XTileAgg*>(group_agg_.get()), done, done + ngroups_,
+                                      done + ngroups_ + nchains_, skip_));
       }
     } else if (nt_ > 0) {
       k_tree<<<nt_ * kTreeBlocks, kBlock, 0, st>>>(reinterpret_cast<const TreeSeg*>(tseg_.get()), partials_.get(),
@@ -815,7 +833,7 @@ class SumPlan {
     }
   }
   int kernel_count() const {
-    return exact_ ? (ntiles_ > 0) + (ngroups_ + nshort_ > 0) : (nt_ > 0 ? 1 : 0);
+    return exact_ ? (ntiles_ > 0) + (nblocks_ + nshort_ > 0) : (nt_ > 0 ? 1 : 0);
   }
   bool empty() const { return jobs_.empty(); }
 
@@ -839,11 +857,11 @@ class SumPlan {
   std::vector<Job> jobs_;
   bool exact_ = false;
   const int* skip_ = nullptr;
-  DevBuf<unsigned char> chains_, xjobs_, tseg_, tile_chain_, group_chain_, short_chain_;
+  DevBuf<unsigned char> chains_, xjobs_, tseg_, tile_chain_, block_chain_, short_chain_;
   mutable DevBuf<unsigned char> tile_agg_, group_agg_;
   mutable DevBuf<double> partials_, stat_;
   mutable DevBuf<unsigned> done_;
-  int nchains_ = 0, nshort_ = 0, nt_ = 0, ntiles_ = 0, ngroups_ = 0;
+  int nchains_ = 0, nshort_ = 0, nt_ = 0, ntiles_ = 0, nblocks_ = 0, ngroups_ = 0;
 };
 
 }  // namespace b200

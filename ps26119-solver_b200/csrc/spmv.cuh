@@ -80,15 +80,6 @@ struct SlabSmem {
 static __device__ unsigned int g_stage_timeouts;
 __device__ __forceinline__ void count_stage_timeout(unsigned* err) { atomicAdd(err ? err : &g_stage_timeouts, 1u); }
 
-// Programmatic dependent launch (sm_90+): a kernel launched with the programmatic-serialisation
-// attribute may start while the kernel before it in the stream is still running; it must not
-// touch that kernel's outputs (or anything a kernel still running may read or write) before
-// pdl_wait(), which returns once every earlier kernel has completed and its writes are visible.
-// pdl_allow_next() lets the next such kernel be scheduled once every block of this one has issued
-// it. In a kernel launched without the attribute both are no-ops.
-__device__ __forceinline__ void pdl_allow_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 __device__ __forceinline__ unsigned smem_u32(const void* p) {
   return static_cast<unsigned>(__cvta_generic_to_shared(p));
 }
