@@ -335,17 +335,8 @@ void Engine::setup() {
   B200_LAUNCH_CHECK();
   kernels_ += 2;
   // the largest slabs (the kernels' tile capacities), rows and columns
-  int ext[4] = {0, 0, 0, 0};
-  {
-    DevBuf<int> d(4);
-    B200_CHECK(cudaMemsetAsync(d.get(), 0, sizeof ext, st_));
-    if (m > 0) k_extents<<<std::min(grid_for(m), 8 * sm_count()), kBlock, 0, st_>>>(m, sp_.a_rp.get(), d.get());
-    if (n > 0) k_extents<<<std::min(grid_for(n), 8 * sm_count()), kBlock, 0, st_>>>(n, sp_.t_rp.get(), d.get() + 2);
-    B200_LAUNCH_CHECK();
-    kernels_ += 2;
-    B200_CHECK(cudaMemcpyAsync(ext, d.get(), sizeof ext, cudaMemcpyDeviceToHost, st_));
-    B200_CHECK(cudaStreamSynchronize(st_));
-  }
+  int ext[4];
+  sp_.extents(ext, st_);
   cap_a_ = fed_tile_capacity(ext[0]);
   cap_t_ = fed_tile_capacity(ext[2]);
   vd_.alloc(n, m);

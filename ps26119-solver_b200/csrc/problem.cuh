@@ -18,6 +18,7 @@
 #include <vector>
 
 #include "engine.hpp"
+#include "lanczos.cuh"
 #include "reduce.cuh"
 #include "setup.cuh"
 #include "spmv.cuh"
@@ -147,6 +148,8 @@ struct ScaledDevice {
   // original-space constants of kkt_general (cpu_backend.cpp:233-262): ‖b‖₂, ‖c‖₂, ‖c‖∞
   double b_norm = 0, c_norm = 0, c_inf = 0;
   long long kernels = 0;
+  int ext[4] = {0, 0, 0, 0};
+  bool have_extents = false;
   int lanczos_launched = 0;  // Lanczos steps launched by the last lanczos() (counted or not)
 
   // Scratch for the setup reductions.
@@ -157,6 +160,7 @@ struct ScaledDevice {
     M = dm;
     m = dm.m, n = dm.n, sense = dm.sense, nnz = dm.nnz;
     exact = exact_order;
+    have_extents = false;
     const std::size_t mm = static_cast<std::size_t>(m), nn = static_cast<std::size_t>(n);
     const std::size_t nz = static_cast<std::size_t>(nnz);
     a_rp.alloc(mm + 1);
@@ -299,6 +303,23 @@ struct ScaledDevice {
   template <class T> const T* rl() const;
   template <class T> const T* ru() const;
 
+  // out: the most nonzeros of a slab of rows, of a row, of a slab of columns, of a column (cached by the
+  // problem; synchronises the stream the first time).
+  void extents(int* out, cudaStream_t st) {
+    if (!have_extents) {
+      DevBuf<int> d(4);
+      B200_CHECK(cudaMemsetAsync(d.get(), 0, sizeof ext, st));
+      if (m > 0) k_extents<<<std::min(grid_for(m), 8 * sm_count()), kBlock, 0, st>>>(m, a_rp.get(), d.get());
+      if (n > 0) k_extents<<<std::min(grid_for(n), 8 * sm_count()), kBlock, 0, st>>>(n, t_rp.get(), d.get() + 2);
+      B200_LAUNCH_CHECK();
+      kernels += 2;
+      B200_CHECK(cudaMemcpyAsync(ext, d.get(), sizeof ext, cudaMemcpyDeviceToHost, st));
+      B200_CHECK(cudaStreamSynchronize(st));
+      have_extents = true;
+    }
+    std::copy(ext, ext + 4, out);
+  }
+
   // ‖Ã‖₂ by Lanczos on ÃᵀÃ (csr.cpp:86-132), on the device: the reference's start vector, the
   // products, and α and β reduced in the reference's order. α and β stay on the device, where the
   // next step's update reads them; the host reads them back a batch of steps at a time (21, then 8)
@@ -317,8 +338,7 @@ struct ScaledDevice {
     SumPlan pal, pbn;
     pal.add(terms.get(), 0, n, 0.0, SumOrder::kSeq, out.get());
     pbn.add(terms.get(), 0, n, 0.0, SumOrder::kSeq, out.get() + 1);
-    pal.build(true, nullptr, st);  // α and β enter η = 0.998/‖Ã‖₂: always the reference's order
-    pbn.build(true, nullptr, st);
+    pbn.build(true, nullptr, st);  // α and β enter η = 0.998/‖Ã‖₂: always the reference's order
     k_lanczos_start<<<grid_for((n + kStartRun - 1) / kStartRun, 64), 64, 0, st>>>(n, jump.get(), v.get(), terms.get());
     B200_LAUNCH_CHECK();
     pbn.launch(st);
@@ -327,7 +347,36 @@ struct ScaledDevice {
     B200_CHECK(cudaMemsetAsync(out.get() + 1, 0, sizeof(double), st));  // no β before the first step
     kernels += 2 + pbn.kernel_count();
     const int tiles = (n + kXTile - 1) / kXTile;
+    // An LP that fits the SMs' shared memory takes a batch of steps in one launch (lanczos.cuh).
+    int ext[4];
+    extents(ext, st);
+    const LanczosShape shape = lanczos_shape(m, n, nnz, ext[1], ext[3]);
+    DevBuf<Cell<double>> cells;
+    DevBuf<XFast> fast;
+    DevBuf<XTileAgg> full;
+    DevBuf<unsigned> count(1);
+    unsigned tag = 1;
+    if (shape.blocks > 0) {
+      cells.alloc(static_cast<std::size_t>(n) + m + shape.blocks + 1);
+      fast.alloc(static_cast<std::size_t>(n / kXTile + shape.blocks));
+      full.alloc(static_cast<std::size_t>(n / kXTile + shape.blocks));
+      B200_CHECK(cudaMemsetAsync(cells.get(), 0, cells.size() * sizeof(Cell<double>), st));
+      B200_CHECK(cudaMemsetAsync(count.get(), 0, sizeof(unsigned), st));
+    } else {
+      pal.build(true, nullptr, st);
+    }
     auto launch = [&](int from, int to) {
+      if (shape.blocks > 0) {
+        Cell<double>* c = cells.get();
+        launch_lanczos({m, n, shape.blocks, t_rp.get(), t_ri.get(), a_rp.get(), a_col.get(), sat.get(), sa.get(),
+                        c, c + n, c + n + m, c + n + m + shape.blocks, v.get(), vprev.get(), terms.get(), hist.get(),
+                        fast.get(), full.get(), count.get(), tag, from, to, err},
+                       shape, st);
+        tag += 3u * static_cast<unsigned>(to - from) + 2u;
+        ++kernels;
+        lanczos_launched = to;
+        return;
+      }
       for (int k = from; k < to; ++k) {
         launch_slab_tma<double>(m, a_rp.get(), a_col.get(), sa.get(), v.get(), EpiStore<double>{{}, t.get()}, st,
                                 nullptr, err);

@@ -58,9 +58,10 @@ __device__ __forceinline__ double block_sum_fixed(double v, double* sh) {
 //   k_xstat   per tile of kXTile terms (one warp): an approximate fp64 sum, in any order; only used
 //             to guess each tile's binade. A kernel that produces the terms may leave it itself.
 //   k_xwalk   one warp per tile, kXWarps tiles per block: the guessed binade's u from the approximate
-//             start (the approximate sums of the chain's earlier tiles), then the tile's XRun (exact
-//             int64: change of S, its lowest and highest running value, parity after, per parity
-//             before); a term with |t/u| ≥ 2^51 (or non-finite) marks the tile. A tile whose running sum
+//             start (the approximate sums of the chain's earlier tiles), then the tile's XRun (change of
+//             S, bounds of its running value, parity after, per parity before): each lane adds its terms
+//             in fp64 to an approximate start of either parity, and the differences of the sums' bits are
+//             the changes of S. A tile whose running sum
 //             changes binade once is summarised in three parts: the run before the term that changes it,
 //             that term, the run after it in the new grid. The block that finishes last of a group of
 //             kXGroup tiles composes the tiles' summaries into the group's, of the same form. The block
@@ -75,13 +76,14 @@ __device__ __forceinline__ double block_sum_fixed(double v, double* sh) {
 // The approximations only choose between two exact paths; the result never depends on them.
 //
 // What bounds it: latency. A dependent fp64 addition takes 8.3 cycles, 10.4 with its operand from
-// shared memory, so a tile added one by one takes 1.4 us, and the walk of a chain pays that for its
-// first tile (the sum starts at zero) and for the few tiles that cross a binade more than once; the
-// other steps are one check over 32 summaries held by the warp's lanes, and a hand-over per crossing.
-// Tiles of 256 terms, one warp's, keep the tiles that must be added one by one cheap. Measured, 15,000
-// terms: 18.5 us a launch (24 with summaries read from shared memory and scanned anew at every crossing,
-// 16 warps of a block on 32 tiles); three launches over tiles of 2,048 terms, the first tile walked in
-// windows of 256 with a scan and a restart per binade crossing, took 68 us.
+// shared memory, so a tile added one by one takes 1.4 us; the first one's terms are added while the others
+// are summarised, and the few tiles that cross a binade more than once cost that in the walk. Its other
+// steps are one check over 32 summaries held by the warp's lanes, and a hand-over per crossing, on
+// integers. Tiles of 256 terms, one warp's, keep the tiles that must be added one by one cheap. Measured,
+// 15,000 terms: 14 us a launch; 18.5 with the terms in units of u by division and rounding, every summary
+// read in full and the first tile left to the walk; 24 with summaries scanned anew in shared memory at
+// every crossing; three launches over tiles of 2,048 terms, the first walked in windows with a scan and a
+// restart per crossing, took 68 us.
 constexpr int kXPer = 8;              // terms per lane
 constexpr int kXTile = 32 * kXPer;    // terms per tile (one warp)
 constexpr int kXGroup = 32;           // tiles per group (one warp lane each)
@@ -107,33 +109,56 @@ struct XJob {
   double* out;
 };
 // The effect of a run of terms on S (the partial sum in units of u), for S even (index 0) and
-// odd (1) at the run's start: K the change of S, mn / mx the lowest / highest running change
-// over positions 1…len (LLONG_MAX / LLONG_MIN for an empty run), out the parity after; bad: a
-// term the integer form cannot take (|t/u| ≥ 2^51 or non-finite); ties: a term is a tie, so that the
-// two parities may differ (without one they agree, and a run is plain integer sums).
+// odd (1) at the run's start: K the change of S; mn / mx bounds of the running change over positions
+// 1…len in units of 2^24, rounded outward (INT_MAX / INT_MIN for an empty run); out the parity after; bad: it
+// cannot be told; ties: the two parities' changes differ somewhere (else a run is plain integer sums).
 struct alignas(16) XRun {
-  long long K[2], mn[2], mx[2];
+  long long K[2];
+  int mn[2], mx[2];
   int out[2];
   int bad, ties;
 };
-// A tile's summary: its terms before `split` counted in the grid u (the binade of the tile's
-// approximate start), the term at `split` (where the approximate running sum leaves that binade;
-// split = −1: it never does) added as a plain fp64 addition, the terms after it counted in the
-// grid u1 of the binade the running sum moved to. u = 0: no usable guess (bad is set). A group's summary
-// has the same form (its split is the tile that changes binade).
+// A tile's summary: its terms before the split counted in the grid of binade e (that of the tile's
+// approximate start), the term where the approximate running sum leaves that binade (split = false: none
+// does) added as a plain fp64 addition, the terms after it counted in the grid of the binade e1 that the
+// running sum moved to. A group's summary has the same form (its split is the tile that changes binade).
 struct alignas(16) XTileAgg {
-  double u, u1;
-  double at;  // the term at `split`
+  double at;  // the term at the split
+  int e, e1;
   XRun pre, suf;
-  int split;
+  bool split;
 };
+// What a walk reads of every summary: a run in one grid without ties is complete here (kXPlain); one with
+// ties or a change of binade is looked up in full (kXFull); kXNone: no summary; kXStart: the chain's
+// first terms, added one by one from its start (the bits of that sum are K). first, len: the tile's terms,
+// where a walk needs them from here.
+enum : int { kXPlain = 0, kXFull = 1, kXNone = 2, kXStart = 3 };
+struct alignas(16) XFast {
+  long long K;
+  int e;
+  int mn, mx;
+  int first;
+  int kind, len;
+};
+struct XSummary {  // as it is made
+  XFast fast;
+  XTileAgg full;
+};
+
 constexpr long long kX52 = 1LL << 52, kX53 = 1LL << 53;
+constexpr int kXShift = 24;  // the bounds' unit
+// x in that unit, rounded down or up; far values (which no check lets pass) stay far.
+__device__ __forceinline__ int x_down(long long x) {
+  x >>= kXShift;
+  return static_cast<int>(x < -(1LL << 29) - 64 ? -(1LL << 29) - 64 : (x > (1LL << 29) + 64 ? (1LL << 29) + 64 : x));
+}
+__device__ __forceinline__ int x_up(long long x) { return x_down(x + ((1LL << kXShift) - 1)); }
 
 __device__ __forceinline__ XRun x_identity() {
   XRun r;
   r.K[0] = r.K[1] = 0;
-  r.mn[0] = r.mn[1] = LLONG_MAX;
-  r.mx[0] = r.mx[1] = LLONG_MIN;
+  r.mn[0] = r.mn[1] = INT_MAX;
+  r.mx[0] = r.mx[1] = INT_MIN;
   r.out[0] = 0, r.out[1] = 1;
   r.bad = r.ties = 0;
   return r;
@@ -146,10 +171,10 @@ __device__ __forceinline__ XRun x_compose(const XRun& a, const XRun& b) {
 #pragma unroll
   for (int p = 0; p < 2; ++p) {
     const bool q = a.out[p] != 0;
-    const long long bK = q ? b.K[1] : b.K[0], bmn = q ? b.mn[1] : b.mn[0], bmx = q ? b.mx[1] : b.mx[0];
-    r.K[p] = a.K[p] + bK;
-    r.mn[p] = bmn == LLONG_MAX ? a.mn[p] : min(a.mn[p], a.K[p] + bmn);
-    r.mx[p] = bmx == LLONG_MIN ? a.mx[p] : max(a.mx[p], a.K[p] + bmx);
+    const int bmn = q ? b.mn[1] : b.mn[0], bmx = q ? b.mx[1] : b.mx[0];
+    r.K[p] = a.K[p] + (q ? b.K[1] : b.K[0]);
+    r.mn[p] = bmn == INT_MAX ? a.mn[p] : min(a.mn[p], x_down(a.K[p]) + bmn);
+    r.mx[p] = bmx == INT_MIN ? a.mx[p] : max(a.mx[p], x_up(a.K[p]) + bmx);
     r.out[p] = q ? b.out[1] : b.out[0];
   }
   return r;
@@ -169,18 +194,6 @@ __device__ __forceinline__ XRun x_shfl_down(const XRun& v, int off) {
   x_unpack(r, __shfl_down_sync(kFull, x_pack(v), off));
   return r;
 }
-__device__ __forceinline__ XRun x_shfl_up(const XRun& v, int off) {
-  XRun r;
-#pragma unroll
-  for (int p = 0; p < 2; ++p) {
-    r.K[p] = __shfl_up_sync(kFull, v.K[p], off);
-    r.mn[p] = __shfl_up_sync(kFull, v.mn[p], off);
-    r.mx[p] = __shfl_up_sync(kFull, v.mx[p], off);
-  }
-  x_unpack(r, __shfl_up_sync(kFull, x_pack(v), off));
-  return r;
-}
-
 // e = floor(log2 |v|) for a normal v whose ulp 2^(e−52) and 2^(52−e) are both normal doubles;
 // otherwise returns false.
 __device__ __forceinline__ bool x_binade(double v, int& e) {
@@ -196,96 +209,45 @@ __device__ __forceinline__ int x_top(double v) { return __double2hiint(v) >> 20;
 __device__ __forceinline__ double x_pow2(int p) {  // 2^p, p in [−1022, 1023]
   return __longlong_as_double(static_cast<long long>(p + 1023) << 52);
 }
-// A term in units of u (inv_u = 1/u, powers of two: t·inv_u is exact unless it under/overflows):
-// false for |t/u| ≥ 2^51 or a non-finite t; else kf = rint(t/u), or floor(t/u) for a tie. Adding and
-// taking away 1.5·2^52 rounds to an integer, and leaves it in the low bits of the sum.
-__device__ __forceinline__ bool x_term(double t, double inv_u, long long& kf, bool& tie) {
-  constexpr double kMagic = 6755399441055744.0;  // 1.5·2^52
-  const double q = t * inv_u;
-  if (!(fabs(q) < 2251799813685248.0)) return false;  // 2^51; also NaN / inf
-  const double m = q + kMagic;
-  kf = __double_as_longlong(m) - __double_as_longlong(kMagic);
-  const double d = q - (m - kMagic);
-  tie = fabs(d) == 0.5;
-  if (d == -0.5) --kf;
-  return true;
+// A normal s as an integer multiple S of its binade's ulp, |S| in [2^52, 2^53), and back (by its bits).
+__device__ __forceinline__ long long x_int(double s) {
+  const long long b = __double_as_longlong(s), m = (b & (kX52 - 1)) | kX52;
+  return b < 0 ? -m : m;
 }
-// The step of S with parity `par` for a term (kf, tie): returns k; par becomes S + k's parity.
-__device__ __forceinline__ long long x_step(long long kf, bool tie, int& par) {
-  long long k = kf;
-  if (tie) {
-    k += (par + kf) & 1;  // to the even neighbour
-    par = 0;
-  } else {
-    par = static_cast<int>((par + k) & 1);
-  }
-  return k;
+__device__ __forceinline__ double x_double(long long S, int e) {
+  const long long a = S < 0 ? -S : S;
+  return __longlong_as_double((a & (kX52 - 1)) | (static_cast<long long>(e + 1023) << 52) | (S < 0 ? LLONG_MIN : 0LL));
 }
-// The XRun of a warp's terms (lane l holds terms 8l … 8l+7; those whose bit q is set in `mask`, the
-// others left out), valid in lane 0. Without a tie both parities make the same steps, and the run is
-// integer sums: about a sixth of the general form's instructions.
-__device__ __forceinline__ XRun x_warp_run(const double* v, unsigned mask, double inv_u) {
+// The composition of the warp's runs in lane order, valid in lane 0.
+__device__ __forceinline__ XRun x_warp_ordered(XRun r) {
   const int lane = threadIdx.x & 31;
-  XRun r = x_identity();
-  long long kf[kXPer];
-  bool tie[kXPer];
-#pragma unroll
-  for (int q = 0; q < kXPer; ++q) {
-    kf[q] = 0, tie[q] = false;
-    if ((mask >> q) & 1u) {
-      if (!x_term(v[q], inv_u, kf[q], tie[q])) r.bad = 1, kf[q] = 0, tie[q] = false;
-      r.ties |= tie[q] ? 1 : 0;
+  if (!__any_sync(kFull, r.ties)) {
+    const long long K = r.K[0];
+    long long inc = K;
+    for (int off = 1; off < 32; off <<= 1) {
+      const long long o = __shfl_up_sync(kFull, inc, off);
+      if (lane >= off) inc += o;
     }
-  }
-  if (__any_sync(kFull, r.ties)) {
-#pragma unroll
-    for (int p = 0; p < 2; ++p) {
-      int par = p;
-      long long K = 0;
-#pragma unroll
-      for (int q = 0; q < kXPer; ++q)
-        if ((mask >> q) & 1u) {
-          K += x_step(kf[q], tie[q], par);
-          r.mn[p] = min(r.mn[p], K);
-          r.mx[p] = max(r.mx[p], K);
-        }
-      r.K[p] = K;
-      r.out[p] = par;
-    }
-    for (int off = 1; off < 32; off <<= 1) {  // ordered reduction (lane order)
-      const XRun o = x_shfl_down(r, off);
-      if ((lane & (2 * off - 1)) == 0 && lane + off < 32) r = x_compose(r, o);
-    }
+    const bool any = r.mn[0] != INT_MAX;
+    r.K[0] = r.K[1] = __shfl_sync(kFull, inc, 31);
+    r.mn[0] = r.mn[1] = __reduce_min_sync(kFull, any ? x_down(inc - K) + r.mn[0] : INT_MAX);
+    r.mx[0] = r.mx[1] = __reduce_max_sync(kFull, any ? x_up(inc - K) + r.mx[0] : INT_MIN);
+    r.out[0] = static_cast<int>(r.K[0] & 1), r.out[1] = r.out[0] ^ 1;
+    r.bad = __any_sync(kFull, r.bad) ? 1 : 0;
     return r;
   }
-  long long K = 0, mn = LLONG_MAX, mx = LLONG_MIN;
-#pragma unroll
-  for (int q = 0; q < kXPer; ++q)
-    if ((mask >> q) & 1u) {
-      K += kf[q];
-      mn = min(mn, K);
-      mx = max(mx, K);
-    }
-  long long inc = K;
   for (int off = 1; off < 32; off <<= 1) {
-    const long long o = __shfl_up_sync(kFull, inc, off);
-    if (lane >= off) inc += o;
+    const XRun o = x_shfl_down(r, off);
+    if ((lane & (2 * off - 1)) == 0 && lane + off < 32) r = x_compose(r, o);
   }
-  if (mask) mn += inc - K, mx += inc - K;
-  for (int off = 16; off > 0; off >>= 1) {
-    mn = min(mn, __shfl_xor_sync(kFull, mn, off));
-    mx = max(mx, __shfl_xor_sync(kFull, mx, off));
-  }
-  r.K[0] = r.K[1] = __shfl_sync(kFull, inc, 31);
-  r.mn[0] = r.mn[1] = mn;
-  r.mx[0] = r.mx[1] = mx;
-  r.out[0] = static_cast<int>(r.K[0] & 1), r.out[1] = r.out[0] ^ 1;
-  r.bad = __any_sync(kFull, r.bad) ? 1 : 0;
   return r;
 }
-// |S| inside [2^52 + 1, 2^53 − 1] with the sign of S0.
-__device__ __forceinline__ bool x_inside(long long S0, long long S) {
-  return S0 > 0 ? (S >= kX52 + 1 && S <= kX53 - 1) : (S <= -(kX52 + 1) && S >= -(kX53 - 1));
+// Whether every S + r, mn ≤ r ≤ mx in units of 2^24, lies inside [2^52 + 1, 2^53 − 1] with the sign of S0
+// (S: S0 plus the change before the run).
+__device__ __forceinline__ bool x_inside(long long S0, long long S, int mn, int mx) {
+  const long long lo = (S >> kXShift) + mn, hi = (S >> kXShift) + 1 + mx;
+  constexpr long long a = (kX52 >> kXShift) + 1, b = (kX53 >> kXShift) - 1;
+  return S0 > 0 ? (lo >= a && hi <= b) : (lo >= -b && hi <= -a);
 }
 
 // A struct of 16-byte words another block wrote, read past this SM's L1.
@@ -374,52 +336,89 @@ __device__ __forceinline__ void x_leave_stat(double* stat, double term) {
   }
 }
 
-// The composition of the warp's runs in lane order, valid in lane 0.
-__device__ __forceinline__ XRun x_warp_ordered(XRun r) {
-  const int lane = threadIdx.x & 31;
-  if (!__any_sync(kFull, r.ties)) {
-    long long inc = r.K[0], mn = r.mn[0], mx = r.mx[0];
-    for (int off = 1; off < 32; off <<= 1) {
-      const long long o = __shfl_up_sync(kFull, inc, off);
-      if (lane >= off) inc += o;
-    }
-    if (mn != LLONG_MAX) mn += inc - r.K[0], mx += inc - r.K[0];
-    for (int off = 16; off > 0; off >>= 1) {
-      mn = min(mn, __shfl_xor_sync(kFull, mn, off));
-      mx = max(mx, __shfl_xor_sync(kFull, mx, off));
-    }
-    r.K[0] = r.K[1] = __shfl_sync(kFull, inc, 31);
-    r.mn[0] = r.mn[1] = mn;
-    r.mx[0] = r.mx[1] = mx;
-    r.out[0] = static_cast<int>(r.K[0] & 1), r.out[1] = r.out[0] ^ 1;
-    r.bad = __any_sync(kFull, r.bad) ? 1 : 0;
-    return r;
-  }
-  for (int off = 1; off < 32; off <<= 1) {
-    const XRun o = x_shfl_down(r, off);
-    if ((lane & (2 * off - 1)) == 0 && lane + off < 32) r = x_compose(r, o);
-  }
-  return r;
+__device__ __forceinline__ XTileAgg x_no_full() {
+  XTileAgg T;
+  T.at = 0.0, T.e = T.e1 = 0;
+  T.pre = T.suf = x_identity();
+  T.split = false;
+  return T;
 }
 
-// The summary of the terms t[a, b) (one tile, one warp; lane l holds terms 8l … 8l+7) for a chain
+// One lane's terms v[q0, q1) added to a start of either parity near `start`, whose binade (top bits `top`)
+// they are meant to stay in: for each parity the change of S, read off the bits; bounds of the running
+// change in units of 2^24; and whether every sum had those top bits. Every double of a binade is a multiple
+// of its ulp, so these are the chain's own steps for any start of that parity as far as it stays inside.
+// The two sums are never more than two ulps apart, so the first one's bounds, widened, serve both: where the
+// other could leave the binade the bounds are too near its end for any commit. start > 0.
+struct XLane {
+  long long K[2];
+  int mn, mx;
+  double end;  // the sum from `start` itself
+  bool clean;
+};
+template <class V>
+__device__ __forceinline__ XLane x_lane(V&& v, int q0, int q1, double start, int top) {
+  XLane r;
+  const double o0 = __longlong_as_double(__double_as_longlong(start) ^ 1);
+  double s = start, o = o0;
+  const auto mid = [](double x) {  // bits 24 … 55: the exponent's lowest and the fraction's highest
+    return static_cast<unsigned>(__funnelshift_r(__double2loint(x), __double2hiint(x), kXShift));
+  };
+  int lo = __double2hiint(start), hi = lo;
+  unsigned mn = mid(start), mx = mn;
+#pragma unroll
+  for (int q = 0; q < kXPer; ++q)
+    if (q >= q0 && q < q1) {
+      s += v(q), o += v(q);
+      lo = min(lo, __double2hiint(s)), hi = max(hi, __double2hiint(s));
+      mn = min(mn, mid(s)), mx = max(mx, mid(s));
+    }
+  r.end = s;
+  r.clean = (lo >> 20) == top && (hi >> 20) == top;
+  const long long b = __double_as_longlong(start);
+  const long long same = __double_as_longlong(s) - b, other = __double_as_longlong(o) - __double_as_longlong(o0);
+  const bool odd = (b & 1) != 0;
+  r.K[0] = odd ? other : same, r.K[1] = odd ? same : other;
+  r.mn = static_cast<int>(mn - mid(start)) - 2;
+  r.mx = static_cast<int>(mx - mid(start)) + 2;
+  return r;
+}
+// The composition of the warp's lanes in lane order (`in`: a lane's part counts, `any`: it has terms), valid
+// in lane 0; flip: the terms' and the sum's signs were turned.
+__device__ __forceinline__ XRun x_compose_lanes(const XLane& r, bool in, bool any, bool flip) {
+  XRun x = x_identity();
+  if (in && any) {
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+      x.K[p] = flip ? -r.K[p] : r.K[p];
+      x.out[p] = static_cast<int>((p + r.K[p]) & 1);
+      x.mn[p] = flip ? -r.mx : r.mn, x.mx[p] = flip ? -r.mn : r.mx;
+    }
+    x.ties = r.K[0] != r.K[1];
+  }
+  return x_warp_ordered(x);
+}
+
+// The summary of the terms t[a, b) (one tile, one warp; lane l holds kXPer terms from l·kXPer) for a chain
 // whose approximate sum before them is s0; valid in lane 0.
-__device__ __forceinline__ XTileAgg x_tile_agg(const double* __restrict__ t, long long a, long long b, double s0) {
+__device__ __forceinline__ XTileAgg x_tile_full(const double* __restrict__ t, long long a, long long b, double s0) {
   const int lane = threadIdx.x & 31;
-  XTileAgg g;
-  g.u = g.u1 = g.at = 0.0;
-  g.split = -1;
-  g.pre = g.suf = x_identity();
+  XTileAgg g = x_no_full();
   int e0;
   if (!x_binade(s0, e0)) {  // uniform over the warp
     g.pre.bad = 1;
     return g;
   }
+  const bool flip = s0 < 0;
   const long long i0 = a + static_cast<long long>(lane) * kXPer;
+  const int cnt = b - i0 >= kXPer ? kXPer : (b > i0 ? static_cast<int>(b - i0) : 0);
   double v[kXPer];
-  double run = 0.0;
 #pragma unroll
-  for (int q = 0; q < kXPer; ++q) v[q] = i0 + q < b ? t[i0 + q] : 0.0;
+  for (int q = 0; q < kXPer; ++q) {
+    v[q] = q < cnt ? t[i0 + q] : 0.0;
+    if (flip) v[q] = -v[q];
+  }
+  double run = 0.0;
 #pragma unroll
   for (int q = 0; q < kXPer; ++q) run += v[q];
   double inc = run;
@@ -427,166 +426,181 @@ __device__ __forceinline__ XTileAgg x_tile_agg(const double* __restrict__ t, lon
     const double o = __shfl_up_sync(kFull, inc, off);
     if (lane >= off) inc += o;
   }
-  const double start = s0 + (inc - run);
-  // the first position whose approximate running sum leaves e0's binade
-  const int base = lane * kXPer;
-  const int top0 = x_top(s0);
-  int first = INT_MAX;
-  double acc = start, at = 0.0, term = 0.0;
-#pragma unroll
-  for (int q = 0; q < kXPer; ++q)
-    if (i0 + q < b) {
-      acc += v[q];
-      if (first == INT_MAX && x_top(acc) != top0) first = base + q, at = acc, term = v[q];
-    }
-  const int split = __reduce_min_sync(kFull, first);
-  // the binade after the split: all later approximate running sums must share it
-  int e1 = e0;
-  bool ok1 = true;
-  if (split != INT_MAX) {
-    const double after = __shfl_sync(kFull, at, split / kXPer);
-    ok1 = x_binade(after, e1);
-    const int top1 = x_top(after);
-    bool same = true;
-    acc = start;
+  const double start = (flip ? -s0 : s0) + (inc - run);  // this lane's approximate start
+  const auto term = [&](int q) { return v[q]; };
+  const int top0 = x_top(flip ? -s0 : s0);
+  const XLane r = x_lane(term, 0, cnt, start, x_top(start));
+  // lanes before k stay in s0's binade; lane k, if there is one, leaves it
+  const unsigned left = __ballot_sync(kFull, cnt > 0 && !(r.clean && x_top(start) == top0));
+  const int k = left ? __ffs(left) - 1 : 32;
+  g.e = e0;
+  if (k == 32) {
+    g.pre = x_compose_lanes(r, true, cnt > 0, flip);
+    return g;
+  }
+  // the term of lane k that leaves it, and its terms before and after that one
+  int split = kXPer, top1 = 0;
+  double at = 0.0, after = 0.0;
+  XLane pre = r, suf = r;
+  bool ok = lane < k || cnt == 0;
+  if (lane == k) {
+    double s = start;
 #pragma unroll
     for (int q = 0; q < kXPer; ++q)
-      if (i0 + q < b) {
-        acc += v[q];
-        if (base + q > split && x_top(acc) != top1) same = false;
+      if (q < cnt && split == kXPer) {
+        s += v[q];
+        if (x_top(s) != top0) split = q, at = v[q], after = s;
       }
-    ok1 = __all_sync(kFull, same) && ok1;
+    int e1;
+    ok = x_top(start) == top0 && split < kXPer && after > 0 && x_binade(after, e1);
+    top1 = x_top(after);
+    pre = x_lane(term, 0, split, start, top0);
+    suf = x_lane(term, split + 1, cnt, after, top1);
+    ok = ok && pre.clean && suf.clean;
   }
-  unsigned mpre = 0, msuf = 0;
-#pragma unroll
-  for (int q = 0; q < kXPer; ++q)
-    if (i0 + q < b) {
-      if (base + q < split) mpre |= 1u << q;
-      else if (split != INT_MAX && base + q > split) msuf |= 1u << q;
-    }
-  g.u = x_pow2(e0 - 52);
-  g.pre = x_warp_run(v, mpre, x_pow2(52 - e0));
-  if (split != INT_MAX) {
-    g.split = split;
-    g.at = __shfl_sync(kFull, term, split / kXPer);
-    if (ok1) {
-      g.u1 = x_pow2(e1 - 52);
-      g.suf = x_warp_run(v, msuf, x_pow2(52 - e1));
-    } else {
-      g.suf.bad = 1;
-    }
+  const int top1k = __shfl_sync(kFull, top1, k);
+  if (lane > k) ok = cnt == 0 || (r.clean && x_top(start) == top1k);
+  if (!__all_sync(kFull, ok)) {
+    g.pre.bad = 1;
+    return g;
   }
+  g.pre = x_compose_lanes(pre, lane <= k, lane < k ? cnt > 0 : split > 0, flip);
+  g.suf = x_compose_lanes(suf, lane >= k, lane > k ? cnt > 0 : split + 1 < cnt, flip);
+  g.e1 = (top1k & 0x7ff) - 1023;
+  g.split = true;
+  at = __shfl_sync(kFull, at, k);
+  g.at = flip ? -at : at;
   return g;
 }
 
-// Commits the run r (counted in the grid u) onto the exact s when s lies in u's binade and every
-// running S stays inside it; returns false (s unchanged) otherwise.
-__device__ __forceinline__ bool x_commit(double& s, double u, const XRun& r) {
-  int e;
-  if (r.bad || u == 0.0 || !x_binade(s, e) || x_pow2(e - 52) != u) return false;
-  const long long S0 = static_cast<long long>(s * x_pow2(52 - e));
-  const bool odd = (S0 & 1) != 0;
-  if (r.mn[0] == LLONG_MAX) return true;  // an empty run
-  const long long mn = odd ? r.mn[1] : r.mn[0], mx = odd ? r.mx[1] : r.mx[0];
-  if (!x_inside(S0, S0 + mn) || !x_inside(S0, S0 + mx)) return false;
-  s = static_cast<double>(S0 + (odd ? r.K[1] : r.K[0])) * u;
-  return true;
+// A full summary's short form.
+__device__ __forceinline__ XSummary x_summary(const XTileAgg& T) {
+  XSummary r;
+  r.full = T;
+  r.fast.K = T.pre.K[0], r.fast.e = T.e, r.fast.mn = T.pre.mn[0], r.fast.mx = T.pre.mx[0];
+  r.fast.first = 0, r.fast.len = 0;
+  r.fast.kind = T.pre.bad ? kXNone : (T.split || T.pre.ties ? kXFull : kXPlain);
+  return r;
+}
+__device__ __forceinline__ XFast x_no_fast() {
+  XFast f;
+  f.K = 0, f.e = 0, f.mn = INT_MAX, f.mx = INT_MIN, f.first = 0, f.kind = kXNone, f.len = 0;
+  return f;
+}
+// The sum after the chain's first terms, as a summary (its walk starts with it).
+__device__ __forceinline__ XSummary x_start(double s) {
+  XSummary r;
+  r.full = x_no_full();
+  r.fast = x_no_fast();
+  r.fast.kind = kXStart, r.fast.K = __double_as_longlong(s);
+  return r;
+}
+__device__ __forceinline__ void x_leave(const XSummary& S, XFast* fast, XTileAgg* full) {  // one lane
+  *fast = S.fast;
+  if (S.fast.kind == kXFull) *full = S.full;
 }
 
-// Commits a whole summary, its change of binade included; returns false (s unchanged) where it cannot.
-__device__ __forceinline__ bool x_commit(double& s, const XTileAgg& T) {
-  double s2 = s;
-  if (!x_commit(s2, T.u, T.pre)) return false;
-  if (T.split >= 0) {
-    s2 += T.at;  // the term that changes the binade, as the chain adds it
-    if (!x_commit(s2, T.u1, T.suf)) return false;
+// Commits a whole summary, its change of binade included, to the sum S·2^(e − 52); returns false (nothing
+// changed) where a running S could leave its binade.
+__device__ __forceinline__ bool x_commit(long long& S, int& e, const XTileAgg& T) {
+  if (T.e != e) return false;
+  bool odd = (S & 1) != 0;
+  long long R = S;
+  if (T.pre.mn[0] != INT_MAX) {
+    if (!x_inside(S, S, odd ? T.pre.mn[1] : T.pre.mn[0], odd ? T.pre.mx[1] : T.pre.mx[0])) return false;
+    R += odd ? T.pre.K[1] : T.pre.K[0];
   }
-  s = s2;
+  int e2 = e;
+  if (T.split) {
+    const double s = x_double(R, e) + T.at;  // the term that changes the binade, as the chain adds it
+    if (!x_binade(s, e2) || e2 != T.e1) return false;
+    R = x_int(s);
+    if (T.suf.mn[0] != INT_MAX) {
+      odd = (R & 1) != 0;
+      if (!x_inside(R, R, odd ? T.suf.mn[1] : T.suf.mn[0], odd ? T.suf.mx[1] : T.suf.mx[0])) return false;
+      R += odd ? T.suf.K[1] : T.suf.K[0];
+    }
+  }
+  S = R, e = e2;
   return true;
 }
 
-// One warp walks cnt consecutive summaries, lane l holding T of the l-th, with the exact s. other(k, s)
-// returns the sum after the k-th where its summary cannot be committed. Every step commits all summaries
-// up to the first that changes binade, is not in s's binade, or whose running S would leave it. Without
-// ties a run's K does not depend on what came before, so one prefix sum over the lanes serves all steps
-// (across a change of grid the sum means nothing, but a step only uses differences within one).
+// What one lane holds of a walk's round of up to 32 summaries.
+struct XRound {
+  XFast fast;
+  XTileAgg full;
+};
+__device__ __forceinline__ XRound x_round(const XFast& f, const XTileAgg* full, bool here) {
+  XRound r;
+  r.fast = f;
+  r.full = x_no_full();
+  if (here && f.kind == kXFull) r.full = x_load(full);
+  return r;
+}
+
+// One warp walks cnt consecutive summaries, lane l holding the l-th, with the exact s. other(k, s) returns
+// the sum after the k-th where its summary cannot be committed. A step commits all plain summaries up to
+// the first that is not one, not in s's binade, or whose running S would leave it; that one is committed
+// by the lane that holds it. Without ties a run's K does not depend on what came before, so one prefix sum
+// over the lanes serves all steps (across a change of grid the sum means nothing, but a step only uses
+// differences within one).
 template <class F>
-__device__ __forceinline__ double x_walk_lanes(double s, const XTileAgg& T, int cnt, F&& other) {
+__device__ __forceinline__ double x_walk_lanes(double s, const XRound& G, int cnt, F&& other) {
   const int lane = threadIdx.x & 31;
   const bool here = lane < cnt;
-  const bool plain = here && !T.pre.bad && T.split < 0 && T.u != 0.0;
-  const unsigned ties = __ballot_sync(kFull, here && T.pre.ties);
-  long long inc = here ? T.pre.K[0] : 0;
+  const bool plain = here && G.fast.kind == kXPlain, empty = plain && G.fast.mn == INT_MAX;
+  long long inc = plain ? G.fast.K : 0;
+#pragma unroll
   for (int off = 1; off < 32; off <<= 1) {
     const long long o = __shfl_up_sync(kFull, inc, off);
     if (lane >= off) inc += o;
   }
-  const long long before = inc - (here ? T.pre.K[0] : 0);
-  int j = 0;
+  const long long before = inc - (plain ? G.fast.K : 0);
+  int j = 0, e;
+  bool have = x_binade(s, e);
+  long long S = x_int(s), base = 0;  // base: `before` at lane j
   while (j < cnt) {
-    int e;
-    const bool have = x_binade(s, e);
-    const double u = have ? x_pow2(e - 52) : 0.0;
-    const unsigned stop = __ballot_sync(kFull, lane >= j && !(plain && have && T.u == u));
-    int f = stop ? __ffs(stop) - 1 : 32;  // the first that cannot be committed with those before it
-    if (f > j) {
-      const long long S0 = static_cast<long long>(s * x_pow2(52 - e));
-      const bool in = lane >= j && lane < f;
-      bool valid;
-      long long K;  // the change of S up to and with this lane's run
-      if ((ties & ((f < 32 ? (1u << f) : 0u) - (1u << j))) == 0) {
-        const long long Kb = before - __shfl_sync(kFull, before, j);
-        K = Kb + T.pre.K[0];
-        valid = x_inside(S0, S0 + Kb + T.pre.mn[0]) && x_inside(S0, S0 + Kb + T.pre.mx[0]);
-      } else {
-        const int p0 = static_cast<int>(S0 & 1);
-        XRun run = in ? T.pre : x_identity();
-        for (int off = 1; off < 32; off <<= 1) {
-          const XRun o = x_shfl_up(run, off);
-          if (lane >= off) run = x_compose(o, run);
-        }
-        XRun ex = x_shfl_up(run, 1);
-        if (lane == 0) ex = x_identity();
-        const long long Kb = p0 ? ex.K[1] : ex.K[0];
-        const bool pb = (p0 ? ex.out[1] : ex.out[0]) != 0;
-        K = p0 ? run.K[1] : run.K[0];
-        valid = x_inside(S0, S0 + Kb + (pb ? T.pre.mn[1] : T.pre.mn[0])) &&
-                x_inside(S0, S0 + Kb + (pb ? T.pre.mx[1] : T.pre.mx[0]));
-      }
-      const unsigned bad = __ballot_sync(kFull, in && !valid);
-      if (bad) f = __ffs(bad) - 1;
-      if (f > j) s = static_cast<double>(S0 + __shfl_sync(kFull, K, f - 1)) * u;
-    }
+    const bool ok = plain && have && (empty || (G.fast.e == e && x_inside(S, S + before - base, G.fast.mn, G.fast.mx)));
+    const unsigned stop = __ballot_sync(kFull, lane >= j && !ok);
+    const int f = stop ? __ffs(stop) - 1 : 32;
+    if (f > j) S += __shfl_sync(kFull, inc, f - 1) - base;
     if (f >= cnt) break;
-    double s2 = s;
-    const int done = lane == f && x_commit(s2, T) ? 1 : 0;
-    s2 = __shfl_sync(kFull, s2, f);
-    s = __shfl_sync(kFull, done, f) ? s2 : other(f, s);
+    // lane f, on its own
+    long long S2 = S;
+    int e2 = e, way = 0;  // 1: committed
+    if (lane == f) {
+      if (G.fast.kind == kXFull && have) way = x_commit(S2, e2, G.full) ? 1 : 0;
+      if (G.fast.kind == kXStart) way = 2, S2 = G.fast.K;
+    }
+    way = __shfl_sync(kFull, way, f);
+    S2 = __shfl_sync(kFull, S2, f);
+    if (way == 1) {
+      S = S2, e = __shfl_sync(kFull, e2, f);
+    } else {
+      s = way == 2 ? __longlong_as_double(S2) : other(f, have ? x_double(S, e) : s);
+      have = x_binade(s, e);
+      S = x_int(s);
+    }
     j = f + 1;
+    base = __shfl_sync(kFull, inc, f);
   }
-  return s;
-}
-__device__ __forceinline__ XTileAgg x_no_summary() {
-  XTileAgg T;
-  T.u = T.u1 = T.at = 0.0;
-  T.pre = T.suf = x_identity();
-  T.split = -1;
-  return T;
+  return have ? x_double(S, e) : s;
 }
 
 // The chain c from its tiles' and groups' summaries (one warp).
-__device__ __forceinline__ double x_walk(const XChain& c, const XTileAgg* ag, const XTileAgg* gg, double* sh) {
+__device__ __forceinline__ double x_walk(const XChain& c, const XFast* tf, const XTileAgg* ag, const XFast* gf,
+                                         const XTileAgg* gg, double* sh) {
   const int lane = threadIdx.x & 31;
   double s = c.init;
   for (int g0 = 0; g0 < c.ngroups; g0 += 32) {
-    const int cntg = c.ngroups - g0 < 32 ? c.ngroups - g0 : 32;
-    const XTileAgg G = lane < cntg ? x_load(gg + c.group0 + g0 + lane) : x_no_summary();
+    const int cntg = c.ngroups - g0 < 32 ? c.ngroups - g0 : 32, gi = c.group0 + g0;
+    const XRound G = x_round(lane < cntg ? x_load(gf + gi + lane) : x_no_fast(), gg + gi + lane, lane < cntg);
     s = x_walk_lanes(s, G, cntg, [&](int g, double sg) {
-      const int t0 = (g0 + g) * kXGroup, cnt = c.ntiles - t0 < kXGroup ? c.ntiles - t0 : kXGroup;
-      const XTileAgg T = lane < cnt ? x_load(ag + c.tile0 + t0 + lane) : x_no_summary();
+      const int t0 = (g0 + g) * kXGroup, cnt = c.ntiles - t0 < kXGroup ? c.ntiles - t0 : kXGroup, ti = c.tile0 + t0;
+      const XRound T = x_round(lane < cnt ? x_load(tf + ti + lane) : x_no_fast(), ag + ti + lane, lane < cnt);
       return x_walk_lanes(sg, T, cnt, [&](int k, double st) {
         long long a, b;
-        x_tile_range(c, c.tile0 + t0 + k, a, b);
+        x_tile_range(c, ti + k, a, b);
         return x_add(c.t, a, b, st, sh);
       });
     });
@@ -594,30 +608,36 @@ __device__ __forceinline__ double x_walk(const XChain& c, const XTileAgg* ag, co
   return s;
 }
 
-// The summary of a group of tiles, lane l holding T of the l-th (valid in lane 0): all tiles in one grid
-// and none that changes binade, or one that does, with the tiles before it in its first grid and those
-// after it in its second. Else u = 0.
-__device__ __forceinline__ XTileAgg x_group(const XTileAgg& T, int cnt) {
+// The summary of a group of tiles (a warp; lane l takes the l-th of cnt), valid in lane 0: all tiles in one
+// grid and none that changes binade, or one that does, with the tiles before it in its first grid and
+// those after it in its second. Else it has none.
+__device__ __forceinline__ XSummary x_group(const XFast* tf, const XTileAgg* ag, int cnt) {
   const int lane = threadIdx.x & 31;
   const bool here = lane < cnt;
-  const unsigned splits = __ballot_sync(kFull, here && T.split >= 0);
+  const XRound R = x_round(here ? x_load(tf + lane) : x_no_fast(), ag + lane, here);
+  XTileAgg T = R.full;
+  if (here && R.fast.kind == kXPlain) {
+    T.e = R.fast.e;
+    T.pre.K[0] = T.pre.K[1] = R.fast.K, T.pre.mn[0] = T.pre.mn[1] = R.fast.mn, T.pre.mx[0] = T.pre.mx[1] = R.fast.mx;
+    T.pre.out[0] = static_cast<int>(R.fast.K & 1), T.pre.out[1] = T.pre.out[0] ^ 1;
+  }
+  const unsigned splits = __ballot_sync(kFull, here && T.split);
   const int k = splits ? __ffs(splits) - 1 : 31;  // the last lane in the first grid
-  XTileAgg G = x_no_summary();
-  const double u0 = __shfl_sync(kFull, T.u, 0), u1 = splits ? __shfl_sync(kFull, T.u1, k) : u0;
-  bool ok = !here || (!T.pre.bad && T.u != 0.0 && T.u == (lane <= k ? u0 : u1));
-  if (lane == k && splits) ok = ok && !T.suf.bad && T.u1 != 0.0;
+  XTileAgg G = x_no_full();
+  const int e0 = __shfl_sync(kFull, T.e, 0), e1 = splits ? __shfl_sync(kFull, T.e1, k) : e0;
+  const bool ok = !here || ((R.fast.kind == kXPlain || R.fast.kind == kXFull) && T.e == (lane <= k ? e0 : e1));
   if (!__all_sync(kFull, ok) || __popc(splits) > 1) {
     G.pre.bad = 1;
-    return G;
+    return x_summary(G);
   }
-  G.u = u0;
+  G.e = e0;
   G.pre = x_warp_ordered(here && lane <= k ? T.pre : x_identity());
   if (splits) {
-    G.u1 = u1, G.split = k;
+    G.e1 = e1, G.split = true;
     G.at = __shfl_sync(kFull, T.at, k);
     G.suf = x_warp_ordered(lane == k ? T.suf : (here && lane > k ? T.pre : x_identity()));
   }
-  return G;
+  return x_summary(G);
 }
 
 // Blocks [0, nblocks): kXWarps tiles of one chain each (block_chain: the chain). The blocks after them:
@@ -627,8 +647,8 @@ __device__ __forceinline__ XTileAgg x_group(const XTileAgg& T, int cnt) {
 static __global__ void __launch_bounds__(32 * kXWarps) k_xwalk(const XChain* __restrict__ ch, const XJob* __restrict__ jobs,
                                                                const int* __restrict__ block_chain, int nblocks,
                                                                const int* __restrict__ short_chain, int nshort,
-                                                               const double* stat, XTileAgg* ag, XTileAgg* gg,
-                                                               unsigned* group_done, unsigned* chain_done,
+                                                               const double* stat, XFast* tf, XTileAgg* ag, XFast* gf,
+                                                               XTileAgg* gg, unsigned* group_done, unsigned* chain_done,
                                                                unsigned* job_done, const int* skip) {
   __shared__ alignas(16) double sh_add[kXWarps][kXTile];
   __shared__ double sh_sum[kXWarps];
@@ -668,18 +688,19 @@ static __global__ void __launch_bounds__(32 * kXWarps) k_xwalk(const XChain* __r
     if (k < c.ntiles) {
       long long a, b;
       x_tile_range(c, c.tile0 + k, a, b);
-      const XTileAgg T = x_tile_agg(c.t, a, b, s0);
-      if (lane == 0) ag[c.tile0 + k] = T;
+      // the first tile's start is known: its terms are added here, while the other tiles are summarised
+      const XSummary T = k == 0 ? x_start(x_add(c.t, a, b, c.init, sh_add[0])) : x_summary(x_tile_full(c.t, a, b, s0));
+      if (lane == 0) x_leave(T, tf + c.tile0 + k, ag + c.tile0 + k);
     }
     __threadfence();
     __syncthreads();
     if (w != 0) return;
     const int g = k0 / kXGroup, t0 = g * kXGroup, cnt = c.ntiles - t0 < kXGroup ? c.ntiles - t0 : kXGroup;
     if (!last_of(group_done + c.group0 + g, (cnt + kXWarps - 1) / kXWarps)) return;
-    const XTileAgg G = x_group(lane < cnt ? x_load(ag + c.tile0 + t0 + lane) : x_no_summary(), cnt);
-    if (lane == 0) gg[c.group0 + g] = G;
+    const XSummary G = x_group(tf + c.tile0 + t0, ag + c.tile0 + t0, cnt);
+    if (lane == 0) x_leave(G, gf + c.group0 + g, gg + c.group0 + g);
     if (!last_of(chain_done + ci, c.ngroups)) return;
-    s = x_walk(c, ag, gg, sh_add[0]);
+    s = x_walk(c, tf, ag, gf, gg, sh_add[0]);
   } else {
     if (ci < 0) return;
     s = x_add(c.t, c.lo, c.hi, c.init, sh_add[w]);
@@ -779,6 +800,8 @@ class SumPlan {
       upload(block_chain, block_chain_, st);
       upload(short_chain, short_chain_, st);
       stat_.alloc(static_cast<std::size_t>(ntiles_ > 0 ? ntiles_ : 1));
+      tile_fast_.alloc(static_cast<std::size_t>(ntiles_ > 0 ? ntiles_ : 1) * sizeof(XFast));
+      group_fast_.alloc(static_cast<std::size_t>(ngroups_ > 0 ? ngroups_ : 1) * sizeof(XFast));
       tile_agg_.alloc(static_cast<std::size_t>(ntiles_ > 0 ? ntiles_ : 1) * sizeof(XTileAgg));
       group_agg_.alloc(static_cast<std::size_t>(ngroups_ > 0 ? ngroups_ : 1) * sizeof(XTileAgg));
       const std::size_t counters = static_cast<std::size_t>(ngroups_) + chains.size() + jobs.size();
@@ -822,7 +845,9 @@ class SumPlan {
         B200_CHECK(cudaLaunchKernelEx(&cfg, k_xwalk, ch, reinterpret_cast<const XJob*>(xjobs_.get()),
                                       reinterpret_cast<const int*>(block_chain_.get()), nblocks_,
                                       reinterpret_cast<const int*>(short_chain_.get()), nshort_,
-                                      static_cast<const double*>(stat_.get()), reinterpret_cast<XTileAgg*>(tile_agg_.get()),
+                                      static_cast<const double*>(stat_.get()), reinterpret_cast<XFast*>(tile_fast_.get()),
+                                      reinterpret_cast<XTileAgg*>(tile_agg_.get()),
+                                      reinterpret_cast<XFast*>(group_fast_.get()),
                                       reinterpret_cast<XTileAgg*>(group_agg_.get()), done, done + ngroups_,
                                       done + ngroups_ + nchains_, skip_));
       }
@@ -858,7 +883,7 @@ class SumPlan {
   bool exact_ = false;
   const int* skip_ = nullptr;
   DevBuf<unsigned char> chains_, xjobs_, tseg_, tile_chain_, block_chain_, short_chain_;
-  mutable DevBuf<unsigned char> tile_agg_, group_agg_;
+  mutable DevBuf<unsigned char> tile_fast_, group_fast_, tile_agg_, group_agg_;
   mutable DevBuf<double> partials_, stat_;
   mutable DevBuf<unsigned> done_;
   int nchains_ = 0, nshort_ = 0, nt_ = 0, ntiles_ = 0, nblocks_ = 0, ngroups_ = 0;

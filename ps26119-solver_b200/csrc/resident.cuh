@@ -248,6 +248,37 @@ struct ResidentSide {
   T *val, *vec;
 };
 
+// Both sides' places in a block's shared memory: columns [c0, c1) of a matrix with row pointers t_rp (of
+// Ãᵀ), rows [r0, r1) of one with a_rp.
+template <class T>
+__device__ __forceinline__ void resident_layout(unsigned char* at, const int* t_rp, int c0, int c1, int col_vecs,
+                                                const int* a_rp, int r0, int r1, int row_vecs, ResidentSide<T>& C,
+                                                ResidentSide<T>& R) {
+  auto take = [&](long long bytes) {
+    unsigned char* r = at;
+    at += (bytes + 7) & ~7LL;
+    return r;
+  };
+  auto side = [&](ResidentSide<T>& S, const int* rp, int from, int to, int vecs) {
+    S.from = from, S.count = to - from, S.stride = S.count;
+    const int nz = __ldg(rp + to) - __ldg(rp + from);
+    S.val = reinterpret_cast<T*>(take(static_cast<long long>(nz) * sizeof(T)));
+    S.vec = reinterpret_cast<T*>(take(static_cast<long long>(vecs) * S.count * sizeof(T)));
+    S.rp = reinterpret_cast<int*>(take((S.count + 1LL) * 4));
+    S.idx = reinterpret_cast<int*>(take(nz * 4LL));
+  };
+  side(C, t_rp, c0, c1, col_vecs);
+  side(R, a_rp, r0, r1, row_vecs);
+}
+// Brings a side's row pointers (rebased), indices and values in.
+template <class T>
+__device__ __forceinline__ void resident_fill(const ResidentSide<T>& S, const int* rp, const int* idx, const T* val) {
+  const int tid = static_cast<int>(threadIdx.x), nt = static_cast<int>(blockDim.x);
+  const int k0 = __ldg(rp + S.from), nz = __ldg(rp + S.from + S.count) - k0;
+  for (int k = tid; k <= S.count; k += nt) S.rp[k] = __ldg(rp + S.from + k) - k0;
+  for (int k = tid; k < nz; k += nt) S.idx[k] = __ldg(idx + k0 + k), S.val[k] = __ldg(val + k0 + k);
+}
+
 // A thread's row: its entries [a, a + len) of the side's arrays, and the first GB of them. (With GB = 4,
 // at 64 registers a thread, the values stay in shared memory until they are used.)
 template <int GB, class T>
@@ -343,38 +374,16 @@ __device__ __forceinline__ void resident_body(const ResidentPart<T, Op>& p, int 
   }
   __syncthreads();
   ResidentSide<T> C, R;
-  {
-    unsigned char* at = resident_smem;
-    auto take = [&](long long bytes) {
-      unsigned char* r = at;
-      at += (bytes + 7) & ~7LL;
-      return r;
-    };
-    auto side = [&](ResidentSide<T>& S, const int* rp, int from, int to, int vecs) {
-      S.from = from, S.count = to - from, S.stride = S.count;
-      const int nz = __ldg(rp + to) - __ldg(rp + from);
-      S.val = reinterpret_cast<T*>(take(static_cast<long long>(nz) * sizeof(T)));
-      S.vec = reinterpret_cast<T*>(take(static_cast<long long>(vecs) * S.count * sizeof(T)));
-      S.rp = reinterpret_cast<int*>(take((S.count + 1LL) * 4));
-      S.idx = reinterpret_cast<int*>(take(nz * 4LL));
-    };
-    side(C, p.t_rp, cut[0], cut[1], Op::kCol);
-    side(R, p.a_rp, cut[2], cut[3], Op::kRow);
-  }
+  resident_layout(resident_smem, p.t_rp, cut[0], cut[1], Op::kCol, p.a_rp, cut[2], cut[3], Op::kRow, C, R);
   const int nt = static_cast<int>(blockDim.x);
-  auto fill = [&](const ResidentSide<T>& S, const int* rp, const int* idx, const T* val) {
-    const int k0 = __ldg(rp + S.from), nz = __ldg(rp + S.from + S.count) - k0;
-    for (int k = tid; k <= S.count; k += nt) S.rp[k] = __ldg(rp + S.from + k) - k0;
-    for (int k = tid; k < nz; k += nt) S.idx[k] = __ldg(idx + k0 + k), S.val[k] = __ldg(val + k0 + k);
-  };
   // y first, and out at once: the columns' first step waits for it
   for (int e = tid; e < R.count; e += nt) {
     const T v = p.op.row_vec(0)[R.from + e];
     R.vec[e] = v;
     cell_store(p.ycell + R.from + e, v, p.tag);
   }
-  fill(C, p.t_rp, p.t_ri, p.t_val);
-  fill(R, p.a_rp, p.a_col, p.a_val);
+  resident_fill(C, p.t_rp, p.t_ri, p.t_val);
+  resident_fill(R, p.a_rp, p.a_col, p.a_val);
   for (int k = 0; k < Op::kCol; ++k)
     for (int e = tid; e < C.count; e += nt) C.vec[k * C.stride + e] = p.op.col_vec(k)[C.from + e];
   for (int k = 1; k < Op::kRow; ++k)
