@@ -123,9 +123,7 @@ __global__ void k_diff(long long n, const T* a, const T* b, T* out) {  // out = 
 
 class Engine {
  public:
-  // grouped: the epochs are launched by a GroupScheduler
-  Engine(const DeviceModel& M, const EngineOptions& o, cudaStream_t st, bool grouped)
-      : M_(M), o_(o), st_(st), grouped_(grouped) {
+  Engine(const DeviceModel& M, const EngineOptions& o, cudaStream_t st) : M_(M), o_(o), st_(st) {
     for (auto& e : ev_) B200_CHECK(cudaEventCreate(&e));
   }
   ~Engine() {
@@ -159,16 +157,19 @@ class Engine {
   EngineResult run_pdlp(const DeviceOutputs& out);
   // run() as steps, for a scheduler that interleaves several engines on one stream:
   // start() once (true: finished already); then per epoch begin_epoch(), the epoch's iteration
-  // kernels (launch_epoch(), or a scheduler's grouped kernels followed by launch_r0()),
+  // kernels (launch_epoch(), or a scheduler's: step kernels with upload_params() before and launch_r0()
+  // after their first step, or a resident launch of resident_part()s, then resident_done()),
   // launch_check(), a synchronisation of the stream, end_epoch() (true: finished). result()
   // holds the outcome once finished.
   bool start(const DeviceOutputs& out);
   void begin_epoch();
+  void upload_params();
   void launch_epoch();
   void launch_r0(cudaStream_t on);
   void launch_check();
   bool end_epoch();
   const EngineResult& result() const { return R_; }
+  bool resident() const { return shape_[mixed_now_ ? 1 : 0].blocks > 0; }
   int check_every() const { return o_.check_every; }
   cudaStream_t stream() const { return st_; }
   bool mixed_now() const { return mixed_now_; }
@@ -184,6 +185,13 @@ class Engine {
   };
   template <class T> SlabOperands primal_operands();
   template <class T> SlabOperands dual_operands();
+  // this engine's part of a resident launch, on `blocks` blocks from block `first`; the bytes it takes
+  // there when `blocks` blocks share it (blocks = 1: all of it)
+  template <class T> ResidentPart<T, ResidentR2h<T>> resident_part(int first, int blocks);
+  long long resident_size(int blocks) const;
+  int num_cols() const { return M_.n; }
+  int num_rows() const { return M_.m; }
+  void resident_done();
   // Bulk-copy waits of this solve's kernels that ran out (synchronises the stream).
   unsigned stage_errors() {
     unsigned v = 0;
@@ -214,12 +222,11 @@ class Engine {
   template <class T> IterVecs<T>& vecs();
   template <class T> void capture_epoch();
   template <class T> void capture_check(int variant);
-  template <class T> void launch_first_residual(const int* skip);
+  template <class T> void launch_first_residual(const int* skip, bool apart);
   template <class T, int kRays> void launch_check_kernels();
-  template <class T> void plan_resident(int max_row, int max_col);
+  template <class T> void plan_resident();
   template <class T> void launch_resident_epoch();
   template <class T> void launch_resident_pdlp(int cur);
-  bool resident() const { return shape_[mixed_now_ ? 1 : 0].blocks > 0; }
   template <class T> void launch_kkt_scaled(const T* xs, const T* ys);
   void launch_kkt_original();
   void make_side_stream();
@@ -255,7 +262,7 @@ class Engine {
   DeviceModel M_;
   const EngineOptions& o_;
   cudaStream_t st_;
-  bool grouped_;
+  int max_row_ = 0, max_col_ = 0;  // the most nonzeros of a row, of a column
   ResidentShape shape_[2];  // resident epochs in fp64 / fp32 (blocks = 0: the step kernels)
   unsigned tag_ = 1;        // the next resident epoch's first tag
   DevBuf<unsigned> stage_err_;  // this solve's bulk-copy timeouts (see count_stage_timeout)
@@ -341,9 +348,10 @@ void Engine::setup() {
   cap_t_ = fed_tile_capacity(ext[2]);
   vd_.alloc(n, m);
   if (o_.mixed) vf_.alloc(n, m);
-  if (!grouped_ && tune_forced() < 0) {  // a forced step-kernel variant runs the step kernels
-    plan_resident<double>(ext[1], ext[3]);
-    if (o_.mixed) plan_resident<float>(ext[1], ext[3]);
+  max_row_ = ext[1], max_col_ = ext[3];
+  if (tune_forced() < 0) {  // a forced step-kernel variant runs the step kernels
+    plan_resident<double>();
+    if (o_.mixed) plan_resident<float>();
   }
   params_.alloc(1);
   hparams_.alloc(1);
@@ -499,20 +507,21 @@ void Engine::build_plans() {
 }
 
 // The residual of a Halpern cycle's first step: dx = x̄ − x̂, adx = Ã dx, dy = ȳ − ŷ and the terms of its
-// three dots. skip: see SumPlan; resident epochs have left the points of that step in buffers of their own.
+// three dots. skip: see SumPlan. apart: a resident epoch has left the points of that step in buffers of their
+// own.
 template <class T>
-void Engine::launch_first_residual(const int* skip) {
+void Engine::launch_first_residual(const int* skip, bool apart) {
   IterVecs<T>& v = vecs<T>();
   const int m = M_.m, n = M_.n;
   double* px = rt_.get();
   double* py = px + 2 * n;
-  const bool f = v.xh0.get() != nullptr;
+  const bool f = apart;
   k_res_x<T><<<grid_for(n), kBlock, 0, st_>>>(n, (f ? v.xb0 : v.xb).get(), (f ? v.xh0 : v.xh).get(), v.dx.get(), px,
                                               skip);
   B200_LAUNCH_CHECK();
   EpiResY<T> e{(f ? v.yb0 : v.yb).get(), (f ? v.yh0 : v.yh).get(), py, py + m, skip};
   launch_slab_tma<T>(m, sp_.a_rp.get(), sp_.a_col.get(), sp_.A_val<T>(), v.dx.get(), e, st_, nullptr, err());
-  plan_r0_.launch(st_);
+  plan_r0_.launch(st_, false, skip != nullptr);
   B200_COUNT(2 + plan_r0_.kernel_count());
 }
 
@@ -662,7 +671,7 @@ void Engine::capture_epoch() {
   B200_CHECK(cudaEventRecordWithFlags(ev_[0], st_, cudaEventRecordExternal));
   step(0);
   B200_CHECK(cudaEventRecordWithFlags(ev_[1], st_, cudaEventRecordExternal));
-  launch_first_residual<T>(r0_skip);  // r⁰ after the first step of a Halpern cycle
+  launch_first_residual<T>(r0_skip, false);  // r⁰ after the first step of a Halpern cycle
   B200_CHECK(cudaEventRecordWithFlags(ev_[2], st_, cudaEventRecordExternal));
   for (int s = 1; s < K; ++s) step(s);
   B200_CHECK(cudaEventRecordWithFlags(ev_[3], st_, cudaEventRecordExternal));
@@ -1017,7 +1026,8 @@ bool Engine::start(const DeviceOutputs& out) {
   return false;
 }
 
-// The step scalars of the next epoch: τ = η/ω, σ = ηω (r2hpdhg.cpp:67), the Halpern counter.
+// The step scalars of the next epoch: τ = η/ω, σ = ηω (r2hpdhg.cpp:67), the Halpern counter. The step
+// kernels read them from the device (upload_params), a resident epoch gets them with its launch.
 void Engine::begin_epoch() {
   StepParams& hp = *hparams_.get();
   hp.tau = eta_ / L_.omega;
@@ -1027,35 +1037,50 @@ void Engine::begin_epoch() {
   hp.K = o_.check_every;
   hp.done = 0;
   hp.skip_r0 = L_.inner != 0 ? 1 : 0;
-  B200_CHECK(cudaMemcpyAsync(params_.get(), &hp, sizeof(StepParams), cudaMemcpyHostToDevice, st_));
   L_.fresh = L_.inner == 0;
+}
+void Engine::upload_params() {
+  B200_CHECK(cudaMemcpyAsync(params_.get(), hparams_.get(), sizeof(StepParams), cudaMemcpyHostToDevice, st_));
 }
 
 // Whether this solve's epochs are resident in precision T, and their buffers: the rule is that the
 // matrix and the updates' vectors fit the SMs' shared memory (resident_shape).
 template <class T>
-void Engine::plan_resident(int max_row, int max_col) {
+void Engine::plan_resident() {
   ResidentShape& s = shape_[std::is_same<T, float>::value ? 1 : 0];
-  s = resident_shape<T, ResidentR2h<T>>(M_.m, M_.n, M_.nnz, max_row, max_col);
+  s = resident_shape<T, ResidentR2h<T>>(M_.m, M_.n, M_.nnz, max_row_, max_col_);
   if (s.blocks > 0) vecs<T>().alloc_resident(M_.n, M_.m, st_);
+}
+long long Engine::resident_size(int blocks) const {
+  return mixed_now_ ? resident_bytes<float, ResidentR2h<float>>(M_.m, M_.n, M_.nnz, max_row_, max_col_, blocks)
+                    : resident_bytes<double, ResidentR2h<double>>(M_.m, M_.n, M_.nnz, max_row_, max_col_, blocks);
+}
+template <class T>
+ResidentPart<T, ResidentR2h<T>> Engine::resident_part(int first, int blocks) {
+  IterVecs<T>& v = vecs<T>();
+  const StepParams& hp = *hparams_.get();
+  return {M_.m, M_.n, first, blocks, sp_.t_rp.get(), sp_.t_ri.get(), sp_.a_rp.get(), sp_.a_col.get(), sp_.At_val<T>(),
+          sp_.A_val<T>(), v.xcell.get(), v.ycell.get(), tag_, err(),
+          {v.x.get(), v.xh.get(), v.xb.get(), v.y.get(), v.yh.get(), v.yb.get(), v.x0.get(), sp_.c<T>(), sp_.l<T>(),
+           sp_.u<T>(), v.y0.get(), sp_.rl<T>(), sp_.ru<T>(), v.xh0.get(), v.xb0.get(), v.yh0.get(), v.yb0.get(), hp.tau,
+           hp.sigma, hp.rho, hp.inner0, hp.K}};
+}
+// After a resident launch of this engine's epoch, on its own stream: the r⁰ of a new Halpern cycle.
+void Engine::resident_done() {
+  tag_ += static_cast<unsigned>(o_.check_every) + 1;
+  ++kernels_;
+  if (!L_.fresh) return;
+  if (mixed_now_) launch_first_residual<float>(nullptr, true);
+  else launch_first_residual<double>(nullptr, true);
 }
 
 template <class T>
 void Engine::launch_resident_epoch() {
-  IterVecs<T>& v = vecs<T>();
-  const StepParams& hp = *hparams_.get();
-  ResidentPart<T, ResidentR2h<T>> p{
-      M_.m, M_.n, 0, shape_[std::is_same<T, float>::value ? 1 : 0].blocks, sp_.t_rp.get(), sp_.t_ri.get(), sp_.a_rp.get(),
-      sp_.a_col.get(), sp_.At_val<T>(), sp_.A_val<T>(), v.xcell.get(), v.ycell.get(), tag_, err(),
-      {v.x.get(), v.xh.get(), v.xb.get(), v.y.get(), v.yh.get(), v.yb.get(), v.x0.get(), sp_.c<T>(), sp_.l<T>(), sp_.u<T>(),
-       v.y0.get(), sp_.rl<T>(), sp_.ru<T>(), v.xh0.get(), v.xb0.get(), v.yh0.get(), v.yb0.get(), hp.tau, hp.sigma, hp.rho,
-       hp.inner0, hp.K}};
+  const ResidentShape& s = shape_[std::is_same<T, float>::value ? 1 : 0];
   B200_CHECK(cudaEventRecord(ev_[0], st_));
-  launch_resident(p, shape_[std::is_same<T, float>::value ? 1 : 0], st_);
+  launch_resident(resident_part<T>(0, s.blocks), s, st_);
   B200_CHECK(cudaEventRecord(ev_[1], st_));
-  tag_ += static_cast<unsigned>(hp.K) + 1;
-  ++kernels_;
-  if (L_.fresh) launch_first_residual<T>(nullptr);
+  resident_done();
 }
 
 template <class T>
@@ -1085,6 +1110,7 @@ void Engine::launch_epoch() {
     else launch_resident_epoch<double>();
     return;
   }
+  upload_params();
   if (mixed_now_) capture_epoch<float>();
   else capture_epoch<double>();
   B200_CHECK(cudaGraphLaunch(g_epoch_[pidx], st_));
@@ -1097,8 +1123,8 @@ void Engine::launch_r0(cudaStream_t on) {
   if (!L_.fresh) return;
   const cudaStream_t own = st_;
   st_ = on;  // launched on the group's stream, between the group's step 0 and step 1
-  if (mixed_now_) launch_first_residual<float>(nullptr);
-  else launch_first_residual<double>(nullptr);
+  if (mixed_now_) launch_first_residual<float>(nullptr, false);
+  else launch_first_residual<double>(nullptr, false);
   st_ = own;
 }
 
@@ -1554,9 +1580,15 @@ class GroupScheduler {
   // A device has PS26119_GROUPS_PER_DEVICE groups (default 2), each with its own host thread
   // and stream, so that one group's host decisions between epochs overlap another group's
   // kernels; a solve joins the group with the fewest solves.
+  struct Registry {
+    std::mutex mu;
+    std::map<int, std::vector<GroupScheduler*>> all;
+  };
+  static Registry& registry() {
+    static Registry* r = new Registry();  // never destroyed: the threads live until exit
+    return *r;
+  }
   static GroupScheduler& for_current_device() {
-    static std::mutex mu;
-    static std::map<int, std::vector<GroupScheduler*>> all;  // never destroyed: the threads live until exit
     static const int per_device = [] {
       const char* e = std::getenv("PS26119_GROUPS_PER_DEVICE");
       const int k = e && *e ? std::atoi(e) : 2;
@@ -1564,8 +1596,8 @@ class GroupScheduler {
     }();
     int dev = 0;
     B200_CHECK(cudaGetDevice(&dev));
-    std::lock_guard<std::mutex> lk(mu);
-    std::vector<GroupScheduler*>& v = all[dev];
+    std::lock_guard<std::mutex> lk(registry().mu);
+    std::vector<GroupScheduler*>& v = registry().all[dev];
     while (static_cast<int>(v.size()) < per_device) v.push_back(new GroupScheduler(dev));
     GroupScheduler* best = v.front();
     for (GroupScheduler* g : v)
@@ -1644,14 +1676,77 @@ class GroupScheduler {
     cfg.numAttrs = (B200_PDL && pdl) ? 1 : 0;
     B200_CHECK(cudaLaunchKernelEx(&cfg, k_group_fed<T, Epi>, parts.get(), nparts, step));
   }
-  // One epoch of every active solve: each solve's step scalars on its own stream; the grouped
-  // iteration kernels on the group's stream once every solve's stream is ready; each solve's
-  // residual section (when its epoch starts a Halpern cycle) on the group's stream after step 0;
-  // then every solve's check graph on its own stream, so the checks of different solves overlap.
+  // One epoch of every active solve as one resident launch (resident.cuh), the device's SMs dealt out to
+  // the groups that have work, and a group's to its solves by their bytes; false (nothing launched) when
+  // they do not fit that way. Against the step kernels, 16 random LPs of 1k to 18k rows in two groups:
+  // 19 us an iteration, checks included, against 27.
+  bool resident_epoch(std::vector<Job*>& active) {
+    int busy = 0;
+    for (GroupScheduler* g : peers_()) busy += g->load_.load() > 0 ? 1 : 0;
+    const int cap = sm_count() / std::max(1, busy), jobs = static_cast<int>(active.size());
+    if (jobs > cap) return false;
+    double total = 0.0;
+    long long elements = 0;
+    for (Job* j : active) {
+      if (!j->e->resident()) return false;
+      total += static_cast<double>(j->e->resident_size(1));
+      elements += static_cast<long long>(j->e->num_rows()) + j->e->num_cols();
+    }
+    if (elements / cap > kResidentElements) return false;
+    // an even share of the bytes each, rounded down and at least one block
+    std::vector<int> blocks(active.size());
+    int used = 0, threads = 64;
+    long long smem = 0;
+    for (std::size_t k = 0; k < active.size(); ++k) {
+      const double share = static_cast<double>(active[k]->e->resident_size(1)) / total;
+      const Engine& e = *active[k]->e;
+      blocks[k] = std::max(1, std::min<int>(static_cast<int>(share * cap), (e.num_rows() + e.num_cols() + 7) / 8));
+      used += blocks[k];
+    }
+    while (used > cap) --*std::max_element(blocks.begin(), blocks.end()), --used;
+    for (std::size_t k = 0; k < active.size(); ++k) {
+      const Engine& e = *active[k]->e;
+      smem = std::max(smem, e.resident_size(blocks[k]));
+      threads = std::max(threads, resident_threads(e.num_rows(), e.num_cols(), blocks[k]));
+    }
+    if (smem > static_cast<long long>(kResidentSmem)) return false;
+    rd_.h.clear(), rf_.h.clear();
+    int first_d = 0, first_f = 0;
+    for (std::size_t k = 0; k < active.size(); ++k) {
+      Engine& e = *active[k]->e;
+      if (e.mixed_now()) rf_.h.push_back(e.resident_part<float>(first_f, blocks[k])), first_f += blocks[k];
+      else rd_.h.push_back(e.resident_part<double>(first_d, blocks[k])), first_d += blocks[k];
+    }
+    rd_.upload(st_), rf_.upload(st_);
+    launch_resident_group<ResidentR2h>(rd_.d.get(), static_cast<int>(rd_.h.size()), first_d, rf_.d.get(),
+                                       static_cast<int>(rf_.h.size()), first_d + first_f, threads,
+                                       static_cast<unsigned>(smem), st_);
+    return true;
+  }
+  // One epoch of every active solve: the resident launch, or the grouped step kernels, on the group's stream
+  // once every solve's stream is ready; each solve's residual section (when its epoch starts a Halpern
+  // cycle) after it on its own stream, or on the group's stream after step 0; then every solve's check
+  // graph on its own stream, so the checks of different solves overlap.
   void epoch(std::vector<Job*>& active) {
-    tf_.clear(), td_.clear();
     for (Job* j : active) {
       j->e->begin_epoch();
+      if (!j->ready) B200_CHECK(cudaEventCreateWithFlags(&j->ready, cudaEventDisableTiming));
+      B200_CHECK(cudaEventRecord(j->ready, j->e->stream()));
+      B200_CHECK(cudaStreamWaitEvent(st_, j->ready, 0));
+    }
+    if (resident_epoch(active)) {
+      B200_CHECK(cudaEventRecord(steps_done_, st_));
+      for (Job* j : active) {
+        B200_CHECK(cudaStreamWaitEvent(j->e->stream(), steps_done_, 0));
+        j->e->resident_done();
+        j->e->launch_check();
+      }
+      for (Job* j : active) B200_CHECK(cudaStreamSynchronize(j->e->stream()));
+      return;
+    }
+    tf_.clear(), td_.clear();
+    for (Job* j : active) {
+      j->e->upload_params();
       if (!j->ready) B200_CHECK(cudaEventCreateWithFlags(&j->ready, cudaEventDisableTiming));
       B200_CHECK(cudaEventRecord(j->ready, j->e->stream()));
       B200_CHECK(cudaStreamWaitEvent(st_, j->ready, 0));
@@ -1716,7 +1811,20 @@ class GroupScheduler {
       }
     }
   }
+  template <class T>
+  struct Parts {  // a resident launch's parts in one working precision (pinned and device)
+    std::vector<ResidentPart<T, ResidentR2h<T>>> h;
+    PinnedBuf<ResidentPart<T, ResidentR2h<T>>> p;
+    DevBuf<ResidentPart<T, ResidentR2h<T>>> d;
+    void upload(cudaStream_t st) {
+      if (h.empty()) return;
+      if (p.size() < h.size()) p.alloc(2 * h.size()), d.alloc(2 * h.size());
+      std::copy(h.begin(), h.end(), p.get());
+      B200_CHECK(cudaMemcpyAsync(d.get(), p.get(), h.size() * sizeof(h[0]), cudaMemcpyHostToDevice, st));
+    }
+  };
   int dev_ = 0;
+  std::vector<GroupScheduler*> peers_() const;  // the device's groups
   std::atomic<int> load_{0};  // solves joined and not yet finished
   cudaStream_t st_ = nullptr;
   cudaEvent_t steps_done_ = nullptr;
@@ -1726,7 +1834,14 @@ class GroupScheduler {
   std::vector<Job*> pending_;
   Tables<double> td_;
   Tables<float> tf_;
+  Parts<double> rd_;
+  Parts<float> rf_;
 };
+
+std::vector<GroupScheduler*> GroupScheduler::peers_() const {
+  std::lock_guard<std::mutex> lk(registry().mu);
+  return registry().all[dev_];
+}
 
 }  // namespace
 
@@ -1765,7 +1880,7 @@ EngineResult run_engine(const DeviceModel& M, const EngineOptions& opt, const De
       return e && *e ? std::atoll(e) : 100000LL;
     }();
     const bool grouped = t_grouped && !opt.pdlp && opt.check_every == 64 && M.nnz <= group_max_nnz;
-    auto e = std::make_unique<Engine>(M, opt, st, grouped);
+    auto e = std::make_unique<Engine>(M, opt, st);
     if (grouped) {
       // setup here, on this caller's stream; the epochs in the device's group
       if (e->start(out)) {

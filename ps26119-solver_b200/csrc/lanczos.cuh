@@ -217,8 +217,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_resident_lanczos(const __grid_c
 // staircase T = 720 (43,200) 21.1 against 21.7; of 60k rows (90,000) 6.5 against 5.2, of T = 1200 (72,000)
 // 27.3 against 22.3.
 constexpr long long kLanczosColumns = 61440;
-// The launch of such a kernel: as few blocks as hold the LP with about 224 columns each, because every
-// block is a summary in the sums and a party to their three exchanges; blocks = 0: it does not fit.
+// Columns a block: few blocks leave SMs to other solves, many make a longer walk and wider exchanges.
+// Setup of 30k random rows with 120 / 224 / 448 / 896 columns a block 4.0 / 4.4 / 3.8 / 4.6 ms, staircase
+// T = 720 19.7 / 20.4 / 18.6 / 24.3; 16 requests' setups side by side 41 / 33 / 30 / 29.
+constexpr long long kLanczosShare = 448;
+// The launch of such a kernel: as few blocks as hold the LP with about kLanczosShare columns each, because
+// every block is a summary in the sums and a party to their three exchanges; blocks = 0: it does not fit.
 struct LanczosShape {
   int blocks = 0, threads = 0;
   unsigned smem = 0;
@@ -228,7 +232,7 @@ inline LanczosShape lanczos_shape(long long m, long long n, long long nnz, long 
   LanczosShape s;
   if (m < 1 || n < 1 || nnz < 1 || n > kLanczosColumns) return s;
   const int sms = sm_count();
-  int blocks = static_cast<int>(std::max(1LL, std::min<long long>(sms, (n + 223) / 224)));
+  int blocks = static_cast<int>(std::max(1LL, std::min<long long>(sms, (n + kLanczosShare - 1) / kLanczosShare)));
   auto bytes = [&](int b) { return resident_bytes<double, LanczosOp>(m, n, nnz, max_row, max_col, b); };
   while (blocks < sms && bytes(blocks) > kResidentSmem / 2) ++blocks;
   if (bytes(blocks) > kResidentSmem - sizeof(LanczosShared) || (m + n) / blocks > kResidentElements) return s;

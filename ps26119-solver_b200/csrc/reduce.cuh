@@ -821,12 +821,14 @@ class SumPlan {
   // The tile sums a producer may leave itself (x_leave_stat) before launch(st, true): of the plan's
   // only chain, starting at its first term. Null when the chain needs none.
   double* stat() { return exact_ && ntiles_ > 0 ? stat_.get() : nullptr; }
-  void launch(cudaStream_t st, bool have_stat = false) const {
+  // skippable: whether the plan's skip flag counts in this launch.
+  void launch(cudaStream_t st, bool have_stat = false, bool skippable = true) const {
+    const int* skip = skippable ? skip_ : nullptr;
     if (exact_) {
       const XChain* ch = reinterpret_cast<const XChain*>(chains_.get());
       if (ntiles_ > 0 && !have_stat) {
         k_xstat<<<(ntiles_ + 7) / 8, 256, 0, st>>>(ch, reinterpret_cast<const int*>(tile_chain_.get()), ntiles_,
-                                                   stat_.get(), skip_);
+                                                   stat_.get(), skip);
         B200_LAUNCH_CHECK();
       }
       const int blocks = nblocks_ + (nshort_ + kXWarps - 1) / kXWarps;
@@ -849,11 +851,11 @@ class SumPlan {
                                       reinterpret_cast<XTileAgg*>(tile_agg_.get()),
                                       reinterpret_cast<XFast*>(group_fast_.get()),
                                       reinterpret_cast<XTileAgg*>(group_agg_.get()), done, done + ngroups_,
-                                      done + ngroups_ + nchains_, skip_));
+                                      done + ngroups_ + nchains_, skip));
       }
     } else if (nt_ > 0) {
       k_tree<<<nt_ * kTreeBlocks, kBlock, 0, st>>>(reinterpret_cast<const TreeSeg*>(tseg_.get()), partials_.get(),
-                                                   done_.get(), skip_);
+                                                   done_.get(), skip);
       B200_LAUNCH_CHECK();
     }
   }

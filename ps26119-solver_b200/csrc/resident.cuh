@@ -77,6 +77,15 @@ __device__ __forceinline__ void cell_store(Cell<T>* p, T v, unsigned tag) {
     asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(t | __float_as_uint(v)) : "memory");
 }
 
+// The lines of the rule, and what lies on both sides (fp64 / mixed, us per iteration, resident against the
+// step kernels): random LPs of 10k rows 3.0 / 3.1 against 6.6 / 6.7, 30k 4.2 / 3.9 against 10.8 / 11.3,
+// 100k 9.8 / 9.0 against 12.9 / 14.1. Past 194 KB a block the next carveout leaves the gathers too little
+// L1: 112k rows (186 KB) 12.0 against 12.7, 121k (201 KB) 20.9 against 12.7. Past 2,560 columns and rows a
+// block the polls crowd out the stores: mixed 150k rows (2,534) 13.6 against 14.1, 180k (3,040) 18.0
+// against 16.9; the staircase T = 3600 (2,651) 6.7 against 9.1.
+constexpr unsigned kResidentSmem = 194u * 1024u;
+constexpr long long kResidentElements = 2688;
+
 constexpr int kResidentPolls = 1 << 20;  // reads of one cell before a wait gives up (about half a second)
 
 // r²HPDHG's updates (EpiPrimal / EpiDual). The vectors named by col_vec / row_vec are held in shared
@@ -448,21 +457,51 @@ __global__ void __launch_bounds__(kThreads, 1) k_resident(const __grid_constant_
   resident_body<GB>(p, static_cast<int>(blockIdx.x));
 }
 
+// Several LPs in one launch (the request loop): blocks [0, blocks_d) are the fp64 LPs', the ones after them
+// the fp32 LPs' (whose `first` counts from there). A block copies its LP's part to shared memory.
+template <int kThreads, int GB, template <class> class Op>
+__global__ void __launch_bounds__(kThreads, 1) k_resident_group(const ResidentPart<double, Op<double>>* __restrict__ pd, int nd,
+                                                                int blocks_d, const ResidentPart<float, Op<float>>* __restrict__ pf,
+                                                                int nf) {
+  auto run = [](const auto* parts, int n, int b) {
+    using Part = std::decay_t<decltype(*parts)>;
+    __shared__ alignas(16) unsigned char held[sizeof(Part)];
+    int k = 0;
+    while (k + 1 < n && __ldg(&parts[k + 1].first) <= b) ++k;
+    for (unsigned q = threadIdx.x; q < sizeof(Part) / 4; q += blockDim.x)
+      reinterpret_cast<unsigned*>(held)[q] = __ldg(reinterpret_cast<const unsigned*>(parts + k) + q);
+    __syncthreads();
+    const Part& p = *reinterpret_cast<const Part*>(held);
+    resident_body<GB>(p, b - p.first);
+  };
+  const int b = static_cast<int>(blockIdx.x);
+  if (b < blocks_d) run(pd, nd, b);
+  else run(pf, nf, b - blocks_d);
+}
+template <template <class> class Op>
+inline void launch_resident_group(const ResidentPart<double, Op<double>>* pd, int nd, int blocks_d,
+                                  const ResidentPart<float, Op<float>>* pf, int nf, int blocks, int threads, unsigned smem,
+                                  cudaStream_t st) {
+  const void* f = threads <= 256   ? reinterpret_cast<const void*>(&k_resident_group<256, 16, Op>)
+                  : threads <= 512 ? reinterpret_cast<const void*>(&k_resident_group<512, 8, Op>)
+                                   : reinterpret_cast<const void*>(&k_resident_group<1024, 4, Op>);
+  B200_CHECK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kResidentSmem)));
+  void* args[] = {&pd, &nd, &blocks_d, &pf, &nf};
+  B200_CHECK(cudaLaunchCooperativeKernel(f, dim3(static_cast<unsigned>(blocks)), dim3(static_cast<unsigned>(threads)), args, smem,
+                                         st));
+}
+
 // How one LP's epochs are launched: blocks, threads and dynamic shared memory; blocks = 0: not this way.
 struct ResidentShape {
   int blocks = 0, threads = 0;
   unsigned smem = 0;
 };
-// The lines of the rule, and what lies on both sides (fp64 / mixed, us per iteration, resident against the
-// step kernels): random LPs of 10k rows 3.0 / 3.1 against 6.6 / 6.7, 30k 4.2 / 3.9 against 10.8 / 11.3,
-// 100k 9.8 / 9.0 against 12.9 / 14.1. Past 194 KB a block the next carveout leaves the gathers too little
-// L1: 112k rows (186 KB) 12.0 against 12.7, 121k (201 KB) 20.9 against 12.7. Past 2,560 columns and rows a
-// block the polls crowd out the stores: mixed 150k rows (2,534) 13.6 against 14.1, 180k (3,040) 18.0
-// against 16.9; the staircase T = 3600 (2,651) 6.7 against 9.1.
-constexpr unsigned kResidentSmem = 194u * 1024u;
-constexpr long long kResidentElements = 2688;
-// One block on each SM (fewer for tiny LPs: at least 8 elements a block), threads for one column or row
-// each as far as 1,024 go.
+// Threads for one column or row each, and a warp for uneven shares, as far as 1,024 go.
+inline int resident_threads(long long m, long long n, int blocks) {
+  const long long warps = (n / blocks + 32) / 32 + (m / blocks + 32) / 32 + 1;
+  return static_cast<int>(32 * std::min(32LL, std::max(2LL, warps)));
+}
+// One block on each SM (fewer for tiny LPs: at least 8 elements a block).
 template <class T, class Op>
 inline ResidentShape resident_shape(long long m, long long n, long long nnz, long long max_row, long long max_col) {
   ResidentShape s;
@@ -470,9 +509,8 @@ inline ResidentShape resident_shape(long long m, long long n, long long nnz, lon
   const int blocks = static_cast<int>(std::max(1LL, std::min<long long>(sm_count(), (m + n + 7) / 8)));
   const long long bytes = resident_bytes<T, Op>(m, n, nnz, max_row, max_col, blocks);
   if (bytes > kResidentSmem || (m + n) / blocks > kResidentElements) return s;
-  const long long warps = (n / blocks + 32) / 32 + (m / blocks + 32) / 32 + 1;
   s.blocks = blocks;
-  s.threads = static_cast<int>(32 * std::min(32LL, std::max(2LL, warps)));
+  s.threads = resident_threads(m, n, blocks);
   s.smem = static_cast<unsigned>(bytes);
   return s;
 }
