@@ -48,6 +48,18 @@ class GpuBackendImpl final : public GpuBackend {
     sp_.make_f32(st_);
     xo_.alloc(n_), yo_.alloc(m_), terms_.alloc(4 * (static_cast<std::size_t>(m_) + n_)), res_.alloc(kNumSlots);
     out_.alloc(4);
+    // the operations' sums, over the term arrays that they share
+    const long long L = static_cast<long long>(m_) + n_;
+    double *K0 = terms_.get(), *R = res_.get();
+    plan_kkt_.add(K0, 0, m_, 0.0, SumOrder::kSeq, R + kRp2);
+    plan_kkt_.add(K0 + L, 0, L, 0.0, SumOrder::kSeq, R + kD);
+    plan_kkt_.add(K0 + 2 * L, 0, L, 0.0, SumOrder::kSeq, R + kRd2);
+    plan_kkt_.add(K0 + 3 * L, m_, L, 0.0, SumOrder::kSeq, R + kP);
+    plan_kkt_.build(exact_, nullptr, st_);
+    plan_n_.add(K0, 0, n_, 0.0, SumOrder::kChunk64, out_.get());
+    plan_n_.build(exact_, nullptr, st_);
+    plan_m_.add(K0, 0, m_, 0.0, SumOrder::kChunk64, out_.get());
+    plan_m_.build(exact_, nullptr, st_);
     B200_CHECK(cudaStreamSynchronize(st_));
   }
   ~GpuBackendImpl() override { cudaStreamDestroy(st_); }
@@ -114,12 +126,12 @@ class GpuBackendImpl final : public GpuBackend {
     B200_LAUNCH_CHECK();
   }
   void spmv(int x, int out) override {
-    if (mixed_) launch_slab_tma<float>(m_, sp_.a_rp.get(), sp_.a_col.get(), sp_.saf.get(), f_[x].get(), EpiStore<float>{{}, f_[out].get()}, st_);
-    else launch_slab_tma<double>(m_, sp_.a_rp.get(), sp_.a_col.get(), sp_.sa.get(), d_[x].get(), EpiStore<double>{{}, d_[out].get()}, st_);
+    if (mixed_) launch_slab_tma<float>(m_, sp_.a_rp.get(), sp_.a_col.get(), sp_.saf.get(), f_[x].get(), EpiStore<float>{{}, f_[out].get()}, st_, nullptr, nullptr, true);
+    else launch_slab_tma<double>(m_, sp_.a_rp.get(), sp_.a_col.get(), sp_.sa.get(), d_[x].get(), EpiStore<double>{{}, d_[out].get()}, st_, nullptr, nullptr, true);
   }
   void spmv_t(int y, int out) override {
-    if (mixed_) launch_slab_tma<float>(n_, cs_.get(), sp_.t_ri.get(), sp_.satf.get(), f_[y].get(), EpiStore<float>{{}, f_[out].get()}, st_);
-    else launch_slab_tma<double>(n_, cs_.get(), sp_.t_ri.get(), sp_.sat.get(), d_[y].get(), EpiStore<double>{{}, d_[out].get()}, st_);
+    if (mixed_) launch_slab_tma<float>(n_, cs_.get(), sp_.t_ri.get(), sp_.satf.get(), f_[y].get(), EpiStore<float>{{}, f_[out].get()}, st_, nullptr, nullptr, true);
+    else launch_slab_tma<double>(n_, cs_.get(), sp_.t_ri.get(), sp_.sat.get(), d_[y].get(), EpiStore<double>{{}, d_[out].get()}, st_, nullptr, nullptr, true);
   }
   double dot(int a, int b) override { return pair_sum(a, b, false); }
   double norm2(int a) override { return std::sqrt(pair_sum(a, a, false)); }
@@ -157,12 +169,12 @@ class GpuBackendImpl final : public GpuBackend {
     B200_LAUNCH_CHECK();
   }
   void fused_primal(int y, int x, int x0, double tau, double w, double rho, int xh, int xb) override {
-    if (mixed_) launch_slab_tma<float>(n_, cs_.get(), sp_.t_ri.get(), sp_.satf.get(), f_[y].get(), epi_primal<float>(x, x0, tau, w, rho, xh, xb), st_);
-    else launch_slab_tma<double>(n_, cs_.get(), sp_.t_ri.get(), sp_.sat.get(), d_[y].get(), epi_primal<double>(x, x0, tau, w, rho, xh, xb), st_);
+    if (mixed_) launch_slab_tma<float>(n_, cs_.get(), sp_.t_ri.get(), sp_.satf.get(), f_[y].get(), epi_primal<float>(x, x0, tau, w, rho, xh, xb), st_, nullptr, nullptr, true);
+    else launch_slab_tma<double>(n_, cs_.get(), sp_.t_ri.get(), sp_.sat.get(), d_[y].get(), epi_primal<double>(x, x0, tau, w, rho, xh, xb), st_, nullptr, nullptr, true);
   }
   void fused_dual(int xb, int y, int y0, double sigma, double w, double rho, int yh, int yb) override {
-    if (mixed_) launch_slab_tma<float>(m_, sp_.a_rp.get(), sp_.a_col.get(), sp_.saf.get(), f_[xb].get(), epi_dual<float>(y, y0, sigma, w, rho, yh, yb), st_);
-    else launch_slab_tma<double>(m_, sp_.a_rp.get(), sp_.a_col.get(), sp_.sa.get(), d_[xb].get(), epi_dual<double>(y, y0, sigma, w, rho, yh, yb), st_);
+    if (mixed_) launch_slab_tma<float>(m_, sp_.a_rp.get(), sp_.a_col.get(), sp_.saf.get(), f_[xb].get(), epi_dual<float>(y, y0, sigma, w, rho, yh, yb), st_, nullptr, nullptr, true);
+    else launch_slab_tma<double>(m_, sp_.a_rp.get(), sp_.a_col.get(), sp_.sa.get(), d_[xb].get(), epi_dual<double>(y, y0, sigma, w, rho, yh, yb), st_, nullptr, nullptr, true);
   }
 
   // Backend::kkt (cpu_backend.cpp:269-276 + 226-284) on the device.
@@ -183,14 +195,7 @@ class GpuBackendImpl final : public GpuBackend {
     launch_slab_tma<double>(m_, sp_.a_rp.get(), sp_.a_col.get(), sp_.a_v0.get(), xo_.get(), er, st_);
     EpiKktCols ec{{}, xo_.get(), M_.c, M_.col_lower, M_.col_upper, static_cast<double>(M_.sense), m_, K0 + 3 * L, K0 + L, K0 + 2 * L, res_.get()};
     launch_slab<double>(n_, M_.col_start, M_.row_index, M_.value, yo_.get(), ec, st_);
-    SumPlan p;
-    double* R = res_.get();
-    p.add(K0, 0, m_, 0.0, SumOrder::kSeq, R + kRp2);
-    p.add(K0 + L, 0, L, 0.0, SumOrder::kSeq, R + kD);
-    p.add(K0 + 2 * L, 0, L, 0.0, SumOrder::kSeq, R + kRd2);
-    p.add(K0 + 3 * L, m_, L, 0.0, SumOrder::kSeq, R + kP);
-    p.build(exact_, nullptr, st_);
-    p.launch(st_);
+    plan_kkt_.launch(st_);
     double h[kNumSlots];
     B200_CHECK(cudaMemcpyAsync(h, res_.get(), sizeof h, cudaMemcpyDeviceToHost, st_));
     B200_CHECK(cudaStreamSynchronize(st_));
@@ -252,10 +257,7 @@ class GpuBackendImpl final : public GpuBackend {
     if (mixed_) k_pair_terms<float><<<grid_for(len), kBlock, 0, st_>>>(len, f_[a].get(), f_[b].get(), diff, terms_.get());
     else k_pair_terms<double><<<grid_for(len), kBlock, 0, st_>>>(len, d_[a].get(), d_[b].get(), diff, terms_.get());
     B200_LAUNCH_CHECK();
-    SumPlan p;
-    p.add(terms_.get(), 0, len, 0.0, SumOrder::kChunk64, out_.get());
-    p.build(exact_, nullptr, st_);
-    p.launch(st_);
+    (len == n_ ? plan_n_ : plan_m_).launch(st_);
     double r = 0;
     B200_CHECK(cudaMemcpyAsync(&r, out_.get(), sizeof r, cudaMemcpyDeviceToHost, st_));
     B200_CHECK(cudaStreamSynchronize(st_));
@@ -268,6 +270,7 @@ class GpuBackendImpl final : public GpuBackend {
   DevBuf<int> cs_, ri_;
   DeviceModel M_;
   ScaledDevice sp_;
+  SumPlan plan_kkt_, plan_n_, plan_m_;
   std::vector<DevBuf<double>> d_;
   std::vector<DevBuf<float>> f_;
   std::vector<long long> sizes_;

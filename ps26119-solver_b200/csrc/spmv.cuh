@@ -56,6 +56,10 @@ namespace b200 {
 #define B200_SLAB_FED 1
 #endif
 
+#ifndef B200_PDL
+#define B200_PDL 1
+#endif
+
 #ifndef B200_SLAB_ROWS
 #define B200_SLAB_ROWS 256
 #endif
@@ -255,6 +259,9 @@ constexpr int kGatherBatch = B200_GATHER_BATCH;  // independent x-gathers issued
 // kTma: the tiles of col/val are staged by TMA bulk copies (the arrays must be this library's
 // own allocations, whose 64-byte tail padding covers the 16-byte widening); otherwise by a
 // batched register copy (caller-owned arrays). epi.active() lets graph-replayed launches exit.
+// Launched with programmatic dependent launch (only with an epilogue that is always active), the row
+// pointers and the first tile come in while the kernel before it ends; x and the epilogue's operands are
+// read after it.
 template <class T, class Epi, bool kTma>
 __global__ void __launch_bounds__(kSlabRows, B200_SLAB_MIN_BLOCKS) k_slab(int rows, const int* __restrict__ rp,
                                                         const int* __restrict__ col,
@@ -262,6 +269,7 @@ __global__ void __launch_bounds__(kSlabRows, B200_SLAB_MIN_BLOCKS) k_slab(int ro
                                                         const T* __restrict__ x, Epi epi,
                                                         const int2* __restrict__ slab, unsigned* err) {
   __shared__ SlabSmem<T> sm;
+  pdl_allow_next();
   if (!epi.active()) return;
   const int r0 = blockIdx.x * kSlabRows;
   const int nr = min(kSlabRows, rows - r0);
@@ -276,13 +284,25 @@ __global__ void __launch_bounds__(kSlabRows, B200_SLAB_MIN_BLOCKS) k_slab(int ro
     k0 = __ldg(rp + r0), k1 = __ldg(rp + r0 + nr);
   }
   const int beg = mine ? __ldg(rp + row) : 0, end = mine ? __ldg(rp + row + 1) : 0;
-  const auto pre = epi_load(epi, mine ? row : r0, 0);
   auto acc = epi_acc(epi, 0);
+  constexpr int kValAlign = 16 / static_cast<int>(sizeof(T));  // elements per 16 bytes
+  auto issue = [&](int t0, int t1) {  // thread 0
+    const int c0 = t0 & ~3, v0 = t0 & ~(kValAlign - 1);
+    const int c1 = (t1 + 3) & ~3, v1 = (t1 + kValAlign - 1) & ~(kValAlign - 1);
+    const unsigned cb = static_cast<unsigned>(c1 - c0) * 4u, vb = static_cast<unsigned>(v1 - v0) * sizeof(T);
+    mbar_expect_tx(&sm.bar, cb + vb);
+    tma_load_1d(sm.col, col + c0, cb, &sm.bar);
+    tma_load_1d(sm.val, val + v0, vb, &sm.bar);
+  };
   if constexpr (kTma) {
-    if (threadIdx.x == 0) mbar_init(&sm.bar);
+    if (threadIdx.x == 0) {
+      mbar_init(&sm.bar);
+      if (k0 < k1) issue(k0, min(k0 + kSlabTile, k1));
+    }
     __syncthreads();
   }
-  constexpr int kValAlign = 16 / static_cast<int>(sizeof(T));  // elements per 16 bytes
+  pdl_wait();
+  const auto pre = epi_load(epi, mine ? row : r0, 0);
   unsigned phase = 0;
   double s = 0.0;
   bool staged = true;
@@ -293,13 +313,9 @@ __global__ void __launch_bounds__(kSlabRows, B200_SLAB_MIN_BLOCKS) k_slab(int ro
     if constexpr (kTma) {
       c0 = t0 & ~3;
       v0 = t0 & ~(kValAlign - 1);
-      const int c1 = (t1 + 3) & ~3, v1 = (t1 + kValAlign - 1) & ~(kValAlign - 1);
-      if (threadIdx.x == 0) {
+      if (t0 != k0 && threadIdx.x == 0) {
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        const unsigned cb = static_cast<unsigned>(c1 - c0) * 4u, vb = static_cast<unsigned>(v1 - v0) * sizeof(T);
-        mbar_expect_tx(&sm.bar, cb + vb);
-        tma_load_1d(sm.col, col + c0, cb, &sm.bar);
-        tma_load_1d(sm.val, val + v0, vb, &sm.bar);
+        issue(t0, t1);
       }
       // thread 0 waits; the others sleep in the barrier instead of spinning on the barrier word
       const int ok = threadIdx.x == 0 ? (mbar_wait_bounded(&sm.bar, phase) ? 1 : 0) : 1;
@@ -632,10 +648,23 @@ inline void slab_prepare() {
 
 template <class T, class Epi, bool kTma = false>
 inline void launch_slab(int rows, const int* rp, const int* col, const T* val, const T* x, const Epi& epi,
-                        cudaStream_t st, const int2* slab = nullptr, unsigned* err = nullptr) {
+                        cudaStream_t st, const int2* slab = nullptr, unsigned* err = nullptr, bool pdl = false) {
   if (rows <= 0) return;
   slab_prepare<T, Epi, kTma>();
   const int grid = (rows + kSlabRows - 1) / kSlabRows;
+  if (B200_PDL && pdl) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(grid));
+    cfg.blockDim = dim3(kSlabRows);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    B200_CHECK(cudaLaunchKernelEx(&cfg, k_slab<T, Epi, kTma>, rows, rp, col, val, x, epi, slab, err));
+    return;
+  }
   k_slab<T, Epi, kTma><<<grid, kSlabRows, 0, st>>>(rows, rp, col, val, x, epi, slab, err);
   B200_LAUNCH_CHECK();
 }
@@ -645,8 +674,8 @@ inline void launch_slab(int rows, const int* rp, const int* col, const T* val, c
 // counter (nullptr: the process-wide one).
 template <class T, class Epi>
 inline void launch_slab_tma(int rows, const int* rp, const int* col, const T* val, const T* x, const Epi& epi,
-                            cudaStream_t st, const int2* slab = nullptr, unsigned* err = nullptr) {
-  launch_slab<T, Epi, B200_STAGE_TMA != 0>(rows, rp, col, val, x, epi, st, B200_SLAB_TABLE ? slab : nullptr, err);
+                            cudaStream_t st, const int2* slab = nullptr, unsigned* err = nullptr, bool pdl = false) {
+  launch_slab<T, Epi, B200_STAGE_TMA != 0>(rows, rp, col, val, x, epi, st, B200_SLAB_TABLE ? slab : nullptr, err, pdl);
 }
 
 // The fully staged form (k_slab_fed) for the iteration epilogues, whose operand vectors are
@@ -656,9 +685,6 @@ inline void launch_slab_tma(int rows, const int* rp, const int* col, const T* va
 // programmatic dependent launch (B200_PDL builds), so the kernel's blocks may start while the
 // previous kernel of the stream finishes: only where Epi::kLiveVecs names every operand vector a
 // kernel still in flight may write. The fallback never uses it.
-#ifndef B200_PDL
-#define B200_PDL 1
-#endif
 
 // Launch variants of k_slab_fed, chosen per matrix by the autotuner (tune.hpp): `gather` = GB
 // (2, 4 or 8 gathers in flight per thread, each thread walking its own row; 0: the spread form,
