@@ -378,6 +378,21 @@ inline int sm_count() {
 __device__ __forceinline__ void pdl_allow_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// Launches a kernel that calls pdl_wait() with programmatic dependent launch.
+template <class... P, class... A>
+inline void launch_pdl(void (*kernel)(P...), int grid, int block, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(grid));
+  cfg.blockDim = dim3(static_cast<unsigned>(block));
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  B200_CHECK(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+}
+
 // Grid-stride helper over [0, n).
 #define B200_FOR(i, n) \
   for (std::int64_t i = blockIdx.x * static_cast<std::int64_t>(blockDim.x) + threadIdx.x; i < (n); \

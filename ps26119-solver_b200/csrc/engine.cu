@@ -409,13 +409,14 @@ void Engine::tune_slab() {
   hp.skip_r0 = 1;
   B200_CHECK(cudaMemcpyAsync(params_.get(), &hp, sizeof hp, cudaMemcpyHostToDevice, st_));
   const StepParams* P = params_.get();
+  const bool stays = stays_in_l2<T>(m, n, M_.nnz);
   auto pair = [&](int vt, int va, bool pdl) {  // one iteration: Ãᵀy + primal update, Ãx̄ + dual update
     EpiPrimal<T> ep{v.x.get(), v.xh.get(), v.xb.get(), v.x0.get(), sp_.c<T>(), sp_.l<T>(), sp_.u<T>(), P, 1, 0, 0, 0};
     launch_slab_fed<T>(n, sp_.t_rp.get(), sp_.t_ri.get(), sp_.At_val<T>(), v.y.get(), ep, st_, slab_t_.get(), cap_t_,
-                       err(), pdl, vt);
+                       err(), pdl, vt, stays);
     EpiDual<T> ed{v.y.get(), v.yh.get(), v.yb.get(), v.y0.get(), sp_.rl<T>(), sp_.ru<T>(), P, 1, 0, 0, 0, 0};
     launch_slab_fed<T>(m, sp_.a_rp.get(), sp_.a_col.get(), sp_.A_val<T>(), v.xb.get(), ed, st_, slab_a_.get(), cap_a_,
-                       err(), true, va);
+                       err(), true, va, stays);
     kernels_ += 2;
   };
   constexpr int kTunePairs = 6;
@@ -659,13 +660,14 @@ void Engine::capture_epoch() {
   B200_CHECK(cudaStreamBeginCapture(st_, cudaStreamCaptureModeThreadLocal));
   // Programmatic dependent launch for every iteration kernel whose predecessor in the stream is
   // another iteration kernel (not the first kernel of the epoch, nor the one after the residual).
+  const bool stays = stays_in_l2<T>(m, n, M_.nnz);
   auto step = [&](int s) {
     EpiPrimal<T> ep{v.x.get(), v.xh.get(), v.xb.get(), v.x0.get(), sp_.c<T>(), sp_.l<T>(), sp_.u<T>(), P, s, 0, 0, 0};
     launch_slab_fed<T>(n, sp_.t_rp.get(), sp_.t_ri.get(), sp_.At_val<T>(), v.y.get(), ep, st_, slab_t_.get(), cap_t_,
-                       err(), s >= 2, var_t_);
+                       err(), s >= 2, var_t_, stays);
     EpiDual<T> ed{v.y.get(), v.yh.get(), v.yb.get(), v.y0.get(), sp_.rl<T>(), sp_.ru<T>(), P, s, 0, 0, 0, 0};
     launch_slab_fed<T>(m, sp_.a_rp.get(), sp_.a_col.get(), sp_.A_val<T>(), v.xb.get(), ed, st_, slab_a_.get(), cap_a_,
-                       err(), true, var_a_);
+                       err(), true, var_a_, stays);
     capture_count_ += 2;
   };
   B200_CHECK(cudaEventRecordWithFlags(ev_[0], st_, cudaEventRecordExternal));
@@ -1275,6 +1277,7 @@ void Engine::capture_pdlp_epoch(int phase) {
   capture_count_ = 0;
   auto capture_scope = std::make_unique<CaptureScope>();  // no device-wide syncs elsewhere meanwhile
   B200_CHECK(cudaStreamBeginCapture(st_, cudaStreamCaptureModeThreadLocal));
+  const bool stays = stays_in_l2<T>(m, n, M_.nnz);
   B200_CHECK(cudaEventRecordWithFlags(ev_[0], st_, cudaEventRecordExternal));
   for (int s = 0; s < K; ++s) {
     const bool odd = ((phase + s) & 1) != 0;
@@ -1284,10 +1287,10 @@ void Engine::capture_pdlp_epoch(int phase) {
     T* yn = odd ? v.y.get() : v.yh.get();
     EpiPdlpPrimal<T> ep{xc, sp_.c<T>(), sp_.l<T>(), sp_.u<T>(), xn, v.xb.get(), v.dx.get(), P, s};
     launch_slab_fed<T>(n, sp_.t_rp.get(), sp_.t_ri.get(), sp_.At_val<T>(), yc, ep, st_, slab_t_.get(), cap_t_, err(),
-                       s >= 1, var_t_);
+                       s >= 1, var_t_, stays);
     EpiPdlpDual<T> ed{yc, sp_.rl<T>(), sp_.ru<T>(), yn, v.dy.get(), P, s};
     launch_slab_fed<T>(m, sp_.a_rp.get(), sp_.a_col.get(), sp_.A_val<T>(), v.xb.get(), ed, st_, slab_a_.get(), cap_a_,
-                       err(), true, var_a_);
+                       err(), true, var_a_, stays);
     capture_count_ += 2;
   }
   B200_CHECK(cudaEventRecordWithFlags(ev_[1], st_, cudaEventRecordExternal));

@@ -114,6 +114,7 @@ static __global__ void __launch_bounds__(kXTile) k_lanczos_update(int n, double*
                                                                   const double* ab, double* terms, double* stat) {
   const int j = blockIdx.x * kXTile + threadIdx.x;
   double term = 0.0;
+  pdl_wait();
   if (j < n) {
     const double e = w[j] - (ab[0] * v[j] + sqrt(ab[1]) * vprev[j]);
     w[j] = e;
@@ -124,6 +125,7 @@ static __global__ void __launch_bounds__(kXTile) k_lanczos_update(int n, double*
 }
 // The next Lanczos vector, w/β; hist receives (α, β²) of this step for the host's later replay.
 static __global__ void k_lanczos_next(int n, const double* w, double* v, double* vprev, const double* ab, double* hist) {
+  pdl_wait();
   const double bn = sqrt(ab[1]);
   if (blockIdx.x == 0 && threadIdx.x == 0) hist[0] = ab[0], hist[1] = ab[1];
   B200_FOR(j, n) {
@@ -378,17 +380,16 @@ struct ScaledDevice {
         return;
       }
       for (int k = from; k < to; ++k) {
+        // every kernel of a step starts while the one before it ends (programmatic dependent launch)
         launch_slab_tma<double>(m, a_rp.get(), a_col.get(), sa.get(), v.get(), EpiStore<double>{{}, t.get()}, st,
-                                nullptr, err);
+                                nullptr, err, true);
         launch_slab_tma<double>(n, t_rp.get(), t_ri.get(), sat.get(), t.get(),
-                                EpiLanczosW{{}, v.get(), w.get(), terms.get(), pal.stat()}, st, nullptr, err);
+                                EpiLanczosW{{}, v.get(), w.get(), terms.get(), pal.stat()}, st, nullptr, err, true);
         pal.launch(st, true);
         // β of the previous step is still in out[1]: this step's β² overwrites it only below
-        k_lanczos_update<<<tiles, kXTile, 0, st>>>(n, w.get(), v.get(), vprev.get(), out.get(), terms.get(), pbn.stat());
-        B200_LAUNCH_CHECK();
+        launch_pdl(k_lanczos_update, tiles, kXTile, st, n, w.get(), v.get(), vprev.get(), out.get(), terms.get(), pbn.stat());
         pbn.launch(st, true);
-        k_lanczos_next<<<grid_for(n), kBlock, 0, st>>>(n, w.get(), v.get(), vprev.get(), out.get(), hist.get() + 2 * k);
-        B200_LAUNCH_CHECK();
+        launch_pdl(k_lanczos_next, grid_for(n), kBlock, st, n, w.get(), v.get(), vprev.get(), out.get(), hist.get() + 2 * k);
         kernels += 6;
       }
       lanczos_launched = to;
