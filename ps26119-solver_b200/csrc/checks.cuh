@@ -143,84 +143,6 @@ struct EpiKktCols : AlwaysActive {
   }
 };
 
-// ---------------------------------------------------------------------- ray test
-// Dual ray r from Δy (rows), primal ray d from Δx (columns), engine.cpp:88-96 / 130-137.
-template <class T>
-static __global__ void k_ray_r(int m, const T* dy, const double* row_scale, double obj_scale, const double* rl,
-                        const double* ru, double* r, double* res, int slot_rmax) {
-  double mx = 0.0;
-  B200_FOR(i, m) {
-    double v = row_scale[i] * static_cast<double>(dy[i]) / obj_scale;
-    if (!isfinite(rl[i])) v = std_min(v, 0.0);
-    if (!isfinite(ru[i])) v = std_max(v, 0.0);
-    r[i] = v;
-    mx = std_max(mx, fabs(v));
-  }
-  warp_max_atomic(max_slot(res, slot_rmax), mx);
-}
-template <class T>
-static __global__ void k_ray_d(int n, const T* dx, const double* col_scale, double bound_scale, const double* cl,
-                        const double* cu, double* d, double* res, int slot_dabs) {
-  double mx = 0.0;
-  B200_FOR(j, n) {
-    double v = col_scale[j] * static_cast<double>(dx[j]) / bound_scale;
-    if (isfinite(cl[j])) v = std_max(v, 0.0);
-    if (isfinite(cu[j])) v = std_min(v, 0.0);
-    d[j] = v;
-    mx = std_max(mx, fabs(v));
-  }
-  warp_max_atomic(max_slot(res, slot_dabs), mx);
-}
-// Columns: g = Aᵀr and gabs = Σ|a r| (CSC order), λ = −g; objective/magnitude terms and the
-// dual-ray violation; plus the primal-ray terms cᵀd and Σ|c d| (engine.cpp:97-116, 138-139).
-static __global__ void k_ray_cols(int n, int m, const int* cp, const int* ri, const double* v, const double* r,
-                           const double* d, const double* c, double sense, const double* cl, const double* cu,
-                           double* t_obj, double* t_mag, double* t_cd, double* t_cmag, double* res, int slot_dviol) {
-  double dviol = 0.0;
-  B200_FOR(j, n) {
-    double g = 0.0, gabs = 0.0;
-    for (int k = cp[j]; k < cp[j + 1]; ++k) {
-      g += v[k] * r[ri[k]];
-      gabs += fabs(v[k] * r[ri[k]]);
-    }
-    const double lam = -g, lo = cl[j], up = cu[j];
-    double ob = 0.0, mg = 0.0;
-    if (lam > 0) {
-      if (isfinite(lo)) ob = lo * lam, mg = gabs * fabs(lo);
-      else dviol = std_max(dviol, lam);
-    } else if (lam < 0) {
-      if (isfinite(up)) ob = up * lam, mg = gabs * fabs(up);
-      else dviol = std_max(dviol, -lam);
-    }
-    t_obj[m + j] = ob;
-    t_mag[m + j] = mg;
-    t_cd[j] = sense * c[j] * d[j];
-    t_cmag[j] = fabs(c[j] * d[j]);
-  }
-  warp_max_atomic(max_slot(res, slot_dviol), dviol);
-}
-// Rows after ad = A_orig·d: primal-ray violation; dual-ray objective/magnitude row terms.
-struct EpiRayRows : AlwaysActive {
-  const double *r, *rl, *ru;
-  double *t_obj, *t_mag;
-  double* res;
-  int slot_pviol;
-  struct Acc {
-    double pviol = 0.0;
-  };
-  __device__ void operator()(int i, double ad, Acc& acc) const {
-    double v = 0.0;
-    if (isfinite(rl[i])) v = std_max(v, -ad);
-    if (isfinite(ru[i])) v = std_max(v, ad);
-    acc.pviol = v;
-    const double ri = r[i];
-    const double term = ri > 0 ? rl[i] * ri : (ri < 0 ? ru[i] * ri : 0.0);
-    t_obj[i] = term;
-    t_mag[i] = fabs(term);
-  }
-  __device__ void flush(const Acc& a) const { warp_max_atomic(max_slot(res, slot_pviol), a.pviol); }
-};
-
 // ---------------------------------------------------------------------- a check in three kernels
 // Everything a check evaluates on the way to its sums, for r²HPDHG: the residual's Δ, the unscaled point,
 // the ray directions (kRays ≥ 1: of the last step; 2: of the drift since the restart anchor as well) and
@@ -228,9 +150,47 @@ struct EpiRayRows : AlwaysActive {
 // products gather: X[j] = {x, Δx̃, d, d₂}, Y[i] = {y, r, r₂, 0}, 32 bytes, one sector. k_check_products then
 // walks every row and every column once for all of them. Each value is the one that the kernels above
 // compute, sums in the same order; the terms go to the same arrays.
+// PDLP's check has the same two kernels (k_pdlp_points, k_pdlp_products): the KKT statistics of the current
+// point and of the average, and the rays of the last step and of the drift; X[j] = {x, x_avg, d, d₂},
+// Y[i] = {y, y_avg, r, r₂}.
 // What bounds it: for LPs up to some 100k rows the number of dependent launches (up to 15 in the longest
 // chain before, 4 now); for large ones the gathers (one of 32 bytes per nonzero and side, against five to
 // seven of 8). A check with the host's part, fp64: 10k rows 87 -> 33 us, 100k 157 -> 71, 1M 560 -> 389.
+// kkt_general's terms of one row and of one column (EpiKktRows, EpiKktCols).
+struct KktTerms {
+  double *rp2, *d, *rd2, *p;  // rows at [0, m), columns at [m, m + n)
+};
+__device__ __forceinline__ void kkt_row(const KktTerms& t, int k, double ax, double yi, double lo, double up, double& pmax,
+                                        double& dmax) {
+  const double out = ax < lo ? lo - ax : (ax > up ? ax - up : 0.0);
+  t.rp2[k] = out * out;
+  pmax = elem_viol(ax, lo, up);
+  double d = 0.0, rd = 0.0;
+  dmax = 0.0;
+  if (yi > 0) {
+    if (isfinite(lo)) d = yi * lo;
+    else rd = yi * yi, dmax = yi;
+  } else if (yi < 0) {
+    if (isfinite(up)) d = yi * up;
+    else rd = yi * yi, dmax = -yi;
+  }
+  t.d[k] = d;
+  t.rd2[k] = rd;
+}
+__device__ __forceinline__ void kkt_col(const KktTerms& t, long long at, double aty, double cj, double x, double lo, double up,
+                                        double& pmax, double& dmax) {
+  t.p[at] = cj * x;
+  pmax = elem_viol(x, lo, up);
+  const double lam = cj - aty;
+  double z;
+  if (isfinite(lo) && isfinite(up)) z = lam;
+  else if (isfinite(lo)) z = std_max(lam, 0.0);
+  else if (isfinite(up)) z = std_min(lam, 0.0);
+  else z = 0.0;
+  t.rd2[at] = (lam - z) * (lam - z);
+  dmax = fabs(lam - z);
+  t.d[at] = z > 0 ? z * lo : (z < 0 ? z * up : 0.0);
+}
 template <class T>
 struct CheckVecs {
   int n, m;
@@ -240,7 +200,7 @@ struct CheckVecs {
   const double *c, *cl, *cu, *rl, *ru;
   double4 *X, *Y;
   double *t_px, *t_dxn, *t_py, *t_cross, *t_dyn;  // residual and restart distances
-  double *k_rp2, *k_d, *k_rd2, *k_p;              // KKT (rows at [0, m), columns at [m, m + n))
+  KktTerms kkt;
   double *r_obj, *r_mag, *r_cd, *r_cmag;          // rays
   double *q_obj, *q_mag, *q_cd, *q_cmag;          // drift rays
   double* res;
@@ -319,7 +279,7 @@ __device__ __forceinline__ double4 load_packed(const double4* p) {
   if constexpr (kAll) b = __ldg(reinterpret_cast<const double2*>(p) + 1);
   return make_double4(a.x, a.y, b.x, b.y);
 }
-// A ray's row terms (EpiRayRows) and column terms (k_ray_cols).
+// A ray's row terms and violation, and its column terms and violation (engine.cpp:97-128).
 __device__ __forceinline__ double ray_row(double ad, double r, double lo, double up, double& obj, double& mag) {
   double viol = 0.0;
   if (isfinite(lo)) viol = std_max(viol, -ad);
@@ -379,20 +339,7 @@ static __global__ void __launch_bounds__(kBlock) k_check_products(const __grid_c
       const double4 Y = v.Y[k];
       const T dy = static_cast<T>(-1.0) * v.yh[k] + static_cast<T>(1.0) * v.yb[k];
       v.t_cross[k] = static_cast<double>(dy) * static_cast<double>(static_cast<T>(adx));
-      const double out = ax < lo ? lo - ax : (ax > up ? ax - up : 0.0);
-      v.k_rp2[k] = out * out;
-      pmax = elem_viol(ax, lo, up);
-      const double yi = Y.x;
-      double d = 0.0, rd = 0.0;
-      if (yi > 0) {
-        if (isfinite(lo)) d = yi * lo;
-        else rd = yi * yi, dmax = yi;
-      } else if (yi < 0) {
-        if (isfinite(up)) d = yi * up;
-        else rd = yi * yi, dmax = -yi;
-      }
-      v.k_d[k] = d;
-      v.k_rd2[k] = rd;
+      kkt_row(v.kkt, k, ax, Y.x, lo, up, pmax, dmax);
       if constexpr (kRays >= 1) {
         double obj, mag;
         viol = ray_row(ad, Y.y, lo, up, obj, mag);
@@ -435,18 +382,7 @@ static __global__ void __launch_bounds__(kBlock) k_check_products(const __grid_c
       const double lo = v.cl[k], up = v.cu[k], c = v.c[k];
       const double4 X = v.X[k];
       const long long at = static_cast<long long>(v.m) + k;
-      const double cj = v.sense * c;
-      v.k_p[at] = cj * X.x;
-      pmax = elem_viol(X.x, lo, up);
-      const double lam = cj - aty;
-      double z;
-      if (isfinite(lo) && isfinite(up)) z = lam;
-      else if (isfinite(lo)) z = std_max(lam, 0.0);
-      else if (isfinite(up)) z = std_min(lam, 0.0);
-      else z = 0.0;
-      v.k_rd2[at] = (lam - z) * (lam - z);
-      dmax = fabs(lam - z);
-      v.k_d[at] = z > 0 ? z * lo : (z < 0 ? z * up : 0.0);
+      kkt_col(v.kkt, at, aty, v.sense * c, X.x, lo, up, pmax, dmax);
       if constexpr (kRays >= 1) {
         double obj, mag;
         viol = ray_col(gr, ga, lo, up, obj, mag);
@@ -467,12 +403,150 @@ static __global__ void __launch_bounds__(kBlock) k_check_products(const __grid_c
   warp_max_atomic(max_slot(v.res, kMaxPmax), pmax);
   warp_max_atomic(max_slot(v.res, kMaxDmax), dmax);
 }
-// The results go to the host's pinned block, and the maxima back to zero for the next check.
-static __global__ void k_check_publish(double* res, double* host) {
+template <class T>
+struct PdlpVecs {
+  int n, m;
+  const T *xc, *xa, *xp, *x0, *yc, *ya, *yp, *y0;  // current, average, the step before, the restart anchor
+  const double *col_scale, *row_scale;
+  double bound_scale, obj_scale, sense;
+  const double *c, *cl, *cu, *rl, *ru;
+  double4 *X, *Y;
+  KktTerms cur, avg;
+  double *r_obj, *r_mag, *r_cd, *r_cmag;  // rays
+  double *q_obj, *q_mag, *q_cd, *q_cmag;  // drift rays
+  double *res, *res_cur;                  // results: of the average and the rays, of the current point
+};
+template <class T, int kRays>
+static __global__ void __launch_bounds__(kBlock) k_pdlp_points(const __grid_constant__ PdlpVecs<T> v, int col_blocks) {
+  const bool cols = static_cast<int>(blockIdx.x) < col_blocks;
+  const int k = (static_cast<int>(blockIdx.x) - (cols ? 0 : col_blocks)) * kBlock + static_cast<int>(threadIdx.x);
+  double mx = 0.0, mx2 = 0.0;
+  if (cols) {
+    if (k < v.n) {
+      const T x = v.xc[k];
+      const double sc = v.col_scale[k], lo = v.cl[k], up = v.cu[k];
+      double4 X;
+      X.x = std_min(std_max(sc * static_cast<double>(x) / v.bound_scale, lo), up);
+      X.y = std_min(std_max(sc * static_cast<double>(v.xa[k]) / v.bound_scale, lo), up);
+      X.z = X.w = 0.0;
+      if constexpr (kRays >= 1) {  // Δ = z_k − z_{k−1}: axpby(1, x, −1, x_prev) (pdlp.cpp:83-85)
+        const T d = static_cast<T>(1.0) * x + static_cast<T>(-1.0) * v.xp[k];
+        X.z = ray_primal(sc * static_cast<double>(d) / v.bound_scale, lo, up);
+        mx = fabs(X.z);
+      }
+      if constexpr (kRays == 2) {  // the drift z − z0: copy + axpby(−1, x0, 1, ·) (pdlp.cpp:89-93)
+        const T d = static_cast<T>(-1.0) * v.x0[k] + static_cast<T>(1.0) * x;
+        X.w = ray_primal(sc * static_cast<double>(d) / v.bound_scale, lo, up);
+        mx2 = fabs(X.w);
+      }
+      v.X[k] = X;
+    }
+    if constexpr (kRays >= 1) warp_max_atomic(max_slot(v.res, kMaxDabs), mx);
+    if constexpr (kRays == 2) warp_max_atomic(max_slot(v.res, kMaxDabs2), mx2);
+  } else {
+    if (k < v.m) {
+      const T y = v.yc[k];
+      const double sc = v.row_scale[k];
+      double4 Y;
+      Y.x = sc * static_cast<double>(y) / v.obj_scale;
+      Y.y = sc * static_cast<double>(v.ya[k]) / v.obj_scale;
+      Y.z = Y.w = 0.0;
+      if constexpr (kRays >= 1) {
+        const T d = static_cast<T>(1.0) * y + static_cast<T>(-1.0) * v.yp[k];
+        Y.z = ray_dual(sc * static_cast<double>(d) / v.obj_scale, v.rl[k], v.ru[k]);
+        mx = fabs(Y.z);
+      }
+      if constexpr (kRays == 2) {
+        const T d = static_cast<T>(-1.0) * v.y0[k] + static_cast<T>(1.0) * y;
+        Y.w = ray_dual(sc * static_cast<double>(d) / v.obj_scale, v.rl[k], v.ru[k]);
+        mx2 = fabs(Y.w);
+      }
+      v.Y[k] = Y;
+    }
+    if constexpr (kRays >= 1) warp_max_atomic(max_slot(v.res, kMaxRmax), mx);
+    if constexpr (kRays == 2) warp_max_atomic(max_slot(v.res, kMaxRmax2), mx2);
+  }
+}
+template <class T, int kRays>
+static __global__ void __launch_bounds__(kBlock) k_pdlp_products(const __grid_constant__ PdlpVecs<T> v, int row_blocks,
+                                                                 const int* __restrict__ rp, const int* __restrict__ col,
+                                                                 const double* __restrict__ a0, const int* __restrict__ cp,
+                                                                 const int* __restrict__ ri, const double* __restrict__ av) {
+  constexpr int GB = 4;
+  const bool rows = static_cast<int>(blockIdx.x) < row_blocks;
+  const int k = (static_cast<int>(blockIdx.x) - (rows ? 0 : row_blocks)) * kBlock + static_cast<int>(threadIdx.x);
+  const bool mine = k < (rows ? v.m : v.n);
+  const int* __restrict__ ptr = rows ? rp : cp;
+  const int* __restrict__ idx = rows ? col : ri;
+  const double* __restrict__ val = rows ? a0 : av;
+  const double4* from = rows ? v.X : v.Y;
+  double sx = 0.0, sy = 0.0, sz = 0.0, sw = 0.0, tz = 0.0, tw = 0.0;  // the four sums, and Σ|·| of the rays'
+  const int b = mine ? ptr[k] : 0, e = mine ? ptr[k + 1] : 0;
+  for (int p = b; p < e; p += GB) {
+    double4 g[GB];
+    double w[GB];
+#pragma unroll
+    for (int q = 0; q < GB; ++q) {
+      const int at = p + q < e ? p + q : p;
+      g[q] = load_packed<(kRays >= 1)>(from + idx[at]);
+      w[q] = val[at];
+    }
+#pragma unroll
+    for (int q = 0; q < GB; ++q)
+      if (p + q < e) {  // each sum in storage order
+        sx += w[q] * g[q].x;
+        sy += w[q] * g[q].y;
+        if constexpr (kRays >= 1) {
+          const double t = w[q] * g[q].z;
+          sz += t, tz += fabs(t);
+        }
+        if constexpr (kRays == 2) {
+          const double t = w[q] * g[q].w;
+          sw += t, tw += fabs(t);
+        }
+      }
+  }
+  double pc = 0.0, dc = 0.0, pa = 0.0, da = 0.0, viol = 0.0, viol2 = 0.0;
+  if (mine && rows) {
+    const double lo = v.rl[k], up = v.ru[k];
+    const double4 Y = v.Y[k];
+    kkt_row(v.cur, k, sx, Y.x, lo, up, pc, dc);
+    kkt_row(v.avg, k, sy, Y.y, lo, up, pa, da);
+    double obj, mag;
+    if constexpr (kRays >= 1) viol = ray_row(sz, Y.z, lo, up, obj, mag), v.r_obj[k] = obj, v.r_mag[k] = mag;
+    if constexpr (kRays == 2) viol2 = ray_row(sw, Y.w, lo, up, obj, mag), v.q_obj[k] = obj, v.q_mag[k] = mag;
+  } else if (mine) {
+    const double lo = v.cl[k], up = v.cu[k], c = v.c[k];
+    const double4 X = v.X[k];
+    const long long at = static_cast<long long>(v.m) + k;
+    kkt_col(v.cur, at, sx, v.sense * c, X.x, lo, up, pc, dc);
+    kkt_col(v.avg, at, sy, v.sense * c, X.y, lo, up, pa, da);
+    double obj, mag;
+    if constexpr (kRays >= 1) {
+      viol = ray_col(sz, tz, lo, up, obj, mag), v.r_obj[at] = obj, v.r_mag[at] = mag;
+      v.r_cd[k] = v.sense * c * X.z, v.r_cmag[k] = fabs(c * X.z);
+    }
+    if constexpr (kRays == 2) {
+      viol2 = ray_col(sw, tw, lo, up, obj, mag), v.q_obj[at] = obj, v.q_mag[at] = mag;
+      v.q_cd[k] = v.sense * c * X.w, v.q_cmag[k] = fabs(c * X.w);
+    }
+  }
+  if constexpr (kRays >= 1) warp_max_atomic(max_slot(v.res, rows ? kMaxPviol : kMaxDviol), viol);
+  if constexpr (kRays == 2) warp_max_atomic(max_slot(v.res, rows ? kMaxPviol2 : kMaxDviol2), viol2);
+  warp_max_atomic(max_slot(v.res_cur, kMaxPmax), pc);
+  warp_max_atomic(max_slot(v.res_cur, kMaxDmax), dc);
+  warp_max_atomic(max_slot(v.res, kMaxPmax), pa);
+  warp_max_atomic(max_slot(v.res, kMaxDmax), da);
+}
+
+// The results go to the host's pinned block, and the maxima back to zero for the next check. (PDLP: a second
+// set, in the second block of threads.)
+static __global__ void k_check_publish(double* res, double* host, double* res2, double* host2) {
   const int k = threadIdx.x;
   if (k >= kNumSlots) return;
-  host[k] = res[k];
-  if (k >= kMaxPmax) res[k] = 0.0;
+  double* r = blockIdx.x ? res2 : res;
+  (blockIdx.x ? host2 : host)[k] = r[k];
+  if (k >= kMaxPmax) r[k] = 0.0;
 }
 // One packed component as a vector (an infeasibility ray).
 static __global__ void k_unpack(int len, const double4* P, int which, double* out) {

@@ -116,11 +116,6 @@ struct IterVecs {
   }
 };
 
-template <class T>
-__global__ void k_diff(long long n, const T* a, const T* b, T* out) {  // out = a − b as axpby(−1, b, 1, out=a)
-  B200_FOR(i, n) out[i] = static_cast<T>(-1.0) * b[i] + static_cast<T>(1.0) * a[i];
-}
-
 class Engine {
  public:
   Engine(const DeviceModel& M, const EngineOptions& o, cudaStream_t st) : M_(M), o_(o), st_(st) {
@@ -230,7 +225,7 @@ class Engine {
   template <class T> void launch_kkt_scaled(const T* xs, const T* ys);
   void launch_kkt_original();
   void make_side_stream();
-  template <class T> void launch_ray(const T* dx, const T* dy, double* r, double* d, int drift);
+  template <class T, int kRays> void launch_pdlp_check_kernels(int phase);
   Kkt read_kkt(const double* h) const;
   Status ray_verdict(const double* h, int which, const Kkt& k, std::string& why) const;
   void setup();
@@ -277,8 +272,8 @@ class Engine {
   DevBuf<double> res_;
   PinnedBuf<double> hres_;
   DevBuf<double4> X4_, Y4_;  // a check's packed points
-  DevBuf<double> rt_, kt_, rayt_, xo_, yo_, r1_, d1_, r2_, d2_, objt_;
-  SumPlan plan_r0_, plan_pid_, plan_kkt_, plan_ray1_, plan_ray2_, plan_obj_, plan_chk_;
+  DevBuf<double> rt_, kt_, kt2_, rayt_, xo_, yo_, r1_, d1_, r2_, d2_, objt_;
+  SumPlan plan_r0_, plan_pid_, plan_kkt_, plan_obj_, plan_chk_;
   SumPlan plan_check_[3];  // a check's sums (residual, KKT, rays), by its variant
   cudaGraphExec_t g_epoch_[2] = {nullptr, nullptr};
   cudaGraphExec_t g_check_[2][3] = {{nullptr, nullptr, nullptr}, {nullptr, nullptr, nullptr}};
@@ -361,8 +356,14 @@ void Engine::setup() {
   const std::size_t mm = static_cast<std::size_t>(m), nn = static_cast<std::size_t>(n);
   rt_.alloc(2 * nn + 3 * mm);
   kt_.alloc(4 * (mm + nn));
-  rayt_.alloc((o_.pdlp ? 1 : 2) * (2 * (mm + nn) + 2 * nn));
-  if (!o_.pdlp) X4_.alloc(nn), Y4_.alloc(mm);
+  rayt_.alloc(2 * (2 * (mm + nn) + 2 * nn));
+  X4_.alloc(nn), Y4_.alloc(mm);
+  if (o_.pdlp) {
+    kt2_.alloc(4 * (mm + nn));
+    res2_.alloc(kNumSlots);
+    hres2_.alloc(kNumSlots);
+    B200_CHECK(cudaMemsetAsync(res2_.get(), 0, kNumSlots * sizeof(double), st_));
+  }
   xo_.alloc(nn), yo_.alloc(mm), r1_.alloc(mm), d1_.alloc(nn), r2_.alloc(mm), d2_.alloc(nn);
   objt_.alloc(mm + 2 * nn);
   build_plans();
@@ -467,33 +468,31 @@ void Engine::build_plans() {
   plan_kkt_.add(K0 + 2 * L, 0, L, 0.0, SumOrder::kSeq, R + kRd2);
   plan_kkt_.add(K0 + 3 * L, m, L, 0.0, SumOrder::kSeq, R + kP);
   double* T0 = rayt_.get();
-  plan_ray1_.add(T0, 0, L, 0.0, SumOrder::kSeq, R + kRayObj);
-  plan_ray1_.add(T0 + L, 0, L, 0.0, SumOrder::kSeq, R + kRayMag);
-  plan_ray1_.add(T0 + 2 * L, 0, n, 0.0, SumOrder::kSeq, R + kRayCd);
-  plan_ray1_.add(T0 + 2 * L + n, 0, n, 0.0, SumOrder::kSeq, R + kRayCmag);
-  plan_ray2_.add(T0, 0, L, 0.0, SumOrder::kSeq, R + kRayObj2);
-  plan_ray2_.add(T0 + L, 0, L, 0.0, SumOrder::kSeq, R + kRayMag2);
-  plan_ray2_.add(T0 + 2 * L, 0, n, 0.0, SumOrder::kSeq, R + kRayCd2);
-  plan_ray2_.add(T0 + 2 * L + n, 0, n, 0.0, SumOrder::kSeq, R + kRayCmag2);
-  if (!o_.pdlp)
-    for (int v = 0; v < 3; ++v) {
-      SumPlan& p = plan_check_[v];
+  for (int v = 0; v < 3; ++v) {
+    SumPlan& p = plan_check_[v];
+    const auto kkt = [&](const double* t, double* r) {
+      p.add(t, 0, m, 0.0, SumOrder::kSeq, r + kRp2);
+      p.add(t + L, 0, L, 0.0, SumOrder::kSeq, r + kD);
+      p.add(t + 2 * L, 0, L, 0.0, SumOrder::kSeq, r + kRd2);
+      p.add(t + 3 * L, m, L, 0.0, SumOrder::kSeq, r + kP);
+    };
+    if (o_.pdlp) {
+      kkt(kt2_.get(), res2_.get());  // the current point's; K0: the average's
+    } else {
       p.add(px, 0, n, 0.0, SumOrder::kChunk64, R + kPx);
       p.add(py, 0, m, 0.0, SumOrder::kChunk64, R + kPy);
       p.add(cross, 0, m, 0.0, SumOrder::kChunk64, R + kCross);
-      p.add(K0, 0, m, 0.0, SumOrder::kSeq, R + kRp2);
-      p.add(K0 + L, 0, L, 0.0, SumOrder::kSeq, R + kD);
-      p.add(K0 + 2 * L, 0, L, 0.0, SumOrder::kSeq, R + kRd2);
-      p.add(K0 + 3 * L, m, L, 0.0, SumOrder::kSeq, R + kP);
-      for (int ray = 0; ray < v; ++ray) {
-        const double* t = T0 + ray * (2 * L + 2 * n);
-        p.add(t, 0, L, 0.0, SumOrder::kSeq, R + (ray ? kRayObj2 : kRayObj));
-        p.add(t + L, 0, L, 0.0, SumOrder::kSeq, R + (ray ? kRayMag2 : kRayMag));
-        p.add(t + 2 * L, 0, n, 0.0, SumOrder::kSeq, R + (ray ? kRayCd2 : kRayCd));
-        p.add(t + 2 * L + n, 0, n, 0.0, SumOrder::kSeq, R + (ray ? kRayCmag2 : kRayCmag));
-      }
-      p.build(o_.exact, nullptr, st_);
     }
+    kkt(K0, R);
+    for (int ray = 0; ray < v; ++ray) {
+      const double* t = T0 + ray * (2 * L + 2 * n);
+      p.add(t, 0, L, 0.0, SumOrder::kSeq, R + (ray ? kRayObj2 : kRayObj));
+      p.add(t + L, 0, L, 0.0, SumOrder::kSeq, R + (ray ? kRayMag2 : kRayMag));
+      p.add(t + 2 * L, 0, n, 0.0, SumOrder::kSeq, R + (ray ? kRayCd2 : kRayCd));
+      p.add(t + 2 * L + n, 0, n, 0.0, SumOrder::kSeq, R + (ray ? kRayCmag2 : kRayCmag));
+    }
+    p.build(o_.exact, nullptr, st_);
+  }
   // finish: objective = offset + Σ c x (Model::objective_value), check sums (solution_checker)
   double* O = objt_.get();
   plan_obj_.add(O, 0, n, M_.offset, SumOrder::kSeq, R + kObjective);
@@ -502,7 +501,6 @@ void Engine::build_plans() {
   plan_r0_.build(o_.exact, skip_r0_flag(params_.get()), st_);
   plan_pid_.build(true, nullptr, st_);
   plan_kkt_.build(o_.exact, nullptr, st_);
-  if (o_.pdlp) plan_ray1_.build(o_.exact, nullptr, st_), plan_ray2_.build(o_.exact, nullptr, st_);
   plan_obj_.build(o_.exact, nullptr, st_);
   plan_chk_.build(o_.exact, nullptr, st_);
 }
@@ -574,7 +572,7 @@ void Engine::launch_check_kernels() {
   CheckVecs<T> c{n, m, v.xb.get(), v.xh.get(), v.x0.get(), v.yb.get(), v.yh.get(), v.y0.get(), sp_.col_scale.get(),
                  sp_.row_scale.get(), sp_.bound_scale, sp_.obj_scale, static_cast<double>(M_.sense), M_.c, M_.col_lower,
                  M_.col_upper, M_.row_lower, M_.row_upper, X4_.get(), Y4_.get(), px, px + n, px + 2 * n, px + 2 * n + m,
-                 px + 2 * n + 2 * m, K0, K0 + L, K0 + 2 * L, K0 + 3 * L, T0, T0 + L, T0 + 2 * L, T0 + 2 * L + n, T1, T1 + L,
+                 px + 2 * n + 2 * m, {K0, K0 + L, K0 + 2 * L, K0 + 3 * L}, T0, T0 + L, T0 + 2 * L, T0 + 2 * L + n, T1, T1 + L,
                  T1 + 2 * L, T1 + 2 * L + n, res_.get()};
   const int cb = (n + kBlock - 1) / kBlock, rb = (m + kBlock - 1) / kBlock;
   if (cb + rb > 0) {
@@ -592,31 +590,9 @@ void Engine::launch_check_kernels() {
   }
   plan_check_[kRays].launch(st_);
   B200_CHECK(cudaStreamWaitEvent(st_, fork_[1], 0));
-  k_check_publish<<<1, 64, 0, st_>>>(res_.get(), hres_.get());
+  k_check_publish<<<1, 64, 0, st_>>>(res_.get(), hres_.get(), nullptr, nullptr);
   B200_LAUNCH_CHECK();
   B200_COUNT(3 + plan_pid_.kernel_count() + plan_check_[kRays].kernel_count());
-}
-
-template <class T>
-void Engine::launch_ray(const T* dx, const T* dy, double* r, double* d, int drift) {
-  const int m = M_.m, n = M_.n;
-  const long long L = static_cast<long long>(m) + n;
-  double* T0 = rayt_.get();
-  const int s_rmax = drift ? kMaxRmax2 : kMaxRmax, s_dabs = drift ? kMaxDabs2 : kMaxDabs;
-  const int s_dviol = drift ? kMaxDviol2 : kMaxDviol, s_pviol = drift ? kMaxPviol2 : kMaxPviol;
-  k_ray_r<T><<<grid_for(m), kBlock, 0, st_>>>(m, dy, sp_.row_scale.get(), sp_.obj_scale, M_.row_lower,
-                                              M_.row_upper, r, res_.get(), s_rmax);
-  k_ray_d<T><<<grid_for(n), kBlock, 0, st_>>>(n, dx, sp_.col_scale.get(), sp_.bound_scale, M_.col_lower,
-                                              M_.col_upper, d, res_.get(), s_dabs);
-  k_ray_cols<<<grid_for(n), kBlock, 0, st_>>>(n, m, M_.col_start, M_.row_index, M_.value, r, d, M_.c,
-                                              static_cast<double>(M_.sense), M_.col_lower, M_.col_upper, T0,
-                                              T0 + L, T0 + 2 * L, T0 + 2 * L + n, res_.get(), s_dviol);
-  B200_LAUNCH_CHECK();
-  EpiRayRows er{{}, r, M_.row_lower, M_.row_upper, T0, T0 + L, res_.get(), s_pviol};
-  launch_slab_tma<double>(m, sp_.a_rp.get(), sp_.a_col.get(), sp_.a_v0.get(), d, er, st_, nullptr, err());
-  SumPlan& p = drift ? plan_ray2_ : plan_ray1_;
-  p.launch(st_);
-  B200_COUNT(4 + p.kernel_count());
 }
 
 template <class T>
@@ -892,7 +868,8 @@ void Engine::finish_p(EngineResult& R, Status status, const T* xs, const T* ys, 
     if (ytmp.get()) B200_CHECK(cudaStreamSynchronize(st_));
   }
   if (status == Status::Infeasible && X4_.get() && ray_test > 0)  // a check left its rays packed
-    k_unpack<<<grid_for(m), kBlock, 0, st_>>>(m, Y4_.get(), ray_test, (ray_test == 2 ? r2_ : r1_).get());
+    k_unpack<<<grid_for(m), kBlock, 0, st_>>>(m, Y4_.get(), o_.pdlp ? ray_test + 1 : ray_test,
+                                               (ray_test == 2 ? r2_ : r1_).get());
   if (status == Status::Unbounded && X4_.get() && ray_test > 0)
     k_unpack<<<grid_for(n), kBlock, 0, st_>>>(n, X4_.get(), ray_test + 1, (ray_test == 2 ? d2_ : d1_).get());
   B200_LAUNCH_CHECK();
@@ -1305,45 +1282,45 @@ void Engine::capture_pdlp_epoch(int phase) {
   pdlp_kernels_[idx][phase] = capture_count_;
 }
 
+// A check's kernels (checks.cuh) in the capture; the KKT statistics of the current point go to res2_, those
+// of the average and the rays to res_.
+template <class T, int kRays>
+void Engine::launch_pdlp_check_kernels(int phase) {
+  IterVecs<T>& v = vecs<T>();
+  const int m = M_.m, n = M_.n;
+  const long long L = static_cast<long long>(m) + n;
+  T *xs[2] = {v.x.get(), v.xh.get()}, *ys[2] = {v.y.get(), v.yh.get()};
+  double *K0 = kt_.get(), *K1 = kt2_.get(), *T0 = rayt_.get(), *T1 = T0 + 2 * L + 2 * n;
+  PdlpVecs<T> c{n, m, xs[phase], v.dx.get(), xs[1 - phase], v.x0.get(), ys[phase], v.dy.get(), ys[1 - phase], v.y0.get(),
+                sp_.col_scale.get(), sp_.row_scale.get(), sp_.bound_scale, sp_.obj_scale, static_cast<double>(M_.sense), M_.c,
+                M_.col_lower, M_.col_upper, M_.row_lower, M_.row_upper, X4_.get(), Y4_.get(),
+                {K1, K1 + L, K1 + 2 * L, K1 + 3 * L}, {K0, K0 + L, K0 + 2 * L, K0 + 3 * L}, T0, T0 + L, T0 + 2 * L,
+                T0 + 2 * L + n, T1, T1 + L, T1 + 2 * L, T1 + 2 * L + n, res_.get(), res2_.get()};
+  const int cb = (n + kBlock - 1) / kBlock, rb = (m + kBlock - 1) / kBlock;
+  if (cb + rb > 0) {
+    k_pdlp_points<T, kRays><<<cb + rb, kBlock, 0, st_>>>(c, cb);
+    k_pdlp_products<T, kRays><<<cb + rb, kBlock, 0, st_>>>(c, rb, sp_.a_rp.get(), sp_.a_col.get(), sp_.a_v0.get(),
+                                                           M_.col_start, M_.row_index, M_.value);
+    B200_LAUNCH_CHECK();
+  }
+  plan_check_[kRays].launch(st_);
+  k_check_publish<<<2, 64, 0, st_>>>(res_.get(), hres_.get(), res2_.get(), hres2_.get());
+  B200_LAUNCH_CHECK();
+  B200_COUNT(3 + plan_check_[kRays].kernel_count());
+}
+
 template <class T>
 void Engine::capture_pdlp_check(int phase, int variant) {
   const int idx = std::is_same<T, float>::value ? 1 : 0;
   if (g_pdlp_chk_[idx][phase][variant]) return;
-  IterVecs<T>& v = vecs<T>();
-  const long long m = M_.m, n = M_.n;
-  T* xc = phase ? v.xh.get() : v.x.get();
-  T* xp = phase ? v.x.get() : v.xh.get();  // z_{k−1}, scratch for the ray directions
-  T* yc = phase ? v.yh.get() : v.y.get();
-  T* yp = phase ? v.y.get() : v.yh.get();
   cudaGraph_t g;
-  slab_prepare<double, EpiKktRows, B200_STAGE_TMA != 0>();
-  slab_prepare<double, EpiKktCols, false>();
-  slab_prepare<double, EpiRayRows, B200_STAGE_TMA != 0>();
   capturing_ = true;
   capture_count_ = 0;
   auto capture_scope = std::make_unique<CaptureScope>();  // no device-wide syncs elsewhere meanwhile
   B200_CHECK(cudaStreamBeginCapture(st_, cudaStreamCaptureModeThreadLocal));
-  clear_maxima();
-  launch_kkt_scaled<T>(xc, yc);  // KKT of the current point -> res2_
-  B200_CHECK(cudaMemcpyAsync(res2_.get(), res_.get(), kNumSlots * sizeof(double), cudaMemcpyDeviceToDevice, st_));
-  clear_maxima();
-  launch_kkt_scaled<T>(v.dx.get(), v.dy.get());  // KKT of the average -> res_
-  if (variant >= 1) {  // Δ = z_k − z_{k−1}: axpby(1, x, −1, x_prev) (pdlp.cpp:83-85)
-    k_axpby<T><<<grid_for(n), kBlock, 0, st_>>>(n, static_cast<T>(1.0), xc, static_cast<T>(-1.0), xp);
-    k_axpby<T><<<grid_for(m), kBlock, 0, st_>>>(m, static_cast<T>(1.0), yc, static_cast<T>(-1.0), yp);
-    B200_LAUNCH_CHECK();
-    capture_count_ += 2;
-    launch_ray<T>(xp, yp, r1_.get(), d1_.get(), 0);
-  }
-  if (variant == 2) {  // the drift z − z0: copy + axpby(−1, x0, 1, ·) (pdlp.cpp:89-93)
-    k_diff<T><<<grid_for(n), kBlock, 0, st_>>>(n, xc, v.x0.get(), xp);
-    k_diff<T><<<grid_for(m), kBlock, 0, st_>>>(m, yc, v.y0.get(), yp);
-    B200_LAUNCH_CHECK();
-    capture_count_ += 2;
-    launch_ray<T>(xp, yp, r2_.get(), d2_.get(), 1);
-  }
-  B200_CHECK(cudaMemcpyAsync(hres_.get(), res_.get(), kNumSlots * sizeof(double), cudaMemcpyDeviceToHost, st_));
-  B200_CHECK(cudaMemcpyAsync(hres2_.get(), res2_.get(), kNumSlots * sizeof(double), cudaMemcpyDeviceToHost, st_));
+  if (variant == 0) launch_pdlp_check_kernels<T, 0>(phase);
+  else if (variant == 1) launch_pdlp_check_kernels<T, 1>(phase);
+  else launch_pdlp_check_kernels<T, 2>(phase);
   const cudaError_t e = cudaStreamEndCapture(st_, &g);
   capture_scope.reset();
   capturing_ = false;
@@ -1406,8 +1383,6 @@ EngineResult Engine::run_pdlp(const DeviceOutputs& out) {
   EngineResult R;
   setup();
   const long long mm = M_.m, nn = M_.n;
-  res2_.alloc(kNumSlots);
-  hres2_.alloc(kNumSlots);
   plan_dist_.add(rt_.get(), 0, nn, 0.0, SumOrder::kChunk64, res_.get() + kPx);
   plan_dist_.add(rt_.get() + 2 * nn, 0, mm, 0.0, SumOrder::kChunk64, res_.get() + kPy);
   plan_dist_.build(true, nullptr, st_);  // the distances enter ω: always the reference's order
@@ -1463,6 +1438,7 @@ EngineResult Engine::run_pdlp(const DeviceOutputs& out) {
   if (mixed_now_) pdlp_restart<float>(cur, false);  // x0 = xa = x, y0 = ya = y
   else pdlp_restart<double>(cur, false);
   const Kkt k0 = kkt_now(false);
+  clear_maxima();  // the first check finds them at zero
   if (fast_it_ < 0 && k0.rel_kkt() <= kFirstOrderFast) fast_it_ = 0;
   double restart_kkt = k0.rel_kkt(), last_candidate = 1e300;
   long long it = 0, inner = 0;

@@ -73,3 +73,26 @@ def test_decisions_are_the_oracles(shape, kind, steps, monkeypatch):
         assert np.array_equal(r.x, o.x) and np.array_equal(r.y, o.y) and r.objective == o.objective
     else:
         assert o.message.split(";")[0] in r.message
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("kind", [infeasible, unbounded])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_pdlp_verdicts_are_certified(shape, kind, precision):
+    """PDLP's check: the ray that it reports passes the gate's own certificate check on the host."""
+    lp = kind(*shape)
+    r = ps26119.solve_lp(lp.c, (lp.col_start, lp.row_index, lp.value), lp.row_lower, lp.row_upper, lp.col_lower,
+                         lp.col_upper, algorithm="pdlp", precision=precision, iteration_limit=64000,
+                         engine={"presolve": False})
+    assert r.status == (ps26119.INFEASIBLE if kind is infeasible else ps26119.UNBOUNDED), r.message
+    assert r.check == "PASS", r.message
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+def test_pdlp_optimum(shape):
+    """PDLP's KKT statistics decide when it ends: its optimum is r²HPDHG's, within both tolerances."""
+    lp = feasible(*shape)
+    args = (lp.c, (lp.col_start, lp.row_index, lp.value), lp.row_lower, lp.row_upper, lp.col_lower, lp.col_upper)
+    a, b = (ps26119.solve_lp(*args, algorithm=alg, tolerance=1e-7, engine={"presolve": False}) for alg in ("pdlp", "r2hpdhg"))
+    assert a.status == b.status == ps26119.OPTIMAL and a.check == b.check == "PASS"
+    assert abs(a.objective - b.objective) <= 1e-6 * (1.0 + abs(b.objective))
