@@ -1101,9 +1101,14 @@ void BatchEngine::finish_slots(const std::vector<Finished>& done) {
   std::vector<double> ho(f);
   B200_CHECK(cudaMemcpyAsync(ho.data(), obj.get(), f * sizeof(double), cudaMemcpyDeviceToHost, st_));
   std::vector<StagedCopy> back;
+  parallel_ranges(F, [&](long long b, long long e) {  // fresh pages, on the host threads
+    for (long long k = b; k < e; ++k) {
+      BatchOutcome& o = *done[static_cast<std::size_t>(k)].out;
+      o.x.resize(n), o.y.resize(m), o.z.resize(n);
+    }
+  }, 2);
   for (std::size_t k = 0; k < f; ++k) {
     BatchOutcome& o = *done[k].out;
-    o.x.resize(n), o.y.resize(m), o.z.resize(n);
     back.push_back({x.get() + k * n, o.x.data(), n * sizeof(double)});
     back.push_back({y.get() + k * m, o.y.data(), m * sizeof(double)});
     back.push_back({z.get() + k * n, o.z.data(), n * sizeof(double)});

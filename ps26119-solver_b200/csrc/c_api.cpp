@@ -616,28 +616,35 @@ extern "C" int ps26119_solve_batch(int num_rows, int num_cols, int sense, double
     if (const char* err = apply_engine_options(engine, o)) return fail(PS26119_INVALID_ARGUMENT, err);
     std::vector<Scenario> sc(static_cast<std::size_t>(num_scenarios));
     auto take = [](const double* a, int len) { return a ? std::vector<double>(a, a + len) : std::vector<double>(); };
-    for (int k = 0; k < num_scenarios; ++k) {
-      const ps26119_scenario& s = scenarios[k];
-      sc[k].obj = take(s.obj, num_cols);
-      sc[k].col_lower = take(s.col_lower, num_cols);
-      sc[k].col_upper = take(s.col_upper, num_cols);
-      sc[k].row_lower = take(s.row_lower, num_rows);
-      sc[k].row_upper = take(s.row_upper, num_rows);
-    }
+    parallel_ranges(num_scenarios, [&](long long b, long long e) {
+      for (long long k = b; k < e; ++k) {
+        const ps26119_scenario& s = scenarios[k];
+        Scenario& to = sc[static_cast<std::size_t>(k)];
+        to.obj = take(s.obj, num_cols);
+        to.col_lower = take(s.col_lower, num_cols);
+        to.col_upper = take(s.col_upper, num_cols);
+        to.row_lower = take(s.row_lower, num_rows);
+        to.row_upper = take(s.row_upper, num_rows);
+      }
+    }, 2);
     const std::vector<Solution> sols = solve_batch(m, sc, o);
     long long launches = 0;
     for (int k = 0; k < num_scenarios; ++k) {
       const Solution& s = sols[k];
       fill(s, &results[k]);
       launches = std::max(launches, s.engine_result.kernel_launches);
-      const std::size_t ok = static_cast<std::size_t>(k);
-      if (x && s.x.size() == static_cast<std::size_t>(num_cols))
-        std::copy(s.x.begin(), s.x.end(), x + ok * num_cols);
-      if (y && s.y.size() == static_cast<std::size_t>(num_rows))
-        std::copy(s.y.begin(), s.y.end(), y + ok * num_rows);
-      if (z && s.z.size() == static_cast<std::size_t>(num_cols))
-        std::copy(s.z.begin(), s.z.end(), z + ok * num_cols);
     }
+    parallel_ranges(num_scenarios, [&](long long b, long long e) {
+      for (std::size_t k = static_cast<std::size_t>(b); k < static_cast<std::size_t>(e); ++k) {
+        const Solution& s = sols[k];
+        if (x && s.x.size() == static_cast<std::size_t>(num_cols))
+          std::copy(s.x.begin(), s.x.end(), x + k * num_cols);
+        if (y && s.y.size() == static_cast<std::size_t>(num_rows))
+          std::copy(s.y.begin(), s.y.end(), y + k * num_rows);
+        if (z && s.z.size() == static_cast<std::size_t>(num_cols))
+          std::copy(s.z.begin(), s.z.end(), z + k * num_cols);
+      }
+    }, 2);
     g_stats = ps26119_stats{};
     g_stats.kernel_launches = launches;
     g_stats.m = num_rows, g_stats.n = num_cols, g_stats.nnz = nnz;

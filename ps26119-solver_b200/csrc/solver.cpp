@@ -13,10 +13,12 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <exception>
 #include <mutex>
 #include <new>
 #include <sstream>
 #include <stdexcept>
+#include <system_error>
 #include <thread>
 
 namespace b200 {
@@ -1537,20 +1539,11 @@ Solution solve(const Model& model, const Options& options) {  // solve.cpp:194-2
 }
 
 // ============================================================ batch (batch.cpp:129-441)
-std::vector<Solution> solve_batch(const Model& base, const std::vector<Scenario>& scenarios, const Options& options) {
+namespace {
+std::vector<Solution> run_batch(const Model& base, const std::vector<Scenario>& scenarios, const Options& options) {
   const auto t0 = clock_t_::now();
   const int K = static_cast<int>(scenarios.size());
   std::vector<Solution> out(K);
-  {  // fingerprints of the scenario models (batch.cpp:113-127): the base with the scenario's vectors
-    const std::vector<std::uint64_t> fp = scenario_fingerprints(base, scenarios);
-    for (int k = 0; k < K; ++k) {
-      char buf[17];
-      std::snprintf(buf, sizeof buf, "%016llx", static_cast<unsigned long long>(fp[k]));
-      out[k].model_fingerprint = buf;
-      out[k].engine = "r2hpdhg-batch";
-      out[k].precision = "fp64";
-    }
-  }
   auto fail_all = [&](const std::string& why) {
     for (auto& s : out) s.status = Status::NotSolved, s.message = why;
     return out;
@@ -1561,30 +1554,37 @@ std::vector<Solution> solve_batch(const Model& base, const std::vector<Scenario>
     const int m = base.num_rows, n = base.num_cols;
     std::vector<BatchScenarioView> views(K);
     std::vector<int> slots;
-    for (int k = 0; k < K; ++k) {  // per-scenario validation (batch.cpp:154-181)
-      const Scenario& s = scenarios[k];
-      bool ok = true;
-      auto pick = [&](const std::vector<double>& v, const std::vector<double>& dflt, std::size_t len) {
-        if (v.empty()) return dflt.data();
-        ok = ok && v.size() == len;
-        return v.data();
-      };
-      BatchScenarioView& vw = views[k];
-      vw.c = pick(s.obj, base.obj, n);
-      vw.col_lower = pick(s.col_lower, base.col_lower, n);
-      vw.col_upper = pick(s.col_upper, base.col_upper, n);
-      vw.row_lower = pick(s.row_lower, base.row_lower, m);
-      vw.row_upper = pick(s.row_upper, base.row_upper, m);
-      for (int j = 0; ok && j < n; ++j)
-        ok = std::isfinite(vw.c[j]) && !std::isnan(vw.col_lower[j]) && !std::isnan(vw.col_upper[j]);
-      for (int i = 0; ok && i < m; ++i) ok = !std::isnan(vw.row_lower[i]) && !std::isnan(vw.row_upper[i]);
-      bool crossed = false;
-      for (int j = 0; ok && !crossed && j < n; ++j) crossed = vw.col_lower[j] > vw.col_upper[j];
-      for (int i = 0; ok && !crossed && i < m; ++i) crossed = vw.row_lower[i] > vw.row_upper[i];
-      if (!ok) {
+    std::vector<char> good(K), cross(K);
+    parallel_ranges(K, [&](long long kb, long long ke) {
+      for (std::size_t k = static_cast<std::size_t>(kb); k < static_cast<std::size_t>(ke); ++k) {
+        // per-scenario validation (batch.cpp:154-181)
+        const Scenario& s = scenarios[k];
+        bool ok = true;
+        auto pick = [&](const std::vector<double>& v, const std::vector<double>& dflt, std::size_t len) {
+          if (v.empty()) return dflt.data();
+          ok = ok && v.size() == len;
+          return v.data();
+        };
+        BatchScenarioView& vw = views[k];
+        vw.c = pick(s.obj, base.obj, n);
+        vw.col_lower = pick(s.col_lower, base.col_lower, n);
+        vw.col_upper = pick(s.col_upper, base.col_upper, n);
+        vw.row_lower = pick(s.row_lower, base.row_lower, m);
+        vw.row_upper = pick(s.row_upper, base.row_upper, m);
+        for (int j = 0; ok && j < n; ++j)
+          ok = std::isfinite(vw.c[j]) && !std::isnan(vw.col_lower[j]) && !std::isnan(vw.col_upper[j]);
+        for (int i = 0; ok && i < m; ++i) ok = !std::isnan(vw.row_lower[i]) && !std::isnan(vw.row_upper[i]);
+        bool crossed = false;
+        for (int j = 0; ok && !crossed && j < n; ++j) crossed = vw.col_lower[j] > vw.col_upper[j];
+        for (int i = 0; ok && !crossed && i < m; ++i) crossed = vw.row_lower[i] > vw.row_upper[i];
+        good[k] = ok, cross[k] = crossed;
+      }
+    }, 2);
+    for (int k = 0; k < K; ++k) {
+      if (!good[k]) {
         out[k].status = Status::NotSolved;
         out[k].message = "scenario has wrong vector sizes or non-finite data";
-      } else if (crossed) {
+      } else if (cross[k]) {
         out[k].status = Status::Infeasible;
         out[k].message = "bounds cross: scenario has a lower bound above its upper bound";
       } else {
@@ -1617,6 +1617,43 @@ std::vector<Solution> solve_batch(const Model& base, const std::vector<Scenario>
   } catch (const std::exception& e) {
     const std::string what = e.what();
     return fail_all(what.rfind("no CUDA device", 0) == 0 ? "CUDA backend unavailable: " + what : what);
+  }
+  return out;
+}
+}  // namespace
+
+// The fingerprints of the scenario models (batch.cpp:113-127: the base with the scenario's vectors) take as
+// long as the device's setup: they are made beside it.
+std::vector<Solution> solve_batch(const Model& base, const std::vector<Scenario>& scenarios, const Options& options) {
+  std::vector<std::uint64_t> fp;
+  std::exception_ptr err;
+  auto make = [&] {
+    try {
+      fp = scenario_fingerprints(base, scenarios);
+    } catch (...) {
+      err = std::current_exception();
+    }
+  };
+  struct Joined {
+    std::thread t;
+    ~Joined() {
+      if (t.joinable()) t.join();
+    }
+  } side;
+  try {
+    side.t = std::thread(make);
+  } catch (const std::system_error&) {
+    make();
+  }
+  std::vector<Solution> out = run_batch(base, scenarios, options);
+  if (side.t.joinable()) side.t.join();
+  if (err) std::rethrow_exception(err);
+  for (std::size_t k = 0; k < out.size(); ++k) {
+    char buf[17];
+    std::snprintf(buf, sizeof buf, "%016llx", static_cast<unsigned long long>(fp[k]));
+    out[k].model_fingerprint = buf;
+    out[k].engine = "r2hpdhg-batch";
+    out[k].precision = "fp64";
   }
   return out;
 }
