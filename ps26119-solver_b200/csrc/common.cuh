@@ -369,6 +369,10 @@ inline int sm_count() {
   return v;
 }
 
+__device__ __forceinline__ unsigned smem_u32(const void* p) {
+  return static_cast<unsigned>(__cvta_generic_to_shared(p));
+}
+
 // Programmatic dependent launch (sm_90+): a kernel launched with the programmatic-serialisation
 // attribute may start while the kernel before it in the stream is still running; it must not
 // touch that kernel's outputs (or anything a kernel still running may read or write) before

@@ -13,9 +13,9 @@
 // Everything is in the kernels' order and arithmetic, so α and β² are the same bits.
 //
 // What bounds it: about ten trips through L2 a step (two half-steps, and four per sum) and the two walks,
-// some 400 cycles for every binade that the sums pass. Measured, Lanczos of 1k random rows 2.3 -> 1.3 ms,
-// 10k 5.6 -> 3.3, staircase T = 168 16.5 -> 9.5 against six launches a step (with the faster walk in both,
-// 10k rows 3.6 ms of setup against 2.8).
+// one x_commit for every binade that the sums pass. Measured, Lanczos of 1k random rows 1.07 against 1.26 ms
+// in six launches a step, 10k 1.65 / 1.88, staircase T = 168 (389 steps) 10.1 / 13.3 (before the walk's steps
+// were shortened in both forms 1.3 / 2.3, 3.3 / 5.6 with 93 steps, 9.5 / 16.5 with 285).
 #pragma once
 
 #include "reduce.cuh"
@@ -94,7 +94,7 @@ __device__ __forceinline__ double lanczos_sum(const LanczosArgs& p, LanczosShare
     for (int off = 16; off > 0; off >>= 1) s0 += __shfl_xor_sync(kFull, s0, off);
     // the chain's first run starts at zero: its terms are added here, while the others are summarised
     XSummary T = sh.tile0 + q == 0 ? x_start(x_add(p.terms, from + a, from + b, 0.0, sh.add))
-                                   : x_summary(x_tile_full(term, a, b, before + s0));
+                                   : x_summary(x_tile_full(x_terms(term, a, b), before + s0));
     T.fast.first = from + a, T.fast.len = b - a;
     if (lane == 0) x_leave(T, p.fast + sh.tile0 + q, p.full + sh.tile0 + q);
   }
@@ -110,12 +110,10 @@ __device__ __forceinline__ double lanczos_sum(const LanczosArgs& p, LanczosShare
     const int all = sh.tiles;
     double r = 0.0;
     // the next round's summaries are on their way while one is walked
-    auto fast_of = [&](int k) { return k + lane < all ? x_load(p.fast + k + lane) : x_no_fast(); };
-    XFast next = fast_of(32);
-    XRound R = x_round(fast_of(0), p.full + lane, lane < all);
+    auto round = [&](int k) { return x_round(p.fast + k + lane, p.full + k + lane, k + lane < all); };
+    XRound R = round(0);
     for (int k0 = 0; k0 < all; k0 += 32) {
-      const XRound N = x_round(next, p.full + k0 + 32 + lane, k0 + 32 + lane < all);
-      next = fast_of(k0 + 64);
+      const XRound N = round(k0 + 32);
       r = x_walk_lanes(r, R, min(32, all - k0), [&](int k, double st) {
         const int a = __shfl_sync(kFull, R.fast.first, k), len = __shfl_sync(kFull, R.fast.len, k);
         return x_add(p.terms, a, a + len, st, sh.add);
@@ -213,10 +211,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_resident_lanczos(const __grid_c
 }
 
 // Past this many columns the walks over one run per 256 of them outweigh the launches saved (the kernels'
-// form composes groups of 32): setup of 40k random rows (60,000 columns) 5.2 against 5.9 ms, of the
-// staircase T = 720 (43,200) 21.1 against 21.7; of 60k rows (90,000) 6.5 against 5.2, of T = 1200 (72,000)
-// 27.3 against 22.3.
-constexpr long long kLanczosColumns = 61440;
+// form composes groups of 32): the steps of 20k random rows (30,000 columns) take 1.78 against 1.88 ms, of
+// the staircase T = 360 (21,600) 12.4 against 13.9; of 30k rows (45,000) 2.34 against 2.24, of T = 720
+// (43,200) 14.8 against 14.3, of 60k rows (90,000) 4.4 against 2.8.
+constexpr long long kLanczosColumns = 40960;
 // Columns a block: few blocks leave SMs to other solves, many make a longer walk and wider exchanges.
 // Setup of 30k random rows with 120 / 224 / 448 / 896 columns a block 4.0 / 4.4 / 3.8 / 4.6 ms, staircase
 // T = 720 19.7 / 20.4 / 18.6 / 24.3; 16 requests' setups side by side 41 / 33 / 30 / 29.

@@ -61,12 +61,12 @@ __device__ __forceinline__ double block_sum_fixed(double v, double* sh) {
 //             start (the approximate sums of the chain's earlier tiles), then the tile's XRun (change of
 //             S, bounds of its running value, parity after, per parity before): each lane adds its terms
 //             in fp64 to an approximate start of either parity, and the differences of the sums' bits are
-//             the changes of S. A tile whose running sum
-//             changes binade once is summarised in three parts: the run before the term that changes it,
-//             that term, the run after it in the new grid. The block that finishes last of a group of
-//             kXGroup tiles composes the tiles' summaries into the group's, of the same form. The block
-//             that finishes last of a chain's walks the chain with the EXACT s, with one warp: a run of
-//             groups is committed as s ← (S0 + K[S0 mod 2])·u as far as s = S0·u lies in their binade and
+//             the changes of S. A tile whose running sum changes binade once is summarised in three parts:
+//             the run before the term that changes it, that term, the run after it in the new grid. The
+//             block that finishes last of a group of kXGroup tiles composes the tiles' summaries into the
+//             group's, of the same form (the first group's start is known, so it is walked instead, as
+//             below, to its exact sum). The block that finishes last of a chain's walks the chain with the
+//             EXACT s, with one warp: a run of groups is committed as s ← (S0 + K[S0 mod 2])·u as far as s = S0·u lies in their binade and
 //             every running S provably stays within [2^52 + 1, 2^53 − 1] (then each exact partial sum
 //             lies inside the binade, at least u/2 from its ends, and rounds to that grid); a group that
 //             changes binade is committed by its three parts; any other one is walked by its tiles in the
@@ -78,12 +78,19 @@ __device__ __forceinline__ double block_sum_fixed(double v, double* sh) {
 // What bounds it: latency. A dependent fp64 addition takes 8.3 cycles, 10.4 with its operand from
 // shared memory, so a tile added one by one takes 1.4 us; the first one's terms are added while the others
 // are summarised, and the few tiles that cross a binade more than once cost that in the walk. Its other
-// steps are one check over 32 summaries held by the warp's lanes, and a hand-over per crossing, on
-// integers. Tiles of 256 terms, one warp's, keep the tiles that must be added one by one cheap. Measured,
-// 15,000 terms: 14 us a launch; 18.5 with the terms in units of u by division and rounding, every summary
-// read in full and the first tile left to the walk; 24 with summaries scanned anew in shared memory at
-// every crossing; three launches over tiles of 2,048 terms, the first walked in windows with a scan and a
-// restart per crossing, took 68 us.
+// steps are one check over 32 summaries held by the warp's lanes, and at a crossing one lane's x_commit, on
+// integers and without a branch, run by every lane before the warp knows which one it is: a warp alone takes
+// 5 or 6 cycles for an instruction, so a step is as long as its longest chain of them. Tiles of 256 terms,
+// one warp's, keep the tiles that must be added one by one cheap. The first group, where most binades are
+// crossed, is walked by its own last block, beside the other groups' composition. Of 14 us for the 525,600
+// terms of the staircase T = 8760 the tiles take 5, the first group 2.5, the count of groups 1, the walk 4.5.
+// Measured, 15,000 / 525,600 / 1.5M uniform terms, one launch by itself from cold caches: 16.8 / 18.5 / 33.8
+// us; 19.3 / 25.1 / 38.9 with the first group in the walk, commits with branches after the ballot, each
+// round's summaries loaded when it began and ties composed pair by pair (Lanczos on T = 8760 23.0 against
+// 28.5 ms, 1M random rows 12.9 / 14.5, 100k 6.6 / 8.4). The forms before: 15,000 terms 18.5 against then 14
+// us with the terms in units of u by division and rounding, every summary read in full and the first tile
+// left to the walk; 24 with summaries scanned anew in shared memory at every crossing; three launches over
+// tiles of 2,048 terms, the first walked in windows with a scan and a restart per crossing, took 68 us.
 constexpr int kXPer = 8;              // terms per lane
 constexpr int kXTile = 32 * kXPer;    // terms per tile (one warp)
 constexpr int kXGroup = 32;           // tiles per group (one warp lane each)
@@ -163,37 +170,6 @@ __device__ __forceinline__ XRun x_identity() {
   r.bad = r.ties = 0;
   return r;
 }
-// a then b (selects instead of indexing with a.out[p], so everything stays in registers)
-__device__ __forceinline__ XRun x_compose(const XRun& a, const XRun& b) {
-  XRun r;
-  r.bad = a.bad | b.bad;
-  r.ties = a.ties | b.ties;
-#pragma unroll
-  for (int p = 0; p < 2; ++p) {
-    const bool q = a.out[p] != 0;
-    const int bmn = q ? b.mn[1] : b.mn[0], bmx = q ? b.mx[1] : b.mx[0];
-    r.K[p] = a.K[p] + (q ? b.K[1] : b.K[0]);
-    r.mn[p] = bmn == INT_MAX ? a.mn[p] : min(a.mn[p], x_down(a.K[p]) + bmn);
-    r.mx[p] = bmx == INT_MIN ? a.mx[p] : max(a.mx[p], x_up(a.K[p]) + bmx);
-    r.out[p] = q ? b.out[1] : b.out[0];
-  }
-  return r;
-}
-__device__ __forceinline__ int x_pack(const XRun& v) { return v.out[0] | (v.out[1] << 1) | (v.bad << 2) | (v.ties << 3); }
-__device__ __forceinline__ void x_unpack(XRun& r, int packed) {
-  r.out[0] = packed & 1, r.out[1] = (packed >> 1) & 1, r.bad = (packed >> 2) & 1, r.ties = (packed >> 3) & 1;
-}
-__device__ __forceinline__ XRun x_shfl_down(const XRun& v, int off) {
-  XRun r;
-#pragma unroll
-  for (int p = 0; p < 2; ++p) {
-    r.K[p] = __shfl_down_sync(kFull, v.K[p], off);
-    r.mn[p] = __shfl_down_sync(kFull, v.mn[p], off);
-    r.mx[p] = __shfl_down_sync(kFull, v.mx[p], off);
-  }
-  x_unpack(r, __shfl_down_sync(kFull, x_pack(v), off));
-  return r;
-}
 // e = floor(log2 |v|) for a normal v whose ulp 2^(e−52) and 2^(52−e) are both normal doubles;
 // otherwise returns false.
 __device__ __forceinline__ bool x_binade(double v, int& e) {
@@ -218,38 +194,68 @@ __device__ __forceinline__ double x_double(long long S, int e) {
   const long long a = S < 0 ? -S : S;
   return __longlong_as_double((a & (kX52 - 1)) | (static_cast<long long>(e + 1023) << 52) | (S < 0 ? LLONG_MIN : 0LL));
 }
-// The composition of the warp's runs in lane order, valid in lane 0.
-__device__ __forceinline__ XRun x_warp_ordered(XRun r) {
+// The composition of the warp's runs in lane order (in every lane). A run's effect on the parity is to
+// keep it, to turn it, or to leave it at 0 or 1 whatever it was, so three ballots tell the parity before each
+// lane, and with it which K is that lane's; then it is one prefix sum for each parity at the start.
+__device__ __forceinline__ XRun x_warp_ordered(const XRun& r) {
   const int lane = threadIdx.x & 31;
-  if (!__any_sync(kFull, r.ties)) {
+  const bool any = r.mn[0] != INT_MAX;
+  XRun x;
+  x.bad = __any_sync(kFull, r.bad) ? 1 : 0;
+  x.ties = __any_sync(kFull, r.ties) ? 1 : 0;
+  if (!x.ties) {
     const long long K = r.K[0];
     long long inc = K;
+#pragma unroll
     for (int off = 1; off < 32; off <<= 1) {
       const long long o = __shfl_up_sync(kFull, inc, off);
       if (lane >= off) inc += o;
     }
-    const bool any = r.mn[0] != INT_MAX;
-    r.K[0] = r.K[1] = __shfl_sync(kFull, inc, 31);
-    r.mn[0] = r.mn[1] = __reduce_min_sync(kFull, any ? x_down(inc - K) + r.mn[0] : INT_MAX);
-    r.mx[0] = r.mx[1] = __reduce_max_sync(kFull, any ? x_up(inc - K) + r.mx[0] : INT_MIN);
-    r.out[0] = static_cast<int>(r.K[0] & 1), r.out[1] = r.out[0] ^ 1;
-    r.bad = __any_sync(kFull, r.bad) ? 1 : 0;
-    return r;
+    x.K[0] = x.K[1] = __shfl_sync(kFull, inc, 31);
+    x.mn[0] = x.mn[1] = __reduce_min_sync(kFull, any ? x_down(inc - K) + r.mn[0] : INT_MAX);
+    x.mx[0] = x.mx[1] = __reduce_max_sync(kFull, any ? x_up(inc - K) + r.mx[0] : INT_MIN);
+    x.out[0] = static_cast<int>(x.K[0] & 1), x.out[1] = x.out[0] ^ 1;
+    return x;
   }
+  const unsigned fixed = __ballot_sync(kFull, r.out[0] == r.out[1]), ones = __ballot_sync(kFull, r.out[0] & r.out[1]);
+  const unsigned turns = __ballot_sync(kFull, r.out[0] & ~r.out[1] & 1);
+  const unsigned below = (1u << lane) - 1u, known = fixed & below;
+  const int last = known ? 31 - __clz(known) : 0;
+  const unsigned after = known ? below & ~((2u << last) - 1u) : below;
+  const int turned = __popc(turns & after) & 1;
+  long long K[2], inc[2];
+  int q[2];
+#pragma unroll
+  for (int p = 0; p < 2; ++p) {
+    q[p] = (known ? static_cast<int>((ones >> last) & 1u) : p) ^ turned;  // the parity before this lane
+    K[p] = inc[p] = q[p] ? r.K[1] : r.K[0];
+  }
+#pragma unroll
   for (int off = 1; off < 32; off <<= 1) {
-    const XRun o = x_shfl_down(r, off);
-    if ((lane & (2 * off - 1)) == 0 && lane + off < 32) r = x_compose(r, o);
+    const long long o0 = __shfl_up_sync(kFull, inc[0], off), o1 = __shfl_up_sync(kFull, inc[1], off);
+    if (lane >= off) inc[0] += o0, inc[1] += o1;
   }
-  return r;
+#pragma unroll
+  for (int p = 0; p < 2; ++p) {
+    x.K[p] = __shfl_sync(kFull, inc[p], 31);
+    x.mn[p] = __reduce_min_sync(kFull, any ? x_down(inc[p] - K[p]) + (q[p] ? r.mn[1] : r.mn[0]) : INT_MAX);
+    x.mx[p] = __reduce_max_sync(kFull, any ? x_up(inc[p] - K[p]) + (q[p] ? r.mx[1] : r.mx[0]) : INT_MIN);
+    x.out[p] = __shfl_sync(kFull, q[p] ? r.out[1] : r.out[0], 31);
+  }
+  return x;
 }
 // Whether every S + r, mn ≤ r ≤ mx in units of 2^24, lies inside [2^52 + 1, 2^53 − 1] with the sign of S0
-// (S: S0 plus the change before the run).
+// (S: S0 plus the change before the run, |S| < 2^53; the answer for any other S means nothing).
 __device__ __forceinline__ bool x_inside(long long S0, long long S, int mn, int mx) {
-  const long long lo = (S >> kXShift) + mn, hi = (S >> kXShift) + 1 + mx;
-  constexpr long long a = (kX52 >> kXShift) + 1, b = (kX53 >> kXShift) - 1;
-  return S0 > 0 ? (lo >= a && hi <= b) : (lo >= -b && hi <= -a);
+  constexpr int a = static_cast<int>(kX52 >> kXShift) + 1, b = static_cast<int>(kX53 >> kXShift) - 1;
+  const int s = static_cast<int>(S >> kXShift);
+  return (s + mn >= (S0 < 0 ? -b : a)) & (s + 1 + mx <= (S0 < 0 ? -a : b));
 }
 
+// 16 bytes another block wrote into shared memory, behind the instructions that follow.
+__device__ __forceinline__ void x_copy16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
 // A struct of 16-byte words another block wrote, read past this SM's L1.
 template <class S>
 __device__ __forceinline__ S x_load(const S* p) {
@@ -399,10 +405,23 @@ __device__ __forceinline__ XRun x_compose_lanes(const XLane& r, bool in, bool an
   return x_warp_ordered(x);
 }
 
-// The summary of the terms t[a, b) (one tile, one warp; lane l holds kXPer terms from l·kXPer) for a chain
-// whose approximate sum before them is s0; valid in lane 0.
-__device__ __forceinline__ XTileAgg x_tile_full(const double* __restrict__ t, long long a, long long b, double s0) {
-  const int lane = threadIdx.x & 31;
+// One lane's terms of a tile t[a, b): kXPer from a + lane·kXPer, zeros past the end.
+struct XTerms {
+  double v[kXPer];
+  int cnt;
+};
+__device__ __forceinline__ XTerms x_terms(const double* __restrict__ t, long long a, long long b) {
+  const long long i0 = a + static_cast<long long>(threadIdx.x & 31) * kXPer;
+  XTerms r;
+  r.cnt = b - i0 >= kXPer ? kXPer : (b > i0 ? static_cast<int>(b - i0) : 0);
+#pragma unroll
+  for (int q = 0; q < kXPer; ++q) r.v[q] = q < r.cnt ? t[i0 + q] : 0.0;
+  return r;
+}
+// The summary of a tile (one warp, its terms in the lanes) for a chain whose approximate sum before it is s0;
+// valid in lane 0.
+__device__ __forceinline__ XTileAgg x_tile_full(XTerms t, double s0) {
+  const int lane = threadIdx.x & 31, cnt = t.cnt;
   XTileAgg g = x_no_full();
   int e0;
   if (!x_binade(s0, e0)) {  // uniform over the warp
@@ -410,14 +429,10 @@ __device__ __forceinline__ XTileAgg x_tile_full(const double* __restrict__ t, lo
     return g;
   }
   const bool flip = s0 < 0;
-  const long long i0 = a + static_cast<long long>(lane) * kXPer;
-  const int cnt = b - i0 >= kXPer ? kXPer : (b > i0 ? static_cast<int>(b - i0) : 0);
-  double v[kXPer];
+  double(&v)[kXPer] = t.v;
 #pragma unroll
-  for (int q = 0; q < kXPer; ++q) {
-    v[q] = q < cnt ? t[i0 + q] : 0.0;
+  for (int q = 0; q < kXPer; ++q)
     if (flip) v[q] = -v[q];
-  }
   double run = 0.0;
 #pragma unroll
   for (int q = 0; q < kXPer; ++q) run += v[q];
@@ -500,55 +515,52 @@ __device__ __forceinline__ void x_leave(const XSummary& S, XFast* fast, XTileAgg
   if (S.fast.kind == kXFull) *full = S.full;
 }
 
-// Commits a whole summary, its change of binade included, to the sum S·2^(e − 52); returns false (nothing
-// changed) where a running S could leave its binade.
+// Commits a whole summary, its change of binade included, to the sum S·2^(e − 52); returns false (S and e
+// mean nothing) where a running S could leave its binade. Without a branch: a chain of about fifty
+// instructions, which every lane can run for its own summary.
 __device__ __forceinline__ bool x_commit(long long& S, int& e, const XTileAgg& T) {
-  if (T.e != e) return false;
-  bool odd = (S & 1) != 0;
-  long long R = S;
-  if (T.pre.mn[0] != INT_MAX) {
-    if (!x_inside(S, S, odd ? T.pre.mn[1] : T.pre.mn[0], odd ? T.pre.mx[1] : T.pre.mx[0])) return false;
-    R += odd ? T.pre.K[1] : T.pre.K[0];
-  }
-  int e2 = e;
-  if (T.split) {
-    const double s = x_double(R, e) + T.at;  // the term that changes the binade, as the chain adds it
-    if (!x_binade(s, e2) || e2 != T.e1) return false;
-    R = x_int(s);
-    if (T.suf.mn[0] != INT_MAX) {
-      odd = (R & 1) != 0;
-      if (!x_inside(R, R, odd ? T.suf.mn[1] : T.suf.mn[0], odd ? T.suf.mx[1] : T.suf.mx[0])) return false;
-      R += odd ? T.suf.K[1] : T.suf.K[0];
-    }
-  }
-  S = R, e = e2;
-  return true;
+  const bool odd = (S & 1) != 0;
+  bool ok = (T.e == e) & ((T.pre.mn[0] == INT_MAX) |
+                          x_inside(S, S, odd ? T.pre.mn[1] : T.pre.mn[0], odd ? T.pre.mx[1] : T.pre.mx[0]));
+  // the term that changes the binade, as the chain adds it (no split: the term is zero)
+  const double s = x_double(S + (odd ? T.pre.K[1] : T.pre.K[0]), e) + T.at;
+  const int e1 = T.split ? T.e1 : T.e;
+  e = ((__double2hiint(s) >> 20) & 0x7ff) - 1023;
+  ok = ok & (e == e1);
+  const long long R = x_int(s);
+  const bool odd1 = (R & 1) != 0;
+  ok = ok & ((T.suf.mn[0] == INT_MAX) |
+             x_inside(R, R, odd1 ? T.suf.mn[1] : T.suf.mn[0], odd1 ? T.suf.mx[1] : T.suf.mx[0]));
+  S = R + (odd1 ? T.suf.K[1] : T.suf.K[0]);
+  return ok;
 }
 
-// What one lane holds of a walk's round of up to 32 summaries.
+// What one lane holds of a walk's round of up to 32 summaries; `full` means something where the kind is
+// kXFull (it is read whatever the kind, so that it need not wait for it).
 struct XRound {
   XFast fast;
   XTileAgg full;
 };
-__device__ __forceinline__ XRound x_round(const XFast& f, const XTileAgg* full, bool here) {
+__device__ __forceinline__ XRound x_round(const XFast* fast, const XTileAgg* full, bool here) {
   XRound r;
-  r.fast = f;
-  r.full = x_no_full();
-  if (here && f.kind == kXFull) r.full = x_load(full);
+  r.fast = x_no_fast(), r.full = x_no_full();
+  if (here) r.fast = x_load(fast), r.full = x_load(full);
   return r;
 }
 
 // One warp walks cnt consecutive summaries, lane l holding the l-th, with the exact s. other(k, s) returns
 // the sum after the k-th where its summary cannot be committed. A step commits all plain summaries up to
-// the first that is not one, not in s's binade, or whose running S would leave it; that one is committed
-// by the lane that holds it. Without ties a run's K does not depend on what came before, so one prefix sum
-// over the lanes serves all steps (across a change of grid the sum means nothing, but a step only uses
-// differences within one).
+// the first that is not one, not in s's binade, or whose running S would leave it, and then that one by
+// itself. Without ties a run's K does not depend on what came before, so one prefix sum over the lanes
+// serves all steps (across a change of grid the sum means nothing, but a step only uses differences within
+// one); and every lane commits its own summary to the sum that the step has there, if it gets that far,
+// before the warp knows which lane that is: a step is then one x_commit long.
 template <class F>
 __device__ __forceinline__ double x_walk_lanes(double s, const XRound& G, int cnt, F&& other) {
   const int lane = threadIdx.x & 31;
   const bool here = lane < cnt;
   const bool plain = here && G.fast.kind == kXPlain, empty = plain && G.fast.mn == INT_MAX;
+  const bool full = here && G.fast.kind == kXFull, start = here && G.fast.kind == kXStart;
   long long inc = plain ? G.fast.K : 0;
 #pragma unroll
   for (int off = 1; off < 32; off <<= 1) {
@@ -560,49 +572,75 @@ __device__ __forceinline__ double x_walk_lanes(double s, const XRound& G, int cn
   bool have = x_binade(s, e);
   long long S = x_int(s), base = 0;  // base: `before` at lane j
   while (j < cnt) {
-    const bool ok = plain && have && (empty || (G.fast.e == e && x_inside(S, S + before - base, G.fast.mn, G.fast.mx)));
+    const long long Sl = S + (before - base);  // the sum before this lane's summary
+    const bool ok = plain & have & (empty | ((G.fast.e == e) & x_inside(S, Sl, G.fast.mn, G.fast.mx)));
+    long long S2 = Sl;
+    int e2 = e;
+    const bool can = x_commit(S2, e2, G.full) & full & have;
     const unsigned stop = __ballot_sync(kFull, lane >= j && !ok);
     const int f = stop ? __ffs(stop) - 1 : 32;
-    if (f > j) S += __shfl_sync(kFull, inc, f - 1) - base;
-    if (f >= cnt) break;
-    // lane f, on its own
-    long long S2 = S;
-    int e2 = e, way = 0;  // 1: committed
-    if (lane == f) {
-      if (G.fast.kind == kXFull && have) way = x_commit(S2, e2, G.full) ? 1 : 0;
-      if (G.fast.kind == kXStart) way = 2, S2 = G.fast.K;
+    if (f >= cnt) {
+      S = __shfl_sync(kFull, Sl + (plain ? G.fast.K : 0), cnt - 1);
+      break;
     }
-    way = __shfl_sync(kFull, way, f);
-    S2 = __shfl_sync(kFull, S2, f);
+    // lane f, on its own. way: 1 committed, 2 the chain's start, 0 neither
+    const int way = __shfl_sync(kFull, can ? 1 : (start ? 2 : 0), f);
+    S = __shfl_sync(kFull, can ? S2 : (start ? G.fast.K : Sl), f);
+    const int ef = __shfl_sync(kFull, e2, f);
+    base = __shfl_sync(kFull, inc, f);
+    j = f + 1;
     if (way == 1) {
-      S = S2, e = __shfl_sync(kFull, e2, f);
+      e = ef;
     } else {
-      s = way == 2 ? __longlong_as_double(S2) : other(f, have ? x_double(S, e) : s);
+      s = way == 2 ? __longlong_as_double(S) : other(f, have ? x_double(S, e) : s);
       have = x_binade(s, e);
       S = x_int(s);
     }
-    j = f + 1;
-    base = __shfl_sync(kFull, inc, f);
   }
   return have ? x_double(S, e) : s;
 }
 
-// The chain c from its tiles' and groups' summaries (one warp).
+// The cnt tiles of chain c from its tile t0 on, from their summaries (one warp), with the exact s before them.
+__device__ __forceinline__ double x_walk_tiles(const XChain& c, int t0, int cnt, double s, const XFast* tf, const XTileAgg* ag,
+                                               double* sh) {
+  const int lane = threadIdx.x & 31, ti = c.tile0 + t0;
+  const XRound T = x_round(tf + ti + lane, ag + ti + lane, lane < cnt);
+  return x_walk_lanes(s, T, cnt, [&](int k, double st) {
+    long long a, b;
+    x_tile_range(c, ti + k, a, b);
+    return x_add(c.t, a, b, st, sh);
+  });
+}
+__device__ __forceinline__ int x_group_tiles(const XChain& c, int g) {
+  return min(kXGroup, c.ntiles - g * kXGroup);
+}
+// The chain c from its groups' summaries (one warp); the first one is its exact sum there. The next round's
+// summaries come into shared memory while one is walked.
 __device__ __forceinline__ double x_walk(const XChain& c, const XFast* tf, const XTileAgg* ag, const XFast* gf,
-                                         const XTileAgg* gg, double* sh) {
+                                         const XTileAgg* gg, XRound (*stage)[32], double* sh) {
   const int lane = threadIdx.x & 31;
+  const auto fetch = [&](int g0) {
+    if (g0 + lane < c.ngroups) {
+      XRound* r = &stage[(g0 >> 5) & 1][lane];
+      const char* f = reinterpret_cast<const char*>(gf + c.group0 + g0 + lane);
+      const char* a = reinterpret_cast<const char*>(gg + c.group0 + g0 + lane);
+#pragma unroll
+      for (unsigned k = 0; k < sizeof(XFast); k += 16) x_copy16(reinterpret_cast<char*>(&r->fast) + k, f + k);
+#pragma unroll
+      for (unsigned k = 0; k < sizeof(XTileAgg); k += 16) x_copy16(reinterpret_cast<char*>(&r->full) + k, a + k);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
   double s = c.init;
+  fetch(0);
   for (int g0 = 0; g0 < c.ngroups; g0 += 32) {
-    const int cntg = c.ngroups - g0 < 32 ? c.ngroups - g0 : 32, gi = c.group0 + g0;
-    const XRound G = x_round(lane < cntg ? x_load(gf + gi + lane) : x_no_fast(), gg + gi + lane, lane < cntg);
-    s = x_walk_lanes(s, G, cntg, [&](int g, double sg) {
-      const int t0 = (g0 + g) * kXGroup, cnt = c.ntiles - t0 < kXGroup ? c.ntiles - t0 : kXGroup, ti = c.tile0 + t0;
-      const XRound T = x_round(lane < cnt ? x_load(tf + ti + lane) : x_no_fast(), ag + ti + lane, lane < cnt);
-      return x_walk_lanes(sg, T, cnt, [&](int k, double st) {
-        long long a, b;
-        x_tile_range(c, ti + k, a, b);
-        return x_add(c.t, a, b, st, sh);
-      });
+    const int cnt = c.ngroups - g0 < 32 ? c.ngroups - g0 : 32;
+    fetch(g0 + 32);
+    asm volatile("cp.async.wait_group 1;" ::: "memory");  // this lane's own, of this round
+    XRound G = stage[(g0 >> 5) & 1][lane];
+    if (lane >= cnt) G.fast = x_no_fast(), G.full = x_no_full();
+    s = x_walk_lanes(s, G, cnt, [&](int g, double sg) {
+      return x_walk_tiles(c, (g0 + g) * kXGroup, x_group_tiles(c, g0 + g), sg, tf, ag, sh);
     });
   }
   return s;
@@ -614,8 +652,8 @@ __device__ __forceinline__ double x_walk(const XChain& c, const XFast* tf, const
 __device__ __forceinline__ XSummary x_group(const XFast* tf, const XTileAgg* ag, int cnt) {
   const int lane = threadIdx.x & 31;
   const bool here = lane < cnt;
-  const XRound R = x_round(here ? x_load(tf + lane) : x_no_fast(), ag + lane, here);
-  XTileAgg T = R.full;
+  const XRound R = x_round(tf + lane, ag + lane, here);
+  XTileAgg T = R.fast.kind == kXFull ? R.full : x_no_full();
   if (here && R.fast.kind == kXPlain) {
     T.e = R.fast.e;
     T.pre.K[0] = T.pre.K[1] = R.fast.K, T.pre.mn[0] = T.pre.mn[1] = R.fast.mn, T.pre.mx[0] = T.pre.mx[1] = R.fast.mx;
@@ -652,6 +690,9 @@ static __global__ void __launch_bounds__(32 * kXWarps) k_xwalk(const XChain* __r
                                                                unsigned* job_done, const int* skip) {
   __shared__ alignas(16) double sh_add[kXWarps][kXTile];
   __shared__ double sh_sum[kXWarps];
+  // the walk's two rounds: in the buffers of the block's other warps, which are done by then
+  static_assert(2 * 32 * sizeof(XRound) <= (kXWarps - 1) * kXTile * sizeof(double), "two rounds fit");
+  XRound(*stage)[32] = reinterpret_cast<XRound(*)[32]>(&sh_add[1][0]);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const bool tiled = static_cast<int>(blockIdx.x) < nblocks;
   const int ks = (static_cast<int>(blockIdx.x) - nblocks) * kXWarps + w;
@@ -675,6 +716,9 @@ static __global__ void __launch_bounds__(32 * kXWarps) k_xwalk(const XChain* __r
   };
   if (tiled) {
     const int k0 = (static_cast<int>(blockIdx.x) - c.block0) * kXWarps, k = k0 + w;
+    long long a, b;
+    x_tile_range(c, c.tile0 + k, a, b);
+    const XTerms mine_t = x_terms(c.t, a, b);  // none past the chain's last tile
     const double mine = lane < w && k0 + lane < c.ntiles ? stat[c.tile0 + k0 + lane] : 0.0;
     double pre = 0.0;  // the approximate sum before this block's tiles
     for (int q = threadIdx.x; q < k0; q += 32 * kXWarps) pre += stat[c.tile0 + q];
@@ -686,21 +730,22 @@ static __global__ void __launch_bounds__(32 * kXWarps) k_xwalk(const XChain* __r
     s0 += c.init;
     for (int q = 0; q < kXWarps; ++q) s0 += sh_sum[q];
     if (k < c.ntiles) {
-      long long a, b;
-      x_tile_range(c, c.tile0 + k, a, b);
       // the first tile's start is known: its terms are added here, while the other tiles are summarised
-      const XSummary T = k == 0 ? x_start(x_add(c.t, a, b, c.init, sh_add[0])) : x_summary(x_tile_full(c.t, a, b, s0));
+      const XSummary T = k == 0 ? x_start(x_add(c.t, a, b, c.init, sh_add[0])) : x_summary(x_tile_full(mine_t, s0));
       if (lane == 0) x_leave(T, tf + c.tile0 + k, ag + c.tile0 + k);
     }
-    __threadfence();
-    __syncthreads();
+    __syncthreads();  // last_of's fence then covers what the other warps left
     if (w != 0) return;
-    const int g = k0 / kXGroup, t0 = g * kXGroup, cnt = c.ntiles - t0 < kXGroup ? c.ntiles - t0 : kXGroup;
+    const int g = k0 / kXGroup, t0 = g * kXGroup, cnt = x_group_tiles(c, g);
     if (!last_of(group_done + c.group0 + g, (cnt + kXWarps - 1) / kXWarps)) return;
-    const XSummary G = x_group(tf + c.tile0 + t0, ag + c.tile0 + t0, cnt);
-    if (lane == 0) x_leave(G, gf + c.group0 + g, gg + c.group0 + g);
-    if (!last_of(chain_done + ci, c.ngroups)) return;
-    s = x_walk(c, tf, ag, gf, gg, sh_add[0]);
+    // the first group's start is known too, so it is walked here, while the others are summarised
+    if (g == 0) s = x_walk_tiles(c, 0, cnt, c.init, tf, ag, sh_add[0]);
+    if (c.ngroups > 1) {
+      const XSummary G = g == 0 ? x_start(s) : x_group(tf + c.tile0 + t0, ag + c.tile0 + t0, cnt);
+      if (lane == 0) x_leave(G, gf + c.group0 + g, gg + c.group0 + g);
+      if (!last_of(chain_done + ci, c.ngroups)) return;
+      s = x_walk(c, tf, ag, gf, gg, stage, sh_add[0]);
+    }
   } else {
     if (ci < 0) return;
     s = x_add(c.t, c.lo, c.hi, c.init, sh_add[w]);

@@ -84,9 +84,6 @@ struct SlabSmem {
 static __device__ unsigned int g_stage_timeouts;
 __device__ __forceinline__ void count_stage_timeout(unsigned* err) { atomicAdd(err ? err : &g_stage_timeouts, 1u); }
 
-__device__ __forceinline__ unsigned smem_u32(const void* p) {
-  return static_cast<unsigned>(__cvta_generic_to_shared(p));
-}
 __device__ __forceinline__ void mbar_init(unsigned long long* bar) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bar)) : "memory");
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");

@@ -15,7 +15,9 @@ pytestmark = pytest.mark.gpu
 MODELS = {"one_tile": lambda: g.random_lp(170, seed=2), "one_by_one": lambda: g.random_lp(680, seed=2),
           "tiles": lambda: g.random_lp(700, seed=2), "jumps": lambda: g.random_lp(30_011, seed=2),
           "long": lambda: g.staircase_lp(40, seed=3), "most_columns": lambda: g.random_lp(9_000, 61_440, 6, seed=2),
-          "too_many_columns": lambda: g.random_lp(9_000, 61_441, 6, seed=2), "holes": lambda: holes(300, 700),
+          "too_many_columns": lambda: g.random_lp(9_000, 61_441, 6, seed=2),
+          "most_in_one_launch": lambda: g.random_lp(9_000, 40_960, 6, seed=2),
+          "first_past_it": lambda: g.random_lp(9_000, 40_961, 6, seed=2), "holes": lambda: holes(300, 700),
           "one_column": lambda: holes(900, 6)}
 
 

@@ -41,3 +41,15 @@ def test_sum_is_sequential(kind, n):
         assert ps26119.ordered_sum(d.data_ptr(), n, init, "seq").hex() == seq(t, init).hex()
         parts = [seq(t[n * c // 64:n * (c + 1) // 64], 0.0) for c in range(64)]
         assert ps26119.ordered_sum(d.data_ptr(), n, init, "chunk64").hex() == seq(np.array(parts), init).hex()
+
+
+@pytest.mark.parametrize("kind", ["positive", "drift", "steps", "return"])
+@pytest.mark.parametrize("n", [524_288, 524_289, 800_001])
+def test_sum_over_rounds_of_groups(kind, n):  # rounds of 32 groups that take turns in two buffers
+    import torch
+    t = terms(kind, n)
+    d = torch.as_tensor(t, device="cuda")
+    torch.cuda.synchronize()
+    for init in (0.0, 3.0 * 2.0 ** 20):
+        want = float(np.add.accumulate(np.concatenate([[init], t]))[-1])
+        assert ps26119.ordered_sum(d.data_ptr(), n, init, "seq").hex() == want.hex()
