@@ -216,7 +216,8 @@ struct ScaledDevice {
     {
       unsigned long long init[2] = {0x7ff0000000000000ULL /* +inf */, 0ULL};
       B200_CHECK(cudaMemcpyAsync(keys.get(), init, sizeof init, cudaMemcpyHostToDevice, st));
-      if (nnz > 0) k_abs_range<<<grid_for(nnz), kBlock, 0, st>>>(nnz, a_v0.get(), keys.get(), keys.get() + 1);
+      if (nnz > 0)
+        k_abs_range<<<std::min(grid_for(nnz), 8 * sm_count()), kBlock, 0, st>>>(nnz, a_v0.get(), keys.get(), keys.get() + 1);
       B200_LAUNCH_CHECK();
       unsigned long long got[2];
       B200_CHECK(cudaMemcpyAsync(got, keys.get(), sizeof got, cudaMemcpyDeviceToHost, st));
@@ -235,10 +236,8 @@ struct ScaledDevice {
                                                    col_scale.get());
         B200_LAUNCH_CHECK();
       }
-      apply(row_scale.get(), col_scale.get(), st);
     }
-    for (int it = 0; it < so.ruiz_iterations; ++it) norm_step(true, st);  // scaling.cpp:81-88
-    if (so.pock_chambolle) norm_step(false, st);                          // scaling.cpp:89-96
+    scale_entries(so, st);
 
     sc.alloc(nn), scl.alloc(nn), scu.alloc(nn), srl.alloc(mm), sru.alloc(mm);
     k_scaled_cols<<<grid_for(nn), kBlock, 0, st>>>(n, sense, dm.c, dm.col_lower, dm.col_upper, col_scale.get(),
@@ -271,7 +270,7 @@ struct ScaledDevice {
       b_norm = std::sqrt(b2);
       c_norm = std::sqrt(c2);
       B200_CHECK(cudaMemsetAsync(keys.get(), 0, sizeof(unsigned long long), st));
-      k_absmax<<<grid_for(nn), kBlock, 0, st>>>(static_cast<long long>(nn), dm.c, keys.get());
+      k_absmax<<<std::min(grid_for(nn), 8 * sm_count()), kBlock, 0, st>>>(static_cast<long long>(nn), dm.c, keys.get());
       B200_LAUNCH_CHECK();
       unsigned long long key = 0;
       B200_CHECK(cudaMemcpyAsync(&key, keys.get(), sizeof key, cudaMemcpyDeviceToHost, st));
@@ -504,23 +503,31 @@ struct ScaledDevice {
     B200_LAUNCH_CHECK();
   }
 
-  void apply(const double* rf, const double* cf, cudaStream_t st) {
-    k_apply_csr<<<grid_for(m), kBlock, 0, st>>>(m, a_rp.get(), a_col.get(), sa.get(), rf, cf);
-    k_apply_csc<<<grid_for(n), kBlock, 0, st>>>(n, M.col_start, t_ri.get(), sat.get(), rf, cf);
-    B200_LAUNCH_CHECK();
-  }
-
-  // One Ruiz (∞-norm) or Pock–Chambolle (1-norm, α = 1) step: factors 1/sqrt(norm), applied to
-  // Ã and Ãᵀ, accumulated into the scales.
-  void norm_step(bool inf_norm, cudaStream_t st) {
-    DevBuf<double>& rf = fac_m;
-    DevBuf<double>& cf = fac_n;
-    k_row_norm<<<grid_for(m), kBlock, 0, st>>>(m, a_rp.get(), sa.get(), inf_norm ? 1 : 0, tmp_m.get());
-    k_row_norm<<<grid_for(n), kBlock, 0, st>>>(n, M.col_start, sat.get(), inf_norm ? 1 : 0, tmp_n.get());
-    k_inv_sqrt_factor<<<grid_for(m), kBlock, 0, st>>>(m, tmp_m.get(), rf.get(), row_scale.get());
-    k_inv_sqrt_factor<<<grid_for(n), kBlock, 0, st>>>(n, tmp_n.get(), cf.get(), col_scale.get());
-    B200_LAUNCH_CHECK();
-    apply(rf.get(), cf.get(), st);
+  // The geometric means' factors (if there are any: the scales so far), then the Ruiz (∞-norm) steps
+  // (scaling.cpp:81-88) and the Pock–Chambolle (1-norm, α = 1) step (scaling.cpp:89-96): each step's factors
+  // 1/√norm, applied to Ã and Ãᵀ by the next step's launches, accumulated into the scales. A step reads the
+  // factors of the one before while it writes its own, so there are two buffers a side.
+  void scale_entries(const ScalingOptions& so, cudaStream_t st) {
+    double* rf[2] = {fac_m.get(), tmp_m.get()};
+    double* cf[2] = {fac_n.get(), tmp_n.get()};
+    int cur = 0;
+    bool pending = gm_applied;
+    if (pending) {
+      B200_CHECK(cudaMemcpyAsync(rf[0], row_scale.get(), sizeof(double) * m, cudaMemcpyDeviceToDevice, st));
+      B200_CHECK(cudaMemcpyAsync(cf[0], col_scale.get(), sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
+    }
+    auto step = [&](auto kernel) {
+      kernel<<<grid_for(m), kBlock, 0, st>>>(m, a_rp.get(), a_col.get(), sa.get(), rf[cur], cf[cur], rf[cur ^ 1],
+                                             row_scale.get());
+      kernel<<<grid_for(n), kBlock, 0, st>>>(n, M.col_start, t_ri.get(), sat.get(), cf[cur], rf[cur], cf[cur ^ 1],
+                                             col_scale.get());
+      B200_LAUNCH_CHECK();
+      cur ^= 1, pending = true;
+    };
+    for (int it = 0; it < so.ruiz_iterations; ++it)
+      step(pending ? &k_scale_step<true, RowNorm::kMax> : &k_scale_step<false, RowNorm::kMax>);
+    if (so.pock_chambolle) step(pending ? &k_scale_step<true, RowNorm::kSum> : &k_scale_step<false, RowNorm::kSum>);
+    if (pending) step(&k_scale_step<true, RowNorm::kNone>);
   }
 
   // Two sequential-order sums: terms over m (into tmp_m) and over n (into tmp_n).

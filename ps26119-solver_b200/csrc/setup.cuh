@@ -156,12 +156,28 @@ static __global__ void k_sort_long(const int* rp, const int* long_rows, const in
 }
 
 // ------------------------------------------------------------------ scaling kernels
+// Bound by bandwidth, and where a pass gathers the other side's factors by the gathers. A thread takes a row
+// and a few of its entries at a time, so that their loads and gathers are in flight together. Measured,
+// structure and scaling of 1M random rows (6M entries) / staircase T = 8760 / 1k random rows: 4.49 / 1.15 /
+// 0.71 ms with a loop of single entries, norms, factors and products in launches of their own and a block per
+// 256 entries in k_abs_range; 3.15 / 0.73 / 0.52 so (4, 6 and 8 entries at a time: 3.22, 3.84 and 4.40 on the
+// first). One launch on it, cold: a side's scaling step 59 us (the three before it about 100), a pass of
+// geometric means 37 (48), k_abs_range 21 (250).
+constexpr int kScaleAhead = 3;
+
+// The smallest and largest |v| over the entries that are not zero. Few blocks with many entries each, because
+// the two atomics of every warp go to the same two places.
 static __global__ void k_abs_range(long long nnz, const double* v, unsigned long long* amin_key,
                                    unsigned long long* amax_key) {
   double lo = INFINITY, hi = 0.0;
-  B200_FOR(k, nnz) {
-    const double a = fabs(v[k]);
-    if (v[k] != 0.0) lo = std_min(lo, a), hi = std_max(hi, a);
+  const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
+  for (long long k = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; k < nnz; k += kScaleAhead * stride) {
+    double x[kScaleAhead];
+#pragma unroll
+    for (int q = 0; q < kScaleAhead; ++q) x[q] = k + q * stride < nnz ? v[k + q * stride] : 0.0;
+#pragma unroll
+    for (int q = 0; q < kScaleAhead; ++q)
+      if (x[q] != 0.0) lo = std_min(lo, fabs(x[q])), hi = std_max(hi, fabs(x[q]));
   }
   warp_min_atomic_pos(amin_key, lo == INFINITY ? 0.0 : lo);
   warp_max_atomic(amax_key, hi);
@@ -176,53 +192,55 @@ static __global__ void k_gm_pass(int rows, const int* rp, const int* idx, const 
                           double* out) {
   B200_FOR(i, rows) {
     double lo = INFINITY, hi = 0.0;
-    for (int k = rp[i]; k < rp[i + 1]; ++k) {
-      const double v = fabs(val[k]) * other[idx[k]];
-      if (v > 0 && isfinite(v)) lo = std_min(lo, v), hi = std_max(hi, v);
+    const int end = rp[i + 1];
+    for (int k = rp[i]; k < end; k += kScaleAhead) {
+      double v[kScaleAhead];
+#pragma unroll
+      for (int q = 0; q < kScaleAhead; ++q) v[q] = k + q < end ? fabs(val[k + q]) * other[idx[k + q]] : 0.0;
+#pragma unroll
+      for (int q = 0; q < kScaleAhead; ++q)
+        if (v[q] > 0 && isfinite(v[q])) lo = std_min(lo, v[q]), hi = std_max(hi, v[q]);
     }
     if (hi > 0) out[i] = clampf_gm(1.0 / (sqrt(lo) * sqrt(hi)));
   }
 }
 
-// Per-row ∞-norm (max |a|) or 1-norm (Σ|a| in storage order) of a CSR (scaling.cpp:18-32).
-static __global__ void k_row_norm(int rows, const int* rp, const double* val, int inf_norm, double* out) {
+// One side's part of a scaling step, over the rows of a CSR (of A, or of Aᵀ for the columns): multiplies the
+// entries by the factors of the step before (kApply: val[k] *= mine_i · other_idx, the same product on both
+// sides), and makes this step's factor, 1/√ of the row's ∞-norm (kMax) or 1-norm in storage order (kSum) of
+// the entries as they are now (scaling.cpp:18-32, 81-96), into out_i and the row's scale. One pass over the
+// entries where the norm, its factor and the product took three launches and two passes.
+enum class RowNorm { kNone, kMax, kSum };
+template <bool kApply, RowNorm kNorm>
+__global__ void k_scale_step(int rows, const int* __restrict__ rp, const int* __restrict__ idx, double* __restrict__ val,
+                             const double* __restrict__ mine, const double* __restrict__ other, double* __restrict__ out,
+                             double* __restrict__ scale) {
   B200_FOR(i, rows) {
+    const double f = kApply ? mine[i] : 1.0;
+    const int end = rp[i + 1];
     double s = 0.0;
-    for (int k = rp[i]; k < rp[i + 1]; ++k) {
-      const double a = fabs(val[k]);
-      if (inf_norm) s = std_max(s, a);
-      else s += a;
+    for (int k = rp[i]; k < end; k += kScaleAhead) {
+      double v[kScaleAhead], g[kScaleAhead];
+#pragma unroll
+      for (int q = 0; q < kScaleAhead; ++q) {
+        const bool in = k + q < end;
+        v[q] = in ? val[k + q] : 0.0;
+        g[q] = kApply && in ? other[idx[k + q]] : 1.0;
+      }
+#pragma unroll
+      for (int q = 0; q < kScaleAhead; ++q)
+        if (k + q < end) {
+          if (kApply) v[q] *= f * g[q], val[k + q] = v[q];
+          if (kNorm == RowNorm::kMax) s = std_max(s, fabs(v[q]));
+          if (kNorm == RowNorm::kSum) s += fabs(v[q]);
+        }
     }
-    out[i] = s;
+    if (kNorm != RowNorm::kNone) {
+      const double r = safe_inv_sqrt(s);
+      out[i] = r;
+      scale[i] *= r;
+    }
   }
-}
-
-static __global__ void k_inv_sqrt_factor(long long n, const double* norm, double* f, double* scale) {
-  B200_FOR(i, n) {
-    f[i] = safe_inv_sqrt(norm[i]);
-    scale[i] *= f[i];
-  }
-}
-
-// val[k] *= rf[row] * cf[col] on a CSR (rows = rows of A) ...
-static __global__ void k_apply_csr(int rows, const int* rp, const int* col, double* val, const double* rf,
-                            const double* cf) {
-  B200_FOR(i, rows) {
-    const double r = rf[i];
-    for (int k = rp[i]; k < rp[i + 1]; ++k) val[k] *= r * cf[col[k]];
-  }
-}
-// ... and on the CSC copy (rows of the CSR = columns of A): same product r_i * c_j.
-static __global__ void k_apply_csc(int cols, const int* cp, const int* row, double* val, const double* rf,
-                            const double* cf) {
-  B200_FOR(j, cols) {
-    const double c = cf[j];
-    for (int k = cp[j]; k < cp[j + 1]; ++k) val[k] *= rf[row[k]] * c;
-  }
-}
-
-static __global__ void k_copy_scale(long long n, const double* src, double* dst) {
-  B200_FOR(i, n) dst[i] = src[i];
 }
 
 // Scaled vectors before the bound/objective scalars (scaling.cpp:111-124).
