@@ -1,6 +1,10 @@
 // checks.cuh — the every-K-iterations work of r²HPDHG on the device: fixed-point residual,
 // KKT statistics on the ORIGINAL problem, infeasibility ray tests, and the final unscaling.
 //
+// A check is three launches and a publication: k_check_points (the points, the residual's and the restart
+// distances' terms), k_check_products (all products with A, Ã and Aᵀ that the check needs, over packed
+// points), one launch of sums, k_check_publish; PDLP's the same with k_pdlp_points / k_pdlp_products.
+//
 // Each kernel writes per-element TERMS of the reference's sums into term arrays (reduced by a
 // SumPlan in the reference's order or a fixed tree) and folds maxima into atomic slots.
 // References:

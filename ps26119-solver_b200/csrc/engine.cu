@@ -3,14 +3,15 @@
 //
 // Execution model:
 //   * One CUDA stream per solve. Setup (structure, scaling, ‖Ã‖₂) runs on the device.
-//   * An EPOCH = K iterations, captured once per precision as a CUDA graph: 2K fused kernels
+//   * An EPOCH = K iterations. Where the LP fits the SMs' shared memory it is one cooperative launch
+//     (resident.cuh); else a CUDA graph, captured once per precision: 2K fused kernels
 //     (Ãᵀy + primal update, Ãx̄ + dual update) plus the epoch-start residual section, which
 //     returns at once unless the epoch starts a Halpern cycle (inner = 0). The step scalars
 //     (τ, σ, the Halpern counter) live in device memory and are refreshed by one small copy
-//     before each replay, so the graph is never rebuilt.
+//     before each epoch, so the graph is never rebuilt.
 //   * A CHECK after each epoch is a second graph (three variants: without ray test, with it,
-//     with the drift test as well). It ends by copying one small status block to pinned host
-//     memory; the host then takes exactly the reference's decisions (termination, ray test,
+//     with the drift test as well): the points, all products, the sums (checks.cuh). It ends by
+//     writing one small status block to pinned host memory; the host then takes exactly the reference's decisions (termination, ray test,
 //     precision promotion, restart, PID primal weight) in fp64 with the same libm calls.
 //   * In exact mode every sum uses the reference's order, so the whole trajectory is
 //     bit-identical to the reference CPU engine; in fast mode only the reductions differ
@@ -1538,7 +1539,8 @@ EngineResult Engine::run_pdlp(const DeviceOutputs& out) {
 }
 // ================================================================ continuous batching
 // The group scheduler: one host thread and one stream per device run the r²HPDHG epochs of every
-// solve in flight together. Per epoch, each half-step is ONE launch of k_group_fed over the slabs
+// solve in flight together. An epoch is one resident launch over all of them where they fit the SMs
+// (resident_epoch); else each half-step is ONE launch of k_group_fed over the slabs
 // of all the solves in that working precision (instead of one launch per solve), each solve with
 // its own step scalars, iterates and epilogue; then every solve's own residual section (when its
 // epoch starts a Halpern cycle) and check graph follow on the same stream, one synchronisation
