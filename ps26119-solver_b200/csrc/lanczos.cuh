@@ -12,6 +12,13 @@
 //      exact sum in a cell that every block waits for.
 // Everything is in the kernels' order and arithmetic, so α and β² are the same bits.
 //
+// Why no cell is overwritten too early: v's and t's as in resident.cuh. A block writes its sums cell anew
+// only after it has had the result of the sum before, which the last block to count in leaves, and a block
+// counts in after it has read the earlier blocks' cells; the result's cell is written anew only once every
+// block has counted in again, after it read the last one. The numbers of runs are read by blocks that the
+// products tie to nothing (an LP whose columns fall into unconnected parts), at any time before they count
+// in first: they have cells of their own, written once a launch, and the next launch follows this one.
+//
 // What bounds it: about ten trips through L2 a step (two half-steps, and four per sum) and the two walks,
 // one x_commit for every binade that the sums pass. Measured, Lanczos of 1k random rows 1.07 against 1.26 ms
 // in six launches a step, 10k 1.65 / 1.88, staircase T = 168 (389 steps) 10.1 / 13.3 (before the walk's steps
@@ -27,12 +34,14 @@ struct LanczosArgs {
   int m, n, blocks;
   const int *t_rp, *t_ri, *a_rp, *a_col;
   const double *t_val, *a_val;
-  Cell<double>*vcell, *tcell, *sums, *scalar;  // sums: one per block
+  Cell<double>*vcell, *tcell, *runs, *sums, *scalar;  // runs, sums: one per block
   double *v, *vprev, *terms, *hist;            // hist: (α, β²) by step
   XFast* fast;      // the runs' summaries, n / kXTile + blocks of them
   XTileAgg* full;
   unsigned* count;  // blocks that have counted in, over all sums
   unsigned tag;     // the first of 2 + 3·(to − from) tags
+  // cells of an LP: n of v, m of t, two per block, the sums' result
+  static long long cells(long long m, long long n, int blocks) { return n + m + 2LL * blocks + 1; }
   int from, to;
   unsigned* err;
 };
@@ -149,11 +158,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_resident_lanczos(const __grid_c
   double *v = C.vec, *vprev = v + C.stride, *wv = vprev + C.stride, *term = wv + C.stride;
   bool dead = false;
   // every block's number of runs, for the places of its own
-  if (tid == 0) cell_store(p.sums + g, static_cast<double>((C.count + kXTile - 1) / kXTile), p.tag);
+  if (tid == 0) cell_store(p.runs + g, static_cast<double>((C.count + kXTile - 1) / kXTile), p.tag);
   if (warp == 0) {
     double mine = 0.0, all = 0.0;
     for (int k = lane; k < p.blocks; k += 32) {
-      const double t = cell_wait(p.sums + k, p.tag, dead);
+      const double t = cell_wait(p.runs + k, p.tag, dead);
       all += t;
       if (k < g) mine += t;
     }

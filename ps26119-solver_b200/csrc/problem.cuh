@@ -358,7 +358,7 @@ struct ScaledDevice {
     DevBuf<unsigned> count(1);
     unsigned tag = 1;
     if (shape.blocks > 0) {
-      cells.alloc(static_cast<std::size_t>(n) + m + shape.blocks + 1);
+      cells.alloc(static_cast<std::size_t>(LanczosArgs::cells(m, n, shape.blocks)));
       fast.alloc(static_cast<std::size_t>(n / kXTile + shape.blocks));
       full.alloc(static_cast<std::size_t>(n / kXTile + shape.blocks));
       B200_CHECK(cudaMemsetAsync(cells.get(), 0, cells.size() * sizeof(Cell<double>), st));
@@ -370,8 +370,8 @@ struct ScaledDevice {
       if (shape.blocks > 0) {
         Cell<double>* c = cells.get();
         launch_lanczos({m, n, shape.blocks, t_rp.get(), t_ri.get(), a_rp.get(), a_col.get(), sat.get(), sa.get(),
-                        c, c + n, c + n + m, c + n + m + shape.blocks, v.get(), vprev.get(), terms.get(), hist.get(),
-                        fast.get(), full.get(), count.get(), tag, from, to, err},
+                        c, c + n, c + n + m, c + n + m + shape.blocks, c + n + m + 2 * shape.blocks, v.get(), vprev.get(),
+                        terms.get(), hist.get(), fast.get(), full.get(), count.get(), tag, from, to, err},
                        shape, st);
         tag += 3u * static_cast<unsigned>(to - from) + 2u;
         ++kernels;
