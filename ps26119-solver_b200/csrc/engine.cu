@@ -402,7 +402,7 @@ void Engine::tune_slab() {
   if (!tune_enabled()) return;
   const int prec = std::is_same<T, float>::value ? 1 : 0;
   const int m = M_.m, n = M_.n;
-  const TuneKey kt = tune_key(0, prec, n, M_.nnz), ka = tune_key(1, prec, m, M_.nnz);
+  const TuneKey kt = tune_key(0, prec, n, M_.nnz, max_col_), ka = tune_key(1, prec, m, M_.nnz, max_row_);
   TuneCache& cache = TuneCache::instance();
   if (cache.get(kt, var_t_) && cache.get(ka, var_a_)) return;
   IterVecs<T>& v = vecs<T>();

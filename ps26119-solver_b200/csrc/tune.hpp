@@ -18,16 +18,18 @@
 namespace b200 {
 
 // A shape class: kernel (0 primal Ãᵀy, 1 dual Ãx̄), working precision (0 fp64, 1 fp32), rows
-// rounded to a power of two, and nonzeros per row in quarters.
+// rounded to a power of two, nonzeros per row in quarters, and the longest row rounded to a power of two where
+// it has more than 64 nonzeros (0: none has): one such row decides the variant. 10k rows of 6 with one of 4,096:
+// 30 us an iteration with the spread form, 234 with the variant measured on 10k rows of 6.
 struct TuneKey {
-  int kernel = 0, precision = 0, log2_rows = 0, nnz_per_row_x4 = 0;
+  int kernel = 0, precision = 0, log2_rows = 0, nnz_per_row_x4 = 0, log2_longest = 0;
   bool operator<(const TuneKey& o) const {
-    return std::tie(kernel, precision, log2_rows, nnz_per_row_x4) <
-           std::tie(o.kernel, o.precision, o.log2_rows, o.nnz_per_row_x4);
+    return std::tie(kernel, precision, log2_rows, nnz_per_row_x4, log2_longest) <
+           std::tie(o.kernel, o.precision, o.log2_rows, o.nnz_per_row_x4, o.log2_longest);
   }
 };
 
-inline TuneKey tune_key(int kernel, int precision, long long rows, long long nnz) {
+inline TuneKey tune_key(int kernel, int precision, long long rows, long long nnz, long long longest = 0) {
   TuneKey k;
   k.kernel = kernel;
   k.precision = precision;
@@ -35,6 +37,8 @@ inline TuneKey tune_key(int kernel, int precision, long long rows, long long nnz
   while (r > 1) r >>= 1, ++k.log2_rows;
   const double per = rows > 0 ? static_cast<double>(nnz) / static_cast<double>(rows) : 0.0;
   k.nnz_per_row_x4 = static_cast<int>(std::lround(per * 4.0));
+  if (longest > 64)
+    while (longest > 1) longest >>= 1, ++k.log2_longest;
   return k;
 }
 
