@@ -37,6 +37,7 @@
 #include "parallel.hpp"
 #include "problem.cuh"
 #include "resident.cuh"
+#include "resident_rule.hpp"
 #include "staging.cuh"
 #include "tune.hpp"
 
@@ -187,6 +188,7 @@ class Engine {
   long long resident_size(int blocks) const;
   int num_cols() const { return M_.n; }
   int num_rows() const { return M_.m; }
+  int longest() const { return std::max(rows_.longest, cols_.longest); }  // the most nonzeros of a row or column
   void resident_done();
   // Bulk-copy waits of this solve's kernels that ran out (synchronises the stream).
   unsigned stage_errors() {
@@ -258,7 +260,7 @@ class Engine {
   DeviceModel M_;
   const EngineOptions& o_;
   cudaStream_t st_;
-  int max_row_ = 0, max_col_ = 0;  // the most nonzeros of a row, of a column
+  RowLengths rows_, cols_;  // the lengths of the rows, of the columns
   ResidentShape shape_[2];  // resident epochs in fp64 / fp32 (blocks = 0: the step kernels)
   unsigned tag_ = 1;        // the next resident epoch's first tag
   DevBuf<unsigned> stage_err_;  // this solve's bulk-copy timeouts (see count_stage_timeout)
@@ -338,13 +340,12 @@ void Engine::setup() {
   B200_LAUNCH_CHECK();
   kernels_ += 2;
   // the largest slabs (the kernels' tile capacities), rows and columns
-  int ext[4];
-  sp_.extents(ext, st_);
-  cap_a_ = fed_tile_capacity(ext[0]);
-  cap_t_ = fed_tile_capacity(ext[2]);
+  const RowLengths* len = sp_.lengths(st_);
+  cap_a_ = fed_tile_capacity(len[0].slab);
+  cap_t_ = fed_tile_capacity(len[1].slab);
   vd_.alloc(n, m);
   if (o_.mixed) vf_.alloc(n, m);
-  max_row_ = ext[1], max_col_ = ext[3];
+  rows_ = len[0], cols_ = len[1];
   if (tune_forced() < 0) {  // a forced step-kernel variant runs the step kernels
     plan_resident<double>();
     if (o_.mixed) plan_resident<float>();
@@ -402,7 +403,7 @@ void Engine::tune_slab() {
   if (!tune_enabled()) return;
   const int prec = std::is_same<T, float>::value ? 1 : 0;
   const int m = M_.m, n = M_.n;
-  const TuneKey kt = tune_key(0, prec, n, M_.nnz, max_col_), ka = tune_key(1, prec, m, M_.nnz, max_row_);
+  const TuneKey kt = tune_key(0, prec, n, M_.nnz, cols_.longest), ka = tune_key(1, prec, m, M_.nnz, rows_.longest);
   TuneCache& cache = TuneCache::instance();
   if (cache.get(kt, var_t_) && cache.get(ka, var_a_)) return;
   IterVecs<T>& v = vecs<T>();
@@ -1024,16 +1025,20 @@ void Engine::upload_params() {
 }
 
 // Whether this solve's epochs are resident in precision T, and their buffers: the rule is that the
-// matrix and the updates' vectors fit the SMs' shared memory (resident_shape).
+// matrix and the updates' vectors fit the SMs' shared memory (resident_shape) and that its long rows and
+// columns do not cost more there than in the step kernels (resident_rule.hpp).
 template <class T>
 void Engine::plan_resident() {
   ResidentShape& s = shape_[std::is_same<T, float>::value ? 1 : 0];
-  s = resident_shape<T, ResidentR2h<T>>(M_.m, M_.n, M_.nnz, max_row_, max_col_);
+  s = resident_shape<T, ResidentR2h<T>>(M_.m, M_.n, M_.nnz, rows_.longest, cols_.longest);
+  if (s.blocks > 0 && !resident_pays(rows_, cols_, static_cast<double>(M_.nnz), s.blocks, s.threads,
+                                     (static_cast<double>(M_.m) + M_.n) / s.blocks, sizeof(T) == 4))
+    s = ResidentShape{};
   if (s.blocks > 0) vecs<T>().alloc_resident(M_.n, M_.m, st_);
 }
 long long Engine::resident_size(int blocks) const {
-  return mixed_now_ ? resident_bytes<float, ResidentR2h<float>>(M_.m, M_.n, M_.nnz, max_row_, max_col_, blocks)
-                    : resident_bytes<double, ResidentR2h<double>>(M_.m, M_.n, M_.nnz, max_row_, max_col_, blocks);
+  return mixed_now_ ? resident_bytes<float, ResidentR2h<float>>(M_.m, M_.n, M_.nnz, rows_.longest, cols_.longest, blocks)
+                    : resident_bytes<double, ResidentR2h<double>>(M_.m, M_.n, M_.nnz, rows_.longest, cols_.longest, blocks);
 }
 template <class T>
 ResidentPart<T, ResidentR2h<T>> Engine::resident_part(int first, int blocks) {
@@ -1676,7 +1681,7 @@ class GroupScheduler {
     if (elements / cap > kResidentElements) return false;
     // an even share of the bytes each, rounded down and at least one block
     std::vector<int> blocks(active.size());
-    int used = 0, threads = 64;
+    int used = 0, threads = 64, longest = 0;
     long long smem = 0;
     for (std::size_t k = 0; k < active.size(); ++k) {
       const double share = static_cast<double>(active[k]->e->resident_size(1)) / total;
@@ -1689,7 +1694,9 @@ class GroupScheduler {
       const Engine& e = *active[k]->e;
       smem = std::max(smem, e.resident_size(blocks[k]));
       threads = std::max(threads, resident_threads(e.num_rows(), e.num_cols(), blocks[k]));
+      longest = std::max(longest, e.longest());
     }
+    smem += resident_chunks(longest, threads);
     if (smem > static_cast<long long>(kResidentSmem)) return false;
     rd_.h.clear(), rf_.h.clear();
     int first_d = 0, first_f = 0;
@@ -1701,7 +1708,7 @@ class GroupScheduler {
     rd_.upload(st_), rf_.upload(st_);
     launch_resident_group<ResidentR2h>(rd_.d.get(), static_cast<int>(rd_.h.size()), first_d, rf_.d.get(),
                                        static_cast<int>(rf_.h.size()), first_d + first_f, threads,
-                                       static_cast<unsigned>(smem), st_);
+                                       longest, static_cast<unsigned>(smem), st_);
     return true;
   }
   // One epoch of every active solve: the resident launch, or the grouped step kernels, on the group's stream

@@ -139,7 +139,7 @@ __device__ __forceinline__ double lanczos_sum(const LanczosArgs& p, LanczosShare
   return sh.value;
 }
 
-template <int kThreads, int GB>
+template <int kThreads, int GB, bool kLong>
 __global__ void __launch_bounds__(kThreads, 1) k_resident_lanczos(const __grid_constant__ LanczosArgs p) {
   using B = ResidentBytes<double, LanczosOp>;
   extern __shared__ __align__(16) unsigned char resident_smem[];
@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_resident_lanczos(const __grid_c
   }
   __syncthreads();
   ResidentSide<double> C, R;
-  resident_layout(resident_smem, p.t_rp, cut[0], cut[1], LanczosOp::kCol, p.a_rp, cut[2], cut[3], LanczosOp::kRow, C, R);
+  resident_layout<kLong>(resident_smem, p.t_rp, cut[0], cut[1], LanczosOp::kCol, p.a_rp, cut[2], cut[3], LanczosOp::kRow, C, R);
   double *v = C.vec, *vprev = v + C.stride, *wv = vprev + C.stride, *term = wv + C.stride;
   bool dead = false;
   // every block's number of runs, for the places of its own
@@ -184,17 +184,17 @@ __global__ void __launch_bounds__(kThreads, 1) k_resident_lanczos(const __grid_c
   __syncthreads();
   double bsq = p.from > 0 ? p.hist[2 * p.from - 1] : 0.0;  // no β before the first step
   for (int k = p.from; k < p.to; ++k) {
-    ResidentRow<GB, double> r;
+    ResidentRow<GB, kLong, double> r;
     for (int e0 = 32 * warp; e0 < R.count; e0 += 32 * warps) {  // t = Ãv
       const int e = e0 + lane < R.count ? e0 + lane : -1;
       r.open(R, e);
-      const double s = resident_sum<GB>(r, R, p.vcell, tag, e0 == 32 * warp, dead);
+      const double s = resident_sum(r, R, p.vcell, tag, e0 == 32 * warp, dead);
       if (e >= 0) cell_store(p.tcell + R.from + e, s, tag);
     }
     for (int e0 = 32 * warp; e0 < C.count; e0 += 32 * warps) {  // w = Ãᵀt
       const int e = e0 + lane < C.count ? e0 + lane : -1;
       r.open(C, e);
-      const double s = resident_sum<GB>(r, C, p.tcell, tag, e0 == 32 * warp, dead);
+      const double s = resident_sum(r, C, p.tcell, tag, e0 == 32 * warp, dead);
       if (e >= 0) wv[e] = s, term[e] = s * v[e];
     }
     __syncthreads();
@@ -232,6 +232,7 @@ constexpr long long kLanczosShare = 448;
 // every block is a summary in the sums and a party to their three exchanges; blocks = 0: it does not fit.
 struct LanczosShape {
   int blocks = 0, threads = 0;
+  int longest = 0;
   unsigned smem = 0;
 };
 inline LanczosShape lanczos_shape(long long m, long long n, long long nnz, long long max_row, long long max_col) {
@@ -242,17 +243,25 @@ inline LanczosShape lanczos_shape(long long m, long long n, long long nnz, long 
   int blocks = static_cast<int>(std::max(1LL, std::min<long long>(sms, (n + kLanczosShare - 1) / kLanczosShare)));
   auto bytes = [&](int b) { return resident_bytes<double, LanczosOp>(m, n, nnz, max_row, max_col, b); };
   while (blocks < sms && bytes(blocks) > kResidentSmem / 2) ++blocks;
-  if (bytes(blocks) > kResidentSmem - sizeof(LanczosShared) || (m + n) / blocks > kResidentElements) return s;
   const long long warps = std::max(n, m) / blocks / 32 + 2;
+  const int threads = static_cast<int>(32 * std::min(32LL, std::max(2LL, warps)));
+  const int longest = static_cast<int>(std::max(max_row, max_col));
+  const long long smem = bytes(blocks) + resident_chunks(longest, threads);
+  if (smem > static_cast<long long>(kResidentSmem - sizeof(LanczosShared)) || (m + n) / blocks > kResidentElements) return s;
   s.blocks = blocks;
-  s.threads = static_cast<int>(32 * std::min(32LL, std::max(2LL, warps)));
-  s.smem = static_cast<unsigned>(bytes(blocks));
+  s.threads = threads;
+  s.longest = longest;
+  s.smem = static_cast<unsigned>(smem);
   return s;
 }
 inline void launch_lanczos(const LanczosArgs& p, const LanczosShape& s, cudaStream_t st) {
-  const void* f = s.threads <= 256   ? reinterpret_cast<const void*>(&k_resident_lanczos<256, 16>)
-                  : s.threads <= 512 ? reinterpret_cast<const void*>(&k_resident_lanczos<512, 8>)
-                                     : reinterpret_cast<const void*>(&k_resident_lanczos<1024, 4>);
+  const auto kernel = [&](auto is_long) {
+    constexpr bool kLong = decltype(is_long)::value;
+    return s.threads <= 256   ? reinterpret_cast<const void*>(&k_resident_lanczos<256, 16, kLong>)
+           : s.threads <= 512 ? reinterpret_cast<const void*>(&k_resident_lanczos<512, 8, kLong>)
+                              : reinterpret_cast<const void*>(&k_resident_lanczos<1024, 4, kLong>);
+  };
+  const void* f = resident_is_long(s.longest, s.threads) ? kernel(std::true_type{}) : kernel(std::false_type{});
   B200_CHECK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kResidentSmem)));
   void* args[] = {const_cast<LanczosArgs*>(&p)};
   B200_CHECK(cudaLaunchCooperativeKernel(f, dim3(static_cast<unsigned>(s.blocks)), dim3(static_cast<unsigned>(s.threads)), args,

@@ -150,8 +150,8 @@ struct ScaledDevice {
   // original-space constants of kkt_general (cpu_backend.cpp:233-262): ‖b‖₂, ‖c‖₂, ‖c‖∞
   double b_norm = 0, c_norm = 0, c_inf = 0;
   long long kernels = 0;
-  int ext[4] = {0, 0, 0, 0};
-  bool have_extents = false;
+  RowLengths lengths_[2];  // of the rows, of the columns
+  bool have_lengths = false;
   int lanczos_launched = 0;  // Lanczos steps launched by the last lanczos() (counted or not)
 
   // Scratch for the setup reductions.
@@ -162,7 +162,7 @@ struct ScaledDevice {
     M = dm;
     m = dm.m, n = dm.n, sense = dm.sense, nnz = dm.nnz;
     exact = exact_order;
-    have_extents = false;
+    have_lengths = false;
     const std::size_t mm = static_cast<std::size_t>(m), nn = static_cast<std::size_t>(n);
     const std::size_t nz = static_cast<std::size_t>(nnz);
     a_rp.alloc(mm + 1);
@@ -304,21 +304,22 @@ struct ScaledDevice {
   template <class T> const T* rl() const;
   template <class T> const T* ru() const;
 
-  // out: the most nonzeros of a slab of rows, of a row, of a slab of columns, of a column (cached by the
-  // problem; synchronises the stream the first time).
-  void extents(int* out, cudaStream_t st) {
-    if (!have_extents) {
-      DevBuf<int> d(4);
-      B200_CHECK(cudaMemsetAsync(d.get(), 0, sizeof ext, st));
+  // The lengths of the rows [0] and of the columns [1] (cached by the problem; synchronises the stream the
+  // first time).
+  const RowLengths* lengths(cudaStream_t st) {
+    if (!have_lengths) {
+      static_assert(sizeof lengths_ == 6 * sizeof(int), "three numbers a side");
+      DevBuf<int> d(6);
+      B200_CHECK(cudaMemsetAsync(d.get(), 0, sizeof lengths_, st));
       if (m > 0) k_extents<<<std::min(grid_for(m), 8 * sm_count()), kBlock, 0, st>>>(m, a_rp.get(), d.get());
-      if (n > 0) k_extents<<<std::min(grid_for(n), 8 * sm_count()), kBlock, 0, st>>>(n, t_rp.get(), d.get() + 2);
+      if (n > 0) k_extents<<<std::min(grid_for(n), 8 * sm_count()), kBlock, 0, st>>>(n, t_rp.get(), d.get() + 3);
       B200_LAUNCH_CHECK();
       kernels += 2;
-      B200_CHECK(cudaMemcpyAsync(ext, d.get(), sizeof ext, cudaMemcpyDeviceToHost, st));
+      B200_CHECK(cudaMemcpyAsync(lengths_, d.get(), sizeof lengths_, cudaMemcpyDeviceToHost, st));
       B200_CHECK(cudaStreamSynchronize(st));
-      have_extents = true;
+      have_lengths = true;
     }
-    std::copy(ext, ext + 4, out);
+    return lengths_;
   }
 
   // ‖Ã‖₂ by Lanczos on ÃᵀÃ (csr.cpp:86-132), on the device: the reference's start vector, the
@@ -349,9 +350,8 @@ struct ScaledDevice {
     kernels += 2 + pbn.kernel_count();
     const int tiles = (n + kXTile - 1) / kXTile;
     // An LP that fits the SMs' shared memory takes a batch of steps in one launch (lanczos.cuh).
-    int ext[4];
-    extents(ext, st);
-    const LanczosShape shape = lanczos_shape(m, n, nnz, ext[1], ext[3]);
+    const RowLengths* len = lengths(st);
+    const LanczosShape shape = lanczos_shape(m, n, nnz, len[0].longest, len[1].longest);
     DevBuf<Cell<double>> cells;
     DevBuf<XFast> fast;
     DevBuf<XTileAgg> full;

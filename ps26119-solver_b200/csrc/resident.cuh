@@ -27,6 +27,7 @@
 // 12.9 -> 9.8; staircase T = 168 6.4 -> 2.7.
 #pragma once
 
+#include "resident_rule.hpp"
 #include "spmv.cuh"
 
 namespace b200 {
@@ -82,7 +83,7 @@ __device__ __forceinline__ void cell_store(Cell<T>* p, T v, unsigned tag) {
 // 100k 9.8 / 9.0 against 12.9 / 14.1. Past 194 KB a block the next carveout leaves the gathers too little
 // L1: 112k rows (186 KB) 12.0 against 12.7, 121k (201 KB) 20.9 against 12.7. Past 2,560 columns and rows a
 // block the polls crowd out the stores: mixed 150k rows (2,534) 13.6 against 14.1, 180k (3,040) 18.0
-// against 16.9; the staircase T = 3600 (2,651) 6.7 against 9.1.
+// against 16.9; the staircase T = 3600 (2,651) 6.7 against 9.1. LPs with long rows: resident_rule.hpp.
 constexpr unsigned kResidentSmem = 194u * 1024u;
 constexpr long long kResidentElements = 2688;
 
@@ -249,17 +250,20 @@ __device__ __forceinline__ int resident_cut(const int* __restrict__ rp, int rows
   return hi;
 }
 
+constexpr int kResidentChunk = 64;  // entries of a long row gathered at a time
+
 // One side of a block's part in shared memory.
 template <class T>
 struct ResidentSide {
   int from, count, stride;
   int *rp, *idx;  // rp rebased to the block's first nonzero
   T *val, *vec;
+  double* chunk;  // the warps' buffers for long rows
 };
 
 // Both sides' places in a block's shared memory: columns [c0, c1) of a matrix with row pointers t_rp (of
 // Ãᵀ), rows [r0, r1) of one with a_rp.
-template <class T>
+template <bool kLong, class T>
 __device__ __forceinline__ void resident_layout(unsigned char* at, const int* t_rp, int c0, int c1, int col_vecs,
                                                 const int* a_rp, int r0, int r1, int row_vecs, ResidentSide<T>& C,
                                                 ResidentSide<T>& R) {
@@ -276,6 +280,7 @@ __device__ __forceinline__ void resident_layout(unsigned char* at, const int* t_
     S.rp = reinterpret_cast<int*>(take((S.count + 1LL) * 4));
     S.idx = reinterpret_cast<int*>(take(nz * 4LL));
   };
+  C.chunk = R.chunk = reinterpret_cast<double*>(take(kLong ? static_cast<long long>(blockDim.x) / 32 * kResidentChunk * 8 : 0));
   side(C, t_rp, c0, c1, col_vecs);
   side(R, a_rp, r0, r1, row_vecs);
 }
@@ -288,18 +293,37 @@ __device__ __forceinline__ void resident_fill(const ResidentSide<T>& S, const in
   for (int k = tid; k < nz; k += nt) S.idx[k] = __ldg(idx + k0 + k), S.val[k] = __ldg(val + k0 + k);
 }
 
+// A long row (resident_rule.hpp) walked by one thread would take a trip to L2 for every GB entries while the whole
+// LP waits for it. Launches with one run kernels in which a warp sums such rows together (resident_long).
+template <int GB>
+constexpr int kResidentLong = resident_long_row(GB > 8 ? 0 : GB > 4 ? 1 : 2);
+inline bool resident_is_long(int longest, int threads) { return longest > resident_long_row(resident_form(threads)); }
+// Their shared memory beside the LP's part: a buffer for a chunk's products per warp.
+inline long long resident_chunks(int longest, int threads) {
+  return resident_is_long(longest, threads) ? threads / 32 * kResidentChunk * 8LL : 0;
+}
+
 // A thread's row: its entries [a, a + len) of the side's arrays, and the first GB of them. (With GB = 4,
 // at 64 registers a thread, the values stay in shared memory until they are used.)
-template <int GB, class T>
+template <int GB, bool kLong, class T>
 struct ResidentRow {
   static constexpr bool kVals = GB > 4;
-  int a, len, longest;  // longest: of the warp's rows
+  int a, len, longest;  // longest: of the warp's rows that have a thread each
+  unsigned together;    // the lanes whose rows the warp sums together (kLong kernels)
   int idx[GB];
   T val[kVals ? GB : 1];
   // e < 0: the lane has no element (a row without entries)
   __device__ __forceinline__ void open(const ResidentSide<T>& S, int e) {
     a = e >= 0 ? S.rp[e] : 0, len = e >= 0 ? S.rp[e + 1] - a : 0;
     longest = __reduce_max_sync(kFull, len);
+    together = 0;
+    if (kLong && longest > kResidentLong<GB>) {
+      const bool is = len > kResidentLong<GB>;
+      if (__reduce_add_sync(kFull, is ? len : 0) < kResidentShare * longest) {
+        together = __ballot_sync(kFull, is);
+        longest = __reduce_max_sync(kFull, is ? 0 : len);
+      }
+    }
     load(S, 0);
   }
   __device__ __forceinline__ void load(const ResidentSide<T>& S, int k) {
@@ -316,15 +340,80 @@ struct ResidentRow {
   }
 };
 
+// The Σ of a long row, entries [0, n) at idx and val, by a whole warp: its lanes gather kResidentChunk entries at
+// a time, the next ones while these are added, and every lane adds their products in CSR order from the warp's
+// buffer `sh` (16-byte aligned). What bounds it: the chain of additions, 13 cycles each by itself (21 with shuffles in
+// place of the buffer), 16 in blocks of 256 threads and 27 in those of 1,024, whose other warps poll beside it;
+// chunks of 128, or two ahead, were no faster. Measured, us per iteration with one thread a long row / so / the
+// step kernels' best variant: 10k rows and one of 512 26.6 / 7.4 / 9.9, of 4,096 190 / 36.9 / 29.7; 60k rows and
+// one of 512 52.7 / 13.1 / 13.7, of 4,096 406 / 63.8 / 33.9.
+struct ResidentLongSum {
+  double s;
+  bool dead;  // a lane's wait ran out
+};
+template <class T>
+__device__ __noinline__ ResidentLongSum resident_long(const int* idx, const T* val, int n, const Cell<T>* cells, unsigned tag,
+                                                      bool dead, double* sh) {
+  constexpr int Q = kResidentChunk / 32;
+  const int lane = static_cast<int>(threadIdx.x) & 31;
+  CellRead<T> g[Q];
+  const auto ask = [&](int k, bool again) {
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      const int e = k + 32 * q + lane;
+      const bool in = e < n;
+      if (!again) g[q] = CellRead<T>{};
+      cell_load(g[q], cells + idx[in ? e : 0], in && !(again && g[q].is(tag)));
+    }
+  };
+  double s = 0.0;
+  ask(0, false);
+  for (int k = 0; k < n; k += kResidentChunk) {
+    for (int polls = 0;; ++polls) {
+      bool late = false;
+#pragma unroll
+      for (int q = 0; q < Q; ++q) late = late || (k + 32 * q + lane < n && !g[q].is(tag));
+      if (!__any_sync(kFull, late && !dead)) break;
+      if (polls > kResidentPolls) dead = true;  // never expected
+      ask(k, true);
+    }
+    __syncwarp();  // the chunk before has been added
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      const int e = k + 32 * q + lane;
+      const double prod = static_cast<double>(val[e < n ? e : 0]) * static_cast<double>(g[q].value());
+      sh[32 * q + lane] = e < n ? prod : -0.0;  // adding −0.0 leaves every sum as it is
+    }
+    __syncwarp();
+    if (k + kResidentChunk < n) ask(k + kResidentChunk, false);
+    const double2* p = reinterpret_cast<const double2*>(sh);
+    double2 v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] = p[q];
+#pragma unroll
+    for (int i = 0; i < kResidentChunk; i += 8) {  // 8 products ahead in registers (wrapping at the buffer's end)
+      double2 w[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) w[q] = p[((i >> 1) + 4 + q) & (kResidentChunk / 2 - 1)];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) s += v[q].x, s += v[q].y;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) v[q] = w[q];
+    }
+  }
+  return {s, __any_sync(kFull, dead) != 0};
+}
+
 // The row's Σ in CSR order, from cells of tag `tag`. `watch`: the warp's first element of this half-step.
 // One lane then watches one cell until it is there before the warp gathers: polls of every gathered cell
 // by every thread slow the stores that they wait for (a step of a 10k LP took 16.3 us that way, 4.4 with the
-// watch). Cells that are late all the same are read again, by the whole warp in step.
-template <int GB, class T>
-__device__ __forceinline__ double resident_sum(ResidentRow<GB, T>& r, const ResidentSide<T>& S, const Cell<T>* cells,
+// watch). Cells that are late all the same are read again, by the whole warp in step. The warp's long rows come
+// after the others.
+template <int GB, bool kLong, class T>
+__device__ __forceinline__ double resident_sum(ResidentRow<GB, kLong, T>& r, const ResidentSide<T>& S, const Cell<T>* cells,
                                                unsigned tag, bool watch, bool& dead) {
   if (watch && r.longest > 0) {
-    const int who = __ffs(__ballot_sync(kFull, r.len > 0)) - 1;
+    const int who = __ffs(__ballot_sync(kFull, r.len > 0) & (kLong ? ~r.together : kFull)) - 1;
     if (static_cast<int>(threadIdx.x & 31) == who) {
       const Cell<T>* c = cells + r.idx[0];
       CellRead<T> g{};
@@ -337,12 +426,13 @@ __device__ __forceinline__ double resident_sum(ResidentRow<GB, T>& r, const Resi
     __syncwarp();
   }
   double s = 0.0;
+  const int lane = static_cast<int>(threadIdx.x) & 31, len = kLong && ((r.together >> lane) & 1u) ? 0 : r.len;
   for (int k = 0;;) {
     CellRead<T> g[GB];
     bool late[GB];
 #pragma unroll
     for (int q = 0; q < GB; ++q) {
-      late[q] = k + q < r.len;
+      late[q] = k + q < len;
       g[q] = CellRead<T>{};
       cell_load(g[q], cells + r.idx[q], late[q]);
     }
@@ -361,16 +451,24 @@ __device__ __forceinline__ double resident_sum(ResidentRow<GB, T>& r, const Resi
 #pragma unroll
     for (int q = 0; q < GB; ++q) {  // in CSR order; adding −0.0 leaves every sum as it is
       const double prod = r.value(S, k, q) * static_cast<double>(g[q].value());
-      s += k + q < r.len ? prod : -0.0;
+      s += k + q < len ? prod : -0.0;
     }
     k += GB;
     if (k >= r.longest) break;
     r.load(S, k);
   }
+  if constexpr (kLong)
+    for (unsigned left = r.together; left != 0; left &= left - 1) {
+      const int who = __ffs(left) - 1, from = __shfl_sync(kFull, r.a, who);
+      const ResidentLongSum t = resident_long(S.idx + from, S.val + from, __shfl_sync(kFull, r.len, who), cells, tag, dead,
+                                              S.chunk + (threadIdx.x >> 5) * kResidentChunk);
+      if (lane == who) s = t.s;
+      dead = t.dead;
+    }
   return dead ? __longlong_as_double(0x7ff8000000000000LL) : s;
 }
 
-template <int GB, class T, class Op>
+template <int GB, bool kLong, class T, class Op>
 __device__ __forceinline__ void resident_body(const ResidentPart<T, Op>& p, int g) {
   using B = ResidentBytes<T, Op>;
   extern __shared__ __align__(16) unsigned char resident_smem[];
@@ -383,7 +481,7 @@ __device__ __forceinline__ void resident_body(const ResidentPart<T, Op>& p, int 
   }
   __syncthreads();
   ResidentSide<T> C, R;
-  resident_layout(resident_smem, p.t_rp, cut[0], cut[1], Op::kCol, p.a_rp, cut[2], cut[3], Op::kRow, C, R);
+  resident_layout<kLong>(resident_smem, p.t_rp, cut[0], cut[1], Op::kCol, p.a_rp, cut[2], cut[3], Op::kRow, C, R);
   const int nt = static_cast<int>(blockDim.x);
   // y first, and out at once: the columns' first step waits for it
   for (int e = tid; e < R.count; e += nt) {
@@ -409,7 +507,7 @@ __device__ __forceinline__ void resident_body(const ResidentPart<T, Op>& p, int 
   // rows of at most GB entries opens its rows once.)
   if (warp < wc) {
     const bool once = C.count <= 32 * wc;
-    ResidentRow<GB, T> r;
+    ResidentRow<GB, kLong, T> r;
     if (once) r.open(C, 32 * warp + lane < C.count ? 32 * warp + lane : -1);
     const bool held = once && r.longest <= GB;
     for (int s = 0; s < K; ++s) {
@@ -420,7 +518,7 @@ __device__ __forceinline__ void resident_body(const ResidentPart<T, Op>& p, int 
         if (!held) r.open(C, e);
         T* v = C.vec + (e >= 0 ? e : 0);
         auto o = p.op.col_before(v, C.stride);
-        const double sum = resident_sum<GB>(r, C, p.ycell, tag, e0 == 32 * warp, dead);
+        const double sum = resident_sum(r, C, p.ycell, tag, e0 == 32 * warp, dead);
         if (e < 0) continue;
         const T xbar = p.op.col(st, sum, o);
         cell_store(p.xcell + C.from + e, xbar, tag + 1);
@@ -430,7 +528,7 @@ __device__ __forceinline__ void resident_body(const ResidentPart<T, Op>& p, int 
   } else {
     const int wr = warps - wc, w = warp - wc;
     const bool once = R.count <= 32 * wr;
-    ResidentRow<GB, T> r;
+    ResidentRow<GB, kLong, T> r;
     if (once) r.open(R, 32 * w + lane < R.count ? 32 * w + lane : -1);
     const bool held = once && r.longest <= GB;
     for (int s = 0; s < K; ++s) {
@@ -441,7 +539,7 @@ __device__ __forceinline__ void resident_body(const ResidentPart<T, Op>& p, int 
         if (!held) r.open(R, e);
         T* v = R.vec + (e >= 0 ? e : 0);
         auto o = p.op.row_before(v, R.stride);
-        const double sum = resident_sum<GB>(r, R, p.xcell, tag, e0 == 32 * w, dead);
+        const double sum = resident_sum(r, R, p.xcell, tag, e0 == 32 * w, dead);
         if (e < 0) continue;
         const T ny = p.op.row(st, sum, o);
         cell_store(p.ycell + R.from + e, ny, tag);
@@ -452,14 +550,15 @@ __device__ __forceinline__ void resident_body(const ResidentPart<T, Op>& p, int 
   if (dead) count_stage_timeout(p.err);
 }
 
-template <int kThreads, int GB, class T, class Op>
+// kLong: with the code for long rows, for LPs that have one (in the kernels of 64 registers it costs spills).
+template <int kThreads, int GB, bool kLong, class T, class Op>
 __global__ void __launch_bounds__(kThreads, 1) k_resident(const __grid_constant__ ResidentPart<T, Op> p) {
-  resident_body<GB>(p, static_cast<int>(blockIdx.x));
+  resident_body<GB, kLong>(p, static_cast<int>(blockIdx.x));
 }
 
 // Several LPs in one launch (the request loop): blocks [0, blocks_d) are the fp64 LPs', the ones after them
 // the fp32 LPs' (whose `first` counts from there). A block copies its LP's part to shared memory.
-template <int kThreads, int GB, template <class> class Op>
+template <int kThreads, int GB, bool kLong, template <class> class Op>
 __global__ void __launch_bounds__(kThreads, 1) k_resident_group(const ResidentPart<double, Op<double>>* __restrict__ pd, int nd,
                                                                 int blocks_d, const ResidentPart<float, Op<float>>* __restrict__ pf,
                                                                 int nf) {
@@ -472,7 +571,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_resident_group(const ResidentPa
       reinterpret_cast<unsigned*>(held)[q] = __ldg(reinterpret_cast<const unsigned*>(parts + k) + q);
     __syncthreads();
     const Part& p = *reinterpret_cast<const Part*>(held);
-    resident_body<GB>(p, b - p.first);
+    resident_body<GB, kLong>(p, b - p.first);
   };
   const int b = static_cast<int>(blockIdx.x);
   if (b < blocks_d) run(pd, nd, b);
@@ -480,11 +579,15 @@ __global__ void __launch_bounds__(kThreads, 1) k_resident_group(const ResidentPa
 }
 template <template <class> class Op>
 inline void launch_resident_group(const ResidentPart<double, Op<double>>* pd, int nd, int blocks_d,
-                                  const ResidentPart<float, Op<float>>* pf, int nf, int blocks, int threads, unsigned smem,
-                                  cudaStream_t st) {
-  const void* f = threads <= 256   ? reinterpret_cast<const void*>(&k_resident_group<256, 16, Op>)
-                  : threads <= 512 ? reinterpret_cast<const void*>(&k_resident_group<512, 8, Op>)
-                                   : reinterpret_cast<const void*>(&k_resident_group<1024, 4, Op>);
+                                  const ResidentPart<float, Op<float>>* pf, int nf, int blocks, int threads, int longest,
+                                  unsigned smem, cudaStream_t st) {
+  const auto kernel = [&](auto is_long) {
+    constexpr bool kLong = decltype(is_long)::value;
+    return threads <= 256   ? reinterpret_cast<const void*>(&k_resident_group<256, 16, kLong, Op>)
+           : threads <= 512 ? reinterpret_cast<const void*>(&k_resident_group<512, 8, kLong, Op>)
+                            : reinterpret_cast<const void*>(&k_resident_group<1024, 4, kLong, Op>);
+  };
+  const void* f = resident_is_long(longest, threads) ? kernel(std::true_type{}) : kernel(std::false_type{});
   B200_CHECK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kResidentSmem)));
   void* args[] = {&pd, &nd, &blocks_d, &pf, &nf};
   B200_CHECK(cudaLaunchCooperativeKernel(f, dim3(static_cast<unsigned>(blocks)), dim3(static_cast<unsigned>(threads)), args, smem,
@@ -494,6 +597,7 @@ inline void launch_resident_group(const ResidentPart<double, Op<double>>* pd, in
 // How one LP's epochs are launched: blocks, threads and dynamic shared memory; blocks = 0: not this way.
 struct ResidentShape {
   int blocks = 0, threads = 0;
+  int longest = 0;  // entries of the longest row or column
   unsigned smem = 0;
 };
 // Threads for one column or row each, and a warp for uneven shares, as far as 1,024 go.
@@ -507,19 +611,25 @@ inline ResidentShape resident_shape(long long m, long long n, long long nnz, lon
   ResidentShape s;
   if (m < 1 || n < 1 || nnz < 1) return s;
   const int blocks = static_cast<int>(std::max(1LL, std::min<long long>(sm_count(), (m + n + 7) / 8)));
-  const long long bytes = resident_bytes<T, Op>(m, n, nnz, max_row, max_col, blocks);
+  const int threads = resident_threads(m, n, blocks), longest = static_cast<int>(std::max(max_row, max_col));
+  const long long bytes = resident_bytes<T, Op>(m, n, nnz, max_row, max_col, blocks) + resident_chunks(longest, threads);
   if (bytes > kResidentSmem || (m + n) / blocks > kResidentElements) return s;
   s.blocks = blocks;
-  s.threads = resident_threads(m, n, blocks);
+  s.threads = threads;
+  s.longest = longest;
   s.smem = static_cast<unsigned>(bytes);
   return s;
 }
 // Launches one epoch cooperatively on `st`.
 template <class T, class Op>
 inline void launch_resident(const ResidentPart<T, Op>& p, const ResidentShape& s, cudaStream_t st) {
-  const void* f = s.threads <= 256   ? reinterpret_cast<const void*>(&k_resident<256, 16, T, Op>)
-                  : s.threads <= 512 ? reinterpret_cast<const void*>(&k_resident<512, 8, T, Op>)
-                                     : reinterpret_cast<const void*>(&k_resident<1024, 4, T, Op>);
+  const auto kernel = [&](auto is_long) {
+    constexpr bool kLong = decltype(is_long)::value;
+    return s.threads <= 256   ? reinterpret_cast<const void*>(&k_resident<256, 16, kLong, T, Op>)
+           : s.threads <= 512 ? reinterpret_cast<const void*>(&k_resident<512, 8, kLong, T, Op>)
+                              : reinterpret_cast<const void*>(&k_resident<1024, 4, kLong, T, Op>);
+  };
+  const void* f = resident_is_long(s.longest, s.threads) ? kernel(std::true_type{}) : kernel(std::false_type{});
   B200_CHECK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kResidentSmem)));
   void* args[] = {const_cast<ResidentPart<T, Op>*>(&p)};
   B200_CHECK(cudaLaunchCooperativeKernel(f, dim3(static_cast<unsigned>(s.blocks)), dim3(static_cast<unsigned>(s.threads)), args,

@@ -813,18 +813,26 @@ static __global__ void k_slab_table(int rows, const int* rp, int2* out) {
 }
 inline int slab_count(int rows) { return rows <= 0 ? 0 : (rows + kSlabRows - 1) / kSlabRows; }
 
-// The most nonzeros of a slab (out[0]) and of a row (out[1]); out zeroed before.
+// The rows' lengths (RowLengths: out[0] slab, [1] longest, [2] together); out zeroed before.
 static __global__ void k_extents(int rows, const int* __restrict__ rp, int* out) {
-  int slab = 0, row = 0;
-  B200_FOR(r, rows) {
-    const int i = static_cast<int>(r), a = rp[i];
-    row = max(row, rp[i + 1] - a);
-    if (i % kSlabRows == 0) slab = max(slab, rp[min(i + kSlabRows, rows)] - a);
+  const int lane = static_cast<int>(threadIdx.x) & 31;
+  int slab = 0, row = 0, together = 0;
+  const std::int64_t stride = static_cast<std::int64_t>(gridDim.x) * blockDim.x;
+  for (std::int64_t r = blockIdx.x * static_cast<std::int64_t>(blockDim.x) + threadIdx.x; r - lane < rows; r += stride) {
+    int len = 0;
+    if (r < rows) {
+      const int i = static_cast<int>(r), a = rp[i];
+      len = rp[i + 1] - a;
+      if (i % kSlabRows == 0) slab = max(slab, rp[min(i + kSlabRows, rows)] - a);
+    }
+    row = max(row, len);
+    together = max(together, static_cast<int>(__reduce_add_sync(kFull, len > 32 ? len : 0)));
   }
   slab = __reduce_max_sync(kFull, slab), row = __reduce_max_sync(kFull, row);
-  if ((threadIdx.x & 31) == 0) {
+  if (lane == 0) {
     if (slab > 0) atomicMax(out, slab);
     if (row > 0) atomicMax(out + 1, row);
+    if (together > 0) atomicMax(out + 2, together);
   }
 }
 
