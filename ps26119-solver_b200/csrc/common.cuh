@@ -9,8 +9,10 @@
 
 #include <atomic>
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <chrono>
 #include <cstdint>
 #include <cstdio>
@@ -23,6 +25,7 @@
 #include <vector>
 #include <stdexcept>
 #include <string>
+#include <type_traits>
 #include <utility>
 
 namespace b200 {
@@ -367,6 +370,48 @@ inline int sm_count() {
     cached[dev].store(v, std::memory_order_relaxed);
   }
   return v;
+}
+
+// The SMs that kernels on stream st may use at the same time: the device's, or the part of them that the green
+// context of the stream holds.
+inline int stream_sm_count(cudaStream_t st) {
+  struct Entries {
+    CUresult (*context)(CUstream, CUgreenCtx*) = nullptr;
+    CUresult (*resource)(CUgreenCtx, CUdevResource*, CUdevResourceType) = nullptr;
+  };
+  static const Entries e = [] {
+    Entries r;
+    const auto find = [](const char* name, auto& fn) {
+      void* p = nullptr;
+      cudaDriverEntryPointQueryResult found;
+      if (cudaGetDriverEntryPoint(name, &p, cudaEnableDefault, &found) == cudaSuccess && found == cudaDriverEntryPointSuccess)
+        fn = reinterpret_cast<std::decay_t<decltype(fn)>>(p);
+    };
+    find("cuStreamGetGreenCtx", r.context);
+    find("cuGreenCtxGetDevResource", r.resource);
+    (void)cudaGetLastError();
+    return r;
+  }();
+  const int all = sm_count();
+  CUgreenCtx ctx = nullptr;
+  CUdevResource part;
+  if (!e.context || !e.resource || e.context(st, &ctx) != CUDA_SUCCESS || !ctx ||
+      e.resource(ctx, &part, CU_DEV_RESOURCE_TYPE_SM) != CUDA_SUCCESS)
+    return all;
+  return std::max(1, std::min(all, static_cast<int>(part.sm.smCount)));
+}
+
+// A cooperative launch; false, with nothing launched, where its blocks cannot all run at the same time (a device
+// shared out between processes): the caller has another way.
+inline bool launch_cooperative(const void* f, int blocks, int threads, void** args, unsigned smem, cudaStream_t st) {
+  const cudaError_t e = cudaLaunchCooperativeKernel(f, dim3(static_cast<unsigned>(blocks)), dim3(static_cast<unsigned>(threads)),
+                                                    args, smem, st);
+  if (e == cudaErrorCooperativeLaunchTooLarge) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  B200_CHECK(e);
+  return true;
 }
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) {

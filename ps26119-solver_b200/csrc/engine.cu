@@ -223,8 +223,9 @@ class Engine {
   template <class T> void launch_first_residual(const int* skip, bool apart);
   template <class T, int kRays> void launch_check_kernels();
   template <class T> void plan_resident();
-  template <class T> void launch_resident_epoch();
-  template <class T> void launch_resident_pdlp(int cur);
+  template <class T> bool launch_resident_epoch();
+  template <class T> bool launch_resident_pdlp(int cur);
+  bool no_resident();
   template <class T> void launch_kkt_scaled(const T* xs, const T* ys);
   void launch_kkt_original();
   void make_side_stream();
@@ -1030,7 +1031,8 @@ void Engine::upload_params() {
 template <class T>
 void Engine::plan_resident() {
   ResidentShape& s = shape_[std::is_same<T, float>::value ? 1 : 0];
-  s = resident_shape<T, ResidentR2h<T>>(M_.m, M_.n, M_.nnz, rows_.longest, cols_.longest);
+  s = resident_shape<T, ResidentR2h<T>>(M_.m, M_.n, M_.nnz, rows_.longest, cols_.longest,
+                                           stream_sm_count(st_));
   if (s.blocks > 0 && !resident_pays(rows_, cols_, static_cast<double>(M_.nnz), s.blocks, s.threads,
                                      (static_cast<double>(M_.m) + M_.n) / s.blocks, sizeof(T) == 4))
     s = ResidentShape{};
@@ -1059,17 +1061,24 @@ void Engine::resident_done() {
   else launch_first_residual<double>(nullptr, true);
 }
 
-template <class T>
-void Engine::launch_resident_epoch() {
-  const ResidentShape& s = shape_[std::is_same<T, float>::value ? 1 : 0];
-  B200_CHECK(cudaEventRecord(ev_[0], st_));
-  launch_resident(resident_part<T>(0, s.blocks), s, st_);
-  B200_CHECK(cudaEventRecord(ev_[1], st_));
-  resident_done();
+// A resident launch was refused (launch_cooperative): this solve's epochs are the step kernels' from here on.
+bool Engine::no_resident() {
+  shape_[0] = shape_[1] = ResidentShape{};
+  return false;
 }
 
 template <class T>
-void Engine::launch_resident_pdlp(int cur) {
+bool Engine::launch_resident_epoch() {
+  const ResidentShape& s = shape_[std::is_same<T, float>::value ? 1 : 0];
+  B200_CHECK(cudaEventRecord(ev_[0], st_));
+  if (!launch_resident(resident_part<T>(0, s.blocks), s, st_)) return no_resident();
+  B200_CHECK(cudaEventRecord(ev_[1], st_));
+  resident_done();
+  return true;
+}
+
+template <class T>
+bool Engine::launch_resident_pdlp(int cur) {
   IterVecs<T>& v = vecs<T>();
   const StepParams& hp = *hparams_.get();
   const bool odd = (hp.K & 1) != 0;
@@ -1082,19 +1091,16 @@ void Engine::launch_resident_pdlp(int cur) {
       {xs[cur], sp_.c<T>(), sp_.l<T>(), sp_.u<T>(), ys[cur], sp_.rl<T>(), sp_.ru<T>(), v.dx.get(), v.dy.get(), xs[out],
        xs[1 - out], v.xb.get(), ys[out], ys[1 - out], hp.tau, hp.sigma, hp.inner0, hp.K}};
   B200_CHECK(cudaEventRecord(ev_[0], st_));
-  launch_resident(p, shape_[std::is_same<T, float>::value ? 1 : 0], st_);
+  if (!launch_resident(p, shape_[std::is_same<T, float>::value ? 1 : 0], st_)) return no_resident();
   B200_CHECK(cudaEventRecord(ev_[1], st_));
   tag_ += static_cast<unsigned>(hp.K) + 1;
   ++kernels_;
+  return true;
 }
 
 void Engine::launch_epoch() {
   const int pidx = mixed_now_ ? 1 : 0;
-  if (resident()) {
-    if (mixed_now_) launch_resident_epoch<float>();
-    else launch_resident_epoch<double>();
-    return;
-  }
+  if (resident() && (mixed_now_ ? launch_resident_epoch<float>() : launch_resident_epoch<double>())) return;
   upload_params();
   if (mixed_now_) capture_epoch<float>();
   else capture_epoch<double>();
@@ -1216,9 +1222,9 @@ EngineResult Engine::run(const DeviceOutputs& out) {
   if (start(out)) return R_;
   const int K = o_.check_every;
   for (;;) {
-    const bool stepped_resident = resident();
     begin_epoch();
     launch_epoch();
+    const bool stepped_resident = resident();
     launch_check();
     B200_CHECK(cudaStreamSynchronize(st_));
     {  // the iteration kernels' time, from the events inside the epoch graph
@@ -1459,10 +1465,7 @@ EngineResult Engine::run_pdlp(const DeviceOutputs& out) {
     hp.skip_r0 = 1;
     B200_CHECK(cudaMemcpyAsync(params_.get(), &hp, sizeof(StepParams), cudaMemcpyHostToDevice, st_));
     const int pidx = mixed_now_ ? 1 : 0;
-    if (resident()) {
-      if (mixed_now_) launch_resident_pdlp<float>(cur);
-      else launch_resident_pdlp<double>(cur);
-    } else {
+    if (!resident() || !(mixed_now_ ? launch_resident_pdlp<float>(cur) : launch_resident_pdlp<double>(cur))) {
       if (mixed_now_) capture_pdlp_epoch<float>(cur);
       else capture_pdlp_epoch<double>(cur);
       B200_CHECK(cudaGraphLaunch(g_pdlp_[pidx][cur], st_));
@@ -1667,6 +1670,7 @@ class GroupScheduler {
   // they do not fit that way. Against the step kernels, 16 random LPs of 1k to 18k rows in two groups:
   // 19 us an iteration, checks included, against 27.
   bool resident_epoch(std::vector<Job*>& active) {
+    if (refused_) return false;  // the device does not run these launches: not asked again at every epoch
     int busy = 0;
     for (GroupScheduler* g : peers_()) busy += g->load_.load() > 0 ? 1 : 0;
     const int cap = sm_count() / std::max(1, busy), jobs = static_cast<int>(active.size());
@@ -1706,10 +1710,10 @@ class GroupScheduler {
       else rd_.h.push_back(e.resident_part<double>(first_d, blocks[k])), first_d += blocks[k];
     }
     rd_.upload(st_), rf_.upload(st_);
-    launch_resident_group<ResidentR2h>(rd_.d.get(), static_cast<int>(rd_.h.size()), first_d, rf_.d.get(),
-                                       static_cast<int>(rf_.h.size()), first_d + first_f, threads,
-                                       longest, static_cast<unsigned>(smem), st_);
-    return true;
+    refused_ = !launch_resident_group<ResidentR2h>(rd_.d.get(), static_cast<int>(rd_.h.size()), first_d, rf_.d.get(),
+                                                   static_cast<int>(rf_.h.size()), first_d + first_f, threads, longest,
+                                                   static_cast<unsigned>(smem), st_);
+    return !refused_;
   }
   // One epoch of every active solve: the resident launch, or the grouped step kernels, on the group's stream
   // once every solve's stream is ready; each solve's residual section (when its epoch starts a Halpern
@@ -1824,6 +1828,7 @@ class GroupScheduler {
   Tables<float> tf_;
   Parts<double> rd_;
   Parts<float> rf_;
+  bool refused_ = false;
 };
 
 std::vector<GroupScheduler*> GroupScheduler::peers_() const {

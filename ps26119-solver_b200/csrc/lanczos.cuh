@@ -235,11 +235,10 @@ struct LanczosShape {
   int longest = 0;
   unsigned smem = 0;
 };
-inline LanczosShape lanczos_shape(long long m, long long n, long long nnz, long long max_row, long long max_col) {
+inline LanczosShape lanczos_shape(long long m, long long n, long long nnz, long long max_row, long long max_col, int sms) {
   using B = ResidentBytes<double, LanczosOp>;
   LanczosShape s;
   if (m < 1 || n < 1 || nnz < 1 || n > kLanczosColumns) return s;
-  const int sms = sm_count();
   int blocks = static_cast<int>(std::max(1LL, std::min<long long>(sms, (n + kLanczosShare - 1) / kLanczosShare)));
   auto bytes = [&](int b) { return resident_bytes<double, LanczosOp>(m, n, nnz, max_row, max_col, b); };
   while (blocks < sms && bytes(blocks) > kResidentSmem / 2) ++blocks;
@@ -254,7 +253,8 @@ inline LanczosShape lanczos_shape(long long m, long long n, long long nnz, long 
   s.smem = static_cast<unsigned>(smem);
   return s;
 }
-inline void launch_lanczos(const LanczosArgs& p, const LanczosShape& s, cudaStream_t st) {
+// false: refused (launch_cooperative).
+inline bool launch_lanczos(const LanczosArgs& p, const LanczosShape& s, cudaStream_t st) {
   const auto kernel = [&](auto is_long) {
     constexpr bool kLong = decltype(is_long)::value;
     return s.threads <= 256   ? reinterpret_cast<const void*>(&k_resident_lanczos<256, 16, kLong>)
@@ -264,8 +264,7 @@ inline void launch_lanczos(const LanczosArgs& p, const LanczosShape& s, cudaStre
   const void* f = resident_is_long(s.longest, s.threads) ? kernel(std::true_type{}) : kernel(std::false_type{});
   B200_CHECK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kResidentSmem)));
   void* args[] = {const_cast<LanczosArgs*>(&p)};
-  B200_CHECK(cudaLaunchCooperativeKernel(f, dim3(static_cast<unsigned>(s.blocks)), dim3(static_cast<unsigned>(s.threads)), args,
-                                         s.smem, st));
+  return launch_cooperative(f, s.blocks, s.threads, args, s.smem, st);
 }
 
 }  // namespace b200

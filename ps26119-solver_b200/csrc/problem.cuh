@@ -351,7 +351,7 @@ struct ScaledDevice {
     const int tiles = (n + kXTile - 1) / kXTile;
     // An LP that fits the SMs' shared memory takes a batch of steps in one launch (lanczos.cuh).
     const RowLengths* len = lengths(st);
-    const LanczosShape shape = lanczos_shape(m, n, nnz, len[0].longest, len[1].longest);
+    LanczosShape shape = lanczos_shape(m, n, nnz, len[0].longest, len[1].longest, stream_sm_count(st));
     DevBuf<Cell<double>> cells;
     DevBuf<XFast> fast;
     DevBuf<XTileAgg> full;
@@ -369,14 +369,19 @@ struct ScaledDevice {
     auto launch = [&](int from, int to) {
       if (shape.blocks > 0) {
         Cell<double>* c = cells.get();
-        launch_lanczos({m, n, shape.blocks, t_rp.get(), t_ri.get(), a_rp.get(), a_col.get(), sat.get(), sa.get(),
-                        c, c + n, c + n + m, c + n + m + shape.blocks, c + n + m + 2 * shape.blocks, v.get(), vprev.get(),
-                        terms.get(), hist.get(), fast.get(), full.get(), count.get(), tag, from, to, err},
-                       shape, st);
-        tag += 3u * static_cast<unsigned>(to - from) + 2u;
-        ++kernels;
-        lanczos_launched = to;
-        return;
+        if (launch_lanczos({m, n, shape.blocks, t_rp.get(), t_ri.get(), a_rp.get(), a_col.get(), sat.get(), sa.get(),
+                            c, c + n, c + n + m, c + n + m + shape.blocks, c + n + m + 2 * shape.blocks, v.get(), vprev.get(),
+                            terms.get(), hist.get(), fast.get(), full.get(), count.get(), tag, from, to, err},
+                           shape, st)) {
+          tag += 3u * static_cast<unsigned>(to - from) + 2u;
+          ++kernels;
+          lanczos_launched = to;
+          return;
+        }
+        shape.blocks = 0;  // refused: the kernels' form, from here on
+        pal.build(true, nullptr, st);
+        if (from > 0)
+          B200_CHECK(cudaMemcpyAsync(out.get() + 1, hist.get() + 2 * from - 1, sizeof(double), cudaMemcpyDeviceToDevice, st));
       }
       for (int k = from; k < to; ++k) {
         // every kernel of a step starts while the one before it ends (programmatic dependent launch)

@@ -577,8 +577,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_resident_group(const ResidentPa
   if (b < blocks_d) run(pd, nd, b);
   else run(pf, nf, b - blocks_d);
 }
+// false: refused (launch_cooperative).
 template <template <class> class Op>
-inline void launch_resident_group(const ResidentPart<double, Op<double>>* pd, int nd, int blocks_d,
+inline bool launch_resident_group(const ResidentPart<double, Op<double>>* pd, int nd, int blocks_d,
                                   const ResidentPart<float, Op<float>>* pf, int nf, int blocks, int threads, int longest,
                                   unsigned smem, cudaStream_t st) {
   const auto kernel = [&](auto is_long) {
@@ -590,8 +591,7 @@ inline void launch_resident_group(const ResidentPart<double, Op<double>>* pd, in
   const void* f = resident_is_long(longest, threads) ? kernel(std::true_type{}) : kernel(std::false_type{});
   B200_CHECK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kResidentSmem)));
   void* args[] = {&pd, &nd, &blocks_d, &pf, &nf};
-  B200_CHECK(cudaLaunchCooperativeKernel(f, dim3(static_cast<unsigned>(blocks)), dim3(static_cast<unsigned>(threads)), args, smem,
-                                         st));
+  return launch_cooperative(f, blocks, threads, args, smem, st);
 }
 
 // How one LP's epochs are launched: blocks, threads and dynamic shared memory; blocks = 0: not this way.
@@ -605,12 +605,12 @@ inline int resident_threads(long long m, long long n, int blocks) {
   const long long warps = (n / blocks + 32) / 32 + (m / blocks + 32) / 32 + 1;
   return static_cast<int>(32 * std::min(32LL, std::max(2LL, warps)));
 }
-// One block on each SM (fewer for tiny LPs: at least 8 elements a block).
+// One block on each of sms SMs (fewer for tiny LPs: at least 8 elements a block).
 template <class T, class Op>
-inline ResidentShape resident_shape(long long m, long long n, long long nnz, long long max_row, long long max_col) {
+inline ResidentShape resident_shape(long long m, long long n, long long nnz, long long max_row, long long max_col, int sms) {
   ResidentShape s;
   if (m < 1 || n < 1 || nnz < 1) return s;
-  const int blocks = static_cast<int>(std::max(1LL, std::min<long long>(sm_count(), (m + n + 7) / 8)));
+  const int blocks = static_cast<int>(std::max(1LL, std::min<long long>(sms, (m + n + 7) / 8)));
   const int threads = resident_threads(m, n, blocks), longest = static_cast<int>(std::max(max_row, max_col));
   const long long bytes = resident_bytes<T, Op>(m, n, nnz, max_row, max_col, blocks) + resident_chunks(longest, threads);
   if (bytes > kResidentSmem || (m + n) / blocks > kResidentElements) return s;
@@ -620,9 +620,9 @@ inline ResidentShape resident_shape(long long m, long long n, long long nnz, lon
   s.smem = static_cast<unsigned>(bytes);
   return s;
 }
-// Launches one epoch cooperatively on `st`.
+// Launches one epoch cooperatively on `st`; false: refused (launch_cooperative).
 template <class T, class Op>
-inline void launch_resident(const ResidentPart<T, Op>& p, const ResidentShape& s, cudaStream_t st) {
+inline bool launch_resident(const ResidentPart<T, Op>& p, const ResidentShape& s, cudaStream_t st) {
   const auto kernel = [&](auto is_long) {
     constexpr bool kLong = decltype(is_long)::value;
     return s.threads <= 256   ? reinterpret_cast<const void*>(&k_resident<256, 16, kLong, T, Op>)
@@ -632,8 +632,7 @@ inline void launch_resident(const ResidentPart<T, Op>& p, const ResidentShape& s
   const void* f = resident_is_long(s.longest, s.threads) ? kernel(std::true_type{}) : kernel(std::false_type{});
   B200_CHECK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kResidentSmem)));
   void* args[] = {const_cast<ResidentPart<T, Op>*>(&p)};
-  B200_CHECK(cudaLaunchCooperativeKernel(f, dim3(static_cast<unsigned>(s.blocks)), dim3(static_cast<unsigned>(s.threads)), args,
-                                         s.smem, st));
+  return launch_cooperative(f, s.blocks, s.threads, args, s.smem, st);
 }
 
 }  // namespace b200
