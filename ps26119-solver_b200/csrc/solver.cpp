@@ -1540,8 +1540,8 @@ Solution solve(const Model& model, const Options& options) {  // solve.cpp:194-2
 
 // ============================================================ batch (batch.cpp:129-441)
 namespace {
-std::vector<Solution> run_batch(const Model& base, const std::vector<Scenario>& scenarios, const Options& options) {
-  const auto t0 = clock_t_::now();
+std::vector<Solution> run_batch(const Model& base, const std::vector<Scenario>& scenarios, const Options& options,
+                                clock_t_::time_point t0) {
   const int K = static_cast<int>(scenarios.size());
   std::vector<Solution> out(K);
   auto fail_all = [&](const std::string& why) {
@@ -1623,8 +1623,9 @@ std::vector<Solution> run_batch(const Model& base, const std::vector<Scenario>& 
 }  // namespace
 
 // The fingerprints of the scenario models (batch.cpp:113-127: the base with the scenario's vectors) take as
-// long as the device's setup: they are made beside it.
+// long as the device's setup: they are made beside it, where the host passes may use more than one thread.
 std::vector<Solution> solve_batch(const Model& base, const std::vector<Scenario>& scenarios, const Options& options) {
+  const auto t0 = clock_t_::now();
   std::vector<std::uint64_t> fp;
   std::exception_ptr err;
   auto make = [&] {
@@ -1640,12 +1641,14 @@ std::vector<Solution> solve_batch(const Model& base, const std::vector<Scenario>
       if (t.joinable()) t.join();
     }
   } side;
-  try {
-    side.t = std::thread(make);
-  } catch (const std::system_error&) {
-    make();
+  if (host_thread_limit() > 1) {
+    try {
+      side.t = std::thread(make);
+    } catch (const std::system_error&) {
+    }
   }
-  std::vector<Solution> out = run_batch(base, scenarios, options);
+  if (!side.t.joinable()) make();
+  std::vector<Solution> out = run_batch(base, scenarios, options, t0);
   if (side.t.joinable()) side.t.join();
   if (err) std::rethrow_exception(err);
   for (std::size_t k = 0; k < out.size(); ++k) {
