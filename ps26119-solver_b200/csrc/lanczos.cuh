@@ -12,6 +12,10 @@
 //      exact sum in a cell that every block waits for.
 // Everything is in the kernels' order and arithmetic, so α and β² are the same bits.
 //
+// A wait that runs out leaves the block with NaN and without its place among the runs: it goes on at place 0, and
+// a walk may then meet summaries of other sums, or none. All of them (the arrays start at zero) name terms that
+// exist, so every access stays inside its array and the kernel ends; the counter `err` makes the estimate an error.
+//
 // Why no cell is overwritten too early: v's and t's as in resident.cuh. A block writes its sums cell anew
 // only after it has had the result of the sum before, which the last block to count in leaves, and a block
 // counts in after it has read the earlier blocks' cells; the result's cell is written anew only once every
@@ -43,6 +47,7 @@ struct LanczosArgs {
   // cells of an LP: n of v, m of t, two per block, the sums' result
   static long long cells(long long m, long long n, int blocks) { return n + m + 2LL * blocks + 1; }
   int from, to;
+  int polls;  // reads of a cell before a wait for the sums gives up
   unsigned* err;
 };
 // What a block holds: three vectors and a term per column, nothing but the entries per row.
@@ -51,12 +56,12 @@ struct LanczosOp {
 };
 
 // Waits (one thread) until the cell has this tag.
-__device__ __forceinline__ double cell_wait(const Cell<double>* c, unsigned tag, bool& dead) {
+__device__ __forceinline__ double cell_wait(const Cell<double>* c, unsigned tag, int limit, bool& dead) {
   CellRead<double> g{};
   for (int polls = 0; !dead; ++polls) {
     cell_load(g, c, true);
     if (g.is(tag)) return g.value();
-    if (polls > kResidentPolls) dead = true;  // never expected
+    if (polls >= limit) dead = true;  // never expected
   }
   return __longlong_as_double(0x7ff8000000000000LL);
 }
@@ -88,12 +93,12 @@ __device__ __forceinline__ double lanczos_sum(const LanczosArgs& p, LanczosShare
   if (tid == 0) cell_store(p.sums + g, s, tag);
   // the earlier blocks' sums: watch the nearest one, then read all of them
   if (g > 0 && w == 0) {
-    if (lane == 0) cell_wait(p.sums + g - 1, tag, dead);
+    if (lane == 0) cell_wait(p.sums + g - 1, tag, p.polls, dead);
     __syncwarp();
   }
   __syncthreads();
   s = 0.0;
-  for (int k = tid; k < g; k += static_cast<int>(blockDim.x)) s += cell_wait(p.sums + k, tag, dead);
+  for (int k = tid; k < g; k += static_cast<int>(blockDim.x)) s += cell_wait(p.sums + k, tag, p.polls, dead);
   const double before = block_sum(s);
   const int tiles = (count + kXTile - 1) / kXTile;
   for (int q = w; q < tiles; q += warps) {
@@ -125,7 +130,7 @@ __device__ __forceinline__ double lanczos_sum(const LanczosArgs& p, LanczosShare
       const XRound N = round(k0 + 32);
       r = x_walk_lanes(r, R, min(32, all - k0), [&](int k, double st) {
         const int a = __shfl_sync(kFull, R.fast.first, k), len = __shfl_sync(kFull, R.fast.len, k);
-        return x_add(p.terms, a, a + len, st, sh.add);
+        return x_add(p.terms, a, min(a + len, p.n), st, sh.add);
       });
       R = N;
     }
@@ -134,7 +139,7 @@ __device__ __forceinline__ double lanczos_sum(const LanczosArgs& p, LanczosShare
       cell_store(p.scalar, r, tag);
     }
   }
-  if (tid == 0) sh.value = cell_wait(p.scalar, tag, dead);
+  if (tid == 0) sh.value = cell_wait(p.scalar, tag, p.polls, dead);
   __syncthreads();
   return sh.value;
 }
@@ -162,7 +167,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_resident_lanczos(const __grid_c
   if (warp == 0) {
     double mine = 0.0, all = 0.0;
     for (int k = lane; k < p.blocks; k += 32) {
-      const double t = cell_wait(p.runs + k, p.tag, dead);
+      const double t = cell_wait(p.runs + k, p.tag, p.polls, dead);
       all += t;
       if (k < g) mine += t;
     }
@@ -170,7 +175,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_resident_lanczos(const __grid_c
       mine += __shfl_xor_sync(kFull, mine, off);
       all += __shfl_xor_sync(kFull, all, off);
     }
-    if (dead) mine = all = 0.0;
+    dead = __any_sync(kFull, dead);
+    if (dead) mine = all = 0.0;  // not NaN, which would become places outside the arrays
     if (lane == 0) sh.tile0 = static_cast<int>(mine), sh.tiles = static_cast<int>(all);
   }
   unsigned tag = p.tag + 1;
@@ -252,6 +258,11 @@ inline LanczosShape lanczos_shape(long long m, long long n, long long nnz, long 
   s.longest = longest;
   s.smem = static_cast<unsigned>(smem);
   return s;
+}
+// PS26119_LANCZOS_POLLS: another limit of those waits (read at every estimate; a test lets them run out).
+inline int lanczos_polls() {
+  const char* e = std::getenv("PS26119_LANCZOS_POLLS");
+  return e && *e ? std::max(0, std::atoi(e)) : kResidentPolls;
 }
 // false: refused (launch_cooperative).
 inline bool launch_lanczos(const LanczosArgs& p, const LanczosShape& s, cudaStream_t st) {

@@ -328,8 +328,16 @@ struct ScaledDevice {
   // and replays the reference's per-step decisions on them (Sturm bisection, breakdown and
   // stagnation tests) in step order while the device runs the next batch. The result and the number
   // of steps that count are the sequential loop's; steps run past the stopping one are discarded.
+  // err: the caller's counter of waits that ran out on the device (nullptr: one of this call's own). When it
+  // counts any the estimate ends there and throws.
   double lanczos(cudaStream_t st, unsigned* err = nullptr) {
     if (n == 0 || nnz == 0) return 0.0;
+    DevBuf<unsigned> own;
+    if (!err) {
+      own.alloc(1);
+      B200_CHECK(cudaMemsetAsync(own.get(), 0, sizeof(unsigned), st));
+      err = own.get();
+    }
     const int K = 400;
     const double rel_tol = 1e-12;
     lanczos_launched = 0;
@@ -357,11 +365,13 @@ struct ScaledDevice {
     DevBuf<XTileAgg> full;
     DevBuf<unsigned> count(1);
     unsigned tag = 1;
+    const int polls = lanczos_polls();
     if (shape.blocks > 0) {
       cells.alloc(static_cast<std::size_t>(LanczosArgs::cells(m, n, shape.blocks)));
       fast.alloc(static_cast<std::size_t>(n / kXTile + shape.blocks));
       full.alloc(static_cast<std::size_t>(n / kXTile + shape.blocks));
       B200_CHECK(cudaMemsetAsync(cells.get(), 0, cells.size() * sizeof(Cell<double>), st));
+      B200_CHECK(cudaMemsetAsync(fast.get(), 0, fast.size() * sizeof(XFast), st));
       B200_CHECK(cudaMemsetAsync(count.get(), 0, sizeof(unsigned), st));
     } else {
       pal.build(true, nullptr, st);
@@ -371,7 +381,7 @@ struct ScaledDevice {
         Cell<double>* c = cells.get();
         if (launch_lanczos({m, n, shape.blocks, t_rp.get(), t_ri.get(), a_rp.get(), a_col.get(), sat.get(), sa.get(),
                             c, c + n, c + n + m, c + n + m + shape.blocks, c + n + m + 2 * shape.blocks, v.get(), vprev.get(),
-                            terms.get(), hist.get(), fast.get(), full.get(), count.get(), tag, from, to, err},
+                            terms.get(), hist.get(), fast.get(), full.get(), count.get(), tag, from, to, polls, err},
                            shape, st)) {
           tag += 3u * static_cast<unsigned>(to - from) + 2u;
           ++kernels;
@@ -399,7 +409,9 @@ struct ScaledDevice {
       lanczos_launched = to;
     };
     PinnedBuf<double> h;
-    h.alloc(2 * static_cast<std::size_t>(K));
+    PinnedBuf<unsigned> ran_out;
+    h.alloc(2 * static_cast<std::size_t>(K)), ran_out.alloc(1);
+    ran_out[0] = 0;
     Event landed[2];
     std::vector<double> alpha, beta;
     double theta = 0, theta_old = -1;
@@ -408,6 +420,7 @@ struct ScaledDevice {
     auto fetch = [&](int a, int b, int s) {
       B200_CHECK(cudaMemcpyAsync(h.get() + 2 * a, hist.get() + 2 * a, 2 * static_cast<std::size_t>(b - a) * sizeof(double),
                                  cudaMemcpyDeviceToHost, st));
+      B200_CHECK(cudaMemcpyAsync(ran_out.get(), err, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
       B200_CHECK(cudaEventRecord(landed[s].get(), st));
     };
     launch(from, to);
@@ -422,6 +435,7 @@ struct ScaledDevice {
       };
       if (ahead) go_on();
       B200_CHECK(cudaEventSynchronize(landed[slot].get()));
+      if (ran_out[0]) break;
       for (int k = from; k < to; ++k) alpha.push_back(h[2 * k]), beta.push_back(std::sqrt(h[2 * k + 1]));
       double thetas[21];
       tridiag_max_eigs(alpha.data(), beta.data(), from + 1, to - from, thetas);
@@ -438,6 +452,7 @@ struct ScaledDevice {
       from = to, to = next, slot ^= 1;
     }
     B200_CHECK(cudaStreamSynchronize(st));  // the steps past the stop, before their buffers go back
+    if (ran_out[0]) throw CudaError("a shared-memory staging wait timed out on the device");
     return std::sqrt(std_max(theta, 0.0)) * (1.0 + 1e-4);
   }
 
