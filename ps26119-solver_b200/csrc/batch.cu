@@ -1072,12 +1072,14 @@ void BatchEngine::compact(const std::vector<int>& keep) {
 }
 
 // The solutions of the slots that end at this check (batch.cpp:276-298): x, y = sense·y_min, z = c − Aᵀy
-// (CSC order) and objective = offset + Σ c x, all of them in a few launches and one staged copy.
+// (CSC order) and objective = offset + Σ c x, all of them in a few launches and one staged copy. They lie in the
+// blocks of terms, which the next check writes anew: a batch that has just fit the device's memory also ends there.
 void BatchEngine::finish_slots(const std::vector<Finished>& done) {
   const int F = static_cast<int>(done.size());
   if (F == 0) return;
   const std::size_t n = static_cast<std::size_t>(n_), m = static_cast<std::size_t>(m_), f = static_cast<std::size_t>(F);
-  DevBuf<double> x(f * n), terms(f * n), z(f * n), y(f * m), obj(f);
+  DevBuf<double>&x = nv_[TPX], &terms = nv_[TDXN], &z = nv_[TP], &y = mv_[TPY];
+  DevBuf<double> obj(f);
   DevBuf<int> slot(f);
   std::vector<int> hs;
   for (const Finished& d : done) hs.push_back(d.slot);
