@@ -93,7 +93,9 @@ static __global__ void k_lanczos_normalise(int n, double* v, double* vprev, cons
     vprev[j] = 0.0;
   }
 }
-// After w = Ãᵀt: the terms of α = wᵀv and their tile sums (reduce.cuh) on the way.
+// After w = Ãᵀt: the terms of α = wᵀv and, where a slab is a tile of terms, their tile sums (reduce.cuh) on the
+// way (stat: null otherwise, and the sum makes its own).
+constexpr bool kLanczosStat = kSlabRows == kXTile;
 struct EpiLanczosW : AlwaysActive {
   const double* v;
   double *w, *terms, *stat;
@@ -398,13 +400,14 @@ struct ScaledDevice {
         launch_slab_tma<double>(m, a_rp.get(), a_col.get(), sa.get(), v.get(), EpiStore<double>{{}, t.get()}, st,
                                 nullptr, err, true);
         launch_slab_tma<double>(n, t_rp.get(), t_ri.get(), sat.get(), t.get(),
-                                EpiLanczosW{{}, v.get(), w.get(), terms.get(), pal.stat()}, st, nullptr, err, true);
-        pal.launch(st, true);
+                                EpiLanczosW{{}, v.get(), w.get(), terms.get(), kLanczosStat ? pal.stat() : nullptr}, st,
+                                nullptr, err, true);
+        pal.launch(st, kLanczosStat);
         // β of the previous step is still in out[1]: this step's β² overwrites it only below
         launch_pdl(k_lanczos_update, tiles, kXTile, st, n, w.get(), v.get(), vprev.get(), out.get(), terms.get(), pbn.stat());
         pbn.launch(st, true);
         launch_pdl(k_lanczos_next, grid_for(n), kBlock, st, n, w.get(), v.get(), vprev.get(), out.get(), hist.get() + 2 * k);
-        kernels += 6;
+        kernels += 5 + (kLanczosStat ? 1 : pal.kernel_count());
       }
       lanczos_launched = to;
     };

@@ -182,9 +182,6 @@ __device__ __forceinline__ bool x_binade(double v, int& e) {
 // The sign and exponent of v: two numbers of which one lies in a binade lie in the same one, with the
 // same sign, where these agree.
 __device__ __forceinline__ int x_top(double v) { return __double2hiint(v) >> 20; }
-__device__ __forceinline__ double x_pow2(int p) {  // 2^p, p in [−1022, 1023]
-  return __longlong_as_double(static_cast<long long>(p + 1023) << 52);
-}
 // A normal s as an integer multiple S of its binade's ulp, |S| in [2^52, 2^53), and back (by its bits).
 __device__ __forceinline__ long long x_int(double s) {
   const long long b = __double_as_longlong(s), m = (b & (kX52 - 1)) | kX52;
