@@ -56,7 +56,8 @@ __device__ __forceinline__ double block_sum_fixed(double v, double* sh) {
 // walk whose only dependence on the past is the parity of S: a run of terms is summarised by its
 // effect for each of the two parities (XRun), and effects compose associatively. So:
 //   k_xstat   per tile of kXTile terms (one warp): an approximate fp64 sum, in any order; only used
-//             to guess each tile's binade. A kernel that produces the terms may leave it itself.
+//             to guess each tile's binade. A kernel that produces the terms may leave it itself. Long chains:
+//             k_xspan adds them up by spans of kXSpan tiles.
 //   k_xwalk   one warp per tile, kXWarps tiles per block: the guessed binade's u from the approximate
 //             start (the approximate sums of the chain's earlier tiles), then the tile's XRun (change of
 //             S, bounds of its running value, parity after, per parity before): each lane adds its terms
@@ -96,6 +97,11 @@ constexpr int kXTile = 32 * kXPer;    // terms per tile (one warp)
 constexpr int kXGroup = 32;           // tiles per group (one warp lane each)
 constexpr int kXWarps = 8;            // warps per block of k_xwalk, tiles per block
 constexpr long long kXShort = 1024;   // chains up to this long are added one by one by a warp
+// Every block adds up the approximate sums of all tiles before its own: the reads grow with the square of the
+// chain. In chains of more than kXSpanMin tiles (3M terms) the tiles come in spans of kXSpan whose sums k_xspan
+// makes first, so that a block reads at most one span's tiles and the spans before it. One call, without / with
+// spans: 8M terms 165 / 157 us, 16M 326 / 257, 64M 1.91 / 0.87 ms, 256M 22.8 / 3.4; 4.5M 108 / 111 us.
+constexpr int kXSpan = 1024, kXSpanMin = 12288;
 
 struct XChain {
   const double* t;
@@ -105,6 +111,7 @@ struct XChain {
   int tile0, ntiles;    // this chain's tiles in the tile arrays (ntiles = 0: added one by one)
   int group0, ngroups;  // its groups of kXGroup tiles
   int block0;           // its first block of kXWarps tiles
+  int span0;            // its first span (−1: none)
   int job;              // its kChunk64 job (−1: *out is the chain's own result)
 };
 // A kChunk64 job: the chains of its chunks leave their sums in part[0, chunks); the chain that
@@ -307,13 +314,14 @@ __device__ __forceinline__ double x_add(const double* t, long long a, long long 
   return s;
 }
 
-static __global__ void __launch_bounds__(256) k_xstat(const XChain* ch, const int* tile_chain, int ntiles,
-                                                      double* stat, const int* skip) {
+// Blocks as k_xwalk's: kXWarps tiles of one chain each.
+static __global__ void __launch_bounds__(32 * kXWarps) k_xstat(const XChain* ch, const int* block_chain, double* stat,
+                                                               const int* skip) {
   if (skip && *skip) return;
-  const int tile = static_cast<int>((blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) >> 5);
+  const XChain& c = ch[block_chain[blockIdx.x]];
   const int lane = threadIdx.x & 31;
-  if (tile >= ntiles) return;
-  const XChain& c = ch[tile_chain[tile]];
+  const int tile = c.tile0 + (static_cast<int>(blockIdx.x) - c.block0) * kXWarps + static_cast<int>(threadIdx.x >> 5);
+  if (tile >= c.tile0 + c.ntiles) return;
   long long a, b;
   x_tile_range(c, tile, a, b);
   double v[kXPer], s = 0.0;
@@ -323,6 +331,18 @@ static __global__ void __launch_bounds__(256) k_xstat(const XChain* ch, const in
   for (int q = 0; q < kXPer; ++q) s += v[q];
   for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(kFull, s, off);
   if (lane == 0) stat[tile] = s;
+}
+// Approximate sums of spans of tiles; one block each. span_chain: the chain.
+static __global__ void __launch_bounds__(256) k_xspan(const XChain* ch, const int* span_chain, const double* stat, double* span,
+                                                      const int* skip) {
+  __shared__ double sh[32];
+  if (skip && *skip) return;
+  const XChain& c = ch[span_chain[blockIdx.x]];
+  const int k0 = (static_cast<int>(blockIdx.x) - c.span0) * kXSpan;
+  double s = 0.0;
+  for (int k = k0 + static_cast<int>(threadIdx.x); k < min(k0 + kXSpan, c.ntiles); k += 256) s += stat[c.tile0 + k];
+  s = block_sum_fixed(s, sh);
+  if (threadIdx.x == 0) span[blockIdx.x] = s;
 }
 // A producer's own tile sum: called by every thread of a block of kXTile threads whose thread i
 // made term i of tile blockIdx.x; stat may be null (a chain that needs none).
@@ -682,7 +702,8 @@ __device__ __forceinline__ XSummary x_group(const XFast* tf, const XTileAgg* ag,
 static __global__ void __launch_bounds__(32 * kXWarps) k_xwalk(const XChain* __restrict__ ch, const XJob* __restrict__ jobs,
                                                                const int* __restrict__ block_chain, int nblocks,
                                                                const int* __restrict__ short_chain, int nshort,
-                                                               const double* stat, XFast* tf, XTileAgg* ag, XFast* gf,
+                                                               const double* stat, const double* span, XFast* tf,
+                                                               XTileAgg* ag, XFast* gf,
                                                                XTileAgg* gg, unsigned* group_done, unsigned* chain_done,
                                                                unsigned* job_done, const int* skip) {
   __shared__ alignas(16) double sh_add[kXWarps][kXTile];
@@ -718,7 +739,12 @@ static __global__ void __launch_bounds__(32 * kXWarps) k_xwalk(const XChain* __r
     const XTerms mine_t = x_terms(c.t, a, b);  // none past the chain's last tile
     const double mine = lane < w && k0 + lane < c.ntiles ? stat[c.tile0 + k0 + lane] : 0.0;
     double pre = 0.0;  // the approximate sum before this block's tiles
-    for (int q = threadIdx.x; q < k0; q += 32 * kXWarps) pre += stat[c.tile0 + q];
+    int from = 0;
+    if (c.span0 >= 0) {
+      from = k0 / kXSpan * kXSpan;
+      for (int q = threadIdx.x; q < k0 / kXSpan; q += 32 * kXWarps) pre += span[c.span0 + q];
+    }
+    for (int q = from + static_cast<int>(threadIdx.x); q < k0; q += 32 * kXWarps) pre += stat[c.tile0 + q];
     for (int off = 16; off > 0; off >>= 1) pre += __shfl_xor_sync(kFull, pre, off);
     if (lane == 0) sh_sum[w] = pre;
     __syncthreads();
@@ -800,22 +826,26 @@ class SumPlan {
     if (exact) {
       std::vector<XChain> chains;
       std::vector<XJob> jobs;
-      ngroups_ = 0;
-      std::vector<int> tile_chain, block_chain, short_chain;
+      ntiles_ = ngroups_ = 0;
+      std::vector<int> block_chain, short_chain, span_chain;
       long long nchunk_jobs = 0;
       for (const Job& j : jobs_)
         if (j.order == SumOrder::kChunk64) ++nchunk_jobs;
       partials_.alloc(static_cast<std::size_t>(nchunk_jobs > 0 ? nchunk_jobs * kChunks : 1));
       auto chain = [&](const double* t, long long lo, long long hi, double init, double* out, int job) {
-        XChain c{t, lo, hi, init, out, static_cast<int>(tile_chain.size()), 0, ngroups_, 0,
-                 static_cast<int>(block_chain.size()), job};
+        XChain c{t, lo, hi, init, out, ntiles_, 0, ngroups_, 0,
+                 static_cast<int>(block_chain.size()), -1, job};
         const int id = static_cast<int>(chains.size());
         if (hi - lo > kXShort) {
           c.ntiles = static_cast<int>((hi - lo + kXTile - 1) / kXTile);
           c.ngroups = (c.ntiles + kXGroup - 1) / kXGroup;
-          tile_chain.insert(tile_chain.end(), static_cast<std::size_t>(c.ntiles), id);
+          ntiles_ += c.ntiles;
           ngroups_ += c.ngroups;
           block_chain.insert(block_chain.end(), static_cast<std::size_t>((c.ntiles + kXWarps - 1) / kXWarps), id);
+          if (c.ntiles > kXSpanMin) {
+            c.span0 = static_cast<int>(span_chain.size());
+            span_chain.insert(span_chain.end(), static_cast<std::size_t>((c.ntiles + kXSpan - 1) / kXSpan), id);
+          }
         } else {
           short_chain.push_back(id);
         }
@@ -833,14 +863,14 @@ class SumPlan {
           jobs.push_back({part, static_cast<int>(chunks), j.init, j.out});
         }
       }
-      ntiles_ = static_cast<int>(tile_chain.size());
       nblocks_ = static_cast<int>(block_chain.size());
       nshort_ = static_cast<int>(short_chain.size());
+      nspans_ = static_cast<int>(span_chain.size());
       upload(chains, chains_, st);
       upload(jobs, xjobs_, st);
-      upload(tile_chain, tile_chain_, st);
       upload(block_chain, block_chain_, st);
       upload(short_chain, short_chain_, st);
+      if (nspans_ > 0) upload(span_chain, span_chain_, st), span_.alloc(span_chain.size());
       stat_.alloc(static_cast<std::size_t>(ntiles_ > 0 ? ntiles_ : 1));
       tile_fast_.alloc(static_cast<std::size_t>(ntiles_ > 0 ? ntiles_ : 1) * sizeof(XFast));
       group_fast_.alloc(static_cast<std::size_t>(ngroups_ > 0 ? ngroups_ : 1) * sizeof(XFast));
@@ -869,8 +899,11 @@ class SumPlan {
     if (exact_) {
       const XChain* ch = reinterpret_cast<const XChain*>(chains_.get());
       if (ntiles_ > 0 && !have_stat) {
-        k_xstat<<<(ntiles_ + 7) / 8, 256, 0, st>>>(ch, reinterpret_cast<const int*>(tile_chain_.get()), ntiles_,
-                                                   stat_.get(), skip);
+        k_xstat<<<nblocks_, 32 * kXWarps, 0, st>>>(ch, reinterpret_cast<const int*>(block_chain_.get()), stat_.get(), skip);
+        B200_LAUNCH_CHECK();
+      }
+      if (nspans_ > 0) {
+        k_xspan<<<nspans_, 256, 0, st>>>(ch, reinterpret_cast<const int*>(span_chain_.get()), stat_.get(), span_.get(), skip);
         B200_LAUNCH_CHECK();
       }
       const int blocks = nblocks_ + (nshort_ + kXWarps - 1) / kXWarps;
@@ -889,7 +922,8 @@ class SumPlan {
         B200_CHECK(cudaLaunchKernelEx(&cfg, k_xwalk, ch, reinterpret_cast<const XJob*>(xjobs_.get()),
                                       reinterpret_cast<const int*>(block_chain_.get()), nblocks_,
                                       reinterpret_cast<const int*>(short_chain_.get()), nshort_,
-                                      static_cast<const double*>(stat_.get()), reinterpret_cast<XFast*>(tile_fast_.get()),
+                                      static_cast<const double*>(stat_.get()), static_cast<const double*>(span_.get()),
+                                      reinterpret_cast<XFast*>(tile_fast_.get()),
                                       reinterpret_cast<XTileAgg*>(tile_agg_.get()),
                                       reinterpret_cast<XFast*>(group_fast_.get()),
                                       reinterpret_cast<XTileAgg*>(group_agg_.get()), done, done + ngroups_,
@@ -902,7 +936,7 @@ class SumPlan {
     }
   }
   int kernel_count() const {
-    return exact_ ? (ntiles_ > 0) + (nblocks_ + nshort_ > 0) : (nt_ > 0 ? 1 : 0);
+    return exact_ ? (ntiles_ > 0) + (nspans_ > 0) + (nblocks_ + nshort_ > 0) : (nt_ > 0 ? 1 : 0);
   }
   bool empty() const { return jobs_.empty(); }
 
@@ -926,11 +960,11 @@ class SumPlan {
   std::vector<Job> jobs_;
   bool exact_ = false;
   const int* skip_ = nullptr;
-  DevBuf<unsigned char> chains_, xjobs_, tseg_, tile_chain_, block_chain_, short_chain_;
+  DevBuf<unsigned char> chains_, xjobs_, tseg_, block_chain_, short_chain_, span_chain_;
   mutable DevBuf<unsigned char> tile_fast_, group_fast_, tile_agg_, group_agg_;
-  mutable DevBuf<double> partials_, stat_;
+  mutable DevBuf<double> partials_, stat_, span_;
   mutable DevBuf<unsigned> done_;
-  int nchains_ = 0, nshort_ = 0, nt_ = 0, ntiles_ = 0, nblocks_ = 0, ngroups_ = 0;
+  int nchains_ = 0, nshort_ = 0, nt_ = 0, ntiles_ = 0, nblocks_ = 0, ngroups_ = 0, nspans_ = 0;
 };
 
 }  // namespace b200
