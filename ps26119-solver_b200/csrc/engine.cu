@@ -104,9 +104,11 @@ struct IterVecs {
   // resident epochs (resident.cuh): the points after a Halpern cycle's first step, the cells of x̄ and y
   DevBuf<T> xh0, xb0, yh0, yb0;
   DevBuf<Cell<T>> xcell, ycell;
-  void alloc(int n, int m) {
-    for (DevBuf<T>* v : {&x, &x0, &xh, &xb, &dx}) v->alloc(static_cast<std::size_t>(n));
-    for (DevBuf<T>* v : {&y, &y0, &yh, &yb, &dy}) v->alloc(static_cast<std::size_t>(m));
+  // dx, dy: PDLP's running averages
+  void alloc(int n, int m, bool pdlp) {
+    for (DevBuf<T>* v : {&x, &x0, &xh, &xb}) v->alloc(static_cast<std::size_t>(n));
+    for (DevBuf<T>* v : {&y, &y0, &yh, &yb}) v->alloc(static_cast<std::size_t>(m));
+    if (pdlp) dx.alloc(static_cast<std::size_t>(n)), dy.alloc(static_cast<std::size_t>(m));
   }
   void alloc_resident(int n, int m, cudaStream_t st) {
     for (DevBuf<T>* v : {&xh0, &xb0}) v->alloc(static_cast<std::size_t>(n));
@@ -275,8 +277,12 @@ class Engine {
   PinnedBuf<StepParams> hparams_;
   DevBuf<double> res_;
   PinnedBuf<double> hres_;
-  DevBuf<double4> X4_, Y4_;  // a check's packed points
-  DevBuf<double> rt_, kt_, kt2_, rayt_, xo_, yo_, r1_, d1_, r2_, d2_, objt_;
+  // A check's packed points and its term arrays (rayt_: of two rays). A solve's end and a warm start's first look
+  // come before or after all checks and lie in the same memory: the unscaled point where the packed points are, the
+  // rays and the objective's terms where the second ray's terms are. (Large LPs are limited by memory.)
+  DevBuf<double4> X4_, Y4_;
+  DevBuf<double> rt_, kt_, rayt_;
+  double *xo_ = nullptr, *yo_ = nullptr, *ray_r_ = nullptr, *ray_d_ = nullptr, *objt_ = nullptr;
   SumPlan plan_r0_, plan_pid_, plan_kkt_, plan_obj_, plan_chk_;
   SumPlan plan_check_[3];  // a check's sums (residual, KKT, rays), by its variant
   cudaGraphExec_t g_epoch_[2] = {nullptr, nullptr};
@@ -344,8 +350,8 @@ void Engine::setup() {
   const RowLengths* len = sp_.lengths(st_);
   cap_a_ = fed_tile_capacity(len[0].slab);
   cap_t_ = fed_tile_capacity(len[1].slab);
-  vd_.alloc(n, m);
-  if (o_.mixed) vf_.alloc(n, m);
+  vd_.alloc(n, m, o_.pdlp);
+  if (o_.mixed) vf_.alloc(n, m, o_.pdlp);
   rows_ = len[0], cols_ = len[1];
   if (tune_forced() < 0) {  // a forced step-kernel variant runs the step kernels
     plan_resident<double>();
@@ -357,18 +363,18 @@ void Engine::setup() {
   hres_.alloc(kNumSlots);
   B200_CHECK(cudaMemsetAsync(res_.get(), 0, kNumSlots * sizeof(double), st_));
   const std::size_t mm = static_cast<std::size_t>(m), nn = static_cast<std::size_t>(n);
-  rt_.alloc(2 * nn + 3 * mm);
+  // (PDLP: the second set of KKT terms, used up when the distances' terms are made)
+  rt_.alloc(o_.pdlp ? 4 * (mm + nn) : 2 * nn + 3 * mm);
   kt_.alloc(4 * (mm + nn));
   rayt_.alloc(2 * (2 * (mm + nn) + 2 * nn));
   X4_.alloc(nn), Y4_.alloc(mm);
   if (o_.pdlp) {
-    kt2_.alloc(4 * (mm + nn));
     res2_.alloc(kNumSlots);
     hres2_.alloc(kNumSlots);
     B200_CHECK(cudaMemsetAsync(res2_.get(), 0, kNumSlots * sizeof(double), st_));
   }
-  xo_.alloc(nn), yo_.alloc(mm), r1_.alloc(mm), d1_.alloc(nn), r2_.alloc(mm), d2_.alloc(nn);
-  objt_.alloc(mm + 2 * nn);
+  xo_ = reinterpret_cast<double*>(X4_.get()), yo_ = reinterpret_cast<double*>(Y4_.get());
+  ray_r_ = rayt_.get() + 2 * (mm + nn) + 2 * nn, ray_d_ = ray_r_ + mm, objt_ = ray_d_ + nn;  // and m + 2n
   build_plans();
   mark("tables+buffers+plans");
   if (o_.mixed) tune_slab<float>();
@@ -480,7 +486,7 @@ void Engine::build_plans() {
       p.add(t + 3 * L, m, L, 0.0, SumOrder::kSeq, r + kP);
     };
     if (o_.pdlp) {
-      kkt(kt2_.get(), res2_.get());  // the current point's; K0: the average's
+      kkt(rt_.get(), res2_.get());  // the current point's; K0: the average's
     } else {
       p.add(px, 0, n, 0.0, SumOrder::kChunk64, R + kPx);
       p.add(py, 0, m, 0.0, SumOrder::kChunk64, R + kPy);
@@ -497,7 +503,7 @@ void Engine::build_plans() {
     p.build(o_.exact, nullptr, st_);
   }
   // finish: objective = offset + Σ c x (Model::objective_value), check sums (solution_checker)
-  double* O = objt_.get();
+  double* O = objt_;
   plan_obj_.add(O, 0, n, M_.offset, SumOrder::kSeq, R + kObjective);
   plan_chk_.add(O + n, 0, L, 0.0, SumOrder::kSeq, R + kChkDual);
   plan_chk_.add(O, 0, n, 0.0, SumOrder::kSeq, R + kChkPrimal);
@@ -518,11 +524,11 @@ void Engine::launch_first_residual(const int* skip, bool apart) {
   double* px = rt_.get();
   double* py = px + 2 * n;
   const bool f = apart;
-  k_res_x<T><<<grid_for(n), kBlock, 0, st_>>>(n, (f ? v.xb0 : v.xb).get(), (f ? v.xh0 : v.xh).get(), v.dx.get(), px,
-                                              skip);
+  T* dx = reinterpret_cast<T*>(X4_.get());  // before the check packs its points there
+  k_res_x<T><<<grid_for(n), kBlock, 0, st_>>>(n, (f ? v.xb0 : v.xb).get(), (f ? v.xh0 : v.xh).get(), dx, px, skip);
   B200_LAUNCH_CHECK();
   EpiResY<T> e{(f ? v.yb0 : v.yb).get(), (f ? v.yh0 : v.yh).get(), py, py + m, skip};
-  launch_slab_tma<T>(m, sp_.a_rp.get(), sp_.a_col.get(), sp_.A_val<T>(), v.dx.get(), e, st_, nullptr, err());
+  launch_slab_tma<T>(m, sp_.a_rp.get(), sp_.a_col.get(), sp_.A_val<T>(), dx, e, st_, nullptr, err());
   plan_r0_.launch(st_, false, skip != nullptr);
   B200_COUNT(2 + plan_r0_.kernel_count());
 }
@@ -532,11 +538,11 @@ void Engine::launch_kkt_original() {
   const int m = M_.m, n = M_.n;
   const long long L = static_cast<long long>(m) + n;
   double* K0 = kt_.get();
-  EpiKktRows er{{}, yo_.get(), M_.row_lower, M_.row_upper, K0, K0 + L, K0 + 2 * L, res_.get()};
-  launch_slab_tma<double>(m, sp_.a_rp.get(), sp_.a_col.get(), sp_.a_v0.get(), xo_.get(), er, s, nullptr, err());
-  EpiKktCols ec{{}, xo_.get(), M_.c, M_.col_lower, M_.col_upper, static_cast<double>(M_.sense), m,
+  EpiKktRows er{{}, yo_, M_.row_lower, M_.row_upper, K0, K0 + L, K0 + 2 * L, res_.get()};
+  launch_slab_tma<double>(m, sp_.a_rp.get(), sp_.a_col.get(), sp_.a_v0.get(), xo_, er, s, nullptr, err());
+  EpiKktCols ec{{}, xo_, M_.c, M_.col_lower, M_.col_upper, static_cast<double>(M_.sense), m,
                 K0 + 3 * L, K0 + L, K0 + 2 * L, res_.get()};
-  launch_slab<double>(n, M_.col_start, M_.row_index, M_.value, yo_.get(), ec, s, nullptr, err());
+  launch_slab<double>(n, M_.col_start, M_.row_index, M_.value, yo_, ec, s, nullptr, err());
   plan_kkt_.launch(s);
   B200_COUNT(2 + plan_kkt_.kernel_count());
 }
@@ -546,8 +552,8 @@ void Engine::launch_kkt_scaled(const T* xs, const T* ys) {
   const cudaStream_t s = st_;
   const int m = M_.m, n = M_.n;
   k_unscale_x<T><<<grid_for(n), kBlock, 0, s>>>(n, xs, sp_.col_scale.get(), sp_.bound_scale, M_.col_lower,
-                                                M_.col_upper, xo_.get());
-  k_unscale_y<T><<<grid_for(m), kBlock, 0, s>>>(m, ys, sp_.row_scale.get(), sp_.obj_scale, yo_.get());
+                                                M_.col_upper, xo_);
+  k_unscale_y<T><<<grid_for(m), kBlock, 0, s>>>(m, ys, sp_.row_scale.get(), sp_.obj_scale, yo_);
   B200_LAUNCH_CHECK();
   B200_COUNT(2);
   launch_kkt_original();
@@ -794,8 +800,8 @@ bool Engine::apply_warm_start() {
     }
   }
   // decide the working precision before uploading (PrecisionPolicy::on_warm_start)
-  B200_CHECK(cudaMemcpyAsync(xo_.get(), xo.data(), n * sizeof(double), cudaMemcpyHostToDevice, st_));
-  B200_CHECK(cudaMemcpyAsync(yo_.get(), yo.data(), m * sizeof(double), cudaMemcpyHostToDevice, st_));
+  B200_CHECK(cudaMemcpyAsync(xo_, xo.data(), n * sizeof(double), cudaMemcpyHostToDevice, st_));
+  B200_CHECK(cudaMemcpyAsync(yo_, yo.data(), m * sizeof(double), cudaMemcpyHostToDevice, st_));
   clear_maxima();
   launch_kkt_original();
   sync_results();
@@ -839,24 +845,37 @@ void Engine::finish_p(EngineResult& R, Status status, const T* xs, const T* ys, 
                       const DeviceOutputs& out, int ray_test) {
   const auto tf = clock::now();
   const int m = M_.m, n = M_.n;
+  // a check has left its rays packed, where the unscaled point is about to go
+  if (status == Status::Infeasible && ray_test > 0) {
+    k_unpack<<<grid_for(m), kBlock, 0, st_>>>(m, Y4_.get(), o_.pdlp ? ray_test + 1 : ray_test, ray_r_);
+    B200_LAUNCH_CHECK();
+    if (out.dual_ray)
+      B200_CHECK(cudaMemcpyAsync(out.dual_ray, ray_r_, m * sizeof(double), cudaMemcpyDeviceToDevice, st_));
+  }
+  if (status == Status::Unbounded && ray_test > 0) {
+    k_unpack<<<grid_for(n), kBlock, 0, st_>>>(n, X4_.get(), ray_test + 1, ray_d_);
+    B200_LAUNCH_CHECK();
+    if (out.primal_ray)
+      B200_CHECK(cudaMemcpyAsync(out.primal_ray, ray_d_, n * sizeof(double), cudaMemcpyDeviceToDevice, st_));
+  }
   clear_maxima();
   launch_kkt_scaled<T>(xs, ys);
   // objective = offset + Σ c_j x_j (Model::objective_value)
-  k_obj_terms<<<grid_for(n), kBlock, 0, st_>>>(n, M_.c, xo_.get(), objt_.get());
+  k_obj_terms<<<grid_for(n), kBlock, 0, st_>>>(n, M_.c, xo_, objt_);
   B200_LAUNCH_CHECK();
   plan_obj_.launch(st_);
   // in-process check (solution_checker.cpp:61-133) on xo and y_min = yo
   double c_scale = std_max(1.0, sp_.c_inf);
-  EpiCheckRows cr{{}, yo_.get(), M_.row_lower, M_.row_upper, c_scale, objt_.get() + n, res_.get()};
-  launch_slab_tma<double>(m, sp_.a_rp.get(), sp_.a_col.get(), sp_.a_v0.get(), xo_.get(), cr, st_, nullptr, err());
+  EpiCheckRows cr{{}, yo_, M_.row_lower, M_.row_upper, c_scale, objt_ + n, res_.get()};
+  launch_slab_tma<double>(m, sp_.a_rp.get(), sp_.a_col.get(), sp_.a_v0.get(), xo_, cr, st_, nullptr, err());
   // t_primal lands in objt_[0, n): the objective terms were consumed by plan_obj_ above
-  EpiCheckCols cc{{}, xo_.get(), M_.c, M_.col_lower, M_.col_upper, static_cast<double>(M_.sense), c_scale, m,
-                  objt_.get() + n, objt_.get(), res_.get()};
-  launch_slab<double>(n, M_.col_start, M_.row_index, M_.value, yo_.get(), cc, st_, nullptr, err());
+  EpiCheckCols cc{{}, xo_, M_.c, M_.col_lower, M_.col_upper, static_cast<double>(M_.sense), c_scale, m,
+                  objt_ + n, objt_, res_.get()};
+  launch_slab<double>(n, M_.col_start, M_.row_index, M_.value, yo_, cc, st_, nullptr, err());
   plan_chk_.launch(st_);
   kernels_ += 3 + plan_obj_.kernel_count() + plan_chk_.kernel_count();
   // outputs
-  if (out.x) B200_CHECK(cudaMemcpyAsync(out.x, xo_.get(), n * sizeof(double), cudaMemcpyDeviceToDevice, st_));
+  if (out.x) B200_CHECK(cudaMemcpyAsync(out.x, xo_, n * sizeof(double), cudaMemcpyDeviceToDevice, st_));
   if (out.y || out.z) {
     DevBuf<double> ytmp;
     double* y = out.y;
@@ -864,24 +883,12 @@ void Engine::finish_p(EngineResult& R, Status status, const T* xs, const T* ys, 
       ytmp.alloc(m);
       y = ytmp.get();
     }
-    k_dual_out<<<grid_for(m), kBlock, 0, st_>>>(m, static_cast<double>(M_.sense), yo_.get(), y);
+    k_dual_out<<<grid_for(m), kBlock, 0, st_>>>(m, static_cast<double>(M_.sense), yo_, y);
     if (out.z) k_reduced_costs<<<grid_for(n), kBlock, 0, st_>>>(n, M_.col_start, M_.row_index, M_.value, M_.c, y, out.z);
     B200_LAUNCH_CHECK();
     kernels_ += 2;
     if (ytmp.get()) B200_CHECK(cudaStreamSynchronize(st_));
   }
-  if (status == Status::Infeasible && X4_.get() && ray_test > 0)  // a check left its rays packed
-    k_unpack<<<grid_for(m), kBlock, 0, st_>>>(m, Y4_.get(), o_.pdlp ? ray_test + 1 : ray_test,
-                                               (ray_test == 2 ? r2_ : r1_).get());
-  if (status == Status::Unbounded && X4_.get() && ray_test > 0)
-    k_unpack<<<grid_for(n), kBlock, 0, st_>>>(n, X4_.get(), ray_test + 1, (ray_test == 2 ? d2_ : d1_).get());
-  B200_LAUNCH_CHECK();
-  if (status == Status::Infeasible && out.dual_ray)
-    B200_CHECK(cudaMemcpyAsync(out.dual_ray, ray_test == 2 ? r2_.get() : r1_.get(), m * sizeof(double),
-                               cudaMemcpyDeviceToDevice, st_));
-  if (status == Status::Unbounded && out.primal_ray)
-    B200_CHECK(cudaMemcpyAsync(out.primal_ray, ray_test == 2 ? d2_.get() : d1_.get(), n * sizeof(double),
-                               cudaMemcpyDeviceToDevice, st_));
   sync_results();
   const double* h = hres_.get();
   const Kkt k = read_kkt(h);
@@ -1302,7 +1309,7 @@ void Engine::launch_pdlp_check_kernels(int phase) {
   const int m = M_.m, n = M_.n;
   const long long L = static_cast<long long>(m) + n;
   T *xs[2] = {v.x.get(), v.xh.get()}, *ys[2] = {v.y.get(), v.yh.get()};
-  double *K0 = kt_.get(), *K1 = kt2_.get(), *T0 = rayt_.get(), *T1 = T0 + 2 * L + 2 * n;
+  double *K0 = kt_.get(), *K1 = rt_.get(), *T0 = rayt_.get(), *T1 = T0 + 2 * L + 2 * n;
   PdlpVecs<T> c{n, m, xs[phase], v.dx.get(), xs[1 - phase], v.x0.get(), ys[phase], v.dy.get(), ys[1 - phase], v.y0.get(),
                 sp_.col_scale.get(), sp_.row_scale.get(), sp_.bound_scale, sp_.obj_scale, static_cast<double>(M_.sense), M_.c,
                 M_.col_lower, M_.col_upper, M_.row_lower, M_.row_upper, X4_.get(), Y4_.get(),
