@@ -165,11 +165,13 @@ typedef struct {
   long long kernel_launches;   /* kernels launched by the solve (graph nodes counted per replay) */
   long long m, n, nnz;         /* size of the problem the engine ran on (after presolve) */
   double spmv_kernel_ms;       /* total device time of the fused iteration kernels (CUDA events) */
-  long long spmv_kernel_launches;
+  long long spmv_kernel_launches; /* half-steps in that time, two an iteration (one launch each, but one for
+                                     all of an epoch's where the LP fits the SMs' shared memory) */
   double teardown_seconds;     /* releasing the engine's device state after the loop */
   double call_seconds;         /* the whole entry-point call, host wall clock */
   int slab_variant_primal;     /* launch variants of the fused iteration kernels picked by the */
-  int slab_variant_dual;       /*   autotuner for this matrix (indices of the library's variant list) */
+  int slab_variant_dual;       /*   autotuner for this matrix (indices of the library's variant list); */
+                               /*   epochs in shared memory do not use them */
   int tuned;                   /* 1: this solve timed the variants itself (first of its shape class) */
   int reserved;
 } ps26119_stats;
@@ -241,7 +243,8 @@ typedef struct {
   double dry_run_seconds;  /* > 0: requests are admitted and timed but not solved (each holds its
                               slot and memory this long); status NOT_SOLVED, engine "dry-run" */
   int solo_engines;        /* 0 (default): the r²HPDHG epochs of all running requests are launched
-                              together, one grouped kernel per half-step over every request's
+                              together: one launch per epoch where they fit the SMs' shared
+                              memory, else one grouped kernel per half-step over every request's
                               slabs; 1: each request's engine launches its own kernels */
 } ps26119_server_options;
 

@@ -74,7 +74,7 @@ struct EngineResult {
   long long kernel_launches = 0;
   double iter_kernel_ms = 0;
   double teardown_seconds = 0;  // releasing the engine's device state after the loop
-  long long iter_kernel_launches = 0;
+  long long iter_kernel_launches = 0;  // half-steps in iter_kernel_ms, two an iteration
   bool have_dual_ray = false, have_primal_ray = false;
   // in-process check of the reported point on the engine's model (device-computed)
   int check = -1;
@@ -93,8 +93,8 @@ struct DeviceOutputs {
   double* primal_ray = nullptr;  // n (Unbounded)
 };
 
-// For the calling thread's later solves: run the r²HPDHG epochs in the device's group (one grouped
-// launch per half-step with every other grouped solve in flight) instead of on the solve's own
+// For the calling thread's later solves: run the r²HPDHG epochs in the device's group (with every other
+// grouped solve in flight, one launch per epoch or per half-step) instead of on the solve's own
 // stream. Results are the same either way. The request loop's slot threads set it.
 void set_grouped_engine(bool on);
 

@@ -22,6 +22,7 @@
 #include "reduce.cuh"
 #include "setup.cuh"
 #include "spmv.cuh"
+#include "tune.hpp"
 
 namespace b200 {
 
@@ -361,7 +362,9 @@ struct ScaledDevice {
     const int tiles = (n + kXTile - 1) / kXTile;
     // An LP that fits the SMs' shared memory takes a batch of steps in one launch (lanczos.cuh).
     const RowLengths* len = lengths(st);
-    LanczosShape shape = lanczos_shape(m, n, nnz, len[0].longest, len[1].longest, stream_sm_count(st));
+    LanczosShape shape;
+    if (tune_forced() < 0)  // a forced step-kernel variant: no cooperative launches
+      shape = lanczos_shape(m, n, nnz, len[0].longest, len[1].longest, stream_sm_count(st));
     DevBuf<Cell<double>> cells;
     DevBuf<XFast> fast;
     DevBuf<XTileAgg> full;

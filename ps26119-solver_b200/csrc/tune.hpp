@@ -6,7 +6,8 @@
 // (src/gpu/cuda_backend.cu:393-394); this measures instead of guessing.
 //
 // Environment: PS26119_AUTOTUNE=0 keeps the default variant (index 0) everywhere;
-// PS26119_SLAB_VARIANT=k forces variant k (tests run every variant this way).
+// PS26119_SLAB_VARIANT=k forces variant k (tests run every variant this way) and the kernels that have variants: no
+// resident epochs and no one-launch Lanczos.
 #pragma once
 
 #include <cmath>

@@ -47,6 +47,14 @@ def test_norm_estimate(name):
     assert [be.norm2_estimate() for _ in range(20)] == [want] * 20
 
 
+@pytest.mark.parametrize("name", list(LPS))
+def test_without_cooperative_launches(name, monkeypatch):
+    """PS26119_SLAB_VARIANT leaves the kernels' form, for processes in which such a launch would have to wait."""
+    monkeypatch.setenv("PS26119_SLAB_VARIANT", "0")
+    lp = LPS[name]()
+    assert ps26119.Backend(lp).norm2_estimate() == oracle.Scaled(lp).norm2()
+
+
 def test_estimates_side_by_side():
     lps = [make() for make in LPS.values()]
     want = [oracle.Scaled(lp).norm2() for lp in lps]
