@@ -305,40 +305,129 @@ __device__ __forceinline__ double ray_col(double g, double gabs, double lo, doub
   }
   return viol;
 }
+// A long row or column would hold up the check: its thread makes two trips to memory (the indices, then the
+// points there) for every four entries. The check of an LP that has one (kLong) sums the long ones of a warp's
+// rows with the whole warp, one after the other, where their entries together are fewer than kCheckShare times
+// the longest's. (A thread takes 0.2 us an entry, so 25 us for 128, no more than a check's launches; the warp 0.01,
+// so that 16 rows one after the other are still quicker than one by its thread.) Ten checks and the first residuals of
+// their cycles, ms, without / with: 60k rows of 6 and one of 4,000 entries 7.5 / 2.8, of 60,000 99 / 28; a column of
+// 60,000 54 / 6.7; 300k rows and one of 300,000 665 / 136. The kernel for LPs without is as it was.
+constexpr int kCheckLong = 128, kCheckShare = 16;
+constexpr int kCheckChunk = 64, kCheckPitch = kCheckChunk + 2;  // entries at a time; of a buffer (free of bank conflicts)
+inline bool check_is_long(int longest) { return longest > kCheckLong; }
+// The lanes whose rows, of len entries each, the warp sums.
+__device__ __forceinline__ unsigned check_together(int len) {
+  const bool is = len > kCheckLong;
+  const long long longest = __reduce_max_sync(kFull, is ? len : 0);
+  return static_cast<long long>(__reduce_add_sync(kFull, is ? len : 0)) < kCheckShare * longest ? __ballot_sync(kFull, is) : 0u;
+}
+// The sums of a long row, entries [b, e) with their indices at idx, by a whole warp: the lanes form kCheckChunk
+// entries' products (load: what those of an entry need; mul: the kSums products of it) while the next ones are
+// on their way, and a lane for each sum adds them in storage order. Lane k < kSums returns the k-th sum, lane kSums + k
+// the sum of the (k + 1)-th products' absolute values. sh: kSums buffers of kCheckPitch.
+template <int kSums, int kAbs, class Load, class Mul>
+__device__ __forceinline__ double check_long(int b, int e, const int* __restrict__ idx, double* sh, const Load& load,
+                                             const Mul& mul) {
+  constexpr int Q = kCheckChunk / 32;
+  const int lane = static_cast<int>(threadIdx.x) & 31;
+  const bool magnitude = lane >= kSums;
+  const double* mine = sh + (lane < kSums ? lane : lane < kSums + kAbs ? lane - kSums + 1 : 0) * kCheckPitch;
+  const auto place = [&](unsigned k, int q) {
+    return static_cast<int>(min(k + static_cast<unsigned>(32 * q + lane), static_cast<unsigned>(e - 1)));
+  };
+  int at[Q];
+  decltype(load(0, 0)) in[Q];
+#pragma unroll
+  for (int q = 0; q < Q; ++q) at[q] = idx[place(b, q)];
+#pragma unroll
+  for (int q = 0; q < Q; ++q) in[q] = load(place(b, q), at[q]), at[q] = idx[place(static_cast<unsigned>(b) + kCheckChunk, q)];
+  double s = 0.0;
+  const auto add = [&](int k) { s += magnitude ? fabs(mine[k]) : mine[k]; };
+  const unsigned end = static_cast<unsigned>(e);
+  for (unsigned k = static_cast<unsigned>(b); k < end; k += kCheckChunk) {
+    __syncwarp();  // the chunk before has been added
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      double prod[kSums];
+      mul(in[q], prod);
+#pragma unroll
+      for (int t = 0; t < kSums; ++t) sh[t * kCheckPitch + 32 * q + lane] = prod[t];
+    }
+    __syncwarp();
+    if (k + kCheckChunk < end) {
+#pragma unroll
+      for (int q = 0; q < Q; ++q) in[q] = load(place(k + kCheckChunk, q), at[q]);
+#pragma unroll
+      for (int q = 0; q < Q; ++q) at[q] = idx[place(k + 2 * kCheckChunk, q)];
+#pragma unroll 16
+      for (int i = 0; i < kCheckChunk; ++i) add(i);
+    } else {
+      for (int i = 0; i < static_cast<int>(end - k); ++i) add(i);
+    }
+  }
+  return s;
+}
 // Rows of A (blocks [0, row_blocks)): original values a0 and scaled values as on one index list; columns
 // (the blocks after them): the caller's CSC.
-template <class T, int kRays>
+template <class T, int kRays, bool kLong>
 static __global__ void __launch_bounds__(kBlock) k_check_products(const __grid_constant__ CheckVecs<T> v, int row_blocks,
                                                                   const int* __restrict__ rp, const int* __restrict__ col,
                                                                   const double* __restrict__ a0, const T* __restrict__ as,
                                                                   const int* __restrict__ cp, const int* __restrict__ ri,
                                                                   const double* __restrict__ av) {
   constexpr int GB = 4;  // entries whose gathers are in flight together
+  __shared__ double sh_long[kLong ? kBlock / 32 : 1][kLong ? (kRays + 2) * kCheckPitch : 1];
   const bool rows = static_cast<int>(blockIdx.x) < row_blocks;
   const int k = (static_cast<int>(blockIdx.x) - (rows ? 0 : row_blocks)) * kBlock + static_cast<int>(threadIdx.x);
+  const int lane = static_cast<int>(threadIdx.x) & 31;
+  double* sh = sh_long[kLong ? threadIdx.x >> 5 : 0];
+  const bool mine = k < (rows ? v.m : v.n);
+  const int* __restrict__ ptr = rows ? rp : cp;
+  const int b = mine ? ptr[k] : 0, all = mine ? ptr[k + 1] : 0;
+  const unsigned together = kLong ? check_together(all - b) : 0u;
+  const int e = kLong && ((together >> lane) & 1u) ? b : all;  // the thread's own walk
   double pmax = 0.0, dmax = 0.0, viol = 0.0, viol2 = 0.0;
   if (rows) {
-    if (k < v.m) {
-      const int b = rp[k], e = rp[k + 1];
-      double ax = 0.0, adx = 0.0, ad = 0.0, ad2 = 0.0;
-      for (int p = b; p < e; p += GB) {
-        double4 g[GB];
-        double w[GB], ws[GB];
+    double ax = 0.0, adx = 0.0, ad = 0.0, ad2 = 0.0;
+    for (int p = b; p < e; p += GB) {
+      double4 g[GB];
+      double w[GB], ws[GB];
 #pragma unroll
-        for (int q = 0; q < GB; ++q) {
-          const int at = p + q < e ? p + q : p;
-          g[q] = load_packed<(kRays >= 1)>(v.X + col[at]);
-          w[q] = a0[at], ws[q] = static_cast<double>(as[at]);
-        }
-#pragma unroll
-        for (int q = 0; q < GB; ++q)
-          if (p + q < e) {  // each sum in CSR order
-            ax += w[q] * g[q].x;
-            adx += ws[q] * g[q].y;
-            if constexpr (kRays >= 1) ad += w[q] * g[q].z;
-            if constexpr (kRays == 2) ad2 += w[q] * g[q].w;
-          }
+      for (int q = 0; q < GB; ++q) {
+        const int at = p + q < e ? p + q : p;
+        g[q] = load_packed<(kRays >= 1)>(v.X + col[at]);
+        w[q] = a0[at], ws[q] = static_cast<double>(as[at]);
       }
+#pragma unroll
+      for (int q = 0; q < GB; ++q)
+        if (p + q < e) {  // each sum in CSR order
+          ax += w[q] * g[q].x;
+          adx += ws[q] * g[q].y;
+          if constexpr (kRays >= 1) ad += w[q] * g[q].z;
+          if constexpr (kRays == 2) ad2 += w[q] * g[q].w;
+        }
+    }
+    if constexpr (kLong) {
+      struct In {
+        double4 g;
+        double w, ws;
+      };
+      for (unsigned left = together; left != 0; left &= left - 1) {
+        const int who = __ffs(left) - 1;
+        const double s = check_long<kRays + 2, 0>(
+            __shfl_sync(kFull, b, who), __shfl_sync(kFull, all, who), col, sh,
+            [&](int p, int at) { return In{load_packed<(kRays >= 1)>(v.X + at), a0[p], static_cast<double>(as[p])}; },
+            [&](const In& in, double* prod) {
+              prod[0] = in.w * in.g.x, prod[1] = in.ws * in.g.y;
+              if constexpr (kRays >= 1) prod[2] = in.w * in.g.z;
+              if constexpr (kRays == 2) prod[3] = in.w * in.g.w;
+            });
+        const double s0 = __shfl_sync(kFull, s, 0), s1 = __shfl_sync(kFull, s, 1), s2 = __shfl_sync(kFull, s, 2),
+                     s3 = __shfl_sync(kFull, s, 3);
+        if (lane == who) ax = s0, adx = s1, ad = s2, ad2 = s3;
+      }
+    }
+    if (mine) {
       const double lo = v.rl[k], up = v.ru[k];
       const double4 Y = v.Y[k];
       const T dy = static_cast<T>(-1.0) * v.yh[k] + static_cast<T>(1.0) * v.yb[k];
@@ -357,32 +446,52 @@ static __global__ void __launch_bounds__(kBlock) k_check_products(const __grid_c
     if constexpr (kRays >= 1) warp_max_atomic(max_slot(v.res, kMaxPviol), viol);
     if constexpr (kRays == 2) warp_max_atomic(max_slot(v.res, kMaxPviol2), viol2);
   } else {
-    if (k < v.n) {
-      const int b = cp[k], e = cp[k + 1];
-      double aty = 0.0, gr = 0.0, ga = 0.0, gr2 = 0.0, ga2 = 0.0;
-      for (int p = b; p < e; p += GB) {
-        double4 g[GB];
-        double w[GB];
+    double aty = 0.0, gr = 0.0, ga = 0.0, gr2 = 0.0, ga2 = 0.0;
+    for (int p = b; p < e; p += GB) {
+      double4 g[GB];
+      double w[GB];
 #pragma unroll
-        for (int q = 0; q < GB; ++q) {
-          const int at = p + q < e ? p + q : p;
-          g[q] = load_packed<kRays == 2>(v.Y + ri[at]);
-          w[q] = av[at];
-        }
-#pragma unroll
-        for (int q = 0; q < GB; ++q)
-          if (p + q < e) {
-            aty += w[q] * g[q].x;
-            if constexpr (kRays >= 1) {
-              const double t = w[q] * g[q].y;
-              gr += t, ga += fabs(t);
-            }
-            if constexpr (kRays == 2) {
-              const double t = w[q] * g[q].z;
-              gr2 += t, ga2 += fabs(t);
-            }
-          }
+      for (int q = 0; q < GB; ++q) {
+        const int at = p + q < e ? p + q : p;
+        g[q] = load_packed<kRays == 2>(v.Y + ri[at]);
+        w[q] = av[at];
       }
+#pragma unroll
+      for (int q = 0; q < GB; ++q)
+        if (p + q < e) {
+          aty += w[q] * g[q].x;
+          if constexpr (kRays >= 1) {
+            const double t = w[q] * g[q].y;
+            gr += t, ga += fabs(t);
+          }
+          if constexpr (kRays == 2) {
+            const double t = w[q] * g[q].z;
+            gr2 += t, ga2 += fabs(t);
+          }
+        }
+    }
+    if constexpr (kLong) {
+      struct In {
+        double4 g;
+        double w;
+      };
+      for (unsigned left = together; left != 0; left &= left - 1) {
+        const int who = __ffs(left) - 1;
+        constexpr int S = kRays + 1;
+        const double s = check_long<S, kRays>(
+            __shfl_sync(kFull, b, who), __shfl_sync(kFull, all, who), ri, sh,
+            [&](int p, int at) { return In{load_packed<kRays == 2>(v.Y + at), av[p]}; },
+            [&](const In& in, double* prod) {
+              prod[0] = in.w * in.g.x;
+              if constexpr (kRays >= 1) prod[1] = in.w * in.g.y;
+              if constexpr (kRays == 2) prod[2] = in.w * in.g.z;
+            });
+        const double s0 = __shfl_sync(kFull, s, 0), s1 = __shfl_sync(kFull, s, 1), a1 = __shfl_sync(kFull, s, S),
+                     s2 = __shfl_sync(kFull, s, 2), a2 = __shfl_sync(kFull, s, S + 1);
+        if (lane == who) aty = s0, gr = s1, ga = a1, gr2 = s2, ga2 = a2;
+      }
+    }
+    if (mine) {
       const double lo = v.cl[k], up = v.cu[k], c = v.c[k];
       const double4 X = v.X[k];
       const long long at = static_cast<long long>(v.m) + k;

@@ -593,8 +593,9 @@ void Engine::launch_check_kernels() {
   plan_pid_.launch(side_);
   B200_CHECK(cudaEventRecord(fork_[1], side_));
   if (cb + rb > 0) {
-    k_check_products<T, kRays><<<cb + rb, kBlock, 0, st_>>>(c, rb, sp_.a_rp.get(), sp_.a_col.get(), sp_.a_v0.get(),
-                                                            sp_.A_val<T>(), M_.col_start, M_.row_index, M_.value);
+    const auto products = check_is_long(longest()) ? &k_check_products<T, kRays, true> : &k_check_products<T, kRays, false>;
+    products<<<cb + rb, kBlock, 0, st_>>>(c, rb, sp_.a_rp.get(), sp_.a_col.get(), sp_.a_v0.get(), sp_.A_val<T>(),
+                                          M_.col_start, M_.row_index, M_.value);
     B200_LAUNCH_CHECK();
   }
   plan_check_[kRays].launch(st_);
