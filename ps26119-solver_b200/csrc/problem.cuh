@@ -423,6 +423,7 @@ struct ScaledDevice {
     double theta = 0, theta_old = -1;
     int stagnant = 0;
     int from = 0, to = std::min(K, 21), slot = 0;
+    const long long walk = static_cast<long long>(len[0].longest) + len[1].longest;
     auto fetch = [&](int a, int b, int s) {
       B200_CHECK(cudaMemcpyAsync(h.get() + 2 * a, hist.get() + 2 * a, 2 * static_cast<std::size_t>(b - a) * sizeof(double),
                                  cudaMemcpyDeviceToHost, st));
@@ -433,8 +434,12 @@ struct ScaledDevice {
     fetch(from, to, slot);
     for (bool done = false; !done;) {
       // The device goes on while the host looks at this batch, where a step is cheap against the
-      // host's look or the run is long; else the steps past the stop would cost more than the wait.
-      const bool ahead = n <= (1 << 18) || to >= 100;
+      // host's look or the run is long; else the steps past the stop would cost more than the wait. What a
+      // step costs is in its columns, its nonzeros, and the longest row and column, which one thread walks each
+      // (0.13 us an entry). Looking ahead regardless / so, ms: 20k rows of 300 columns, dense, 7,350 / 5,220; 2,000 of
+      // 3,000, dense, 1,452 / 1,258; 20k rows of 200 17.2 / 12.4; 100k rows of 30 2.9 / 2.4; a band of 150k rows of 24
+      // 2.8 / 2.2 (without these steps the first three took 5,550, 1,280 and 15.2 ms).
+      const bool ahead = (n <= (1 << 18) && nnz <= (1 << 21) && walk <= 512) || (to >= 100 && nnz <= (1 << 24) && walk <= 4096);
       const int next = std::min(K, to + 8);
       auto go_on = [&] {
         if (next > to) launch(to, next), fetch(to, next, slot ^ 1);
