@@ -23,10 +23,9 @@
 // products tie to nothing (an LP whose columns fall into unconnected parts), at any time before they count
 // in first: they have cells of their own, written once a launch, and the next launch follows this one.
 //
-// What bounds it: about ten trips through L2 a step (two half-steps, and four per sum) and the two walks,
-// one x_commit for every binade that the sums pass. Measured, Lanczos of 1k random rows 1.07 against 1.26 ms
-// in six launches a step, 10k 1.65 / 1.88, staircase T = 168 (389 steps) 10.1 / 13.3 (before the walk's steps
-// were shortened in both forms 1.3 / 2.3, 3.3 / 5.6 with 93 steps, 9.5 / 16.5 with 285).
+// What bounds it: about ten trips through L2 a step (two half-steps, and four per sum) and the two walks, one
+// x_commit for every binade that the sums pass. Measured, the whole estimate in ms, in six launches a step / so:
+// 1k random rows 1.15 / 1.05, 10k 1.87 / 1.61, staircase T = 168 (389 steps) 12.6 / 10.1.
 #pragma once
 
 #include "reduce.cuh"
@@ -226,13 +225,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_resident_lanczos(const __grid_c
 }
 
 // Past this many columns the walks over one run per 256 of them outweigh the launches saved (the kernels'
-// form composes groups of 32): the steps of 20k random rows (30,000 columns) take 1.78 against 1.88 ms, of
-// the staircase T = 360 (21,600) 12.4 against 13.9; of 30k rows (45,000) 2.34 against 2.24, of T = 720
-// (43,200) 14.8 against 14.3, of 60k rows (90,000) 4.4 against 2.8.
+// form composes groups of 32). The estimate in one launch / by kernels, ms: staircase T = 360 (21,600 columns) 12.4 /
+// 13.4, T = 680 (40,800) 13.9 / 14.1, 27k random rows (40,500) 1.94 / 1.91; past the line, in an earlier build, T = 720
+// (43,200) 14.8 / 14.3, 30k rows (45,000) 2.34 / 2.24, 60k (90,000) 4.4 / 2.8.
 constexpr long long kLanczosColumns = 40960;
-// Columns a block: few blocks leave SMs to other solves, many make a longer walk and wider exchanges.
-// Setup of 30k random rows with 120 / 224 / 448 / 896 columns a block 4.0 / 4.4 / 3.8 / 4.6 ms, staircase
-// T = 720 19.7 / 20.4 / 18.6 / 24.3; 16 requests' setups side by side 41 / 33 / 30 / 29.
+// Columns a block: few blocks leave SMs to other solves, many make a longer walk and wider exchanges. The
+// estimate with 112 / 224 / 448 / 896 columns a block, ms: 10k random rows 1.79 / 1.63 / 1.61 / 1.83, 27k 2.17 / 2.18 /
+// 1.94 / 2.43, staircase T = 360 13.4 / 12.4 / 12.4 / 15.4, T = 680 16.3 / 16.2 / 13.9 / 17.8; 16 solves of 64 iterations side by
+// side 38.5 / 34.7 / 33.4 / 29.4.
 constexpr long long kLanczosShare = 448;
 // The launch of such a kernel: as few blocks as hold the LP with about kLanczosShare columns each, because
 // every block is a summary in the sums and a party to their three exchanges; blocks = 0: it does not fit.

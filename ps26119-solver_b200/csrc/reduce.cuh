@@ -85,13 +85,9 @@ __device__ __forceinline__ double block_sum_fixed(double v, double* sh) {
 // one warp's, keep the tiles that must be added one by one cheap. The first group, where most binades are
 // crossed, is walked by its own last block, beside the other groups' composition. Of 14 us for the 525,600
 // terms of the staircase T = 8760 the tiles take 5, the first group 2.5, the count of groups 1, the walk 4.5.
-// Measured, 15,000 / 525,600 / 1.5M uniform terms, one launch by itself from cold caches: 16.8 / 18.5 / 33.8
-// us; 19.3 / 25.1 / 38.9 with the first group in the walk, commits with branches after the ballot, each
-// round's summaries loaded when it began and ties composed pair by pair (Lanczos on T = 8760 23.0 against
-// 28.5 ms, 1M random rows 12.9 / 14.5, 100k 6.6 / 8.4). The forms before: 15,000 terms 18.5 against then 14
-// us with the terms in units of u by division and rounding, every summary read in full and the first tile
-// left to the walk; 24 with summaries scanned anew in shared memory at every crossing; three launches over
-// tiles of 2,048 terms, the first walked in windows with a scan and a restart per crossing, took 68 us.
+// Measured, 15,000 / 525,600 / 1.5M uniform terms, one launch by itself from cold caches: 16.8 / 18.5 / 33.8 us
+// (15,000 in three launches over tiles of 2,048 terms, walked in windows with a scan and a restart per crossing:
+// 68 us).
 constexpr int kXPer = 8;              // terms per lane
 constexpr int kXTile = 32 * kXPer;    // terms per tile (one warp)
 constexpr int kXGroup = 32;           // tiles per group (one warp lane each)

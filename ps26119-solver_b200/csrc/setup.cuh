@@ -160,8 +160,9 @@ static __global__ void k_sort_long(const int* rp, const int* long_rows, const in
 // and a few of its entries at a time, so that their loads and gathers are in flight together. Measured,
 // structure and scaling of 1M random rows (6M entries) / staircase T = 8760 / 1k random rows: 4.49 / 1.15 /
 // 0.71 ms with a loop of single entries, norms, factors and products in launches of their own and a block per
-// 256 entries in k_abs_range; 3.15 / 0.73 / 0.52 so (4, 6 and 8 entries at a time: 3.22, 3.84 and 4.40 on the
-// first). One launch on it, cold: a side's scaling step 59 us (the three before it about 100), a pass of
+// 256 entries in k_abs_range; 3.15 / 0.79 / 0.47 so. With 2 / 3 / 4 / 8 entries at a time: 1M rows of 6 3.21 / 3.15 / 3.21 /
+// 4.42, 100k rows of 30 2.39 / 2.34 / 2.47 / 4.25, 20k rows of 200 7.63 / 7.33 / 8.38 / 13.7, a band of 150k rows of 24 1.97 /
+// 1.96 / 1.96 / 3.47. One launch on it, cold: a side's scaling step 59 us (the three before it about 100), a pass of
 // geometric means 37 (48), k_abs_range 21 (250).
 constexpr int kScaleAhead = 3;
 
