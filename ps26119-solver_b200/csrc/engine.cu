@@ -225,6 +225,7 @@ class Engine {
   template <class T> void launch_first_residual(const int* skip, bool apart);
   template <class T, int kRays> void launch_check_kernels();
   template <class T> void plan_resident();
+  bool epoch_is_resident() const;
   template <class T> bool launch_resident_epoch();
   template <class T> bool launch_resident_pdlp(int cur);
   bool no_resident();
@@ -266,6 +267,7 @@ class Engine {
   RowLengths rows_, cols_;  // the lengths of the rows, of the columns
   ResidentShape shape_[2];  // resident epochs in fp64 / fp32 (blocks = 0: the step kernels)
   unsigned tag_ = 1;        // the next resident epoch's first tag
+  bool stepped_resident_ = false;  // the last epoch of launch_epoch()
   DevBuf<unsigned> stage_err_;  // this solve's bulk-copy timeouts (see count_stage_timeout)
   clock::time_point t0_;
   ScaledDevice sp_;
@@ -1069,6 +1071,35 @@ void Engine::resident_done() {
   else launch_first_residual<double>(nullptr, true);
 }
 
+// The solves that run their epochs on a device by themselves (run, run_pdlp), while one of them lives.
+class SolvesRunning {
+ public:
+  SolvesRunning() {
+    B200_CHECK(cudaGetDevice(&dev_));
+    ++count(dev_);
+  }
+  ~SolvesRunning() { --count(dev_); }
+  SolvesRunning(const SolvesRunning&) = delete;
+  SolvesRunning& operator=(const SolvesRunning&) = delete;
+  static std::atomic<int>& count(int dev) {
+    static std::atomic<int> n[64];
+    return n[dev & 63];
+  }
+
+ private:
+  int dev_ = 0;
+};
+
+// Whether the next epoch is resident: not beside more than one other solve, because such launches, which must have
+// all their blocks on the SMs at once, then take turns where step kernels share the device. 32 random LPs of 1k to 20k
+// rows, 16 at a time on their own kernels, at most 300,000 iterations each: 17.2 s all resident, 8.0 so, 8.1 by the step
+// kernels alone. Two at a time, 1,920 iterations of 10k rows each: 22 ms resident, 41 by step kernels (with the checks of then).
+bool Engine::epoch_is_resident() const {
+  int dev = 0;
+  B200_CHECK(cudaGetDevice(&dev));
+  return resident() && SolvesRunning::count(dev).load(std::memory_order_relaxed) <= 2;
+}
+
 // A resident launch was refused (launch_cooperative): this solve's epochs are the step kernels' from here on.
 bool Engine::no_resident() {
   shape_[0] = shape_[1] = ResidentShape{};
@@ -1108,7 +1139,8 @@ bool Engine::launch_resident_pdlp(int cur) {
 
 void Engine::launch_epoch() {
   const int pidx = mixed_now_ ? 1 : 0;
-  if (resident() && (mixed_now_ ? launch_resident_epoch<float>() : launch_resident_epoch<double>())) return;
+  if ((stepped_resident_ = epoch_is_resident() && (mixed_now_ ? launch_resident_epoch<float>() : launch_resident_epoch<double>())))
+    return;
   upload_params();
   if (mixed_now_) capture_epoch<float>();
   else capture_epoch<double>();
@@ -1228,17 +1260,17 @@ bool Engine::end_epoch() {
 
 EngineResult Engine::run(const DeviceOutputs& out) {
   if (start(out)) return R_;
+  const SolvesRunning running;
   const int K = o_.check_every;
   for (;;) {
     begin_epoch();
     launch_epoch();
-    const bool stepped_resident = resident();
     launch_check();
     B200_CHECK(cudaStreamSynchronize(st_));
     {  // the iteration kernels' time, from the events inside the epoch graph
       float a = 0, b = 0;
       B200_CHECK(cudaEventElapsedTime(&a, ev_[0], ev_[1]));
-      if (!stepped_resident) B200_CHECK(cudaEventElapsedTime(&b, ev_[2], ev_[3]));
+      if (!stepped_resident_) B200_CHECK(cudaEventElapsedTime(&b, ev_[2], ev_[3]));
       iter_ms_ += a + b;
       iter_launches_ += 2LL * K;
     }
@@ -1459,6 +1491,7 @@ EngineResult Engine::run_pdlp(const DeviceOutputs& out) {
   else pdlp_restart<double>(cur, false);
   const Kkt k0 = kkt_now(false);
   clear_maxima();  // the first check finds them at zero
+  const SolvesRunning running;
   if (fast_it_ < 0 && k0.rel_kkt() <= kFirstOrderFast) fast_it_ = 0;
   double restart_kkt = k0.rel_kkt(), last_candidate = 1e300;
   long long it = 0, inner = 0;
@@ -1473,7 +1506,7 @@ EngineResult Engine::run_pdlp(const DeviceOutputs& out) {
     hp.skip_r0 = 1;
     B200_CHECK(cudaMemcpyAsync(params_.get(), &hp, sizeof(StepParams), cudaMemcpyHostToDevice, st_));
     const int pidx = mixed_now_ ? 1 : 0;
-    if (!resident() || !(mixed_now_ ? launch_resident_pdlp<float>(cur) : launch_resident_pdlp<double>(cur))) {
+    if (!epoch_is_resident() || !(mixed_now_ ? launch_resident_pdlp<float>(cur) : launch_resident_pdlp<double>(cur))) {
       if (mixed_now_) capture_pdlp_epoch<float>(cur);
       else capture_pdlp_epoch<double>(cur);
       B200_CHECK(cudaGraphLaunch(g_pdlp_[pidx][cur], st_));
